@@ -14,13 +14,14 @@ constexpr float kC2 = 0.0009f;      // cl/kernelGetGlobalSsim2D.cl:104
 constexpr int kMaxK = 512;          // largest ellipse block size accepted
 
 enum Metric { kPearson = 0, kSsim = 1, kNrmse = 2, kAbsDiff = 3, kCosine = 4,
-              kDebugDot = 5 /* diagnostics: num += G a_p a_q, den += r_p + r_q */,
+              kDebugDot = 5 /* diagnostics: num += G a_p a_q */,
               kHu = 6, kPhase = 7 /* block-map shape metrics */,
               kNrmseW = 8 /* NRMSE with each term weighted (the 3D global kernel) */,
               // NRMSE from the accumulated squared difference of the unit
               // vectors (FP32 engine): unweighted (2D) and weighted (3D)
               kNrmseD = 9, kNrmseDW = 10,
-              kHu7 = 11 /* block map: distance of the seven Hu invariants */ };
+              kHu7 = 11 /* block map: distance of the seven Hu invariants */,
+              kDebugSum = 12 /* diagnostics: num += r_p + r_q */ };
 
 // The FP32 engine's accumulator holds sum_i (u_p,i - u_q,i)^2 instead of the
 // dot product for these metrics.
@@ -115,6 +116,9 @@ struct EpiConsts {
   const float* U = nullptr;
   int kp = 0, K = 0;
   float nrmse_near = 1.0f;
+  float gscale = 1.0f;      // G = gscale x the contraction's accumulator
+  float inv_wscale = 0.0f;  // sigma / a
+  float c2h = 0.0f;         // c2 / (2 gscale)
 };
 
 // Near-identical pairs (G > 1 - 2^-7) of tensor-core NRMSE take the exact
@@ -124,26 +128,26 @@ constexpr float kNrmseNear = 1.0f - 1.0f / 128.0f;
 
 // Launch the FP32 CUDA-core all-pairs kernel (global_fp32.cu), on the same
 // symmetric schedule as the tensor-core engine with 128 x 128 tiles.
-// U: n_pad x kp floats (unit vectors), params: n_pad entries, num/den: n
+// U: n_pad x kp floats (unit vectors), params: n_pad entries, num: n
 // doubles (zeroed). The work items are split into n_shards equal ranges; this
 // launch runs range `shard`.
 cudaError_t launch_gram_fp32(const float* U, int kp, const BlockParams* params, const float* tile_rmax,
-                             EpiConsts ec, double* num, double* den, int num_sms, cudaStream_t st,
-                             int shard = 0, int n_shards = 1);
+                             EpiConsts ec, double* num, int num_sms, cudaStream_t st, int shard = 0,
+                             int n_shards = 1);
 
 // Column parameters of one BN-column tile as the tensor-core engine copies
-// them into shared memory: [a x BN | r x BN | sigma x BN | mu x BN | max r of
-// the tile | 3 x pad], each array permuted within every 16-column group so that
-// an epilogue thread's four columns of the group (2j, 2j + 1, 8 + 2j, 9 + 2j for
-// j = t % 4) are one float4.
-__host__ __device__ constexpr int col_soa_floats(int bn) { return 4 * bn + 4; }
+// them into shared memory: [a x BN | r x BN | sigma x BN | mu x BN | per group
+// of BN/4 columns {centre of a, half range of a, centre of r, half range of r}],
+// each array permuted within every 16-column group so that an epilogue thread's
+// four columns of the group (2j, 2j + 1, 8 + 2j, 9 + 2j for j = t % 4) are one
+// float4.
+__host__ __device__ constexpr int col_soa_floats(int bn) { return 4 * bn + 16; }
 __host__ __device__ constexpr int col_soa_pos(int i) {
   return (i & ~15) + 4 * ((i & 7) >> 1) + 2 * ((i >> 3) & 1) + (i & 1);
 }
-// Row parameters of one 128-row block: per row the pairs (a, a, -eps r, -eps r,
-// sigma, sigma, mu, mu) as the epilogue's f32x2 operands, then r x 128, then
-// max r and 3 x pad.
-constexpr int kRowSoaFloats = 8 * 128 + 128 + 4;
+// Row parameters of one 128-row block: [a | r | sigma | mu] x 128, then the same
+// four values per group of 32 rows.
+constexpr int kRowSoaFloats = 4 * 128 + 16;
 
 // Launch shape of the tensor-core engine for a K': column tile width (256 or
 // 128), whole-tile A buffers or a ring of 64-column chunks, dynamic shared
@@ -183,13 +187,13 @@ long long gram_tc_items(int n, int bn, int* L, int num_sms, int max_L = 0);
 
 // Launch the split-BF16 tcgen05 all-pairs kernel (global_tc.cu).
 // A, B: n_pad x kq bf16 (store_split); params: n_pad entries (rows past n
-// zero); soa_ws: gram_tc_soa_floats(n_pad) floats of workspace; num/den: n
-// doubles (zeroed), to which every pair's terms are added for both blocks.
+// zero); soa_ws: gram_tc_soa_floats(n_pad) floats of workspace; num: n
+// doubles (zeroed), to which every pair's term is added for both blocks.
 // The upper-triangle work items are split into n_shards equal ranges; this
-// launch runs range `shard` (the shards' num/den add up to the whole map).
+// launch runs range `shard` (the shards' num add up to the whole map).
 cudaError_t launch_gram_tc(const __nv_bfloat16* A, const __nv_bfloat16* B, int kq, int n_pad,
-                           const BlockParams* params, float* soa_ws, EpiConsts ec, double* num, double* den,
-                           int num_sms, int* status, cudaStream_t st, int shard = 0, int n_shards = 1,
+                           const BlockParams* params, float* soa_ws, EpiConsts ec, double* num, int num_sms,
+                           int* status, cudaStream_t st, int shard = 0, int n_shards = 1,
                            const TcDebug* dbg = nullptr, const TcChoice* choice = nullptr);
 
 }  // namespace sred

@@ -17,6 +17,7 @@
 // |x_p|^2 + |x_q|^2 - 2<x_p, x_q> never cancels in FP32.
 // 1/(1+t) is evaluated to first or second order, or exactly, according to the
 // tile's largest t (c_mode below), with relative error below 6e-8.
+// The weight's sums over q alone (the denominators) are computed in weights.cu.
 // The self pair (q == p) uses G = 1 exactly, as the reference's direct
 // evaluation gives; only tiles that contain the diagonal check for it.
 #pragma once
@@ -41,6 +42,19 @@ __device__ __forceinline__ float ex2_approx(float x) {
 __device__ __forceinline__ float rcp_approx(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// PTX sqrt.approx: relative error at most 2^-23.
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float y;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
   return y;
 }
 
@@ -78,19 +92,15 @@ __device__ __forceinline__ int c_mode(float tmax) {
   return tmax < kTFirst ? kCFirst : (tmax < kTFast ? kCSecond : kCExact);
 }
 
-// The two per-pair terms (numerator tn, denominator td); symmetric in p, q.
-// CMODE is used by Pearson only.
+// The per-pair numerator term; symmetric in p, q (the denominators, sums of the
+// weight alone, are weights.cu's). CMODE is used by Pearson only.
 template <int METRIC, int CMODE>
-__device__ __forceinline__ void pair_terms(float G, const RowState& rp, const BlockParams& cq,
-                                           const EpiConsts& ec, float& tn, float& td) {
-  if (METRIC == kDebugDot) {  // symmetric diagnostic terms
-    tn = G * rp.a * cq.a;
-    td = rp.r + cq.r;
-    return;
-  }
+__device__ __forceinline__ float pair_term(float G, const RowState& rp, const BlockParams& cq, const EpiConsts& ec) {
+  if (METRIC == kDebugDot) return G * rp.a * cq.a;  // symmetric diagnostic terms
+  if (METRIC == kDebugSum) return rp.r + cq.r;
   const float d = rp.a - cq.a;
   const float w = ex2_approx(-d * d);
-  td = w;
+  float tn;
   if (METRIC == kPearson) {
     float gc;
     if (CMODE == kCFirst) {
@@ -120,6 +130,7 @@ __device__ __forceinline__ void pair_terms(float G, const RowState& rp, const Bl
   } else {  // Abs-diff of stds
     tn = fabsf(rp.sigma - cq.sigma) * w;
   }
+  return tn;
 }
 
 // ---------------------------------------------------------------------------

@@ -39,7 +39,6 @@ struct Fp32Args {
   const float* tile_rmax;
   EpiConsts ec;
   double* num;
-  double* den;
   int n_rb;              // 128-blocks holding valid rows (= column tiles)
   int L;                 // row blocks per item
   long long item0, item1;
@@ -76,14 +75,13 @@ __device__ __forceinline__ void load_tile_t(float* S, const float* __restrict__ 
   }
 }
 
-// Pair terms of this thread's 8 x 8 pairs into the row sums rn/rd (per tile)
-// and the column sums cn/cd (per item). MASKED: the diagonal or ragged tile
+// Pair terms of this thread's 8 x 8 pairs into the row sums rn (per tile)
+// and the column sums cn (per item). MASKED: the diagonal or ragged tile
 // (q >= p for the rows, q > p for the columns, both below n).
 template <int METRIC, int CMODE, bool MASKED>
 __device__ __forceinline__ void tile_epilogue(const float (&acc)[TM][TM], const BlockParams* __restrict__ rowp,
                                               const BlockParams* __restrict__ colp, int row0, int col0,
-                                              const EpiConsts& ec, float (&rn)[TM], float (&rd)[TM],
-                                              float (&cn)[TM], float (&cd)[TM]) {
+                                              const EpiConsts& ec, float (&rn)[TM], float (&cn)[TM]) {
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
 #pragma unroll
   for (int i = 0; i < TM; i++) {
@@ -94,50 +92,42 @@ __device__ __forceinline__ void tile_epilogue(const float (&acc)[TM][TM], const 
       const int q = col0 + tx * TM + j;
       float G = acc[i][j];
       if (!diff_metric(METRIC) && MASKED && q == p && rs.r > 0.0f) G = 1.0f;
-      float tn, td;
-      pair_terms<METRIC, CMODE>(G, rs, colp[tx * TM + j], ec, tn, td);
+      const float tn = pair_term<METRIC, CMODE>(G, rs, colp[tx * TM + j], ec);
       if (!MASKED) {
         rn[i] += tn;
-        rd[i] += td;
         cn[j] += tn;
-        cd[j] += td;
       } else {
         const bool rv = p < ec.n && q >= p && q < ec.n, cv = rv && q != p;
         rn[i] += rv ? tn : 0.0f;
-        rd[i] += rv ? td : 0.0f;
         cn[j] += cv ? tn : 0.0f;
-        cd[j] += cv ? td : 0.0f;
       }
     }
   }
 }
 
-// Sums of 16 values over the 16 lanes that share them (lanes with equal
-// lane >> 4): stages xor 1, 2, 4, 8 each keep half the values; lane l ends with
-// the full sum of value index (bit3 = l&1, bit2 = (l>>1)&1, bit1 = (l>>2)&1, bit0 = (l>>3)&1).
-__device__ __forceinline__ float reduce16(const float (&x)[16], int& idx) {
+// Sums of 8 values over the 16 lanes that share them (lanes with equal
+// lane >> 4): stages xor 1, 2, 4 each keep half the values, xor 8 adds the two
+// halves; lane l ends with the full sum of value index (bit2 = l&1, bit1 =
+// (l>>1)&1, bit0 = (l>>2)&1).
+__device__ __forceinline__ float reduce16(const float (&x)[8], int& idx) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  float y8[8], y4[4], y2[2];
-  const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4, b3 = lane & 8;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const float keep = b0 ? x[8 + i] : x[i], send = b0 ? x[i] : x[8 + i];
-    y8[i] = keep + __shfl_xor_sync(full, send, 1);
-  }
+  float y4[4], y2[2];
+  const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4;
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    const float keep = b1 ? y8[4 + i] : y8[i], send = b1 ? y8[i] : y8[4 + i];
-    y4[i] = keep + __shfl_xor_sync(full, send, 2);
+    const float keep = b0 ? x[4 + i] : x[i], send = b0 ? x[i] : x[4 + i];
+    y4[i] = keep + __shfl_xor_sync(full, send, 1);
   }
 #pragma unroll
   for (int i = 0; i < 2; i++) {
-    const float keep = b2 ? y4[2 + i] : y4[i], send = b2 ? y4[i] : y4[2 + i];
-    y2[i] = keep + __shfl_xor_sync(full, send, 4);
+    const float keep = b1 ? y4[2 + i] : y4[i], send = b1 ? y4[i] : y4[2 + i];
+    y2[i] = keep + __shfl_xor_sync(full, send, 2);
   }
-  const float keep = b3 ? y2[1] : y2[0], send = b3 ? y2[0] : y2[1];
-  idx = 8 * (int)b0 + 4 * (int)b1 + 2 * (int)b2 + (int)b3;
-  return keep + __shfl_xor_sync(full, send, 8);
+  const float keep = b2 ? y2[1] : y2[0], send = b2 ? y2[0] : y2[1];
+  const float s = keep + __shfl_xor_sync(full, send, 4);
+  idx = 4 * (int)b0 + 2 * (int)b1 + (int)b2;
+  return s + __shfl_xor_sync(full, s, 8);
 }
 
 template <int METRIC>
@@ -159,9 +149,9 @@ __global__ void __launch_bounds__(NT, 2) k_gram_fp32(Fp32Args g) {
     for (int i = threadIdx.x; i < BM; i += NT) Bp[i] = g.params[col0 + i];
     const float rmax_c = g.tile_rmax[ct];
     const bool full = col0 + BM <= g.ec.n;
-    float cn[TM], cd[TM];
+    float cn[TM];
 #pragma unroll
-    for (int j = 0; j < TM; j++) cn[j] = cd[j] = 0.0f;
+    for (int j = 0; j < TM; j++) cn[j] = 0.0f;
 
     for (int rb = rb0; rb < rb1; rb++) {
       const int row0 = rb * BM;
@@ -199,45 +189,35 @@ __global__ void __launch_bounds__(NT, 2) k_gram_fp32(Fp32Args g) {
       }
       const int cm = METRIC == kPearson ? c_mode(kEps * g.tile_rmax[rb] * rmax_c) : kCFirst;
       const bool masked = !full || rb == ct;
-      float rn[TM], rd[TM];
+      float rn[TM];
 #pragma unroll
-      for (int i = 0; i < TM; i++) rn[i] = rd[i] = 0.0f;
+      for (int i = 0; i < TM; i++) rn[i] = 0.0f;
       if (masked)
-        tile_epilogue<METRIC, kCExact, true>(acc, Ap, Bp, row0, col0, g.ec, rn, rd, cn, cd);
+        tile_epilogue<METRIC, kCExact, true>(acc, Ap, Bp, row0, col0, g.ec, rn, cn);
       else if (cm == kCFirst)
-        tile_epilogue<METRIC, kCFirst, false>(acc, Ap, Bp, row0, col0, g.ec, rn, rd, cn, cd);
+        tile_epilogue<METRIC, kCFirst, false>(acc, Ap, Bp, row0, col0, g.ec, rn, cn);
       else if (cm == kCSecond)
-        tile_epilogue<METRIC, kCSecond, false>(acc, Ap, Bp, row0, col0, g.ec, rn, rd, cn, cd);
+        tile_epilogue<METRIC, kCSecond, false>(acc, Ap, Bp, row0, col0, g.ec, rn, cn);
       else
-        tile_epilogue<METRIC, kCExact, false>(acc, Ap, Bp, row0, col0, g.ec, rn, rd, cn, cd);
+        tile_epilogue<METRIC, kCExact, false>(acc, Ap, Bp, row0, col0, g.ec, rn, cn);
       // Row sums of the 16 column-threads of each row group (a half-warp),
-      // then one FP64 atomic per row and sum.
-      float x[16];
-#pragma unroll
-      for (int i = 0; i < TM; i++) {
-        x[2 * i] = rn[i];
-        x[2 * i + 1] = rd[i];
-      }
+      // then one FP64 atomic per row.
       int idx;
-      const float s = reduce16(x, idx);
-      const int r = row0 + ty * TM + (idx >> 1);
-      if (r < g.ec.n) atomicAdd(((idx & 1) ? g.den : g.num) + r, (double)s);
+      const float s = reduce16(rn, idx);
+      const int r = row0 + ty * TM + idx;
+      if (!(threadIdx.x & 8) && r < g.ec.n) atomicAdd(g.num + r, (double)s);
     }
-    // Column sums of the item: the two row groups of a warp (xor 16), then one
-    // FP64 atomic per column, sum and warp.
+    // Column sums of the item: the two row groups of a warp (xor 16, each half
+    // keeps four columns), then one FP64 atomic per column and warp.
     {
       const unsigned full_mask = 0xffffffffu;
       const bool hi = threadIdx.x & 16;
-      float y[TM];
 #pragma unroll
-      for (int j = 0; j < TM; j++) {
-        const float keep = hi ? cd[j] : cn[j], send = hi ? cn[j] : cd[j];
-        y[j] = keep + __shfl_xor_sync(full_mask, send, 16);
-      }
-#pragma unroll
-      for (int j = 0; j < TM; j++) {
-        const int q = col0 + tx * TM + j;
-        if (q < g.ec.n) atomicAdd((hi ? g.den : g.num) + q, (double)y[j]);
+      for (int j = 0; j < TM / 2; j++) {
+        const float keep = hi ? cn[TM / 2 + j] : cn[j], send = hi ? cn[j] : cn[TM / 2 + j];
+        const float y = keep + __shfl_xor_sync(full_mask, send, 16);
+        const int q = col0 + tx * TM + (hi ? TM / 2 : 0) + j;
+        if (q < g.ec.n) atomicAdd(g.num + q, (double)y);
       }
     }
   }
@@ -246,8 +226,7 @@ __global__ void __launch_bounds__(NT, 2) k_gram_fp32(Fp32Args g) {
 }  // namespace
 
 cudaError_t launch_gram_fp32(const float* U, int kp, const BlockParams* params, const float* tile_rmax,
-                             EpiConsts ec, double* num, double* den, int num_sms, cudaStream_t st, int shard,
-                             int n_shards) {
+                             EpiConsts ec, double* num, int num_sms, cudaStream_t st, int shard, int n_shards) {
   if (n_shards < 1 || shard < 0 || shard >= n_shards) return cudaErrorInvalidValue;
   if (ec.n <= 0) return cudaSuccess;
   Fp32Args g;
@@ -257,7 +236,6 @@ cudaError_t launch_gram_fp32(const float* U, int kp, const BlockParams* params, 
   g.tile_rmax = tile_rmax;
   g.ec = ec;
   g.num = num;
-  g.den = den;
   g.n_rb = (ec.n + BM - 1) / BM;
   // Items of up to 16 row blocks, fewer when that leaves under ~4 per SM slot.
   int L = 16;
@@ -282,6 +260,7 @@ cudaError_t launch_gram_fp32(const float* U, int kp, const BlockParams* params, 
     case kNrmseD: SRED_LAUNCH(kNrmseD); break;
     case kNrmseDW: SRED_LAUNCH(kNrmseDW); break;
     case kDebugDot: SRED_LAUNCH(kDebugDot); break;
+    case kDebugSum: SRED_LAUNCH(kDebugSum); break;
     default: SRED_LAUNCH(kAbsDiff); break;
   }
 #undef SRED_LAUNCH

@@ -65,10 +65,10 @@ constexpr int kEpiWarps = 16;                     // 4 per SM sub-partition
 constexpr int kThreads = (kEpiWarps + 2) * 32;
 constexpr int kEpiThreads = kEpiWarps * 32;
 constexpr int kRSlots = 2;                        // row-parameter ring depth
-constexpr int kRowR = 8 * kBM;                    // offset of r in a row-parameter slot
-constexpr int kRowMax = kRowR + kBM;              // offset of max r
+constexpr int kRowR = kBM, kRowS = 2 * kBM, kRowMu = 3 * kBM;  // r, sigma, mu in a row-parameter slot (a at 0)
+constexpr int kRowGrp = 4 * kBM;                  // the four 32-row groups' centres and half ranges
 constexpr int kRowFloats = kRowSoaFloats;         // one 128-row block's parameters
-constexpr int kRowPartBytes = 2 * 4 * kBM * 8;    // [2 buffers][4 column groups][128 rows] float2
+constexpr int kRowPartBytes = 2 * 4 * kBM * 4;    // [2 buffers][4 column groups][128 rows] floats
 constexpr int kMaxRun = 32;                       // row blocks per run (work item), at most
 constexpr int kBarBytes = 512;
 constexpr size_t kSmemBudget = 227 * 1024;
@@ -82,7 +82,7 @@ struct Cfg {
   static constexpr int kM = BN / kBM;               // row blocks per column tile
   static constexpr int kCSoa = col_soa_floats(BN);  // floats per column tile's parameters
   static constexpr int kBChunkBytes = BN * kChunk * 2;
-  static constexpr int kColAccBytes = kEpiThreads * 8 * kCH * 4;  // per thread: 2 sums x 4 columns x chunks
+  static constexpr int kScratch = 32 + kColW;       // floats of f and g per epilogue warp
 };
 
 struct TcArgs {
@@ -98,7 +98,6 @@ struct TcArgs {
   const float* rowsoa;          // per 128-row block, natural order
   EpiConsts ec;
   double* num;
-  double* den;
   int* status;
   unsigned long long timeout_ns;
   long long withhold;           // test hook: the producer never issues this tile's loads (-1: none)
@@ -260,9 +259,74 @@ __device__ __forceinline__ void tmem_wait8(uint32_t (&v)[8]) {
 
 // ---------------------------------------------------------------------------
 // Epilogue arithmetic on f32x2 pairs (two neighbouring columns of one row).
+//
+// The blocks are ordered by sigma, so the 32 rows and BN/4 columns of a warp's
+// slab have nearly equal a (the weight's argument). With a_p = alpha + dp and
+// a_q = beta + dq (alpha, beta: the slab's group centres),
+//   2^-(a_p - a_q)^2 = 2^-(a_p - beta)^2 * 2^(dq (2 (alpha - beta) - dq)) * 2^(2 dp dq)
+//                    = f_p * g_q * 2^(2 dp dq),
+// and the last factor is 1 + 2 ln2 dp dq + O((dp dq)^2). A slab whose largest
+// 2 ln2 |dp dq| is below kPureTol therefore needs no exponential per pair, and
+// no weight: its row sums are f_p sum_q g_q x_pq and its column sums
+// g_q sum_p f_p x_pq, with f and g computed once per row and column of the
+// slab (96 exponentials for 2,048 pairs). Up to kFirstTol the first-order
+// factor is applied per pair. The other smooth factors of a metric (Pearson's
+// 1/(1 + t), SSIM's 1/(sigma_p^2 + sigma_q^2 + c2)) split the same way; what
+// the split neglects is bounded per slab, and a slab over any bound (or with a
+// non-finite parameter) takes the pairwise form.
 // ---------------------------------------------------------------------------
 
-// Row constants, both halves equal (only the fields a metric uses survive).
+// Largest neglected relative term of a factorised weight: 2^-21 (4.8e-7, in one
+// corner of a slab; it changes sign with dp and dq, so the sums are off by far
+// less), the rounding error of the pairwise argument (a_p - a_q)^2 at weights
+// near 2^-8. First order: (6.9e-4)^2 / 2 = 2.4e-7.
+constexpr float kPureTol = 4.8e-7f;
+constexpr float kFirstTol = 6.9e-4f;
+// 2^-161 flushes to 0 in ex2.approx.ftz with any FP32 partner: all pair terms are 0.
+constexpr float kZeroDist = 12.7f;
+
+enum SlabMode { kPure = 0, kFirst = 1, kPairFirst = 2, kPairExact = 3, kZero = 4 };
+
+template <int METRIC>
+constexpr bool weighted_num() {
+  return METRIC == kPearson || METRIC == kSsim || METRIC == kNrmseW;
+}
+template <int METRIC>
+constexpr bool nrmse_tc() {
+  return METRIC == kNrmse || METRIC == kNrmseW;
+}
+
+// Coefficient of dp dq in the neglected factor: 2 ln2 for the weight, plus for
+// SSIM the mixed second derivative of 1 / (sigma_p^2 + sigma_q^2 + c2).
+template <int METRIC>
+__device__ __forceinline__ float mixed_coeff(float alpha, float beta, const EpiConsts& ec) {
+  float k = 1.3862944f;
+  if (METRIC == kSsim) {
+    const float sa = alpha * ec.inv_wscale, sb = beta * ec.inv_wscale;
+    const float S = fmaf(sa, sa, fmaf(sb, sb, ec.c2));
+    k += 4.0f * sa * sb * ec.inv_wscale * ec.inv_wscale / (S * S);
+  }
+  return k;
+}
+
+// The form a slab takes. rg, cg: {centre of a, half range of a, centre of r, half range of r}.
+template <int METRIC>
+__device__ __forceinline__ int slab_mode(const float4& rg, const float4& cg, const EpiConsts& ec) {
+  if (!weighted_num<METRIC>()) return kPairExact;
+  const float D = fabsf(rg.x - cg.x);
+  if (D - rg.y - cg.y > kZeroDist) return kZero;
+  const float e = mixed_coeff<METRIC>(rg.x, cg.x, ec) * rg.y * cg.y;
+  bool ok = e <= kFirstTol && D * cg.y <= 24.0f;
+  // Pearson: 1/(1+t) = its values through the group centres up to eps dr_p dr_q
+  if (METRIC == kPearson) ok = ok && kEps * rg.w * cg.w <= 1.2e-7f;
+  // SSIM: 2 sp sq G + c2 = 2 sp sq (G + c2/2 rp rq), so no block of sigma 0 and no overflow
+  if (METRIC == kSsim) ok = ok && rg.z - rg.w > 0.0f && cg.z - cg.w > 0.0f && (rg.z + rg.w) * (cg.z + cg.w) < 1e25f;
+  if (ok) return e <= kPureTol ? kPure : kFirst;
+  if (METRIC == kPearson && kEps * (rg.z + rg.w) * (cg.z + cg.w) < kTFirst) return kPairFirst;
+  return kPairExact;
+}
+
+// Row constants of the pairwise forms, both halves equal (only the fields a metric uses survive).
 struct RowC {
   F2 a, ne, r;                 // weight argument, -eps/sigma, 1/sigma (diagnostic terms)
   F2 mu2, sg2, mumu, s2, sg;   // 2 mu, 2 sigma, mu^2, sigma^2 + c2, sigma
@@ -271,19 +335,15 @@ struct RowC {
 template <int METRIC>
 __device__ __forceinline__ RowC make_rowc(const float* __restrict__ rs, int row, const EpiConsts& ec) {
   RowC c;
-  const float4 lo = *reinterpret_cast<const float4*>(rs + 8 * row);  // a, a, -eps r, -eps r
-  c.a = f2(lo.x, lo.y);
-  if (METRIC == kPearson) c.ne = f2(lo.z, lo.w);
-  if (METRIC == kDebugDot) {
-    const float r = rs[kRowR + row];
-    c.r = f2(r, r);
-  }
-  if (METRIC == kSsim || METRIC == kNrmse || METRIC == kNrmseW) {
-    const float4 hi = *reinterpret_cast<const float4*>(rs + 8 * row + 4);  // sigma, sigma, mu, mu
-    c.sg = f2(hi.x, hi.y);
+  auto dup = [](float v) { return f2(v, v); };
+  c.a = dup(rs[row]);
+  if (METRIC == kPearson) c.ne = dup(-kEps * rs[kRowR + row]);
+  if (METRIC == kDebugDot || METRIC == kDebugSum) c.r = dup(rs[kRowR + row]);
+  if (METRIC == kSsim || nrmse_tc<METRIC>()) {
+    c.sg = dup(rs[kRowS + row]);
     c.sg2 = add2(c.sg, c.sg);
     if (METRIC == kSsim) {
-      const F2 m = f2(hi.z, hi.w);
+      const F2 m = dup(rs[kRowMu + row]);
       c.mu2 = add2(m, m);
       c.mumu = mul2(m, m);
       c.s2 = fma2(c.sg, c.sg, f2(ec.c2, ec.c2));
@@ -292,16 +352,34 @@ __device__ __forceinline__ RowC make_rowc(const float* __restrict__ rs, int row,
   return c;
 }
 
-// Numerator factor x and weight w of two pairs; the numerator term is x w for
-// the weighted metrics and x for unweighted NRMSE (2D) and the diagnostic dot
-// product (whose "weight" is r_p + r_q). Same arithmetic as pair_terms.
-template <int METRIC, int CMODE>
+// NRMSE term of two pairs: sqrt(((K-1)/K)((s_p - s_q)^2 + 2 s_p s_q (1 - G))).
+// sqrt.approx (PTX: relative error at most 2^-23) instead of the correctly
+// rounded root, whose multi-instruction sequence took a third of the loop.
+__device__ __forceinline__ F2 nrmse_term2(F2 G, F2 sg, F2 sg2, F2 qs, const EpiConsts& ec) {
+  const F2 one = f2(1.0f, 1.0f), sc = f2(ec.nrmse_scale, ec.nrmse_scale);
+  const F2 ds = sub2(sg, qs);
+  float x0, x1;
+  f2_split(mul2(sc, fma2(ds, ds, mul2(mul2(sg2, qs), sub2(one, G)))), x0, x1);
+  return f2(sqrt_approx(fmaxf(x0, 0.0f)), sqrt_approx(fmaxf(x1, 0.0f)));
+}
+
+// Pairwise form: numerator factor x and weight w of two pairs; the term is x w
+// for the weighted metrics and x for unweighted NRMSE (2D) and the diagnostic
+// metrics. Same arithmetic as pair_terms.
+template <int METRIC, bool EXACT>
 __device__ __forceinline__ void terms2(F2 G, const RowC& rc, F2 qa, F2 qr, F2 qs, F2 qm, const EpiConsts& ec,
                                        F2& x, F2& w) {
   const F2 one = f2(1.0f, 1.0f);
   if (METRIC == kDebugDot) {
     x = mul2(G, mul2(rc.a, qa));
-    w = add2(rc.r, qr);
+    return;
+  }
+  if (METRIC == kDebugSum) {
+    x = add2(rc.r, qr);
+    return;
+  }
+  if (METRIC == kNrmse) {
+    x = nrmse_term2(G, rc.sg, rc.sg2, qs, ec);
     return;
   }
   const F2 d = sub2(rc.a, qa);
@@ -311,11 +389,8 @@ __device__ __forceinline__ void terms2(F2 G, const RowC& rc, F2 qa, F2 qr, F2 qs
   float x0, x1;
   if (METRIC == kPearson) {
     F2 gc;
-    if (CMODE == kCFirst) {
+    if (!EXACT) {
       gc = fma2(mul2(G, rc.ne), qr, G);  // G (1 - t)
-    } else if (CMODE == kCSecond) {
-      const F2 nt = mul2(rc.ne, qr);     // -t
-      gc = mul2(G, fma2(nt, add2(nt, one), one));  // G (1 - t + t^2)
     } else {
       float d0, d1;
       f2_split(sub2(one, mul2(rc.ne, qr)), d0, d1);  // 1 + t
@@ -331,17 +406,9 @@ __device__ __forceinline__ void terms2(F2 G, const RowC& rc, F2 qa, F2 qr, F2 qs
     f2_split(den, e0, e1);
     f2_split(mul2(num, f2(rcp_approx(e0), rcp_approx(e1))), q0, q1);
     x = f2(fmaxf(q0, 0.0f), fmaxf(q1, 0.0f));
-  } else {  // kNrmse, kNrmseW: ((K-1)/K)((s_p - s_q)^2 + 2 s_p s_q (1 - G))
-    const F2 sc = f2(ec.nrmse_scale, ec.nrmse_scale);
-    const F2 ds = sub2(rc.sg, qs);
-    f2_split(mul2(sc, fma2(ds, ds, mul2(mul2(rc.sg2, qs), sub2(one, G)))), x0, x1);
-    x = f2(sqrtf(fmaxf(x0, 0.0f)), sqrtf(fmaxf(x1, 0.0f)));
+  } else {  // kNrmseW
+    x = nrmse_term2(G, rc.sg, rc.sg2, qs, ec);
   }
-}
-
-template <int METRIC>
-constexpr bool weighted_num() {
-  return METRIC == kPearson || METRIC == kSsim || METRIC == kNrmseW;
 }
 
 // Exact squared distance of two FP32 unit vectors (NRMSE near-identical pairs).
@@ -354,6 +421,17 @@ __device__ __noinline__ float exact_diff2(const float* __restrict__ up, const fl
   return acc;
 }
 
+// Correction of a near-identical NRMSE pair: the term of the exact squared
+// difference minus the one nrmse_term2 added (recomputed with its arithmetic).
+__device__ __noinline__ float nrmse_correction(float g, float sp, float sq, int p, int q, const float* __restrict__ U,
+                                               int kp, int K, float scale) {
+  const float ds = __fsub_rn(sp, sq);
+  const float approx = sqrt_approx(fmaxf(
+      __fmul_rn(scale, __fmaf_rn(ds, ds, __fmul_rn(__fmul_rn(__fadd_rn(sp, sp), sq), __fsub_rn(1.0f, g)))), 0.0f));
+  const float D = (q == p) ? 0.0f : exact_diff2(U + (size_t)p * kp, U + (size_t)q * kp, K);
+  return sqrtf(__fmul_rn(scale, __fmaf_rn(ds, ds, __fmul_rn(__fmul_rn(sp, sq), D)))) - approx;
+}
+
 __device__ __forceinline__ void f2_add_half(F2& v, int half, float x) {
   float lo, hi;
   f2_split(v, lo, hi);
@@ -362,32 +440,173 @@ __device__ __forceinline__ void f2_add_half(F2& v, int half, float x) {
   v = f2(lo, hi);
 }
 
-template <int METRIC>
-constexpr bool nrmse_tc() {
-  return METRIC == kNrmse || METRIC == kNrmseW;
+// One 32-row x BN/4-column slab of a tile for this warp: BN/64 chunks of 16
+// columns, each read for both 16-lane halves of the warp's 32 TMEM lanes. Each
+// thread has 4 rows (32(w%4) + t/4 + 8k) and 4 columns per chunk (2(t%4) + {0, 1},
+// 8 + 2(t%4) + {0, 1}). rs: the tile's row parameters; cs: this warp's column
+// parameters (permuted); cacc[c][rep]: the item's column sums of this thread,
+// in registers; p0: block index of tile row 0; q0: of the slab's first column;
+// fs: this warp's scratch (32 + BN/4 floats). Row sums go to rsum[k].
+//
+// Factorised slab (FIRST: with the first-order weight factor per pair).
+template <int METRIC, int BN, bool FIRST>
+__device__ __forceinline__ void slab_factor(uint32_t taddr, const float* __restrict__ rs, const float* __restrict__ cs,
+                                            const float4& rg, const float4& cg, float* __restrict__ fs,
+                                            F2 (&cacc)[Cfg<BN>::kCH][2], const EpiConsts& ec, int p0, int q0,
+                                            float (&rsum)[4]) {
+  constexpr int CH = Cfg<BN>::kCH, W = Cfg<BN>::kColW;
+  const int lane = threadIdx.x & 31, rsub = lane >> 2, csub = lane & 3;
+  const int quarter = (threadIdx.x >> 5) & 3;
+  uint32_t buf[2][8];
+  tmem_ld8(taddr, buf[0]);
+  // f of row `lane` and g of columns (permuted positions) 2 lane, 2 lane + 1
+  const float sa = rg.x * ec.inv_wscale, sb = cg.x * ec.inv_wscale;
+  {
+    const int row = quarter * 32 + lane;
+    const float d = rs[row] - cg.x;
+    float f = ex2_approx(-d * d);
+    if (METRIC == kPearson) f *= ec.gscale * rcp_approx(fmaf(kEps * rs[kRowR + row], cg.z, 1.0f));
+    if (METRIC == kSsim) {
+      const float s = rs[kRowS + row];
+      f *= ec.gscale * 2.0f * s * rcp_approx(fmaf(s, s, fmaf(sb, sb, ec.c2)));
+    }
+    fs[(lane & 7) * 4 + (lane >> 3)] = f;
+    const float D2 = 2.0f * (rg.x - cg.x);
+    const float cn = METRIC == kPearson ? fmaf(kEps * rg.z, cg.z, 1.0f)
+                                        : (METRIC == kSsim ? fmaf(sa, sa, fmaf(sb, sb, ec.c2)) : 1.0f);
+#pragma unroll
+    for (int j = 0; j < W / 32; j++) {
+      const int i = lane + 32 * j;
+      const float dq = cs[i] - cg.x;
+      float g = ex2_approx(dq * (D2 - dq));
+      if (METRIC == kPearson) g *= cn * rcp_approx(fmaf(kEps * rg.z, cs[BN + i], 1.0f));
+      if (METRIC == kSsim) {
+        const float s = cs[2 * BN + i];
+        g *= s * cn * rcp_approx(fmaf(s, s, fmaf(sa, sa, ec.c2)));
+      }
+      fs[32 + i] = g;
+    }
+  }
+  __syncwarp();
+  const float4 f4 = *reinterpret_cast<const float4*>(fs + 4 * rsub);
+  const F2 fr[4] = {f2(f4.x, f4.x), f2(f4.y, f4.y), f2(f4.z, f4.z), f2(f4.w, f4.w)};
+  F2 rn[4], dp[4], mu[4], rr[4], sg[4];
+  const float kc = FIRST ? mixed_coeff<METRIC>(rg.x, cg.x, ec) : 0.0f;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    rn[k] = f2(0.0f, 0.0f);
+    const int row = quarter * 32 + rsub + 8 * k;
+    if (FIRST) {
+      const float v = kc * (rs[row] - rg.x);
+      dp[k] = f2(v, v);
+    }
+    if (METRIC == kSsim) {
+      const float m = rs[kRowMu + row], r = ec.c2h * rs[kRowR + row];
+      mu[k] = f2(m, m);
+      rr[k] = f2(r, r);
+    }
+    if (METRIC == kNrmseW) {
+      const float v = rs[kRowS + row];
+      sg[k] = f2(v, v);
+    }
+  }
+  tmem_wait8(buf[0]);
+#pragma unroll
+  for (int c = 0; c < CH; c++) {
+    const int cb = 16 * c + 4 * csub;
+    const float4 g4 = *reinterpret_cast<const float4*>(fs + 32 + cb);
+    float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f), s4 = r4, m4 = r4, a4 = r4;
+    if (FIRST) a4 = *reinterpret_cast<const float4*>(cs + cb);
+    if (METRIC == kSsim) {
+      r4 = *reinterpret_cast<const float4*>(cs + BN + cb);
+      m4 = *reinterpret_cast<const float4*>(cs + 3 * BN + cb);
+    }
+    if (METRIC == kNrmseW) s4 = *reinterpret_cast<const float4*>(cs + 2 * BN + cb);
+    const F2 qg[2] = {f2(g4.x, g4.y), f2(g4.z, g4.w)};
+    F2 cn[2] = {f2(0.0f, 0.0f), f2(0.0f, 0.0f)};
+#pragma unroll
+    for (int hh = 0; hh < 2; hh++) {
+      const int step = c * 2 + hh;
+      uint32_t(&cur)[8] = buf[step & 1];
+      uint32_t(&nxt)[8] = buf[(step + 1) & 1];
+      if (step + 1 < CH * 2) tmem_ld8(taddr + ((uint32_t)(16 * ((step + 1) & 1)) << 16) + 16 * ((step + 1) >> 1), nxt);
+      float near = 1.0f;  // NRMSE: smallest 1 - G
+#pragma unroll
+      for (int rep = 0; rep < 2; rep++) {
+        const F2 dq = FIRST ? sub2(rep ? f2(a4.z, a4.w) : f2(a4.x, a4.y), f2(cg.x, cg.x)) : f2(0.0f, 0.0f);
+        const F2 qr = rep ? f2(r4.z, r4.w) : f2(r4.x, r4.y);
+        const F2 qs = rep ? f2(s4.z, s4.w) : f2(s4.x, s4.y);
+        const F2 qm = rep ? f2(m4.z, m4.w) : f2(m4.x, m4.y);
+#pragma unroll
+        for (int kk = 0; kk < 2; kk++) {
+          const int kr = 2 * hh + kk;
+          const float g0 = __uint_as_float(cur[4 * rep + 2 * kk]), g1 = __uint_as_float(cur[4 * rep + 2 * kk + 1]);
+          F2 x;
+          if (METRIC == kPearson) {
+            x = f2(fmaxf(g0, 0.0f), fmaxf(g1, 0.0f));
+          } else if (METRIC == kSsim) {
+            const F2 c1 = f2(ec.c1, ec.c1), two = f2(2.0f, 2.0f);
+            const F2 m = mul2(mu[kr], qm);
+            float e0, e1, x0, x1;
+            f2_split(fma2(m, m, c1), e0, e1);
+            const F2 y = mul2(fma2(rr[kr], qr, f2(g0, g1)), fma2(m, two, c1));
+            f2_split(mul2(y, f2(rcp_approx(e0), rcp_approx(e1))), x0, x1);
+            x = f2(fmaxf(x0, 0.0f), fmaxf(x1, 0.0f));
+          } else {
+            const F2 G = mul2(f2(g0, g1), f2(ec.gscale, ec.gscale));
+            float t0, t1;
+            f2_split(G, t0, t1);
+            near = min3(near, 1.0f - t0, 1.0f - t1);
+            x = nrmse_term2(G, sg[kr], add2(sg[kr], sg[kr]), qs, ec);
+          }
+          if (FIRST) x = fma2(mul2(x, dp[kr]), dq, x);
+          rn[kr] = fma2(x, qg[rep], rn[kr]);
+          cn[rep] = fma2(x, fr[kr], cn[rep]);
+        }
+      }
+      if (METRIC == kNrmseW && near < 1.0f - ec.nrmse_near) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const int rep = j >> 2, kk = (j >> 1) & 1, lh = j & 1, kr = 2 * hh + kk;
+          const float g = __fmul_rn(__uint_as_float(cur[4 * rep + 2 * kk + lh]), ec.gscale);
+          if (!(g > ec.nrmse_near)) continue;
+          const int row = quarter * 32 + rsub + 8 * kr, q = q0 + 16 * c + 8 * rep + 2 * csub + lh;
+          const int ci = 16 * c + 4 * csub + 2 * rep + lh;  // permuted column slot
+          float corr = nrmse_correction(g, rs[kRowS + row], cs[2 * BN + ci], p0 + row, q, ec.U, ec.kp, ec.K,
+                                        ec.nrmse_scale);
+          if (FIRST) corr = fmaf(corr * kc * (rs[row] - rg.x), cs[ci] - cg.x, corr);
+          float glo, ghi, flo, fhi;
+          f2_split(qg[rep], glo, ghi);
+          f2_split(fr[kr], flo, fhi);
+          f2_add_half(rn[kr], lh, corr * (lh ? ghi : glo));
+          f2_add_half(cn[rep], lh, corr * flo);
+        }
+      }
+      if (step + 1 < CH * 2) tmem_wait8(nxt);
+    }
+    cacc[c][0] = fma2(cn[0], qg[0], cacc[c][0]);
+    cacc[c][1] = fma2(cn[1], qg[1], cacc[c][1]);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    float lo, hi, f, fh;
+    f2_split(rn[k], lo, hi);
+    f2_split(fr[k], f, fh);
+    rsum[k] = f * (lo + hi);
+  }
 }
 
-// One 32-row x BN/4-column slab of a tile for this warp: BN/64 chunks of 16
-// columns, each read for both 16-lane halves of the warp's 32 TMEM lanes.
-// rs: the tile's row parameters; cs: this warp's column parameters (permuted);
-// cacc: this thread's column accumulators in shared memory, float4 j at
-// cacc[j * kEpiThreads] for j = 2c + {0: num, 1: den}, each holding the
-// thread's four columns of chunk c (2(t%4) + {0, 1}, 8 + 2(t%4) + {0, 1});
-// p0: block index of tile row 0; q0: block index of the slab's first column.
-// The tile's row sums are returned in rsum[2k + {0: num, 1: den}] for rows
-// 32(w%4) + t/4 + 8k.
-// Row passes of the epilogue: the metrics with many row constants (SSIM,
-// NRMSE) take the 4 rows in two passes of 2 so that their constants fit in
-// registers; the column accumulators are then read and written once per pass.
+// Pairwise slab. Row passes: the metrics with many row constants (SSIM, NRMSE)
+// take the 4 rows in two passes of 2 so that their constants fit in registers.
 template <int METRIC>
 constexpr int row_passes() {
   return (METRIC == kSsim || METRIC == kNrmse || METRIC == kNrmseW) ? 2 : 1;
 }
 
-template <int METRIC, int BN, int CMODE, bool MASKED>
-__device__ __forceinline__ void sym_tile(uint32_t taddr, const float* __restrict__ rs, const float* __restrict__ cs,
-                                         float4* __restrict__ cacc, int p0, int q0, const EpiConsts& ec,
-                                         float (&rsum)[8]) {
+template <int METRIC, int BN, bool EXACT, bool MASKED>
+__device__ __forceinline__ void slab_pairs(uint32_t taddr, const float* __restrict__ rs, const float* __restrict__ cs,
+                                           F2 (&cacc)[Cfg<BN>::kCH][2], int p0, int q0, const EpiConsts& ec,
+                                           float (&rsum)[4]) {
   constexpr int CH = Cfg<BN>::kCH;
   constexpr int NP = row_passes<METRIC>(), R = 4 / NP;  // passes, rows per pass
   constexpr int HP = R / 2;                              // 16-lane halves per pass
@@ -396,14 +615,14 @@ __device__ __forceinline__ void sym_tile(uint32_t taddr, const float* __restrict
 #pragma unroll 1
   for (int pass = 0; pass < NP; pass++) {
     RowC rc[R];
-    F2 rn[R], rd[R];
+    F2 rn[R];
     int prow[R];
     bool force[R];
 #pragma unroll
     for (int kr = 0; kr < R; kr++) {
       const int row = quarter * 32 + rsub + 8 * (pass * R + kr);
       rc[kr] = make_rowc<METRIC>(rs, row, ec);
-      rn[kr] = rd[kr] = f2(0.0f, 0.0f);
+      rn[kr] = f2(0.0f, 0.0f);
       prow[kr] = p0 + row;
       force[kr] = MASKED && rs[kRowR + row] > 0.0f;
     }
@@ -415,15 +634,11 @@ __device__ __forceinline__ void sym_tile(uint32_t taddr, const float* __restrict
     tmem_wait8(buf[0]);
 #pragma unroll
     for (int c = 0; c < CH; c++) {
-      const float4 cnv = cacc[(2 * c) * kEpiThreads], cdv = cacc[(2 * c + 1) * kEpiThreads];
-      F2 cn[2] = {f2(cnv.x, cnv.y), f2(cnv.z, cnv.w)};
-      F2 cd[2] = {f2(cdv.x, cdv.y), f2(cdv.z, cdv.w)};
       const int cb = 16 * c + 4 * csub;
-      const float4 a4 = *reinterpret_cast<const float4*>(cs + cb);
-      float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f), s4 = r4, m4 = r4;
-      if (METRIC == kPearson || METRIC == kDebugDot) r4 = *reinterpret_cast<const float4*>(cs + BN + cb);
-      if (METRIC == kSsim || METRIC == kNrmse || METRIC == kNrmseW)
-        s4 = *reinterpret_cast<const float4*>(cs + 2 * BN + cb);
+      float4 a4 = make_float4(0.f, 0.f, 0.f, 0.f), r4 = a4, s4 = a4, m4 = a4;
+      if (METRIC != kNrmse && METRIC != kDebugSum) a4 = *reinterpret_cast<const float4*>(cs + cb);
+      if (METRIC == kPearson || METRIC == kDebugSum) r4 = *reinterpret_cast<const float4*>(cs + BN + cb);
+      if (METRIC == kSsim || nrmse_tc<METRIC>()) s4 = *reinterpret_cast<const float4*>(cs + 2 * BN + cb);
       if (METRIC == kSsim) m4 = *reinterpret_cast<const float4*>(cs + 3 * BN + cb);
 #pragma unroll
       for (int hh = 0; hh < HP; hh++) {
@@ -434,7 +649,7 @@ __device__ __forceinline__ void sym_tile(uint32_t taddr, const float* __restrict
           const int nc = (step + 1) / HP, nh = (step + 1) % HP;
           tmem_ld8(tp + ((uint32_t)(16 * nh) << 16) + 16 * nc, nxt);
         }
-        uint32_t near = 0;  // NRMSE: sign bits of (1 - delta) - G, any set = a near-identical pair
+        float near = 1.0f;  // NRMSE: smallest 1 - G
 #pragma unroll
         for (int rep = 0; rep < 2; rep++) {
           const F2 qa = rep ? f2(a4.z, a4.w) : f2(a4.x, a4.y);
@@ -445,52 +660,50 @@ __device__ __forceinline__ void sym_tile(uint32_t taddr, const float* __restrict
 #pragma unroll
           for (int kk = 0; kk < 2; kk++) {
             const int kr = 2 * hh + kk;
-            float g0 = __uint_as_float(cur[4 * rep + 2 * kk]), g1 = __uint_as_float(cur[4 * rep + 2 * kk + 1]);
+            F2 G = mul2(f2(__uint_as_float(cur[4 * rep + 2 * kk]), __uint_as_float(cur[4 * rep + 2 * kk + 1])),
+                        f2(ec.gscale, ec.gscale));
             const int p = prow[kr];
             if (MASKED) {
+              float g0, g1;
+              f2_split(G, g0, g1);
               if (force[kr] && qlo == p) g0 = 1.0f;
               if (force[kr] && qlo + 1 == p) g1 = 1.0f;
+              G = f2(g0, g1);
             }
             F2 x, w;
-            terms2<METRIC, CMODE>(f2(g0, g1), rc[kr], qa, qr, qs, qm, ec, x, w);
+            terms2<METRIC, EXACT>(G, rc[kr], qa, qr, qs, qm, ec, x, w);
             if (nrmse_tc<METRIC>()) {
-              float t0, t1;
-              f2_split(sub2(f2(ec.nrmse_near, ec.nrmse_near), f2(g0, g1)), t0, t1);
-              asm("lop3.b32 %0, %0, %1, %2, 0xFE;" : "+r"(near) : "r"(__float_as_uint(t0)), "r"(__float_as_uint(t1)));
+              float g0, g1;
+              f2_split(G, g0, g1);
+              near = min3(near, 1.0f - g0, 1.0f - g1);
             }
             if (!MASKED) {
               if (weighted_num<METRIC>()) {
                 rn[kr] = fma2(x, w, rn[kr]);
-                cn[rep] = fma2(x, w, cn[rep]);
+                cacc[c][rep] = fma2(x, w, cacc[c][rep]);
               } else {
                 rn[kr] = add2(rn[kr], x);
-                cn[rep] = add2(cn[rep], x);
+                cacc[c][rep] = add2(cacc[c][rep], x);
               }
-              rd[kr] = add2(rd[kr], w);
-              cd[rep] = add2(cd[rep], w);
             } else {
-              float x0, x1, w0, w1;
+              float x0, x1;
               f2_split(weighted_num<METRIC>() ? mul2(x, w) : x, x0, x1);
-              f2_split(w, w0, w1);
               const bool pv = p < ec.n;
               const bool r0 = pv && qlo >= p && qlo < ec.n, r1 = pv && qlo + 1 >= p && qlo + 1 < ec.n;
               const bool c0 = r0 && qlo != p, c1 = r1 && qlo + 1 != p;
               rn[kr] = add2(rn[kr], f2(r0 ? x0 : 0.0f, r1 ? x1 : 0.0f));
-              rd[kr] = add2(rd[kr], f2(r0 ? w0 : 0.0f, r1 ? w1 : 0.0f));
-              cn[rep] = add2(cn[rep], f2(c0 ? x0 : 0.0f, c1 ? x1 : 0.0f));
-              cd[rep] = add2(cd[rep], f2(c0 ? w0 : 0.0f, c1 ? w1 : 0.0f));
+              cacc[c][rep] = add2(cacc[c][rep], f2(c0 ? x0 : 0.0f, c1 ? x1 : 0.0f));
             }
           }
         }
-        if (nrmse_tc<METRIC>() && (int)near < 0) {
+        if (nrmse_tc<METRIC>() && near < 1.0f - ec.nrmse_near) {
           // Near-identical pairs: replace the accumulated term by the one of the
-          // exact squared difference (the same arithmetic as terms2 recomputes
-          // the term to remove).
+          // exact squared difference.
 #pragma unroll
           for (int j = 0; j < 8; j++) {
             const int rep = j >> 2, kk = (j >> 1) & 1, lh = j & 1;
             const int kr = 2 * hh + kk;
-            const float g = __uint_as_float(cur[4 * rep + 2 * kk + lh]);
+            const float g = __fmul_rn(__uint_as_float(cur[4 * rep + 2 * kk + lh]), ec.gscale);
             const int row = quarter * 32 + rsub + 8 * (pass * R + kr);
             const int p = prow[kr], q = q0 + 16 * c + 8 * rep + 2 * csub + lh;
             const bool rv = !MASKED || (p < ec.n && q >= p && q < ec.n);
@@ -498,79 +711,51 @@ __device__ __forceinline__ void sym_tile(uint32_t taddr, const float* __restrict
             float ge = g;
             if (MASKED && force[kr] && q == p) ge = 1.0f;
             if (!(ge > ec.nrmse_near) || !rv) continue;
-            const float sp = rs[8 * row + 4];
             const int ci = 16 * c + 4 * csub + 2 * rep + lh;  // permuted column slot
-            const float sq = cs[2 * BN + ci];
-            const float ds = __fsub_rn(sp, sq);
-            const float approx = sqrtf(fmaxf(
-                __fmul_rn(ec.nrmse_scale, __fmaf_rn(ds, ds, __fmul_rn(__fmul_rn(__fadd_rn(sp, sp), sq), __fsub_rn(1.0f, ge)))),
-                0.0f));
-            const float D = (q == p) ? 0.0f : exact_diff2(ec.U + (size_t)p * ec.kp, ec.U + (size_t)q * ec.kp, ec.K);
-            const float exact = sqrtf(__fmul_rn(ec.nrmse_scale, __fmaf_rn(ds, ds, __fmul_rn(__fmul_rn(sp, sq), D))));
-            float corr = exact - approx;
+            float corr = nrmse_correction(ge, rs[kRowS + row], cs[2 * BN + ci], p, q, ec.U, ec.kp, ec.K, ec.nrmse_scale);
             if (METRIC == kNrmseW) {
-              const float d = __fsub_rn(rs[8 * row], cs[ci]);
+              const float d = __fsub_rn(rs[row], cs[ci]);
               corr *= ex2_approx(-__fmul_rn(d, d));
             }
             f2_add_half(rn[kr], lh, corr);
-            if (cv) f2_add_half(cn[rep], lh, corr);
+            if (cv) f2_add_half(cacc[c][rep], lh, corr);
           }
         }
         if (step + 1 < CH * HP) tmem_wait8(nxt);
       }
-      float4 o;
-      f2_split(cn[0], o.x, o.y);
-      f2_split(cn[1], o.z, o.w);
-      cacc[(2 * c) * kEpiThreads] = o;
-      f2_split(cd[0], o.x, o.y);
-      f2_split(cd[1], o.z, o.w);
-      cacc[(2 * c + 1) * kEpiThreads] = o;
     }
 #pragma unroll
     for (int kr = 0; kr < R; kr++) {
-      float lo, hi, n, d;
+      float lo, hi;
       f2_split(rn[kr], lo, hi);
-      n = lo + hi;
-      f2_split(rd[kr], lo, hi);
-      d = lo + hi;
-      if (pass == 0) {  // compile-time indices into rsum (the pass loop is not unrolled)
-        rsum[2 * kr] = n;
-        rsum[2 * kr + 1] = d;
-      } else {
-        rsum[2 * (R + kr)] = n;
-        rsum[2 * (R + kr) + 1] = d;
-      }
+      // compile-time indices into rsum (the pass loop is not unrolled)
+      if (pass == 0) rsum[kr] = lo + hi;
+      else rsum[(NP - 1) * R + kr] = lo + hi;
     }
   }
 }
 
-// Row sums of the 4 lanes that share rows (lanes 4i..4i+3): x[2k + s] holds
-// row k's sum s; lane t ends with (num, den) of row k = 2 (t & 1) + ((t >> 1) & 1).
-__device__ __forceinline__ float2 reduce_rows4(const float (&x)[8]) {
+// Row sums of the 4 lanes that share rows (lanes 4i..4i+3): x[k] holds row k's
+// partial; lane t ends with row k = 2 (t & 1) + ((t >> 1) & 1).
+__device__ __forceinline__ float reduce_rows4(const float (&x)[4]) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const bool b0 = lane & 1, b1 = lane & 2;
-  float y[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const float keep = b0 ? x[4 + i] : x[i], send = b0 ? x[i] : x[4 + i];
-    y[i] = keep + __shfl_xor_sync(full, send, 1);
-  }
-  float z[2];
+  float y[2];
 #pragma unroll
   for (int i = 0; i < 2; i++) {
-    const float keep = b1 ? y[2 + i] : y[i], send = b1 ? y[i] : y[2 + i];
-    z[i] = keep + __shfl_xor_sync(full, send, 2);
+    const float keep = b0 ? x[2 + i] : x[i], send = b0 ? x[i] : x[2 + i];
+    y[i] = keep + __shfl_xor_sync(full, send, 1);
   }
-  return make_float2(z[0], z[1]);
+  const float keep = b1 ? y[1] : y[0], send = b1 ? y[0] : y[1];
+  return keep + __shfl_xor_sync(full, send, 2);
 }
 
 // Column sums of the 8 lanes that share columns (lanes with equal t % 4),
-// then one FP64 atomic add per column and sum. x index:
-// ((c * 2 + rep) * 2 + lohi) * 2 + sum, column 16c + 8rep + 2(t % 4) + lohi.
+// then one FP64 atomic add per column. x index: (c * 2 + rep) * 2 + lohi,
+// column 16c + 8rep + 2(t % 4) + lohi.
 template <int NV>
-__device__ __forceinline__ void flush_columns(const float (&x)[NV], int q0, const EpiConsts& ec, double* num,
-                                              double* den) {
+__device__ __forceinline__ void flush_columns(const float (&x)[NV], int q0, const EpiConsts& ec, double* num) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, csub = lane & 3;
   const int b1 = (lane >> 2) & 1, b2 = (lane >> 3) & 1, b3 = (lane >> 4) & 1;
@@ -593,9 +778,9 @@ __device__ __forceinline__ void flush_columns(const float (&x)[NV], int q0, cons
 #pragma unroll
   for (int j = 0; j < NV / 8; j++) {
     const int i = b1 * (NV / 2) + b2 * (NV / 4) + b3 * (NV / 8) + j;
-    const int c = i >> 3, rep = (i >> 2) & 1, lohi = (i >> 1) & 1, s = i & 1;
+    const int c = i >> 2, rep = (i >> 1) & 1, lohi = i & 1;
     const int q = q0 + 16 * c + 8 * rep + 2 * csub + lohi;
-    if (q < ec.n) atomicAdd((s ? den : num) + q, (double)u[j]);
+    if (q < ec.n) atomicAdd(num + q, (double)u[j]);
   }
 }
 
@@ -754,12 +939,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t sC = sA + (TR ? 2 * g.a_bytes : S * kAChunkBytes);    // 2 column-parameter slots
   const uint32_t sR = sC + 2 * C::kCSoa * 4;                           // kRSlots row-parameter slots
   const uint32_t sP = sR + kRSlots * kRowFloats * 4;                   // row partials
-  const uint32_t sQ = sP + kRowPartBytes;                              // column accumulators
-  const uint32_t sBar = sQ + C::kColAccBytes;
+  const uint32_t sF = sP + kRowPartBytes;                              // f and g of each epilogue warp
+  const uint32_t sBar = sF + kEpiWarps * C::kScratch * 4;
   const float* cslots = reinterpret_cast<const float*>(sbase + (sC - base));
   const float* rslots = reinterpret_cast<const float*>(sbase + (sR - base));
-  float2* rowpart = reinterpret_cast<float2*>(sbase + (sP - base));
-  float4* colacc = reinterpret_cast<float4*>(sbase + (sQ - base));
+  float* rowpart = reinterpret_cast<float*>(sbase + (sP - base));
+  float* scratch = reinterpret_cast<float*>(sbase + (sF - base));
   // barriers: a_full[16], a_empty[16], b_full, b_empty, acc_full[2], acc_empty[2],
   //           c_full[2], c_empty[2], r_full[2], r_empty[2], done; then the TMEM
   //           address and 8 row-partial counters
@@ -987,11 +1172,11 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (!mbar_wait(b_cfull + 8 * cs, (item_i >> 1) & 1, g, ST_TIMEOUT_EPI)) { ok = false; break; }
       item_i++;
       const float* csl = cslots + cs * C::kCSoa;
-      const float rmax_c = csl[4 * BN];
+      const float4 cg = *reinterpret_cast<const float4*>(csl + 4 * BN + 4 * group);
       const int q0 = ct * BN + group * C::kColW;
-      float4* cacc = colacc + threadIdx.x;
+      F2 cacc[CH][2];
 #pragma unroll
-      for (int j = 0; j < 2 * CH; j++) cacc[j * kEpiThreads] = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int c = 0; c < CH; c++) cacc[c][0] = cacc[c][1] = f2(0.0f, 0.0f);
       for (int rb = rb0; ok && rb < rb1; rb++, tile++) {
         const uint32_t b = (uint32_t)(tile & 1);
         const uint32_t rsl = (uint32_t)(tile & (kRSlots - 1));
@@ -1005,17 +1190,23 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + b * BN + group * C::kColW;
         const int p0 = rb * kBM;
         const float* csw = csl + group * C::kColW;
-        float rsum[8];
+        float rsum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if constexpr (kPhase == 1) {
-          sym_tile<METRIC, BN, kCExact, true>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
+          slab_pairs<METRIC, BN, true, true>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
+        } else if constexpr (!weighted_num<METRIC>()) {
+          slab_pairs<METRIC, BN, true, false>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
         } else {
-          const int cm = METRIC == kPearson ? c_mode(kEps * rsp[kRowMax] * rmax_c) : kCFirst;
-          if (cm == kCFirst)
-            sym_tile<METRIC, BN, kCFirst, false>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
-          else if (METRIC == kPearson && cm == kCSecond)
-            sym_tile<METRIC, BN, kCSecond, false>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
-          else
-            sym_tile<METRIC, BN, kCExact, false>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
+          const float4 rg = *reinterpret_cast<const float4*>(rsp + kRowGrp + 4 * quarter);
+          float* fs = scratch + warp * C::kScratch;
+          const int mode = slab_mode<METRIC>(rg, cg, g.ec);
+          if (mode == kPure)
+            slab_factor<METRIC, BN, false>(taddr, rsp, csw, rg, cg, fs, cacc, g.ec, p0, q0, rsum);
+          else if (mode == kFirst)
+            slab_factor<METRIC, BN, true>(taddr, rsp, csw, rg, cg, fs, cacc, g.ec, p0, q0, rsum);
+          else if (METRIC == kPearson && mode == kPairFirst)
+            slab_pairs<METRIC, BN, false, false>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
+          else if (mode == kPairExact)
+            slab_pairs<METRIC, BN, true, false>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
         }
         tc_fence_before();
         // Row sums: 4 lanes per row, then the 4 column-group warps of this
@@ -1023,9 +1214,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         // partials adds the four (fixed order) and issues one atomic per row
         // and sum. It releases the accumulator only after reading, so no warp
         // overwrites these partials (two tiles later) before they are read.
-        const float2 z = reduce_rows4(rsum);
+        const float z = reduce_rows4(rsum);
         const int krow = 2 * (lane & 1) + ((lane >> 1) & 1);
-        float2* rp = rowpart + b * (4 * kBM);
+        float* rp = rowpart + b * (4 * kBM);
         rp[group * kBM + quarter * 32 + (lane >> 2) + 8 * krow] = z;
         __syncwarp();
         unsigned last = 0;
@@ -1043,18 +1234,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (last) {
           __syncwarp();
           const int row = quarter * 32 + lane;
-          float sn = 0.0f, sd = 0.0f;
+          float sn = 0.0f;
 #pragma unroll
-          for (int gg = 0; gg < 4; gg++) {
-            const float2 v = rp[gg * kBM + row];
-            sn += v.x;
-            sd += v.y;
-          }
+          for (int gg = 0; gg < 4; gg++) sn += rp[gg * kBM + row];
           const int p = p0 + row;
-          if (p < g.ec.n) {
-            atomicAdd(g.num + p, (double)sn);
-            atomicAdd(g.den + p, (double)sd);
-          }
+          if (p < g.ec.n) atomicAdd(g.num + p, (double)sn);
         }
         __syncwarp();
         if (lane == 0) {
@@ -1064,21 +1248,12 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       if (!ok) break;
       // Column sums of the item.
-      float x[8 * CH];
+      float x[4 * CH];
 #pragma unroll
-      for (int c = 0; c < CH; c++) {
-        const float4 nv = cacc[(2 * c) * kEpiThreads], dv = cacc[(2 * c + 1) * kEpiThreads];
-        const float ns[4] = {nv.x, nv.y, nv.z, nv.w}, ds[4] = {dv.x, dv.y, dv.z, dv.w};
+      for (int c = 0; c < CH; c++)
 #pragma unroll
-        for (int r = 0; r < 2; r++)
-#pragma unroll
-          for (int lh = 0; lh < 2; lh++) {
-            const int i = ((c * 2 + r) * 2 + lh) * 2;
-            x[i] = ns[2 * r + lh];
-            x[i + 1] = ds[2 * r + lh];
-          }
-      }
-      flush_columns<8 * CH>(x, q0, g.ec, g.num, g.den);
+        for (int r = 0; r < 2; r++) f2_split(cacc[c][r], x[(c * 2 + r) * 2], x[(c * 2 + r) * 2 + 1]);
+      flush_columns<4 * CH>(x, q0, g.ec, g.num);
       __syncwarp();
       if (lane == 0) mbar_arrive(b_cempty + 8 * cs);
     }
@@ -1091,44 +1266,52 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // Column parameters of each BN-column tile, permuted so that thread t of an
 // epilogue warp finds its four columns of a 16-column chunk (2(t%4) + {0, 1}
-// and 8 + 2(t%4) + {0, 1}) in one float4 (col_soa_pos), with the tile's
-// largest 1/sigma; and the row parameters of each 128-row block as the
-// epilogue's f32x2 pairs (kRowSoaFloats) with the block's largest 1/sigma.
+// and 8 + 2(t%4) + {0, 1}) in one float4 (col_soa_pos), and the row parameters
+// of each 128-row block, in order; each followed by the centre and half range
+// of a and r over its four groups (BN/4 columns, 32 rows), which the epilogue's
+// slab forms are chosen by. A NaN makes its group's ranges NaN.
 // Blocks [0, n_ctp): column tiles; [n_ctp, n_ctp + n_rbp): row blocks.
 template <int BN>
 __global__ void k_sym_soa(const BlockParams* __restrict__ params, int n_ctp, float* __restrict__ colsoa,
                           float* __restrict__ rowsoa) {
   const int i = threadIdx.x;
-  __shared__ float wm[8];
+  __shared__ float4 wm[8];
   const bool col = blockIdx.x < n_ctp;
   const int width = col ? BN : kBM;
   const int tile = col ? blockIdx.x : blockIdx.x - n_ctp;
   float* o = col ? colsoa + (size_t)tile * col_soa_floats(BN) : rowsoa + (size_t)tile * kRowSoaFloats;
-  float r = 0.0f;
   if (i < width) {
     const BlockParams p = params[(size_t)tile * width + i];
-    if (col) {
-      const int pos = col_soa_pos(i);
-      o[pos] = p.a;
-      o[width + pos] = p.r;
-      o[2 * width + pos] = p.sigma;
-      o[3 * width + pos] = p.mu;
-    } else {
-      const float ne = -kEps * p.r;
-      reinterpret_cast<float4*>(o + 8 * i)[0] = make_float4(p.a, p.a, ne, ne);
-      reinterpret_cast<float4*>(o + 8 * i)[1] = make_float4(p.sigma, p.sigma, p.mu, p.mu);
-      o[kRowR + i] = p.r;
+    const int pos = col ? col_soa_pos(i) : i;
+    o[pos] = p.a;
+    o[width + pos] = p.r;
+    o[2 * width + pos] = p.sigma;
+    o[3 * width + pos] = p.mu;
+    float4 m = make_float4(p.a, p.a, p.r, p.r);
+    const bool bad = !(p.a - p.a == 0.0f) || !(p.r - p.r == 0.0f);
+    for (int s = 16; s; s >>= 1) {
+      m.x = fminf(m.x, __shfl_xor_sync(0xffffffffu, m.x, s));
+      m.y = fmaxf(m.y, __shfl_xor_sync(0xffffffffu, m.y, s));
+      m.z = fminf(m.z, __shfl_xor_sync(0xffffffffu, m.z, s));
+      m.w = fmaxf(m.w, __shfl_xor_sync(0xffffffffu, m.w, s));
     }
-    r = p.r;
+    if (__any_sync(0xffffffffu, bad)) m = make_float4(nanf(""), nanf(""), nanf(""), nanf(""));
+    if ((i & 31) == 0) wm[i >> 5] = m;
   }
-  for (int s = 16; s; s >>= 1) r = fmaxf(r, __shfl_xor_sync(0xffffffffu, r, s));
-  if ((i & 31) == 0) wm[i >> 5] = r;
   __syncthreads();
   if (i < 4) {
-    float m = 0.0f;
-    if (i == 0)
-      for (int w = 0; w < (int)(blockDim.x >> 5); w++) m = fmaxf(m, wm[w]);
-    o[(col ? 4 * width : kRowMax) + i] = m;
+    const int per = width / 128;  // warps per group
+    float4 m = wm[i * per];
+    if (per == 2) {
+      const float4 b = wm[i * per + 1];
+      const bool bad = m.x != m.x || b.x != b.x;
+      m = make_float4(fminf(m.x, b.x), fmaxf(m.y, b.y), fminf(m.z, b.z), fmaxf(m.w, b.w));
+      if (bad) m.x = m.y = m.z = m.w = nanf("");
+    }
+    // half ranges rounded up, so that they bound the distance to the rounded centre
+    const float ca = 0.5f * (m.x + m.y), cr = 0.5f * (m.z + m.w);
+    reinterpret_cast<float4*>(o + 4 * width)[i] =
+        make_float4(ca, fmaxf(m.y - ca, ca - m.x) * 1.0000002f, cr, fmaxf(m.w - cr, cr - m.z) * 1.0000002f);
   }
 }
 
@@ -1161,7 +1344,7 @@ bool make_map(CUtensorMap* m, const __nv_bfloat16* ptr, int kq, int rows, int bo
 
 size_t fixed_smem(int bn) {
   return 1024 + 2 * (size_t)col_soa_floats(bn) * 4 + kRSlots * kRowFloats * 4 + kRowPartBytes +
-         (size_t)kEpiThreads * 8 * (bn / 64) * 4 + kBarBytes;
+         (size_t)kEpiWarps * (32 + bn / 4) * 4 + kBarBytes;
 }
 
 }  // namespace
@@ -1220,8 +1403,8 @@ long long gram_tc_items(int n, int bn, int* L_out, int num_sms, int max_L) {
 }
 
 cudaError_t launch_gram_tc(const __nv_bfloat16* A, const __nv_bfloat16* B, int kq, int n_pad,
-                           const BlockParams* params, float* soa_ws, EpiConsts ec, double* num, double* den,
-                           int num_sms, int* status, cudaStream_t st, int shard, int n_shards,
+                           const BlockParams* params, float* soa_ws, EpiConsts ec, double* num, int num_sms,
+                           int* status, cudaStream_t st, int shard, int n_shards,
                            const TcDebug* dbg, const TcChoice* choice) {
   TcPlan plan;
   const bool planned = choice && choice->bn ? plan_shape(kq, choice->bn, choice->tr != 0, &plan)
@@ -1256,7 +1439,6 @@ cudaError_t launch_gram_tc(const __nv_bfloat16* A, const __nv_bfloat16* B, int k
   g.rowsoa = rowsoa;
   g.ec = ec;
   g.num = num;
-  g.den = den;
   g.status = status;
   g.timeout_ns = dbg && dbg->timeout_ns ? dbg->timeout_ns : 4000000000ull;
   g.withhold = dbg ? dbg->withhold_tile : -1;
@@ -1290,6 +1472,7 @@ cudaError_t launch_gram_tc(const __nv_bfloat16* A, const __nv_bfloat16* B, int k
     case kNrmse: SRED_TC(kNrmse); break;
     case kNrmseW: SRED_TC(kNrmseW); break;
     case kDebugDot: SRED_TC(kDebugDot); break;
+    case kDebugSum: SRED_TC(kDebugSum); break;
     default: return cudaErrorInvalidValue;
   }
 #undef SRED_TC

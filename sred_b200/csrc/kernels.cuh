@@ -24,7 +24,7 @@ __global__ void k_scatter(const uint8_t* flags, size_t n, const int2* offs, int*
                           int* slot);
 __global__ void k_pack(const float* img, int W, Ellipse e, const int* gram_pix, int n, float wscale, int mode,
                        float* U, int kp, __nv_bfloat16* A, __nv_bfloat16* B, int kq, BlockParams* params,
-                       float* tile_rmax, double* sums);
+                       float* tile_rmax, double* sums, unsigned* arange);
 __global__ void k_finalize(const int* slot, int W, int H, int rw, int rh, const double* num, const double* den,
                            const BlockParams* params, const double* sums, int n_flat, int metric, double sk,
                            double n_pixels, const float* mask, int apply_mask, float* out);

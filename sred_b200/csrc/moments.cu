@@ -233,6 +233,7 @@ __global__ void k_scatter(const uint8_t* __restrict__ flags, size_t n, const int
 //   sums[0] = sum_q 2^-(a_q)^2           (weight of a pair with a flat block)
 //   sums[1] = sum_q sqrt((K-1)/K) sigma_q (NRMSE against a flat block)
 //   sums[2] = sum_q sigma_q 2^-(a_q)^2     (Abs-diff against a flat block)
+// and the range of a (arange: launch_den, weights.cuh).
 // The block sums are warp-wide reductions, one block after another; the
 // per-block scalar work (square roots, quotients, exp2, params) then runs on
 // lane k for block k of the 32, instead of on one lane per block while the
@@ -245,7 +246,7 @@ __global__ void k_pack(const float* __restrict__ img, int W, Ellipse e, const in
                        int n, float wscale, int mode, float* __restrict__ U, int kp,
                        __nv_bfloat16* __restrict__ A, __nv_bfloat16* __restrict__ B, int kq,
                        BlockParams* __restrict__ params, float* __restrict__ tile_rmax,
-                       double* __restrict__ sums) {
+                       double* __restrict__ sums, unsigned* __restrict__ arange) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -254,6 +255,7 @@ __global__ void k_pack(const float* __restrict__ img, int W, Ellipse e, const in
   const double sk = sqrt((double)(K - 1) / (double)K);
   const double rK = __drcp_rn((double)K);  // s / K as div_fixed: the correctly rounded quotient
   double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
+  unsigned a_lo = 0u, a_hi = 0u;  // ~bits of the smallest a, bits of the largest
   for (long long j0 = 32LL * gw; j0 < n; j0 += 32LL * nw) {
     const int nb = (int)min(32LL, (long long)n - j0);
     // The sum and centred sum of squares of each block; lane k keeps block k's.
@@ -292,6 +294,8 @@ __global__ void k_pack(const float* __restrict__ img, int W, Ellipse e, const in
       bp.mu = (float)mu;
       bp.pad0 = bp.pad1 = bp.pad2 = 0.0f;
       params[j] = bp;
+      a_lo = max(a_lo, ~__float_as_uint(bp.a));
+      a_hi = max(a_hi, __float_as_uint(bp.a));
       atomicMax(reinterpret_cast<int*>(tile_rmax) + (j >> 7), __float_as_int(bp.r));
       const double a = sigma * (double)wscale;
       const double w0 = exp2(-(a * a));
@@ -319,6 +323,12 @@ __global__ void k_pack(const float* __restrict__ img, int W, Ellipse e, const in
         }
       }
     }
+  }
+  a_lo = __reduce_max_sync(full, a_lo);
+  a_hi = __reduce_max_sync(full, a_hi);
+  if (lane == 0) {
+    atomicMax(arange, a_lo);
+    atomicMax(arange + 1, a_hi);
   }
   for (int o = 16; o; o >>= 1) {
     acc0 += __shfl_xor_sync(full, acc0, o);

@@ -16,11 +16,13 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "order.cuh"
 #include "shape.cuh"
 #include "cluster.cuh"
 #include "gat_tree.cuh"
 #include "relevance.cuh"
 #include "volume.cuh"
+#include "weights.cuh"
 
 using namespace sred;
 
@@ -29,7 +31,7 @@ namespace {
 enum BufId {
   B_IMG, B_MEANS, B_STDS, B_MASK, B_MASKIN, B_FLAGS, B_SLOT, B_GPIX, B_FPIX, B_COUNTS, B_U, B_A, B_B,
   B_PARAMS, B_RMAX, B_NUM, B_DEN, B_SUMS, B_OUT, B_VARS, B_MM, B_NMASK, B_BAD, B_STATUS, B_STDS2, B_COLSOA,
-  B_FEAT, B_SIG, B_FR, B_FI, B_GAT, B_OFF3, B_REF3, B_STAT, B_THR, B_KMX, B_KMD2, B_KMLAB, B_KMB, B_TBOX, B_TSTAT, B_TMEAN, B_TVAR, B_STKIN, B_STKOUT,
+  B_FEAT, B_SIG, B_FR, B_FI, B_GAT, B_OFF3, B_REF3, B_STAT, B_THR, B_KMX, B_KMD2, B_KMLAB, B_KMB, B_TBOX, B_TSTAT, B_TMEAN, B_TVAR, B_STKIN, B_STKOUT, B_SORT, B_NODES, B_SLICES,
   B_NBUF
 };
 
@@ -47,8 +49,8 @@ struct GState {
   int d = 1, rd = 0;
   int metric = 0, w = 0, h = 0, rw = 0, rh = 0, K = 0, n_g = 0, n_flat = 0, engine = 0, kp = 0, kq = 0;
   size_t n = 0, n_pad = 0;
-  float nv = 0, thr = 0, npx = 0, relc = 0;
-  bool given = false;
+  float nv = 0, thr = 0, npx = 0, relc = 0, wscale = 0;
+  bool given = false, sorted = false;
 };
 
 }  // namespace
@@ -251,6 +253,27 @@ struct GivenStats {
 };
 
 
+// The tensor-core engine's weighted metrics run on blocks in order of sigma
+// (their weights factorise, global_tc.cu); unweighted NRMSE and the FP32 engine
+// take the blocks in raster order, whose pixels overlap while packing.
+bool sort_for(int engine, int metric) {
+  return engine == SRED_ENGINE_TC && (metric == kPearson || metric == kSsim || metric == kNrmseW);
+}
+
+sred_status sort_blocks(sred_ctx* c, const float* d_stds, int n_g, cudaStream_t st) {
+  int* d_ws;
+  CKS(ensure(c, B_SORT, sort_workspace_ints(n_g), &d_ws));
+  CK(launch_sort_blocks(d_stds, static_cast<int*>(c->buf[B_GPIX].p), n_g, d_ws, static_cast<int*>(c->buf[B_SLOT].p),
+                        st));
+  return SRED_OK;
+}
+
+// Kernels of a map between the statistics and the finalisation.
+int contraction_launches(int n_g, int engine, bool sorted) {
+  if (n_g == 0) return 0;
+  return (engine == SRED_ENGINE_TC ? 3 : 2) + kDenLaunches + (sorted ? kSortLaunches : 0);
+}
+
 // Phase 1: everything before the all-pairs contraction.
 sred_status global_prepare(sred_ctx* c, int metric, const float* d_img, int w, int h, int bw, int bh, float relc,
                            cudaStream_t st, const GivenStats* given, GState* gs) {
@@ -326,7 +349,7 @@ sred_status global_prepare(sred_ctx* c, int metric, const float* d_img, int w, i
   CKS(ensure(c, B_RMAX, n_pad / 128, &d_rmax));
   CKS(ensure(c, B_NUM, n_pad, &d_num));
   CKS(ensure(c, B_DEN, n_pad, &d_den));
-  CKS(ensure(c, B_SUMS, 4, &d_sums));
+  CKS(ensure(c, B_SUMS, 8, &d_sums));  // the flat blocks' sums, then the range of a
   if (engine == SRED_ENGINE_FP32 || metric == kNrmse) {  // tensor-core NRMSE reads U for near-identical pairs
     CKS(ensure(c, B_U, n_pad * kp, &d_U));
     CK(cudaMemsetAsync(d_U + (size_t)n_g * kp, 0, (n_pad - n_g) * kp * sizeof(float), st));
@@ -340,8 +363,9 @@ sred_status global_prepare(sred_ctx* c, int metric, const float* d_img, int w, i
   CK(cudaMemsetAsync(d_params + n_g, 0, (n_pad - n_g) * sizeof(BlockParams), st));
   CK(cudaMemsetAsync(d_rmax, 0, (n_pad / 128) * sizeof(float), st));
   CK(cudaMemsetAsync(d_num, 0, n_pad * sizeof(double), st));
-  CK(cudaMemsetAsync(d_den, 0, n_pad * sizeof(double), st));
-  CK(cudaMemsetAsync(d_sums, 0, 4 * sizeof(double), st));
+  CK(cudaMemsetAsync(d_sums, 0, 8 * sizeof(double), st));
+  const bool sorted = sort_for(engine, metric);
+  if (sorted) CKS(sort_blocks(c, d_stds, n_g, st));
   // weight = exp(-(s_p - s_q)^2 / (FILTER_PARAM + EPSILON)) = 2^-(a_p - a_q)^2,
   // FILTER_PARAM + EPSILON summed in FP32 as the reference kernel does.
   const float hden = nv + kEps;
@@ -351,7 +375,7 @@ sred_status global_prepare(sred_ctx* c, int metric, const float* d_img, int w, i
     const int pgrid = grid_for(((size_t)n_g + 31) / 32 * 32, 256, 8 * c->num_sms);
     const int mode = engine == SRED_ENGINE_FP32 ? 0 : split_levels_for(metric, K) - 1;
     k_pack<<<pgrid, 256, 0, st>>>(d_img, w, e, d_gpix, n_g, wscale, mode, d_U, kp, d_A, d_B, kq, d_params,
-                                  d_rmax, d_sums);
+                                  d_rmax, d_sums, reinterpret_cast<unsigned*>(d_sums + 4));
     CK(cudaGetLastError());
   }
   if (engine == SRED_ENGINE_TC) {
@@ -376,13 +400,32 @@ sred_status global_prepare(sred_ctx* c, int metric, const float* d_img, int w, i
   gs->thr = thr;
   gs->npx = npx;
   gs->relc = relc;
+  gs->wscale = wscale;
+  gs->sorted = sorted;
   gs->given = given != nullptr;
   gs->valid = true;
   return SRED_OK;
 }
 
+// The denominators of a prepared map's blocks into the den workspace. They are
+// one pass over all blocks: shard 0's share of the sums; the other shards' is 0.
+sred_status denominators(sred_ctx* c, const GState& gs, cudaStream_t st, int shard) {
+  double *d_den = static_cast<double*>(c->buf[B_DEN].p), *d_nodes;
+  if (shard != 0) {
+    CK(cudaMemsetAsync(d_den, 0, gs.n_g * sizeof(double), st));
+    return SRED_OK;
+  }
+  float2* d_slices;
+  CKS(ensure(c, B_NODES, kDenNodes, &d_nodes));
+  CKS(ensure(c, B_SLICES, den_slices(gs.n_g), &d_slices));
+  CK(launch_den(static_cast<const BlockParams*>(c->buf[B_PARAMS].p), gs.n_g,
+                reinterpret_cast<const unsigned*>(static_cast<double*>(c->buf[B_SUMS].p) + 4), d_nodes, d_slices, d_den,
+                st));
+  return SRED_OK;
+}
+
 // Phase 2: the all-pairs contraction (work-item range `shard` of n_shards of
-// the upper triangle) into the num/den workspaces.
+// the upper triangle) into the num workspace, and the denominators.
 sred_status global_gram(sred_ctx* c, const GState& gs, cudaStream_t st, int shard, int n_shards) {
   if (gs.n_g > 0) {
     EpiConsts ec;
@@ -400,13 +443,15 @@ sred_status global_gram(sred_ctx* c, const GState& gs, cudaStream_t st, int shar
       ec.K = gs.K;
       ec.nrmse_near = kNrmseNear;
     }
+    ec.inv_wscale = 1.0f / gs.wscale;
+    ec.c2h = 0.5f * kC2 / ec.gscale;
     double* d_num = static_cast<double*>(c->buf[B_NUM].p);
-    double* d_den = static_cast<double*>(c->buf[B_DEN].p);
     const BlockParams* d_params = static_cast<const BlockParams*>(c->buf[B_PARAMS].p);
     const float* d_rmax = static_cast<const float*>(c->buf[B_RMAX].p);
+    CKS(denominators(c, gs, st, shard));
     if (gs.engine == SRED_ENGINE_FP32) {
-      CK(launch_gram_fp32(static_cast<const float*>(c->buf[B_U].p), gs.kp, d_params, d_rmax, ec, d_num, d_den,
-                          c->num_sms, st, shard, n_shards));
+      CK(launch_gram_fp32(static_cast<const float*>(c->buf[B_U].p), gs.kp, d_params, d_rmax, ec, d_num, c->num_sms,
+                          st, shard, n_shards));
     } else {
       int* d_status;
       CKS(ensure(c, B_STATUS, 4, &d_status));
@@ -414,7 +459,7 @@ sred_status global_gram(sred_ctx* c, const GState& gs, cudaStream_t st, int shar
         CK(cudaMemsetAsync(d_status, 0, 4 * sizeof(int), st));
         CK(launch_gram_tc(static_cast<const __nv_bfloat16*>(c->buf[B_A].p),
                           static_cast<const __nv_bfloat16*>(c->buf[B_B].p), gs.kq, (int)gs.n_pad, d_params,
-                          static_cast<float*>(c->buf[B_COLSOA].p), ec, d_num, d_den, c->num_sms, d_status, st, shard,
+                          static_cast<float*>(c->buf[B_COLSOA].p), ec, d_num, c->num_sms, d_status, st, shard,
                           n_shards, &c->tc_debug, ch));
         return SRED_OK;
       };
@@ -441,7 +486,6 @@ sred_status global_gram(sred_ctx* c, const GState& gs, cudaStream_t st, int shar
         float best = 3.4e38f;
         for (int i = 0; i < nc; i++) {
           CK(cudaMemsetAsync(d_num, 0, gs.n_pad * sizeof(double), st));
-          CK(cudaMemsetAsync(d_den, 0, gs.n_pad * sizeof(double), st));
           CK(cudaEventRecord(c->ev[4], st));
           CKS(run(&cand[i]));
           CK(cudaEventRecord(c->ev[5], st));
@@ -459,7 +503,6 @@ sred_status global_gram(sred_ctx* c, const GState& gs, cudaStream_t st, int shar
           g_tune[key] = TuneEntry{chosen, best};
         }
         CK(cudaMemsetAsync(d_num, 0, gs.n_pad * sizeof(double), st));
-        CK(cudaMemsetAsync(d_den, 0, gs.n_pad * sizeof(double), st));
         CK(cudaEventRecord(c->ev[1], st));  // ms_gram times the map's own contraction, not the tuning
       }
       CKS(run(have ? &chosen : nullptr));
@@ -507,7 +550,7 @@ sred_status global_finish(sred_ctx* c, const GState& gs, cudaStream_t st, int no
     info->ms_gram = t12;
     info->ms_finalize = t23;
     info->ms_total = t03;
-    info->launches = (gs.given ? 0 : 2) + 4 + (gs.n_g > 0 ? (gs.engine == SRED_ENGINE_TC ? 3 : 2) : 0) + 1 +
+    info->launches = (gs.given ? 0 : 2) + 4 + contraction_launches(gs.n_g, gs.engine, gs.sorted) + 1 +
                      (normalize ? 3 : 0);
   }
   if (c->log_cb) {
@@ -848,11 +891,12 @@ sred_status global3d_prepare(sred_ctx* c, int metric, const float* d_vol, int w,
   __nv_bfloat16 *d_A = nullptr, *d_B = nullptr;
   BlockParams* d_params;
   float* d_rmax;
-  double *d_num, *d_den;
+  double *d_num, *d_den, *d_sums;
   CKS(ensure(c, B_PARAMS, n_pad, &d_params));
   CKS(ensure(c, B_RMAX, n_pad / 128, &d_rmax));
   CKS(ensure(c, B_NUM, n_pad, &d_num));
   CKS(ensure(c, B_DEN, n_pad, &d_den));
+  CKS(ensure(c, B_SUMS, 8, &d_sums));  // the range of a, after the 2D maps' sums
   if (engine == SRED_ENGINE_FP32 || metric == kNrmse) {  // tensor-core NRMSE reads U for near-identical pairs
     CKS(ensure(c, B_U, n_pad * kp, &d_U));
     CK(cudaMemsetAsync(d_U + (size_t)n_g * kp, 0, (n_pad - n_g) * kp * sizeof(float), st));
@@ -866,14 +910,16 @@ sred_status global3d_prepare(sred_ctx* c, int metric, const float* d_vol, int w,
   CK(cudaMemsetAsync(d_params + n_g, 0, (n_pad - n_g) * sizeof(BlockParams), st));
   CK(cudaMemsetAsync(d_rmax, 0, (n_pad / 128) * sizeof(float), st));
   CK(cudaMemsetAsync(d_num, 0, n_pad * sizeof(double), st));
-  CK(cudaMemsetAsync(d_den, 0, n_pad * sizeof(double), st));
+  CK(cudaMemsetAsync(d_sums, 0, 8 * sizeof(double), st));
+  const bool sorted = sort_for(engine, metric == kNrmse ? kNrmseW : metric);
+  if (sorted) CKS(sort_blocks(c, d_stds, n_g, st));
   // weight = exp(-(s_p - s_q)^2 / (FILTER_PARAM + EPSILON)) = 2^-(a_p - a_q)^2
   const float hden = nv + kEps;
   const float wscale = (float)std::sqrt(1.4426950408889634 / (double)hden);
   if (n_g > 0) {
     k_pack3d<<<grid_for((size_t)n_g * 32, 256, 8 * c->num_sms), 256, 0, st>>>(
         d_vol, v, d_off, d_gpix, n_g, wscale, engine == SRED_ENGINE_FP32 ? 0 : split_levels_for(metric, K) - 1, d_U, kp, d_A,
-        d_B, kq, d_params, d_rmax);
+        d_B, kq, d_params, d_rmax, reinterpret_cast<unsigned*>(d_sums + 4));
     CK(cudaGetLastError());
   }
   if (engine == SRED_ENGINE_TC) {
@@ -901,6 +947,8 @@ sred_status global3d_prepare(sred_ctx* c, int metric, const float* d_vol, int w,
   gs->thr = thr;
   gs->npx = npx;
   gs->relc = relc;
+  gs->wscale = wscale;
+  gs->sorted = sorted;
   gs->valid = true;
   return SRED_OK;
 }
@@ -949,7 +997,7 @@ sred_status global3d_finish(sred_ctx* c, const GState& gs, cudaStream_t st, int 
     info->ms_gram = t12;
     info->ms_finalize = t23;
     info->ms_total = t03;
-    info->launches = 5 + (gs.n_g > 0 ? (gs.engine == SRED_ENGINE_TC ? 3 : 2) : 0) + 1 + (normalize ? 3 : 0);
+    info->launches = 5 + contraction_launches(gs.n_g, gs.engine, gs.sorted) + 1 + (normalize ? 3 : 0);
   }
   if (c->log_cb) {
     float t03 = 0;
@@ -1675,6 +1723,7 @@ sred_status reserve_global(sred_ctx* c, const sred_job* jobs, int n_jobs) {
   uint8_t* u8;
   int* i32;
   int2* i2;
+  float2* f2;
   BlockParams* bp;
   double* d;
   __nv_bfloat16* bf;
@@ -1686,7 +1735,10 @@ sred_status reserve_global(sred_ctx* c, const sred_job* jobs, int n_jobs) {
   CKS(ensure(c, B_RMAX, n_pad / 128, &f));
   CKS(ensure(c, B_NUM, n_pad, &d));
   CKS(ensure(c, B_DEN, n_pad, &d));
+  CKS(ensure(c, B_NODES, kDenNodes, &d));
+  CKS(ensure(c, B_SLICES, den_slices((int)n_pad), &f2));
   if (tc) {
+    CKS(ensure(c, B_SORT, sort_workspace_ints((int)n_pad), &i32));
     CKS(ensure(c, B_A, a, &bf));
     CKS(ensure(c, B_B, a, &bf));
     CKS(ensure(c, B_COLSOA, cols, &f));
@@ -2054,9 +2106,11 @@ sred_status sred_debug_gram_rowdot(sred_ctx* c, int engine, const float* u, cons
   k_pack_vectors<<<grid_for((size_t)n * 32, 256, 8 * c->num_sms), 256, 0, st>>>(
       d_u, n, k, engine == SRED_ENGINE_FP32 ? 0 : 1, d_U, kp, d_A, d_B, kq);
   CK(cudaGetLastError());
-  EpiConsts ec{kDebugDot, n, 1.0f, kC1, kC2};
+  // num and den are two sums over the same schedule
+  EpiConsts ec{kDebugDot, n, 1.0f, kC1, kC2}, ed{kDebugSum, n, 1.0f, kC1, kC2};
   if (engine == SRED_ENGINE_FP32) {
-    CK(launch_gram_fp32(d_U, kp, d_params, d_rmax, ec, d_num, d_den, c->num_sms, st));
+    CK(launch_gram_fp32(d_U, kp, d_params, d_rmax, ec, d_num, c->num_sms, st));
+    CK(launch_gram_fp32(d_U, kp, d_params, d_rmax, ed, d_den, c->num_sms, st));
   } else {
     int* d_status;
     CKS(ensure(c, B_STATUS, 4, &d_status));
@@ -2065,7 +2119,9 @@ sred_status sred_debug_gram_rowdot(sred_ctx* c, int engine, const float* u, cons
     CKS(ensure(c, B_COLSOA, gram_tc_soa_floats((int)n_pad), &d_soa));
     TcPlan plan;
     if (!plan_gram_tc(kq, &plan)) return fail(c, SRED_ERR_ARG, "K too large for the tensor-core engine");
-    CK(launch_gram_tc(d_A, d_B, kq, (int)n_pad, d_params, d_soa, ec, d_num, d_den, c->num_sms, d_status, st, 0, 1,
+    CK(launch_gram_tc(d_A, d_B, kq, (int)n_pad, d_params, d_soa, ec, d_num, c->num_sms, d_status, st, 0, 1,
+                      &c->tc_debug));
+    CK(launch_gram_tc(d_A, d_B, kq, (int)n_pad, d_params, d_soa, ed, d_den, c->num_sms, d_status, st, 0, 1,
                       &c->tc_debug));
     int status = 0;
     CK(cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -300,7 +300,9 @@ __global__ void k_flags3d(const float* __restrict__ stds, Vol3 v, float thr, int
 __global__ void k_pack3d(const float* __restrict__ img, Vol3 v, const int* __restrict__ off,
                          const int* __restrict__ gram_pix, int n, float wscale, int mode, float* __restrict__ U,
                          int kp, __nv_bfloat16* __restrict__ A, __nv_bfloat16* __restrict__ B, int kq,
-                         BlockParams* __restrict__ params, float* __restrict__ tile_rmax) {
+                         BlockParams* __restrict__ params, float* __restrict__ tile_rmax,
+                         unsigned* __restrict__ arange) {
+  unsigned a_lo = 0u, a_hi = 0u;  // ~bits of the smallest a, bits of the largest (launch_den, weights.cuh)
   const int lane = threadIdx.x & 31;
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -342,8 +344,14 @@ __global__ void k_pack3d(const float* __restrict__ img, Vol3 v, const int* __res
       bp.mu = (float)mu;
       bp.pad0 = bp.pad1 = bp.pad2 = 0.0f;
       params[j] = bp;
+      a_lo = max(a_lo, ~__float_as_uint(bp.a));
+      a_hi = max(a_hi, __float_as_uint(bp.a));
       atomicMax(reinterpret_cast<int*>(tile_rmax) + (j >> 7), __float_as_int(bp.r));
     }
+  }
+  if (lane == 0 && a_hi | a_lo) {
+    atomicMax(arange, a_lo);
+    atomicMax(arange + 1, a_hi);
   }
 }
 

@@ -1,0 +1,213 @@
+// Denominators of the global maps: den_p = sum_q 2^-(a_p - a_q)^2 over the
+// contracted blocks (the weight's own sum, java/CLUtils.java:1747-1770), the
+// self pair included.
+//
+// The weight depends on the two blocks' scalars a alone, so the n sums are one
+// function of one variable, F(x) = sum_q 2^-(x - a_q)^2, at the points a_p. F is
+// a sum of Gaussians of one width: between nodes 1/8 apart a 12-point Lagrange
+// polynomial reproduces it to 6e-11 relative (the 12th derivative of 2^-x^2 is
+// at most 7.4e4; times 5.5e-5 h^12). So the sums take n terms at some tens of
+// nodes (FP64) and n interpolations instead of n^2 / 2 pair terms; accumulating
+// them beside the numerators was a sixth of the pair arithmetic and half of the
+// contraction's accumulators.
+//
+// k_den_nodes: one CTA per 2,048 blocks, eight nodes at a time; consecutive
+// nodes of a block follow from two multiplications,
+//   2^-(x + h - a)^2 = 2^-(x - a)^2 * r,  r = 2^-(2 (x - a) h + h^2),  r' = r 2^(-2 h^2),
+// and one FP64 atomic add per node and CTA. Nodes further than 14 from every
+// block of the slice (terms below 2^-169) are skipped.
+// k_den_eval: one thread per block. Where the range of a does not fit the node
+// table (2,046 at h = 1/8) or is not finite, the same kernel sums the pair terms
+// directly (FP32 terms, FP64 sums of 256), slice by slice within that distance.
+#include "epilogue.cuh"
+#include "weights.cuh"
+
+namespace sred {
+
+namespace {
+
+constexpr double kH = 0.125;
+constexpr int kPad = 6;            // nodes below the smallest a
+constexpr int kThreads = 256;
+constexpr int kPer = kDenSlice / kThreads;
+constexpr int kGroup = 8;          // nodes per step
+constexpr float kFar = 14.0f;
+
+// Node grid of the a-range (arange: see launch_den): first node and count (0: no grid).
+__device__ __forceinline__ int node_grid(const unsigned* __restrict__ arange, double* x0) {
+  const unsigned lo = ~arange[0], hi = arange[1];
+  if (hi >= 0x7f800000u) return 0;  // infinite or NaN (either sign)
+  const double a0 = (double)__uint_as_float(lo), a1 = (double)__uint_as_float(hi);
+  *x0 = a0 - kPad * kH;
+  const double m = floor((a1 - a0) / kH) + 2 * kPad + 2;
+  return m <= (double)kDenNodes ? (int)m : 0;
+}
+
+__global__ void __launch_bounds__(kThreads) k_den_nodes(const BlockParams* __restrict__ params, int n,
+                                                        const unsigned* __restrict__ arange,
+                                                        double* __restrict__ nodes, float2* __restrict__ slices) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i0 = blockIdx.x * kDenSlice;
+  __shared__ float2 wr[kThreads / 32];
+  __shared__ double red[kThreads / 32][kGroup];
+  float v[kPer];
+  float lo = 3.4e38f, hi = -3.4e38f;
+  bool bad = false;
+#pragma unroll
+  for (int j = 0; j < kPer; j++) {
+    const int i = i0 + j * kThreads + threadIdx.x;
+    v[j] = i < n ? params[i].a : 3.4e38f;  // past the end: further than kFar from every node
+    if (i < n) {
+      lo = fminf(lo, v[j]);
+      hi = fmaxf(hi, v[j]);
+      bad |= !(v[j] - v[j] == 0.0f);
+    }
+  }
+  for (int o = 16; o; o >>= 1) {
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if (__any_sync(0xffffffffu, bad)) lo = hi = nanf("");
+  if (lane == 0) wr[w] = make_float2(lo, hi);
+  __syncthreads();
+  lo = wr[0].x;
+  hi = wr[0].y;
+  bad = lo != lo;
+  for (int k = 1; k < kThreads / 32; k++) {
+    bad |= wr[k].x != wr[k].x;
+    lo = fminf(lo, wr[k].x);
+    hi = fmaxf(hi, wr[k].y);
+  }
+  if (bad) lo = hi = nanf("");
+  if (threadIdx.x == 0) slices[blockIdx.x] = make_float2(lo, hi);
+  double x0;
+  const int m = node_grid(arange, &x0);
+  if (m == 0) return;
+  const int g0 = max(0, (int)floor(((double)lo - kFar - x0) / (kH * kGroup)));
+  const int g1 = min((m - 1) / kGroup, (int)floor(((double)hi + kFar - x0) / (kH * kGroup)));
+  const double q = exp2(-2.0 * kH * kH);
+  for (int g = g0; g <= g1; g++) {
+    const double xb = x0 + (double)(g * kGroup) * kH;
+    double acc[kGroup];
+#pragma unroll
+    for (int k = 0; k < kGroup; k++) acc[k] = 0.0;
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+      const double d = xb - (double)v[j];
+      if (fabs(d + 0.5 * kH * kGroup) > (double)kFar) continue;  // (2^-182 at most)
+      double e = exp2(-d * d), r = exp2(-(2.0 * d + kH) * kH);
+#pragma unroll
+      for (int k = 0; k < kGroup; k++) {
+        acc[k] += e;
+        e *= r;
+        r *= q;
+      }
+    }
+    // 8 sums over 32 lanes: three halving steps leave lane l sum index l & 7, two more finish it
+#pragma unroll
+    for (int s = 0; s < 3; s++) {
+      const bool up = (lane >> s) & 1;
+#pragma unroll
+      for (int k = 0; k < (kGroup >> (s + 1)); k++) {
+        const double keep = up ? acc[2 * k + 1] : acc[2 * k], send = up ? acc[2 * k] : acc[2 * k + 1];
+        acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, 1 << s);
+      }
+    }
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 8);
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 16);
+    __syncthreads();
+    if (lane < kGroup) red[w][lane] = acc[0];
+    __syncthreads();
+    if (threadIdx.x < kGroup && g * kGroup + (int)threadIdx.x < m) {
+      double t = 0.0;
+      for (int k = 0; k < kThreads / 32; k++) t += red[k][threadIdx.x];
+      atomicAdd(nodes + g * kGroup + threadIdx.x, t);
+    }
+  }
+}
+
+// 1 / prod_{j != k} (k - j) for the nodes 0..11.
+__device__ __forceinline__ double lagrange_scale(int k) {
+  const double f[12] = {1.0, 1.0, 2.0, 6.0, 24.0, 120.0, 720.0, 5040.0, 40320.0, 362880.0, 3628800.0, 39916800.0};
+  const double v = 1.0 / (f[k] * f[11 - k]);
+  return (k & 1) ? v : -v;  // sign (-1)^(11 - k)
+}
+
+__global__ void __launch_bounds__(kThreads) k_den_eval(const BlockParams* __restrict__ params, int n,
+                                                       const unsigned* __restrict__ arange,
+                                                       const double* __restrict__ nodes,
+                                                       const float2* __restrict__ slices, int nslices,
+                                                       double* __restrict__ den) {
+  const int i = blockIdx.x * kThreads + threadIdx.x;
+  double x0;
+  if (node_grid(arange, &x0) > 0) {
+    if (i >= n) return;
+    const double t = ((double)params[i].a - x0) / kH;
+    const int k0 = (int)floor(t) - (kPad - 1);
+    const double s = t - (double)k0;  // in [5, 6)
+    double suf[12];
+    suf[11] = 1.0;
+#pragma unroll
+    for (int k = 11; k > 0; k--) suf[k - 1] = suf[k] * (s - (double)k);
+    double pre = 1.0, sum = 0.0;
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+      sum += lagrange_scale(k) * pre * suf[k] * nodes[k0 + k];
+      pre *= s - (double)k;
+    }
+    den[i] = sum;
+    return;
+  }
+  __shared__ float sa[kThreads];
+  __shared__ float2 wr[kThreads / 32];
+  const float a = i < n ? params[i].a : 0.0f;
+  float lo = i < n ? a : 3.4e38f, hi = i < n ? a : -3.4e38f;
+  const bool bad = i < n && !(a - a == 0.0f);
+  for (int o = 16; o; o >>= 1) {
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  const bool any_bad = __syncthreads_or(bad);
+  if ((threadIdx.x & 31) == 0) wr[threadIdx.x >> 5] = make_float2(lo, hi);
+  __syncthreads();
+  for (int k = 0; k < kThreads / 32; k++) {
+    lo = fminf(lo, wr[k].x);
+    hi = fmaxf(hi, wr[k].y);
+  }
+  double sum = 0.0;
+  for (int s = 0; s < nslices; s++) {
+    const float2 r = slices[s];
+    if (!any_bad && (r.x - hi > kFar || lo - r.y > kFar)) continue;  // (a NaN range is not skipped)
+    const int q0 = s * kDenSlice, q1 = min(n, q0 + kDenSlice);
+    for (int qb = q0; qb < q1; qb += kThreads) {
+      const int m = min(kThreads, q1 - qb);
+      __syncthreads();
+      if ((int)threadIdx.x < m) sa[threadIdx.x] = params[qb + threadIdx.x].a;
+      __syncthreads();
+      float part = 0.0f;
+      for (int k = 0; k < m; k++) {
+        const float d = a - sa[k];
+        part += ex2_approx(-d * d);
+      }
+      sum += (double)part;
+    }
+  }
+  if (i < n) den[i] = sum;
+}
+
+}  // namespace
+
+int den_slices(int n) { return (n + kDenSlice - 1) / kDenSlice; }
+
+cudaError_t launch_den(const BlockParams* params, int n, const unsigned* arange, double* nodes, float2* slices,
+                       double* den, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  const cudaError_t e = cudaMemsetAsync(nodes, 0, kDenNodes * sizeof(double), st);
+  if (e != cudaSuccess) return e;
+  const int ns = den_slices(n);
+  k_den_nodes<<<ns, kThreads, 0, st>>>(params, n, arange, nodes, slices);
+  k_den_eval<<<(n + kThreads - 1) / kThreads, kThreads, 0, st>>>(params, n, arange, nodes, slices, ns, den);
+  return cudaGetLastError();
+}
+
+}  // namespace sred
