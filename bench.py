@@ -262,7 +262,7 @@ def run_ours(args, rank, local, world):
         "higher_is_better": True,
         "scaling": "weak",
         "vs_baseline": None,
-        "dtype": "bf16x3 split (hi/lo) tensor-core Gram, f32 accumulate, f64 moments" if r["info"]["engine"] == 0
+        "dtype": "fp16x3 split (hi/mid) tensor-core Gram, f32 accumulate, f64 moments" if r["info"]["engine"] == 0
                  else "f32 CUDA-core Gram, f64 moments",
         "data": "synthetic (seeded spot image, numpy default_rng; no dataset)",
         "config": {"workload": WORKLOAD, "image": f"{W_IMG}x{H_IMG}", "block": f"{BW}x{BH}", "K": K,
@@ -285,7 +285,7 @@ def run_ours(args, rank, local, world):
             "note": f"all-pairs Gram kernel; algorithmic FLOPs = contracted pairs x 2K (K={K}), contracted pairs = "
                     f"n(n+1)/2 of the n non-flat relevant blocks (symmetric schedule: each unordered pair once; "
                     f"value counts all relevant^2 ordered pairs the map is defined over); peak = {pk['source']} "
-                    f"sustained BF16 / 3 (three hi/lo products per FP32-accurate product)"}
+                    f"sustained BF16 / 3 (the FP16 rate; three hi/mid products per FP32-accurate product)"}
     if "fp32" in results and args.engine != "fp32":
         f = results["fp32"]
         fv = f["pairs"] / (f["total_ms"] / 1e3)
@@ -579,7 +579,7 @@ def run_volume_global(args, rank, local, world):
     line = {"metric": "3D global-map block-pairs/s at 192x192x64/5x5x5", "value": pairs / (total_ms / 1e3),
             "unit": "block-pairs/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": total_ms / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "bf16x3 split tensor-core Gram, f32 accumulate, f64 sums" if args.engine == "tc"
+            "dtype": "fp16x3 split tensor-core Gram, f32 accumulate, f64 sums" if args.engine == "tc"
                      else "f32 CUDA-core Gram, f64 sums",
             "data": "synthetic (seeded spot volume, numpy default_rng; no dataset)",
             "config": {"workload": "3D global repetition map, 192x192x64 float32 spot volume (24x24x8 lattice), "
@@ -729,7 +729,7 @@ def run_shard(args, rank, local, world):
     line = {"metric": METRIC.replace("split-BF16 vs FP32 speedup @≤1e-5 err", "one map sharded across GPUs by work items"),
             "value": pairs / (ms / 1e3), "unit": "block-pairs/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "strong",
-            "vs_baseline": None, "dtype": "bf16x3 split (hi/lo) tensor-core Gram, f32 accumulate, f64 moments",
+            "vs_baseline": None, "dtype": "fp16x3 split (hi/mid) tensor-core Gram, f32 accumulate, f64 moments",
             "data": "synthetic",
             "config": {"workload": WORKLOAD, "image": f"{W_IMG}x{H_IMG}", "block": f"{BW}x{BH}",
                        "pairs_per_step": pairs,
@@ -806,7 +806,7 @@ def run_batch(args, rank, local, world):
     line = {"metric": "batched global maps: block-pairs/s summed over maps (wall time, host buffers)",
             "value": pairs / dt, "unit": "block-pairs/s", "n_gpus": world, "steps": 1, "warmup": args.warmup,
             "ms_per_step": dt * 1e3, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "bf16x3 split (hi/lo) tensor-core Gram, f32 accumulate, f64 moments", "data": "synthetic",
+            "dtype": "fp16x3 split (hi/mid) tensor-core Gram, f32 accumulate, f64 moments", "data": "synthetic",
             "config": {"workload": f"{args.images} images x 5 block sizes x 2 metrics = {len(jobs)} global maps, "
                                    "sides 256-1024, relevance 1.0; warm-up: the largest image's 10 maps",
                        "images": args.images, "maps": len(jobs),

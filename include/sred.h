@@ -32,14 +32,14 @@ typedef enum {
     SRED_ERR_INVALID_INPUT = 8   /* NaN/Inf pixel in a noise tile (java/Utils.java:886-889) */
 } sred_status;
 
-/* Contraction engine of the global map. SRED_ENGINE_TC: split-BF16 tcgen05
- * tensor-core Gram with FP32 accumulation (u = hi + mid, or hi + mid + lo
- * when 6K <= 128 and for NRMSE); SRED_ENGINE_FP32: plain FP32 CUDA-core Gram.
+/* Contraction engine of the global map. SRED_ENGINE_TC: split-FP16 tcgen05
+ * tensor-core Gram with FP32 accumulation (u = hi + mid, 22 significand bits);
+ * SRED_ENGINE_FP32: plain FP32 CUDA-core Gram.
  * Both share moments, the symmetric schedule (each unordered block pair
- * evaluated once) and the fused epilogue. Abs-diff needs no contraction and
- * runs on the FP32 engine's kernel; a map whose operands do not fit the
- * tensor-core kernel's shared memory (K' above 576) falls back to the FP32
- * engine, where NRMSE accumulates |u_p - u_q|^2 directly. */
+ * evaluated once), the pair terms and the denominators. Abs-diff needs no
+ * contraction and runs on the FP32 engine's kernel. On the FP32 engine NRMSE
+ * accumulates |u_p - u_q|^2 directly. The other metrics' blocks are limited to
+ * K = 212 pixels on either engine (SRED_ERR_LAUNCH above). */
 typedef enum { SRED_ENGINE_TC = 0, SRED_ENGINE_FP32 = 1 } sred_engine;
 
 typedef struct sred_ctx sred_ctx;
@@ -337,7 +337,7 @@ sred_status sred_block_map_2d_device_noalloc(const char *metric, const float *d_
  * num[p] = sum_q <u_p, u_q> w1[p] w1[q] and den[p] = sum_q (w2[p] + w2[q]),
  * symmetric pair terms like the maps' own, computed by the
  * chosen engine's all-pairs kernel (the tensor-core engine splits u into
- * bf16 hi/lo without normalising it). */
+ * fp16 hi/mid without normalising or scaling it: |u| below 65504). */
 sred_status sred_debug_gram_rowdot(sred_ctx *ctx, int engine, const float *u, const float *w1,
                                    const float *w2, int n, int k, double *num, double *den);
 
@@ -353,14 +353,13 @@ sred_status sred_debug_set_tc_wait(sred_ctx *ctx, unsigned long long timeout_ns,
 
 /* Launch-shape tuner of the tensor-core engine (no counterpart in the
  * reference, whose OpenCL kernels run one fixed work-group size,
- * java/CLUtils.java:432-433). A global map's contraction can run as
- * 128 x 256 or 128 x 128 tiles, with each tile's A operand resident or
- * streamed through a ring of 16 KB chunks, and with 32, 16, 8 or 4 row blocks
- * per run of work items. The process keeps one table, shared by every context:
+ * java/CLUtils.java:432-433). A global map's contraction can stream its row
+ * blocks as whole tiles or in 16 KB chunks, and take 128, 32, 16, 8 or 4 row
+ * blocks per run of work items. The process keeps one table, shared by every context:
  * key (K' = padded contraction length, metric code, size class of the
  * contracted block count n: 0 below 65,536, 1 below 262,144, else 2) ->
  * shape. A map whose key is in the table runs that shape; other maps run the
- * default shape (128 x 256, A resident when it fits, 32 row blocks).
+ * default shape (whole tiles when three fit, 128 row blocks).
  *
  * sred_set_gram_tuning(ctx, 1) makes later unsharded maps on ctx (and its
  * batch workers) whose key is missing time every shape on their own
@@ -371,8 +370,9 @@ sred_status sred_debug_set_tc_wait(sred_ctx *ctx, unsigned long long timeout_ns,
 sred_status sred_set_gram_tuning(sred_ctx *ctx, int on);
 
 /* Copies at most `cap` table entries: entries[6 i .. 6 i + 5] = K', metric
- * code, size class, tile columns (256 or 128), A resident (1) or chunk ring
- * (0), row blocks per run; ms[i] = that shape's timed contraction in ms.
+ * code, size class, tile columns (256; 128 in tables of earlier versions, which
+ * runs as 256), whole tiles (1) or chunks (0), row blocks per run; ms[i] = that
+ * shape's timed contraction in ms.
  * Returns the number of entries in the table (call with cap 0 to size). */
 int sred_gram_tuning_entries(int *entries, float *ms, int cap);
 
@@ -454,7 +454,7 @@ sred_status sred_block_map_3d_device(sred_ctx *ctx, const char *metric, const fl
  * and Abs-diff inverted where the mask is 1, the mask applied when
  * relevance_constant > 0, normalizeImage3D over the mask. Sums in FP64 from
  * FP32 terms (the tensor-core engine computes the block dot products in split
- * BF16, as the 2D global map). Repairs of the reference, which does not run as
+ * FP16, as the 2D global map). Repairs of the reference, which does not run as
  * shipped: the relevance mask is getRelevanceMask3D's (noise variance = mean
  * local variance over the interior; the command passes the 2D mask,
  * java/GlobalRepetition3D_.java:126-128, whose indexing fails on the first

@@ -269,8 +269,8 @@ def _panel_items_before_run(j: int, c0: int, c1: int, h: int) -> int:
 
 
 def gram_panel(bn: int, kq: int) -> int:
-    """Column tiles per panel: as many bn-column B tiles of K' = kq bf16 as fit
-    in 48 MB (the rule libsred applies, global_tc.cu: launch_gram_tc)."""
+    """Column tiles per panel: as many bn-column tiles of kq fp16 per
+    block as fit in 48 MB (the rule libsred applies, global_tc.cu: launch_gram_tc)."""
     return max(1, (48 << 20) // (bn * kq * 2))
 
 
@@ -278,7 +278,7 @@ def gram_items(n_gram: int, bn: int = 256, num_sms: int = 148) -> tuple[int, int
     """(items, L) of the tensor-core engine's symmetric schedule for n_gram
     blocks and bn-column tiles: the upper triangle of 128-row x bn-column
     tiles, cut into items (a run of L row blocks against one column tile that
-    reaches it), L the largest of 32, 16, 8, 4, 2 that leaves at least 4 items
+    reaches it), L the largest of 128, 64, ..., 2 that leaves at least 16 items
     per SM (the rule libsred applies, global_tc.cu: gram_tc_items)."""
     m = bn // 128
     n_rb, n_ct = (n_gram + 127) // 128, (n_gram + bn - 1) // bn
@@ -286,8 +286,8 @@ def gram_items(n_gram: int, bn: int = 256, num_sms: int = 148) -> tuple[int, int
     def items(L):
         return _items_before_run((n_rb + L - 1) // L, n_ct, L // m)
 
-    L = 32
-    while L > 2 and items(L) < 4 * num_sms:
+    L = 128
+    while L > 2 and items(L) < 16 * num_sms:
         L //= 2
     L = max(L, m)
     return items(L), L

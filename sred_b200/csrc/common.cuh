@@ -1,7 +1,7 @@
 // Shared definitions of libsred's device code and host orchestration.
 #pragma once
 #include <cuda_runtime.h>
-#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <stdint.h>
 
 #include "../../include/sred.h"
@@ -12,6 +12,7 @@ constexpr float kEps = 0.0000001f;  // java/Utils.java:20 (Utils.EPSILON)
 constexpr float kC1 = 0.0001f;      // cl/kernelGetGlobalSsim2D.cl:102
 constexpr float kC2 = 0.0009f;      // cl/kernelGetGlobalSsim2D.cl:104
 constexpr int kMaxK = 512;          // largest ellipse block size accepted
+constexpr int kMaxGlobalK = 212;    // largest block of a global map with a contraction
 
 enum Metric { kPearson = 0, kSsim = 1, kNrmse = 2, kAbsDiff = 3, kCosine = 4,
               kDebugDot = 5 /* diagnostics: num += G a_p a_q */,
@@ -52,37 +53,55 @@ struct BlockParams {
   float pad0, pad1, pad2;
 };
 
-// Split-BF16 operands of the tensor-core engine, u = hi + mid (+ lo), each
-// part the BF16 rounding of what the previous parts leave of u:
-//   two levels:   A = [hi|mid|hi], B = [hi|hi|mid] (3K columns); the products
-//                 carry about 16 significand bits (dot-product error up to
-//                 ~1e-5 for unit vectors);
-//   three levels: A = [hi|mid|lo|hi|mid|hi], B = [hi|hi|hi|mid|mid|lo] (6K
-//                 columns); every product down to 2^-18 relative, an FP32-level
-//                 dot product. Used while 6K fits in 128 columns, where the
-//                 tiles are bound by the epilogue and the deeper MMA is free,
-//                 and always for NRMSE, whose 1 - G term needs it.
-inline int split_levels(int K) { return 6 * K <= 128 ? 3 : 2; }
-inline int split_cols(int K) { return split_levels(K) == 3 ? (6 * K + 31) / 32 * 32 : (3 * K + 31) / 32 * 32; }
-inline bool nrmse_metric(int m) { return m == 2 /* kNrmse */ || m == 8 /* kNrmseW */; }
-inline int split_levels_for(int metric, int K) { return nrmse_metric(metric) ? 3 : split_levels(K); }
-inline int split_cols_for(int metric, int K) {
-  return split_levels_for(metric, K) == 3 ? (6 * K + 31) / 32 * 32 : (3 * K + 31) / 32 * 32;
+// Split-FP16 operand of the tensor-core engine: u = hi + mid, hi = fp16(u 2^14) and
+// mid = fp16(u 2^14 - hi) (|u| <= 1, so hi <= 2^14 and every mid down to u = 2^-16
+// keeps its 11 bits). Dot products hi.hi + mid.hi + hi.mid carry 22 significand
+// bits; G = 2^-28 of the accumulated value.
+//
+// A row holds each part once. The row and the column operand are the same array:
+// the MMAs pair blocks of 16 elements of one with blocks of the other. K = 16 nb + r:
+//   [hi: nb blocks | mid: nb blocks | row tail: nt | column tail: nt],
+// the tails holding the last r elements of every part side by side, as
+// [hi|mid|hi] in the row tail and [hi|hi|mid] in the column tail, nt = ceil(3r / 16)
+// blocks: 3 nb + nt steps of 16 instead of 3 ceil(K / 16).
+struct SplitLayout {
+  int nb, r, nt, pitch;  // pitch: fp16 per row, a multiple of 32
+};
+__host__ __device__ inline SplitLayout split_layout(int K) {
+  const int nb = K / 16, r = K % 16, nt = (3 * r + 15) / 16;
+  return SplitLayout{nb, r, nt, 32 * (nb + nt)};
 }
+constexpr float kSplitScale = 16384.0f;
+constexpr float kSplitGScale = 1.0f / (16384.0f * 16384.0f);
+constexpr int kSplitSlack = 32;  // fp16 past the last row that a copy may read
+// K': the padded contraction length (the key of the launch-shape table).
+inline int split_cols(int K) { return (3 * K + 31) / 32 * 32; }
+inline bool nrmse_metric(int m) { return m == 2 /* kNrmse */ || m == 8 /* kNrmseW */; }
 
-__device__ __forceinline__ void store_split(__nv_bfloat16* a, __nv_bfloat16* b, int K, int i, double u,
-                                            int levels) {
-  const __nv_bfloat16 hi = __float2bfloat16_rn((float)u);
-  const double r = u - (double)__bfloat162float(hi);
-  const __nv_bfloat16 mid = __float2bfloat16_rn((float)r);
-  if (levels == 2) {
-    a[i] = hi; a[K + i] = mid; a[2 * K + i] = hi;
-    b[i] = hi; b[K + i] = hi; b[2 * K + i] = mid;
-    return;
+// Element i of a block's vector (already scaled) into its row.
+__device__ __forceinline__ void store_split(__half* row, const SplitLayout& l, int i, double u) {
+  const __half hi = __float2half_rn((float)u);
+  const __half mid = __float2half_rn((float)(u - (double)__half2float(hi)));
+  if (i < 16 * l.nb) {
+    row[i] = hi;
+    row[16 * l.nb + i] = mid;
+  } else {
+    __half* a = row + 32 * l.nb + (i - 16 * l.nb);
+    __half* b = a + 16 * l.nt;
+    a[0] = hi;
+    a[l.r] = mid;
+    a[2 * l.r] = hi;
+    b[0] = hi;
+    b[l.r] = hi;
+    b[2 * l.r] = mid;
   }
-  const __nv_bfloat16 lo = __float2bfloat16_rn((float)(r - (double)__bfloat162float(mid)));
-  a[i] = hi; a[K + i] = mid; a[2 * K + i] = lo; a[3 * K + i] = hi; a[4 * K + i] = mid; a[5 * K + i] = hi;
-  b[i] = hi; b[K + i] = hi; b[2 * K + i] = hi; b[3 * K + i] = mid; b[4 * K + i] = mid; b[5 * K + i] = lo;
+}
+// The zeros behind the tails, one of 32 lanes' share.
+__device__ __forceinline__ void store_split_pad(__half* row, const SplitLayout& l, int lane) {
+  for (int i = 3 * l.r + lane; i < 16 * l.nt; i += 32) {
+    row[32 * l.nb + i] = __float2half_rn(0.0f);
+    row[32 * l.nb + 16 * l.nt + i] = __float2half_rn(0.0f);
+  }
 }
 
 // a / b, correctly rounded, for many a and one b: y = RN(1/b) once, then
@@ -118,6 +137,7 @@ struct EpiConsts {
   float nrmse_near = 1.0f;
   float gscale = 1.0f;      // G = gscale x the contraction's accumulator
   float inv_wscale = 0.0f;  // sigma / a
+  float tau = 0.0f;         // eps (a / sigma)^2: Pearson's t = tau / (a_p a_q)
   float c2h = 0.0f;         // c2 / (2 gscale)
 };
 
@@ -149,16 +169,15 @@ __host__ __device__ constexpr int col_soa_pos(int i) {
 // four values per group of 32 rows.
 constexpr int kRowSoaFloats = 4 * 128 + 16;
 
-// Launch shape of the tensor-core engine for a K': column tile width (256 or
-// 128), whole-tile A buffers or a ring of 64-column chunks, dynamic shared
-// memory. False if the B tile does not fit in shared memory.
+// Ring shape of the tensor-core engine for K ellipse pixels: stages of whole
+// row-block tiles or of single 64-column chunks (sc chunks each), dynamic shared
+// memory. False if the operands do not fit in shared memory (K above 288).
 struct TcPlan {
-  int bn;
-  bool tr;
-  int stages;
+  int ctas;  // CTAs that share a tile (1 or 2)
+  int sc, stages;
   size_t smem;
 };
-bool plan_gram_tc(int kq, TcPlan* plan);
+bool plan_gram_tc(int K, TcPlan* plan);
 
 // Test hooks of the tensor-core engine: a wait limit (0: 4 s) and a tile whose
 // operand copies the producer never issues (-1: none), so that the pipeline
@@ -168,14 +187,16 @@ struct TcDebug {
   long long withhold_tile;
 };
 
-// A launch shape of the tensor-core engine (bn 0: the default plan): column
-// tile width, whole-tile A buffers (tr 1) or the chunk ring (tr 0), and the
-// largest run of row blocks per work item (L; the item-count rule may lower it).
+// A launch shape of the tensor-core engine (bn 0: the default plan): tr 1 for
+// whole-tile stages, 0 for single chunks; L: the largest run of row blocks per
+// work item (the item-count rule may lower it). The tiles are 256 columns wide;
+// 128, a width of earlier tables, runs as 256.
 struct TcChoice {
   int bn = 0, tr = 0, L = 0;
 };
-// The launch shapes that fit in shared memory for a K' (at most cap).
-int gram_tc_candidates(int kq, TcChoice* out, int cap);
+// The launch shapes to time for K (at most cap), and whether one can run.
+int gram_tc_candidates(int K, TcChoice* out, int cap);
+bool gram_tc_valid(int K, const TcChoice& c);
 
 // Floats of the parameter workspace launch_gram_tc fills (column tiles and
 // row blocks) for n_pad blocks.
@@ -185,15 +206,15 @@ size_t gram_tc_soa_floats(int n_pad);
 // upper triangle of 128-row x bn-column tiles in runs of L row blocks).
 long long gram_tc_items(int n, int bn, int* L, int num_sms, int max_L = 0);
 
-// Launch the split-BF16 tcgen05 all-pairs kernel (global_tc.cu).
-// A, B: n_pad x kq bf16 (store_split); params: n_pad entries (rows past n
-// zero); soa_ws: gram_tc_soa_floats(n_pad) floats of workspace; num: n
-// doubles (zeroed), to which every pair's term is added for both blocks.
-// The upper-triangle work items are split into n_shards equal ranges; this
-// launch runs range `shard` (the shards' num add up to the whole map).
-cudaError_t launch_gram_tc(const __nv_bfloat16* A, const __nv_bfloat16* B, int kq, int n_pad,
-                           const BlockParams* params, float* soa_ws, EpiConsts ec, double* num, int num_sms,
-                           int* status, cudaStream_t st, int shard = 0, int n_shards = 1,
+// Launch the split-FP16 tcgen05 all-pairs kernel (global_tc.cu).
+// U: n_pad rows of split_layout(K).pitch fp16 (store_split; rows past n zero);
+// params: n_pad entries (rows past n zero); soa_ws: gram_tc_soa_floats(n_pad)
+// floats of workspace; num: n doubles (zeroed), to which every pair's term is
+// added for both blocks. The upper-triangle work items are split into n_shards
+// equal ranges; this launch runs range `shard` (the shards' num add up to the
+// whole map).
+cudaError_t launch_gram_tc(const __half* U, int K, int n_pad, const BlockParams* params, float* soa_ws, EpiConsts ec,
+                           double* num, int num_sms, int* status, cudaStream_t st, int shard = 0, int n_shards = 1,
                            const TcDebug* dbg = nullptr, const TcChoice* choice = nullptr);
 
 }  // namespace sred

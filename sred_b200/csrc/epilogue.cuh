@@ -1,5 +1,5 @@
 // Fused per-pair epilogue of the global repetition map, shared by the FP32
-// CUDA-core engine and the split-BF16 tensor-core engine.
+// CUDA-core engine and the split-FP16 tensor-core engine.
 //
 // Input per pair (p, q): G = <u_p, u_q>, the dot product of the two blocks'
 // zero-mean unit vectors (the contraction engine's output), and the blocks'

@@ -1,53 +1,51 @@
-// Split-BF16 tcgen05 engine of the global repetition map (sm_100a).
+// Split-FP16 tcgen05 engine of the global repetition map (sm_100a).
 //
-// G = A' B'^T on the 5th-generation tensor cores, where each block's FP64 unit
-// vector u is split into bf16 parts (common.cuh: store_split), so one BF16
-// MMA chain with FP32 accumulation yields an FP32-accurate <u_p, u_q>.
+// G = <u_p, u_q> on the 5th-generation tensor cores, where each block's FP64 unit
+// vector u is split into two fp16 parts, u = hi + mid (common.cuh: SplitLayout),
+// and G = hi.hi + mid.hi + hi.mid with FP32 accumulation: an FP32-accurate dot
+// product (what is left out is below 2^-22 |u_p| |u_q|).
 //
 // Symmetric schedule. Every per-pair term of the global map (weight, Pearson,
-// global SSIM, NRMSE, Abs-diff; epilogue.cuh) is symmetric in (p, q), so each
-// unordered pair is evaluated once: only tiles of the upper triangle are
-// scheduled (a 128-row block rb against a BN-column tile ct with
-// 128 rb <= BN ct + BN - 1), pairs below the diagonal are masked in the
-// diagonal tiles, and each pair's numerator and denominator terms are added to
-// the sums of both blocks (the self pair once).
+// global SSIM, NRMSE; epilogue.cuh) is symmetric in (p, q), so each unordered
+// pair is evaluated once: only tiles of the upper triangle are scheduled (a
+// 128-row block rb against a 256-column tile ct with 128 rb <= 256 ct + 255), pairs
+// below the diagonal are masked in the diagonal tiles, and each pair's term is
+// added to the sums of both blocks (the self pair once).
 //
-// Work item = (column tile ct, a run of up to L row blocks). The item's B tile
-// (BN x K') and column parameters stay in shared memory for the whole item;
-// the A tiles of its row blocks stream through (two whole tiles when they fit,
-// else a ring of 64-column chunks). Items are ordered panel-major (decode_item):
-// all CTAs work on the same row blocks at a time and share their A tiles in
-// L2, and a panel's B tiles stay in L2 while the runs pass over them; the
-// producer prefetches A two row blocks ahead and the next item's B into L2.
-// Each CTA walks its items twice: first their full tiles, then their masked
+// Work item = (column tile ct, a run of up to L row blocks). A cluster of two
+// CTAs (two SMs) works on an item together: row blocks go in pairs, CTA r of the
+// cluster takes row block rb + r, and one M = 256 tcgen05.mma (cta_group::2)
+// computes both CTAs' 128 x 256 tiles. Each CTA keeps half of the column tile's
+// operand (128 rows of U) in its shared memory for the whole item and streams its
+// own row blocks through a ring of stages. One CTA per tile (M = 128) read 96 bytes
+// of shared memory per clock for the MMAs alone, of 128 there are, and wrote 32 more
+// for the row blocks; the pair reads 64. Items are ordered panel-major
+// (decode_item): all clusters work on the same row blocks at a time and share them
+// in L2, and a panel's column tiles stay in L2 while the runs pass over them.
+// Each cluster walks its items twice: first their full tiles, then their masked
 // ones (diagonal and ragged tiles, about 0.2% of all), so that the masked
 // epilogue form sits in a loop of its own (with it in the main loop the full
 // tiles ran 3% slower).
-// The launch shape (BN = 256 or 128, whole-tile or chunk-ring A, L) is the
-// default of plan_gram_tc or a tuned TcChoice. CTA = 1 per SM, persistent.
-// Warp roles:
+// Warp roles (one CTA per SM, persistent):
 //   warp 16     TMA producer (one thread)
-//   warp 17     MMA issuer (one thread): tcgen05.mma M=128 N=BN K=16 into one
-//               of two TMEM accumulators, tcgen05.commit to publish it
-//   warps 0-15  epilogue: warp w reads TMEM lanes 32(w%4).. and BN/4 columns
-//               from BN/4 (w/4) with tcgen05.ld.16x256b, which gives each
-//               thread 4 rows x (BN/16) columns of the warp's slab. The fused
-//               per-pair metric runs on f32x2 pairs of neighbouring columns.
-//               Column sums of the item accumulate in per-thread shared
-//               memory slots (BN/16 values per thread and sum, read and
-//               written once per 16-column chunk of each tile) and leave once
-//               per item after a butterfly over the 8 lanes that share
-//               columns; row sums of a tile leave
-//               once per tile after a butterfly over the 4 lanes that share
-//               rows and a combine of the 4 column-group warps in shared
-//               memory: one FP64 atomic add per row per tile.
+//   warp 17     CTA 0: MMA issuer (one thread): tcgen05.mma M=256 N=256 K=16 into
+//               one of two TMEM accumulators, tcgen05.commit to both CTAs'
+//               barriers. CTA 1: relays its producer's arrivals to CTA 0.
+//   warps 0-15  epilogue: tcgen05.ld.16x256b gives each thread 4 rows x 4 columns
+//               of a 32 x 16 block; the fused per-pair metric runs on f32x2 pairs
+//               of neighbouring columns. Column sums of the item stay in registers
+//               and leave once per item (a butterfly over the 8 lanes that share
+//               columns); row sums leave once per tile (a butterfly over 4 lanes):
+//               one FP64 atomic add per row and warp.
 // Every mbarrier wait is bounded by wall time (a host-set limit); on expiry the
 // kernel records a status code, stops issuing work, waits (bounded) for its own
 // copies in flight, frees TMEM and returns. No TMA multicast is used.
 #include <cuda.h>
 #include <cudaTypedefs.h>
+#include <cuda_fp16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
@@ -57,38 +55,47 @@ namespace sred {
 
 namespace {
 
-constexpr int kBM = 128;                          // rows per tile (TMEM lanes)
-constexpr int kChunk = 64;                        // bf16 per K chunk (128 B: one SWIZZLE_128B atom row)
-constexpr int kAChunkBytes = kBM * kChunk * 2;    // 16 KB
+constexpr int kBM = 128;                          // rows per CTA and tile (TMEM lanes)
+constexpr int kBN = 256;                          // columns per tile
+constexpr int kChunk = 64;                        // fp16 per chunk (128 B: one SWIZZLE_128B atom row)
+constexpr int kChunkBytes = kBM * kChunk * 2;     // 128 rows of a chunk: 16 KB
 constexpr int kMaxStages = 16;
 constexpr int kEpiWarps = 16;                     // 4 per SM sub-partition
 constexpr int kThreads = (kEpiWarps + 2) * 32;
-constexpr int kEpiThreads = kEpiWarps * 32;
-constexpr int kRSlots = 2;                        // row-parameter ring depth
-constexpr int kRowR = kBM, kRowS = 2 * kBM, kRowMu = 3 * kBM;  // r, sigma, mu in a row-parameter slot (a at 0)
+constexpr int kRSlots = 4;                        // row-parameter ring depth
+constexpr int kRowR = kBM, kRowS = 2 * kBM, kRowMu = 3 * kBM;  // r, sigma, mu of a row block (a at 0)
 constexpr int kRowGrp = 4 * kBM;                  // the four 32-row groups' centres and half ranges
 constexpr int kRowFloats = kRowSoaFloats;         // one 128-row block's parameters
-constexpr int kRowPartBytes = 2 * 4 * kBM * 4;    // [2 buffers][4 column groups][128 rows] floats
-constexpr int kMaxRun = 32;                       // row blocks per run (work item), at most
+constexpr int kColFloats = col_soa_floats(kBN);   // one column tile's parameters
+constexpr int kMaxRun = 128;                      // row blocks per run (work item), at most
 constexpr int kBarBytes = 512;
+constexpr int kMaxMma = 64;                       // entries of the MMA table (3 nb + nt + 1 at most 58)
+constexpr int kTabBytes = kMaxMma * 8 + 16 * 4;
 constexpr size_t kSmemBudget = 227 * 1024;
 
-enum { ST_OK = 0, ST_TIMEOUT_PRODUCER = 1, ST_TIMEOUT_MMA = 2, ST_TIMEOUT_EPI = 3, ST_TIMEOUT_DRAIN = 4 };
+enum { ST_OK = 0, ST_TIMEOUT_PRODUCER = 1, ST_TIMEOUT_MMA = 2, ST_TIMEOUT_EPI = 3, ST_TIMEOUT_DRAIN = 4, ST_ALIGNMENT = 5 };
 
-template <int BN>
+// Epilogue sets. Two: warps 0-7 take the even tiles, warps 8-15 the odd ones, each
+// warp 32 rows x 128 columns, so that one set's fixed work per tile (waits, row
+// and column factors, row sums) is spread over more pairs and runs under the
+// other set's pair loop. One: all 16 warps share every tile, 32 x 64 each, which
+// halves the column sums a thread holds and leaves registers for the row
+// constants of SSIM and NRMSE (96 per thread).
+template <int METRIC>
+constexpr int epi_sets() {
+  return METRIC == kPearson ? 2 : 1;
+}
+template <int METRIC>
 struct Cfg {
-  static constexpr int kColW = BN / 4;              // columns per epilogue warp
-  static constexpr int kCH = kColW / 16;            // 16-column chunks per warp and tile
-  static constexpr int kM = BN / kBM;               // row blocks per column tile
-  static constexpr int kCSoa = col_soa_floats(BN);  // floats per column tile's parameters
-  static constexpr int kBChunkBytes = BN * kChunk * 2;
-  static constexpr int kScratch = 32 + kColW;       // floats of f and g per epilogue warp
+  static constexpr int kSets = epi_sets<METRIC>();
+  static constexpr int kColW = 64 * kSets;          // columns per epilogue warp (a slab)
+  static constexpr int kCH = kColW / 16;            // 16-column chunks per slab
 };
+constexpr int kScratch = 32 + 128;                  // floats of f and g per epilogue warp
 
 struct TcArgs {
-  int kq, nkc, stages;          // K', K chunks per tile (nfull + tail), chunk-ring depth
-  int nfull, tail;              // whole-tile mode: 64-column chunks and a 32-column tail (0 or 1)
-  uint32_t a_bytes, b_bytes;    // whole A tile and whole B tile (64-column chunks + 32-column tail)
+  int nb, nt;                   // blocks of 16 per part and tail blocks (SplitLayout)
+  int nch, sc, nst, stages;     // chunks per tile, chunks per stage, stages per tile, ring depth
   int n_rb, n_ct;               // row blocks holding valid rows, column tiles
   int L, h;                     // row blocks per item (a run), L / (BN / 128)
   int n_runs;                   // runs of L row blocks
@@ -100,7 +107,7 @@ struct TcArgs {
   double* num;
   int* status;
   unsigned long long timeout_ns;
-  long long withhold;           // test hook: the producer never issues this tile's loads (-1: none)
+  long long withhold;           // test hook: the producers never issue this tile's loads (-1: none)
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -121,8 +128,28 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+// Address of the same shared-memory location in CTA 0 of the cluster.
+__device__ __forceinline__ uint32_t leader_addr(uint32_t a) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(a));
+  return r;
+}
+
+// Arrive on a barrier of either CTA of the cluster (a shared::cluster address).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// The epilogue's arrivals only say that this warp's reads of a buffer are done
+// (their values are in registers), so they are relaxed: a releasing arrive waits
+// for the warp's row-sum atomics in flight to reach L2, 550 clocks a tile at CTA
+// scope and 1,500 at cluster scope.
+__device__ __forceinline__ void mbar_arrive_done_reading(uint32_t bar) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
@@ -141,43 +168,53 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 // records `code`) if the wait exceeded the limit or another role of any CTA
 // already gave up. Drain waits (for copies or MMAs this CTA issued) pass
 // abort = false: they keep waiting, within the same bound, after another
-// role has given up. The single-thread roles (producer, MMA issuer) wait
-// mostly for the epilogue; they back off with nanosleep (up to 0.5 us) so
-// that their polling does not take issue slots from the epilogue warps of
-// their SM sub-partition.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const TcArgs& g, int code,
-                                          bool abort = true, bool backoff = false) {
-  if (mbar_test(bar, parity)) return true;
+// role has given up. The producer, which runs buffers ahead, backs off with a
+// short nanosleep so that its polling does not take issue slots from the
+// epilogue warps of its SM sub-partition; the MMA issuer does not (a late wake
+// is idle tensor time: with a back-off of up to 0.5 us for both roles the 9x9
+// map's MMAs waited for operands that had landed).
+__device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, int* status, unsigned long long limit_ns,
+                                            int code, bool abort, bool backoff) {
   const unsigned long long t0 = globaltimer();
-  uint32_t ns = 32;
   for (uint32_t i = 1;; i++) {
-    if (backoff) {
-      __nanosleep(ns);
-      ns = ns < 512 ? 2 * ns : 512;
-    }
+    if (backoff) __nanosleep(40);
     if (mbar_test(bar, parity)) return true;
-    if ((i & (backoff ? 7u : 255u)) == 0) {
-      if (abort && *reinterpret_cast<volatile int*>(g.status) != ST_OK) return false;
-      if (globaltimer() - t0 > g.timeout_ns) {
-        atomicCAS(g.status, ST_OK, code);
+    if ((i & (backoff ? 63u : 255u)) == 0) {
+      if (abort && *reinterpret_cast<volatile int*>(status) != ST_OK) return false;
+      if (globaltimer() - t0 > limit_ns) {
+        atomicCAS(status, ST_OK, code);
         return false;
       }
     }
   }
 }
 
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const TcArgs& g, int code, bool abort = true,
+                                          bool backoff = false) {
+  return mbar_test(bar, parity) || mbar_wait_slow(bar, parity, g.status, g.timeout_ns, code, abort, backoff);
+}
+
+// The same for a whole warp, with one answer for all its lanes.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, const TcArgs& g, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, g, code));
+}
+// One box of U: g.sc chunks of 64 columns of 128 rows (a stage, or the whole half
+// of a column tile), from chunk c and row y. One instruction per operand tile: the
+// producer thread needs some 150 clocks for each, and seven a tile (one per chunk,
+// one L2 prefetch per chunk, the row parameters) bounded the pipeline at 1,700.
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int y, int c) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::
           "r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(0), "r"(y), "r"(c)
       : "memory");
 }
 
-// L2 prefetch of one tensor-map box (no shared memory, no completion).
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)),
-               "r"(x), "r"(y)
+// L2 prefetch of one box (no shared memory, no completion).
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int y, int c) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(
+                   reinterpret_cast<uint64_t>(map)),
+               "r"(0), "r"(y), "r"(c)
                : "memory");
 }
 
@@ -188,50 +225,52 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                : "memory");
 }
 
-// Shared-memory matrix descriptor: K-major, SWIZZLE_128B (128-byte rows),
-// 8-row groups 1024 B apart.
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>(1) << 16;           // leading byte offset (unused for swizzled K-major)
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;   // stride byte offset
-  d |= static_cast<uint64_t>(1) << 46;           // descriptor version (sm_100)
-  d |= static_cast<uint64_t>(2) << 61;           // SWIZZLE_128B
-  return d;
-}
+// Shared-memory matrix descriptors: K-major, SWIZZLE_128B (128-byte rows), 8-row
+// groups 1,024 B apart. Only the start address (16-byte units, low word) differs
+// between operands; the rest is the constant high word (stride 64 units,
+// descriptor version 1, swizzle mode 2).
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | (1u << 16); }
 
-// Same for SWIZZLE_64B (64-byte rows, 8-row groups 512 B apart): the 32-column
-// tail of K' in the whole-tile mode.
-__device__ __forceinline__ uint64_t desc_sw64(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>(1) << 16;
-  d |= static_cast<uint64_t>(512 >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(4) << 61;  // SWIZZLE_64B
-  return d;
-}
-
-// Instruction descriptor, kind::f16: D = F32, A = B = BF16, both K-major, M = 128, N = BN.
-template <int BN>
+// Instruction descriptor, kind::f16: D = F32, A = B = FP16, both K-major, M = 128
+// rows per CTA of the group, N = 256.
+template <int CTAS>
 constexpr uint32_t idesc() {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BN >> 3) << 17) |
-         (static_cast<uint32_t>(kBM >> 4) << 24);
+  return (1u << 4) | (static_cast<uint32_t>(kBN >> 3) << 17) | (static_cast<uint32_t>(CTAS * kBM >> 4) << 24);
 }
 
-template <int BN>
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(da), "l"(db), "r"(idesc<BN>()), "r"(accumulate)
-      : "memory");
+template <int CTAS>
+__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint32_t da_lo, uint32_t db_lo, uint32_t accumulate) {
+  if constexpr (CTAS == 2)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+        "mov.b64 a, {%1, %3};\n\t"
+        "mov.b64 b, {%2, %3};\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %4, p;\n\t}" ::"r"(tmem_d),
+        "r"(da_lo), "r"(db_lo), "n"(kDescHi), "n"(idesc<2>()), "r"(accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+        "mov.b64 a, {%1, %3};\n\t"
+        "mov.b64 b, {%2, %3};\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}" ::"r"(tmem_d),
+        "r"(da_lo), "r"(db_lo), "n"(kDescHi), "n"(idesc<1>()), "r"(accumulate)
+        : "memory");
 }
 
+// Arrive on this barrier (in both CTAs of a pair) once every MMA issued so far is complete.
+template <int CTAS>
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
+  if constexpr (CTAS == 2)
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+        "h"((unsigned short)3)
+        : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -244,8 +283,13 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "r"(taddr)
-               : "memory");
+               : "r"(taddr));
+}
+
+// A batch: 16 columns of all 32 lanes.
+__device__ __forceinline__ void tmem_ld_batch(uint32_t taddr, uint32_t (&v)[2][8]) {
+  tmem_ld8(taddr, v[0]);
+  tmem_ld8(taddr + (16u << 16), v[1]);
 }
 
 // Wait for every TMEM load this thread issued; the register operands tie
@@ -253,8 +297,11 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
 __device__ __forceinline__ void tmem_wait8(uint32_t (&v)[8]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;"
                : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])
-               :
-               : "memory");
+               :);
+}
+__device__ __forceinline__ void tmem_wait_batch(uint32_t (&v)[2][8]) {
+  tmem_wait8(v[0]);
+  tmem_wait8(v[1]);
 }
 
 // ---------------------------------------------------------------------------
@@ -285,7 +332,7 @@ constexpr float kFirstTol = 6.9e-4f;
 // 2^-161 flushes to 0 in ex2.approx.ftz with any FP32 partner: all pair terms are 0.
 constexpr float kZeroDist = 12.7f;
 
-enum SlabMode { kPure = 0, kFirst = 1, kPairFirst = 2, kPairExact = 3, kZero = 4 };
+enum SlabMode { kZero = 0, kPure = 1, kFirst = 2, kPairFirst = 3, kPairExact = 4 };
 
 template <int METRIC>
 constexpr bool weighted_num() {
@@ -296,32 +343,49 @@ constexpr bool nrmse_tc() {
   return METRIC == kNrmse || METRIC == kNrmseW;
 }
 
-// Coefficient of dp dq in the neglected factor: 2 ln2 for the weight, plus for
-// SSIM the mixed second derivative of 1 / (sigma_p^2 + sigma_q^2 + c2).
-template <int METRIC>
-__device__ __forceinline__ float mixed_coeff(float alpha, float beta, const EpiConsts& ec) {
-  float k = 1.3862944f;
-  if (METRIC == kSsim) {
-    const float sa = alpha * ec.inv_wscale, sb = beta * ec.inv_wscale;
-    const float S = fmaf(sa, sa, fmaf(sb, sb, ec.c2));
-    k += 4.0f * sa * sb * ec.inv_wscale * ec.inv_wscale / (S * S);
-  }
-  return k;
-}
+// What a factorised slab needs beside its parameters: the row factor is
+// f_p = 2^(-(a_p - beta)^2 + sf (a_p - alpha)) cf, the column factor
+// g_q = 2^(dq (eg - dq)), and kc dp dq the first-order term. Pearson's
+// 1/(1 + t), t = eps / (sigma_p sigma_q) = tau / (a_p a_q), is cf = 1/(1 + t0)
+// at the centres and, to first order in dp and dq, a linear term in each
+// exponent (sf and part of eg).
+struct SlabC {
+  float alpha, beta, cf, sf, eg, kc;
+};
 
 // The form a slab takes. rg, cg: {centre of a, half range of a, centre of r, half range of r}.
 template <int METRIC>
-__device__ __forceinline__ int slab_mode(const float4& rg, const float4& cg, const EpiConsts& ec) {
-  if (!weighted_num<METRIC>()) return kPairExact;
-  const float D = fabsf(rg.x - cg.x);
-  if (D - rg.y - cg.y > kZeroDist) return kZero;
-  const float e = mixed_coeff<METRIC>(rg.x, cg.x, ec) * rg.y * cg.y;
-  bool ok = e <= kFirstTol && D * cg.y <= 24.0f;
-  // Pearson: 1/(1+t) = its values through the group centres up to eps dr_p dr_q
-  if (METRIC == kPearson) ok = ok && kEps * rg.w * cg.w <= 1.2e-7f;
-  // SSIM: 2 sp sq G + c2 = 2 sp sq (G + c2/2 rp rq), so no block of sigma 0 and no overflow
-  if (METRIC == kSsim) ok = ok && rg.z - rg.w > 0.0f && cg.z - cg.w > 0.0f && (rg.z + rg.w) * (cg.z + cg.w) < 1e25f;
-  if (ok) return e <= kPureTol ? kPure : kFirst;
+__device__ __forceinline__ int slab_mode(const float4& rg, const float4& cg, const EpiConsts& ec, SlabC& sc) {
+  const float D = rg.x - cg.x;
+  sc.alpha = rg.x;
+  sc.beta = cg.x;
+  sc.cf = nrmse_tc<METRIC>() ? 1.0f : ec.gscale;  // (NRMSE scales G itself)
+  sc.sf = 0.0f;
+  sc.eg = 2.0f * D;
+  sc.kc = 1.3862944f;  // 2 ln2
+  if (fabsf(D) - rg.y - cg.y > kZeroDist) return kZero;
+  bool ok = fabsf(D) * cg.y <= 24.0f;
+  if (METRIC == kPearson) {
+    const float ra = rcp_approx(rg.x), rb = rcp_approx(cg.x);
+    const float t0 = ec.tau * ra * rb, c = rcp_approx(1.0f + t0), u = 1.442695f * t0 * c;
+    sc.cf *= c;
+    sc.sf = u * ra;
+    sc.eg = fmaf(u, rb, sc.eg);
+    // the neglected second order of t: t0 times the squared relative ranges
+    const float q = rg.y * ra + cg.y * rb;
+    ok = ok && q <= 0.25f && t0 * q * q <= 1.2e-7f && t0 < 0.125f;
+  }
+  if (METRIC == kSsim) {
+    // 1/(sigma_p^2 + sigma_q^2 + c2) splits through the centres; its mixed second
+    // derivative joins the first-order term. 2 sp sq G + c2 = 2 sp sq (G + c2/2 rp rq)
+    // needs sigma > 0 and no overflow.
+    const float sa = rg.x * ec.inv_wscale, sb = cg.x * ec.inv_wscale;
+    const float S = fmaf(sa, sa, fmaf(sb, sb, ec.c2));
+    sc.kc += 4.0f * sa * sb * ec.inv_wscale * ec.inv_wscale / (S * S);
+    ok = ok && rg.z - rg.w > 0.0f && cg.z - cg.w > 0.0f && (rg.z + rg.w) * (cg.z + cg.w) < 1e25f;
+  }
+  const float e = sc.kc * rg.y * cg.y;
+  if (ok && e <= kFirstTol) return e <= kPureTol ? kPure : kFirst;
   if (METRIC == kPearson && kEps * (rg.z + rg.w) * (cg.z + cg.w) < kTFirst) return kPairFirst;
   return kPairExact;
 }
@@ -440,64 +504,72 @@ __device__ __forceinline__ void f2_add_half(F2& v, int half, float x) {
   v = f2(lo, hi);
 }
 
-// One 32-row x BN/4-column slab of a tile for this warp: BN/64 chunks of 16
-// columns, each read for both 16-lane halves of the warp's 32 TMEM lanes. Each
-// thread has 4 rows (32(w%4) + t/4 + 8k) and 4 columns per chunk (2(t%4) + {0, 1},
-// 8 + 2(t%4) + {0, 1}). rs: the tile's row parameters; cs: this warp's column
-// parameters (permuted); cacc[c][rep]: the item's column sums of this thread,
-// in registers; p0: block index of tile row 0; q0: of the slab's first column;
-// fs: this warp's scratch (32 + BN/4 floats). Row sums go to rsum[k].
+// A warp's part of a tile, a slab: 32 rows x W columns, in chunks of 16
+// columns, each read for both 16-lane halves of the warp's 32 TMEM lanes. Each thread has 4
+// rows (32(w%4) + t/4 + 8k) and 4 columns per chunk (2(t%4) + {0, 1}, 8 + 2(t%4) +
+// {0, 1}). rs: the tile's row parameters; cs: the slab's column parameters
+// (permuted); cacc[c][rep]: the item's column sums of this thread, in registers;
+// p0: block index of tile row 0; q0: of the slab's first column; fs: this warp's
+// scratch (f by row, then g by permuted column). Row sums go to rsum[k].
 //
-// Factorised slab (FIRST: with the first-order weight factor per pair).
-template <int METRIC, int BN, bool FIRST>
-__device__ __forceinline__ void slab_factor(uint32_t taddr, const float* __restrict__ rs, const float* __restrict__ cs,
-                                            const float4& rg, const float4& cg, float* __restrict__ fs,
-                                            F2 (&cacc)[Cfg<BN>::kCH][2], const EpiConsts& ec, int p0, int q0,
+// Row and column factors of the slab: row 32(w%4) + lane and columns (permuted
+// positions) lane + 32 j of this lane. They need no accumulator, so they are
+// computed while its MMAs run.
+template <int METRIC>
+__device__ __forceinline__ void slab_factors(const float* __restrict__ rs, const float* __restrict__ cs,
+                                             const SlabC& sc, float* __restrict__ fs, const EpiConsts& ec) {
+  const int lane = threadIdx.x & 31;
+  const int row = (threadIdx.x & 96) + lane;
+  const float sa = sc.alpha * ec.inv_wscale, sb = sc.beta * ec.inv_wscale;
+  const float a = rs[row], d = a - sc.beta;
+  float f = ex2_approx(fmaf(-d, d, sc.sf * (a - sc.alpha))) * sc.cf;
+  if (METRIC == kSsim) {
+    const float s = rs[kRowS + row];
+    f *= 2.0f * s * rcp_approx(fmaf(s, s, fmaf(sb, sb, ec.c2)));
+  }
+  fs[(lane & 7) * 4 + (lane >> 3)] = f;
+  const float S = fmaf(sa, sa, fmaf(sb, sb, ec.c2));
+#pragma unroll
+  for (int j = 0; j < Cfg<METRIC>::kColW / 32; j++) {
+    const int i = lane + 32 * j;
+    const float dq = cs[i] - sc.beta;
+    float g = ex2_approx(dq * (sc.eg - dq));
+    if (METRIC == kSsim) {
+      const float s = cs[2 * kBN + i];
+      g *= s * S * rcp_approx(fmaf(s, s, fmaf(sa, sa, ec.c2)));
+    }
+    fs[32 + i] = g;
+  }
+}
+
+// The slab's pair loop (FIRST: with the first-order weight factor per pair;
+// unweighted NRMSE has no factors). TMEM is read 16 columns at a time, the next
+// 16 issued before the current ones are evaluated.
+template <int METRIC, bool FIRST>
+__device__ __forceinline__ void tile_factor(uint32_t taddr, const float* __restrict__ rs, const float* __restrict__ cs,
+                                            const SlabC& sc, const float* __restrict__ fs,
+                                            F2 (&cacc)[Cfg<METRIC>::kCH][2], const EpiConsts& ec, int p0, int q0,
                                             float (&rsum)[4]) {
-  constexpr int CH = Cfg<BN>::kCH, W = Cfg<BN>::kColW;
+  constexpr int CH = Cfg<METRIC>::kCH;
+  constexpr bool WGT = weighted_num<METRIC>();
   const int lane = threadIdx.x & 31, rsub = lane >> 2, csub = lane & 3;
   const int quarter = (threadIdx.x >> 5) & 3;
-  uint32_t buf[2][8];
-  tmem_ld8(taddr, buf[0]);
-  // f of row `lane` and g of columns (permuted positions) 2 lane, 2 lane + 1
-  const float sa = rg.x * ec.inv_wscale, sb = cg.x * ec.inv_wscale;
-  {
-    const int row = quarter * 32 + lane;
-    const float d = rs[row] - cg.x;
-    float f = ex2_approx(-d * d);
-    if (METRIC == kPearson) f *= ec.gscale * rcp_approx(fmaf(kEps * rs[kRowR + row], cg.z, 1.0f));
-    if (METRIC == kSsim) {
-      const float s = rs[kRowS + row];
-      f *= ec.gscale * 2.0f * s * rcp_approx(fmaf(s, s, fmaf(sb, sb, ec.c2)));
-    }
-    fs[(lane & 7) * 4 + (lane >> 3)] = f;
-    const float D2 = 2.0f * (rg.x - cg.x);
-    const float cn = METRIC == kPearson ? fmaf(kEps * rg.z, cg.z, 1.0f)
-                                        : (METRIC == kSsim ? fmaf(sa, sa, fmaf(sb, sb, ec.c2)) : 1.0f);
-#pragma unroll
-    for (int j = 0; j < W / 32; j++) {
-      const int i = lane + 32 * j;
-      const float dq = cs[i] - cg.x;
-      float g = ex2_approx(dq * (D2 - dq));
-      if (METRIC == kPearson) g *= cn * rcp_approx(fmaf(kEps * rg.z, cs[BN + i], 1.0f));
-      if (METRIC == kSsim) {
-        const float s = cs[2 * BN + i];
-        g *= s * cn * rcp_approx(fmaf(s, s, fmaf(sa, sa, ec.c2)));
-      }
-      fs[32 + i] = g;
-    }
+  uint32_t buf[2][2][8];
+  tmem_ld_batch(taddr, buf[0]);
+  F2 fr[4], rn[4], dp[4], mu[4], rr[4], sg[4];
+  if (WGT) {
+    const float4 f4 = *reinterpret_cast<const float4*>(fs + 4 * rsub);
+    fr[0] = f2(f4.x, f4.x);
+    fr[1] = f2(f4.y, f4.y);
+    fr[2] = f2(f4.z, f4.z);
+    fr[3] = f2(f4.w, f4.w);
   }
-  __syncwarp();
-  const float4 f4 = *reinterpret_cast<const float4*>(fs + 4 * rsub);
-  const F2 fr[4] = {f2(f4.x, f4.x), f2(f4.y, f4.y), f2(f4.z, f4.z), f2(f4.w, f4.w)};
-  F2 rn[4], dp[4], mu[4], rr[4], sg[4];
-  const float kc = FIRST ? mixed_coeff<METRIC>(rg.x, cg.x, ec) : 0.0f;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     rn[k] = f2(0.0f, 0.0f);
     const int row = quarter * 32 + rsub + 8 * k;
     if (FIRST) {
-      const float v = kc * (rs[row] - rg.x);
+      const float v = sc.kc * (rs[row] - sc.alpha);
       dp[k] = f2(v, v);
     }
     if (METRIC == kSsim) {
@@ -505,42 +577,41 @@ __device__ __forceinline__ void slab_factor(uint32_t taddr, const float* __restr
       mu[k] = f2(m, m);
       rr[k] = f2(r, r);
     }
-    if (METRIC == kNrmseW) {
+    if (nrmse_tc<METRIC>()) {
       const float v = rs[kRowS + row];
       sg[k] = f2(v, v);
     }
   }
-  tmem_wait8(buf[0]);
+  tmem_wait_batch(buf[0]);
 #pragma unroll
   for (int c = 0; c < CH; c++) {
-    const int cb = 16 * c + 4 * csub;
-    const float4 g4 = *reinterpret_cast<const float4*>(fs + 32 + cb);
-    float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f), s4 = r4, m4 = r4, a4 = r4;
-    if (FIRST) a4 = *reinterpret_cast<const float4*>(cs + cb);
-    if (METRIC == kSsim) {
-      r4 = *reinterpret_cast<const float4*>(cs + BN + cb);
-      m4 = *reinterpret_cast<const float4*>(cs + 3 * BN + cb);
-    }
-    if (METRIC == kNrmseW) s4 = *reinterpret_cast<const float4*>(cs + 2 * BN + cb);
-    const F2 qg[2] = {f2(g4.x, g4.y), f2(g4.z, g4.w)};
-    F2 cn[2] = {f2(0.0f, 0.0f), f2(0.0f, 0.0f)};
-#pragma unroll
-    for (int hh = 0; hh < 2; hh++) {
-      const int step = c * 2 + hh;
-      uint32_t(&cur)[8] = buf[step & 1];
-      uint32_t(&nxt)[8] = buf[(step + 1) & 1];
-      if (step + 1 < CH * 2) tmem_ld8(taddr + ((uint32_t)(16 * ((step + 1) & 1)) << 16) + 16 * ((step + 1) >> 1), nxt);
+    uint32_t(&cur)[2][8] = buf[c & 1];
+    uint32_t(&nxt)[2][8] = buf[(c + 1) & 1];
+    if (c + 1 < CH) tmem_ld_batch(taddr + 16 * (c + 1), nxt);
+    {
+      const int cb = 16 * c + 4 * csub;
+      float4 g4 = make_float4(0.f, 0.f, 0.f, 0.f), r4 = g4, s4 = g4, m4 = g4, a4 = g4;
+      if (WGT) g4 = *reinterpret_cast<const float4*>(fs + 32 + cb);
+      if (FIRST) a4 = *reinterpret_cast<const float4*>(cs + cb);
+      if (METRIC == kSsim) {
+        r4 = *reinterpret_cast<const float4*>(cs + kBN + cb);
+        m4 = *reinterpret_cast<const float4*>(cs + 3 * kBN + cb);
+      }
+      if (nrmse_tc<METRIC>()) s4 = *reinterpret_cast<const float4*>(cs + 2 * kBN + cb);
+      const F2 qg[2] = {f2(g4.x, g4.y), f2(g4.z, g4.w)};
+      F2 cn[2] = {f2(0.0f, 0.0f), f2(0.0f, 0.0f)};
       float near = 1.0f;  // NRMSE: smallest 1 - G
 #pragma unroll
       for (int rep = 0; rep < 2; rep++) {
-        const F2 dq = FIRST ? sub2(rep ? f2(a4.z, a4.w) : f2(a4.x, a4.y), f2(cg.x, cg.x)) : f2(0.0f, 0.0f);
+        const F2 dq = FIRST ? sub2(rep ? f2(a4.z, a4.w) : f2(a4.x, a4.y), f2(sc.beta, sc.beta))
+                            : f2(0.0f, 0.0f);
         const F2 qr = rep ? f2(r4.z, r4.w) : f2(r4.x, r4.y);
         const F2 qs = rep ? f2(s4.z, s4.w) : f2(s4.x, s4.y);
         const F2 qm = rep ? f2(m4.z, m4.w) : f2(m4.x, m4.y);
 #pragma unroll
-        for (int kk = 0; kk < 2; kk++) {
-          const int kr = 2 * hh + kk;
-          const float g0 = __uint_as_float(cur[4 * rep + 2 * kk]), g1 = __uint_as_float(cur[4 * rep + 2 * kk + 1]);
+        for (int kr = 0; kr < 4; kr++) {
+          const int vi = 4 * rep + 2 * (kr & 1);
+          const float g0 = __uint_as_float(cur[kr >> 1][vi]), g1 = __uint_as_float(cur[kr >> 1][vi + 1]);
           F2 x;
           if (METRIC == kPearson) {
             x = f2(fmaxf(g0, 0.0f), fmaxf(g1, 0.0f));
@@ -560,54 +631,63 @@ __device__ __forceinline__ void slab_factor(uint32_t taddr, const float* __restr
             x = nrmse_term2(G, sg[kr], add2(sg[kr], sg[kr]), qs, ec);
           }
           if (FIRST) x = fma2(mul2(x, dp[kr]), dq, x);
-          rn[kr] = fma2(x, qg[rep], rn[kr]);
-          cn[rep] = fma2(x, fr[kr], cn[rep]);
+          if (WGT) {
+            rn[kr] = fma2(x, qg[rep], rn[kr]);
+            cn[rep] = kr == 0 ? mul2(x, fr[kr]) : fma2(x, fr[kr], cn[rep]);
+          } else {
+            rn[kr] = add2(rn[kr], x);
+            cn[rep] = kr == 0 ? x : add2(cn[rep], x);
+          }
         }
       }
-      if (METRIC == kNrmseW && near < 1.0f - ec.nrmse_near) {
+      if (nrmse_tc<METRIC>() && near < 1.0f - ec.nrmse_near) {
+        // Near-identical pairs: replace the accumulated term by the one of the
+        // exact squared difference.
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-          const int rep = j >> 2, kk = (j >> 1) & 1, lh = j & 1, kr = 2 * hh + kk;
-          const float g = __fmul_rn(__uint_as_float(cur[4 * rep + 2 * kk + lh]), ec.gscale);
+        for (int j = 0; j < 16; j++) {
+          const int rep = j >> 3, kr = (j >> 1) & 3, lh = j & 1;
+          const float g = __fmul_rn(__uint_as_float(cur[kr >> 1][4 * rep + 2 * (kr & 1) + lh]), ec.gscale);
           if (!(g > ec.nrmse_near)) continue;
           const int row = quarter * 32 + rsub + 8 * kr, q = q0 + 16 * c + 8 * rep + 2 * csub + lh;
           const int ci = 16 * c + 4 * csub + 2 * rep + lh;  // permuted column slot
-          float corr = nrmse_correction(g, rs[kRowS + row], cs[2 * BN + ci], p0 + row, q, ec.U, ec.kp, ec.K,
+          float corr = nrmse_correction(g, rs[kRowS + row], cs[2 * kBN + ci], p0 + row, q, ec.U, ec.kp, ec.K,
                                         ec.nrmse_scale);
-          if (FIRST) corr = fmaf(corr * kc * (rs[row] - rg.x), cs[ci] - cg.x, corr);
-          float glo, ghi, flo, fhi;
-          f2_split(qg[rep], glo, ghi);
-          f2_split(fr[kr], flo, fhi);
+          if (FIRST) corr = fmaf(corr * sc.kc * (rs[row] - sc.alpha), cs[ci] - sc.beta, corr);
+          float glo = 1.0f, ghi = 1.0f, flo = 1.0f, fhi;
+          if (WGT) {
+            f2_split(qg[rep], glo, ghi);
+            f2_split(fr[kr], flo, fhi);
+          }
           f2_add_half(rn[kr], lh, corr * (lh ? ghi : glo));
           f2_add_half(cn[rep], lh, corr * flo);
         }
       }
-      if (step + 1 < CH * 2) tmem_wait8(nxt);
+#pragma unroll
+      for (int rep = 0; rep < 2; rep++)
+        cacc[c][rep] = WGT ? fma2(cn[rep], qg[rep], cacc[c][rep]) : add2(cn[rep], cacc[c][rep]);
     }
-    cacc[c][0] = fma2(cn[0], qg[0], cacc[c][0]);
-    cacc[c][1] = fma2(cn[1], qg[1], cacc[c][1]);
+    if (c + 1 < CH) tmem_wait_batch(nxt);
   }
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    float lo, hi, f, fh;
+    float lo, hi;  // f is applied to the reduced row sums
     f2_split(rn[k], lo, hi);
-    f2_split(fr[k], f, fh);
-    rsum[k] = f * (lo + hi);
+    rsum[k] = lo + hi;
   }
 }
 
-// Pairwise slab. Row passes: the metrics with many row constants (SSIM, NRMSE)
+// Pairwise form. Row passes: the metrics with many row constants (SSIM, NRMSE)
 // take the 4 rows in two passes of 2 so that their constants fit in registers.
 template <int METRIC>
 constexpr int row_passes() {
   return (METRIC == kSsim || METRIC == kNrmse || METRIC == kNrmseW) ? 2 : 1;
 }
 
-template <int METRIC, int BN, bool EXACT, bool MASKED>
-__device__ __forceinline__ void slab_pairs(uint32_t taddr, const float* __restrict__ rs, const float* __restrict__ cs,
-                                           F2 (&cacc)[Cfg<BN>::kCH][2], int p0, int q0, const EpiConsts& ec,
+template <int METRIC, bool EXACT, bool MASKED>
+__device__ __forceinline__ void tile_pairs(uint32_t taddr, const float* __restrict__ rs, const float* __restrict__ cs,
+                                           F2 (&cacc)[Cfg<METRIC>::kCH][2], int p0, int q0, const EpiConsts& ec,
                                            float (&rsum)[4]) {
-  constexpr int CH = Cfg<BN>::kCH;
+  constexpr int CH = Cfg<METRIC>::kCH;
   constexpr int NP = row_passes<METRIC>(), R = 4 / NP;  // passes, rows per pass
   constexpr int HP = R / 2;                              // 16-lane halves per pass
   const int lane = threadIdx.x & 31, rsub = lane >> 2, csub = lane & 3;
@@ -637,9 +717,9 @@ __device__ __forceinline__ void slab_pairs(uint32_t taddr, const float* __restri
       const int cb = 16 * c + 4 * csub;
       float4 a4 = make_float4(0.f, 0.f, 0.f, 0.f), r4 = a4, s4 = a4, m4 = a4;
       if (METRIC != kNrmse && METRIC != kDebugSum) a4 = *reinterpret_cast<const float4*>(cs + cb);
-      if (METRIC == kPearson || METRIC == kDebugSum) r4 = *reinterpret_cast<const float4*>(cs + BN + cb);
-      if (METRIC == kSsim || nrmse_tc<METRIC>()) s4 = *reinterpret_cast<const float4*>(cs + 2 * BN + cb);
-      if (METRIC == kSsim) m4 = *reinterpret_cast<const float4*>(cs + 3 * BN + cb);
+      if (METRIC == kPearson || METRIC == kDebugSum) r4 = *reinterpret_cast<const float4*>(cs + kBN + cb);
+      if (METRIC == kSsim || nrmse_tc<METRIC>()) s4 = *reinterpret_cast<const float4*>(cs + 2 * kBN + cb);
+      if (METRIC == kSsim) m4 = *reinterpret_cast<const float4*>(cs + 3 * kBN + cb);
 #pragma unroll
       for (int hh = 0; hh < HP; hh++) {
         const int step = c * HP + hh;
@@ -712,7 +792,7 @@ __device__ __forceinline__ void slab_pairs(uint32_t taddr, const float* __restri
             if (MASKED && force[kr] && q == p) ge = 1.0f;
             if (!(ge > ec.nrmse_near) || !rv) continue;
             const int ci = 16 * c + 4 * csub + 2 * rep + lh;  // permuted column slot
-            float corr = nrmse_correction(ge, rs[kRowS + row], cs[2 * BN + ci], p, q, ec.U, ec.kp, ec.K, ec.nrmse_scale);
+            float corr = nrmse_correction(ge, rs[kRowS + row], cs[2 * kBN + ci], p, q, ec.U, ec.kp, ec.K, ec.nrmse_scale);
             if (METRIC == kNrmseW) {
               const float d = __fsub_rn(rs[row], cs[ci]);
               corr *= ex2_approx(-__fmul_rn(d, d));
@@ -902,172 +982,188 @@ struct ItemCursor {
   }
 };
 
+template <int CTAS>
 __device__ __forceinline__ ItemCursor first_item(const TcArgs& g) {
   ItemCursor c;
-  c.init(g, g.item0 + blockIdx.x);
+  c.init(g, g.item0 + blockIdx.x / CTAS);
   return c;
 }
 
-// End of a role: all warps meet, then the MMA warp frees TMEM.
-__device__ __forceinline__ void role_exit(uint32_t tmem, int tmem_cols, bool owner) {
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  if (owner) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols) : "memory");
+template <int CTAS>
+__device__ __forceinline__ void group_sync() {
+  if constexpr (CTAS == 2) cluster_sync();
+  else __syncthreads();
 }
 
-// TR (whole-tile mode, when two A tiles and the B tile fit): A moves one
-// whole 128-row tile at a time through two buffers, and the single
-// tcgen05.commit per tile both publishes the accumulator and frees the tile's
-// A buffer (the producer waits on the accumulator barrier). K' = 64 c + 32 t:
-// c SWIZZLE_128B chunks and an optional SWIZZLE_64B tail.
-// !TR (chunk ring): A moves in 64-column chunks through S stages, one commit
-// per chunk.
-template <int METRIC, int BN, bool TR>
-__global__ void __launch_bounds__(kThreads, 1)
-    k_gram_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-              const __grid_constant__ CUtensorMap tmA64, const __grid_constant__ CUtensorMap tmB64, TcArgs g) {
-  using C = Cfg<BN>;
-  constexpr int CH = C::kCH;
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t raw = smem_u32(smem_raw);
-  const uint32_t base = (raw + 1023u) & ~1023u;
-  uint8_t* sbase = smem_raw + (base - raw);
-  const int S = g.stages, nkc = g.nkc;
-  const uint32_t sB = base;                                            // resident B tile
-  const uint32_t sA = sB + g.b_bytes;                                  // TR: 2 x a_bytes; else S x 16 KB
-  const uint32_t sC = sA + (TR ? 2 * g.a_bytes : S * kAChunkBytes);    // 2 column-parameter slots
-  const uint32_t sR = sC + 2 * C::kCSoa * 4;                           // kRSlots row-parameter slots
-  const uint32_t sP = sR + kRSlots * kRowFloats * 4;                   // row partials
-  const uint32_t sF = sP + kRowPartBytes;                              // f and g of each epilogue warp
-  const uint32_t sBar = sF + kEpiWarps * C::kScratch * 4;
+// End of a role: all warps (of both CTAs of a pair) meet (no CTA leaves while the
+// other may still arrive on its barriers or an MMA reads its shared memory), then
+// the MMA warps free TMEM.
+template <int CTAS>
+__device__ __forceinline__ void role_exit(uint32_t tmem, bool owner) {
+  tc_fence_before();
+  group_sync<CTAS>();
+  tc_fence_after();
+  if (!owner) return;
+  if constexpr (CTAS == 2)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kBN) : "memory");
+  else
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kBN) : "memory");
+}
+
+template <int METRIC, int CTAS>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
+    k_gram_tc(const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUtensorMap tmB, TcArgs g) {
+  using C = Cfg<METRIC>;
+  constexpr int CH = C::kCH, EW = kEpiWarps, W = C::kColW, SETS = C::kSets;
+  constexpr int M = CTAS;            // row blocks per tile
+  constexpr int BH = 2 / CTAS;       // halves of the column tile in this CTA
+  extern __shared__ __align__(1024) uint8_t sbase[];  // (swizzled tiles need 1,024-byte alignment)
+  const uint32_t base = smem_u32(sbase);
+  const int S = g.stages;
+  const uint32_t rank = CTAS == 2 ? blockIdx.x & 1 : 0, n_clusters = gridDim.x / CTAS;
+  const uint32_t stage_bytes = (uint32_t)g.sc * kChunkBytes;
+  const uint32_t sB = base;                                            // this CTA's part of the column tile
+  const uint32_t sA = sB + BH * g.nch * kChunkBytes;                   // S stages of row-block chunks
+  const uint32_t sC = sA + S * stage_bytes;                            // 2 column-parameter slots
+  const uint32_t sR = sC + 2 * kColFloats * 4;                         // kRSlots row-parameter slots
+  const uint32_t sF = sR + kRSlots * kRowFloats * 4;                   // f and g of each epilogue warp
+  const uint32_t sBar = sF + EW * kScratch * 4;
   const float* cslots = reinterpret_cast<const float*>(sbase + (sC - base));
   const float* rslots = reinterpret_cast<const float*>(sbase + (sR - base));
-  float* rowpart = reinterpret_cast<float*>(sbase + (sP - base));
   float* scratch = reinterpret_cast<float*>(sbase + (sF - base));
   // barriers: a_full[16], a_empty[16], b_full, b_empty, acc_full[2], acc_empty[2],
-  //           c_full[2], c_empty[2], r_full[2], r_empty[2], done; then the TMEM
-  //           address and 8 row-partial counters
+  //           c_full[2], c_empty[2], r_full[4], r_empty[4], done; then the TMEM
+  //           address
   const uint32_t b_afull = sBar, b_aempty = b_afull + 8 * kMaxStages, b_bfull = b_aempty + 8 * kMaxStages,
                  b_bempty = b_bfull + 8, b_accf = b_bempty + 8, b_acce = b_accf + 16, b_cfull = b_acce + 16,
                  b_cempty = b_cfull + 16, b_rfull = b_cempty + 16, b_rempty = b_rfull + 8 * kRSlots,
                  b_done = b_rempty + 8 * kRSlots;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sbase + (b_done + 8 - base));
-  // per (accumulator buffer, quarter): column-group warps that have written
-  // their row partials of the current tile (the fourth combines them)
-  unsigned* rowcnt = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // (warp: uniform)
   if (threadIdx.x == 0) {
+    // operand barriers of CTA 0: its own producer and CTA 1's relay
+    const uint32_t full = CTAS == 2 && rank == 0 ? 2 : 1;
     for (int s = 0; s < kMaxStages; s++) {
-      mbar_init(b_afull + 8 * s, 1);
+      mbar_init(b_afull + 8 * s, full);
       mbar_init(b_aempty + 8 * s, 1);
     }
-    mbar_init(b_bfull, 1);
+    mbar_init(b_bfull, full);
     mbar_init(b_bempty, 1);
     for (int b = 0; b < 2; b++) {
       mbar_init(b_accf + 8 * b, 1);
-      mbar_init(b_acce + 8 * b, kEpiWarps);
+      mbar_init(b_acce + 8 * b, CTAS * EW / SETS);  // (CTA 0's: the epilogue warps of both CTAs)
       mbar_init(b_cfull + 8 * b, 1);
-      mbar_init(b_cempty + 8 * b, kEpiWarps);
+      mbar_init(b_cempty + 8 * b, EW);
     }
     for (int r = 0; r < kRSlots; r++) {
       mbar_init(b_rfull + 8 * r, 1);
-      mbar_init(b_rempty + 8 * r, kEpiWarps);
+      mbar_init(b_rempty + 8 * r, EW / SETS);
     }
-    for (int i = 0; i < 8; i++) rowcnt[i] = 0;
     mbar_init(b_done, 1);
+    if (base & 1023) atomicCAS(g.status, ST_OK, ST_ALIGNMENT);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == kEpiWarps + 1) {  // MMA warp owns the TMEM allocation
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(2 * BN)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  // Operand offsets (16-byte units, within a stage and the column tile) of the
+  // tile's MMAs, in the order of the row operand's blocks: hi blocks with hi and
+  // mid, mid blocks with hi, row tails with column tails. A block of 16 fp16 is 32 B,
+  // four to a chunk.
+  uint2* mma_tab = reinterpret_cast<uint2*>(sbase + (sBar + kBarBytes - base));
+  uint32_t* mma_end = reinterpret_cast<uint32_t*>(mma_tab + kMaxMma);  // MMAs up to the end of each stage
+  if (warp == 2) {
+    const int nb = g.nb, nt = g.nt, n = 3 * nb + nt;
+    constexpr uint32_t kChunkU = kChunkBytes >> 4;
+    for (int m = lane; m <= n; m += 32) {  // (entry n: read ahead, never used)
+      int qa, qb;
+      if (m < 2 * nb) {
+        qa = m >> 1;
+        qb = (m & 1) ? nb + qa : qa;
+      } else if (m < 3 * nb) {
+        qa = m - nb;
+        qb = qa - nb;
+      } else {
+        qa = min(m - nb, 2 * nb + nt - 1);
+        qb = qa + nt;
+      }
+      const uint32_t ca = (uint32_t)(qa >> 2) % (uint32_t)g.sc, cb = (uint32_t)(qb >> 2);
+      mma_tab[m] = make_uint2(ca * kChunkU + 2 * (qa & 3), cb * (BH * kChunkU) + 2 * (qb & 3));
+    }
+    for (int st = lane; st < g.nst; st += 32) {
+      const int q1 = min(2 * nb + nt, 4 * (st + 1) * g.sc);
+      mma_end[st] = q1 <= nb ? 2 * q1 : q1 + nb;
+    }
+  }
+  if (warp == 1) {  // the MMA warps of both CTAs own the TMEM allocation
+    if constexpr (CTAS == 2) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                   "r"(2 * kBN)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                   "r"(2 * kBN)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   tc_fence_before();
-  __syncthreads();
+  group_sync<CTAS>();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (warp == kEpiWarps) {
+  if (warp == 0) {
     // ---------------------------------------------------------------- TMA
     if (lane == 0) {
       long long tile = 0;
-      uint32_t item_i = 0, n_r = 0, n_a = 0;  // items, row-parameter loads, A loads (tiles or chunks) issued
-      uint32_t s = 0, eph = 0;                // chunk ring: stage, parity of the round being refilled
+      uint32_t item_i = 0, n_r = 0, n_a = 0;  // items, row-parameter loads, stage loads issued
+      uint32_t s = 0, eph = 0;                // ring: stage, parity of the round being refilled
       bool ok = true;
       for (int phase = 0; ok && phase < 2; phase++)
-      for (ItemCursor cur = first_item(g); ok && cur.it < g.item1; cur.advance(g, gridDim.x)) {
+      for (ItemCursor cur = first_item<CTAS>(g); ok && cur.it < g.item1; cur.advance(g, n_clusters)) {
         int ct, rb0, rb1;
-        if (!cur.part(g, C::kM, BN, phase, ct, rb0, rb1)) continue;
+        if (!cur.part(g, kBN / kBM, kBN, phase, ct, rb0, rb1)) continue;
         const uint32_t cs = item_i & 1;
         // the column-parameter slot the epilogue released two items ago, and the
         // B buffer once the MMAs of the previous item are complete
         if (!mbar_wait(b_cempty + 8 * cs, ((item_i >> 1) & 1) ^ 1, g, ST_TIMEOUT_PRODUCER, true, true)) { ok = false; break; }
         if (item_i > 0 && !mbar_wait(b_bempty, (item_i - 1) & 1, g, ST_TIMEOUT_PRODUCER, true, true)) { ok = false; break; }
-        mbar_expect_tx(b_cfull + 8 * cs, C::kCSoa * 4);
-        bulk_load(sC + cs * C::kCSoa * 4, g.colsoa + (size_t)ct * C::kCSoa, C::kCSoa * 4, b_cfull + 8 * cs);
-        mbar_expect_tx(b_bfull, g.b_bytes);
-        for (int c = 0; c < g.nfull; c++) tma_load_2d(sB + c * C::kBChunkBytes, &tmB, b_bfull, c * kChunk, ct * BN);
-        if (g.tail) tma_load_2d(sB + g.nfull * C::kBChunkBytes, &tmB64, b_bfull, g.nfull * kChunk, ct * BN);
+        mbar_expect_tx(b_bfull, BH * g.nch * kChunkBytes);
+        const int yb = ct * kBN + (int)rank * kBM;
+        for (int c = 0; c < g.nch; c += g.sc) tma_load_3d(sB + BH * c * kChunkBytes, &tmB, b_bfull, yb, c);
+        mbar_expect_tx(b_cfull + 8 * cs, kColFloats * 4);
+        bulk_load(sC + cs * kColFloats * 4, g.colsoa + (size_t)ct * kColFloats, kColFloats * 4, b_cfull + 8 * cs);
         item_i++;
-        {  // the B tile of this CTA's next item into L2
+        {  // the B tile of this cluster's next item into L2
           int nct, nrb0, nrb1;
           ItemCursor nx = cur;
-          nx.advance(g, gridDim.x);
-          if (nx.it < g.item1 && nx.part(g, C::kM, BN, phase, nct, nrb0, nrb1) && nct != ct) {
-            for (int c = 0; c < g.nfull; c++) tma_prefetch_2d(&tmB, c * kChunk, nct * BN);
-            if (g.tail) tma_prefetch_2d(&tmB64, g.nfull * kChunk, nct * BN);
-          }
+          nx.advance(g, n_clusters);
+          if (nx.it < g.item1 && nx.part(g, kBN / kBM, kBN, phase, nct, nrb0, nrb1) && nct != ct)
+            for (int c = 0; c < g.nch; c += g.sc) tma_prefetch_3d(&tmB, nct * kBN + (int)rank * kBM, c);
         }
-        for (int rb = rb0; ok && rb < rb1; rb++, tile++) {
+        for (int rb = rb0; ok && rb < rb1; rb += M, tile++) {
           if (tile == g.withhold) { ok = false; break; }
-          // A two row blocks ahead into L2, so that the copies below hit L2
-          if (rb + 2 < rb1) {
-            for (int c = 0; c < g.nfull; c++) tma_prefetch_2d(&tmA, c * kChunk, (rb + 2) * kBM);
-            if (g.tail) tma_prefetch_2d(&tmA64, g.nfull * kChunk, (rb + 2) * kBM);
-          }
-          // The A operand first (the MMA waits for it), then the row parameters
-          // (the epilogue needs them only once the accumulator is ready).
-          if (TR) {
-            // A buffer tile & 1 is free once the accumulator of tile - 2 is published
-            if (tile >= 2 && !mbar_wait(b_accf + 8 * (tile & 1), ((tile - 2) >> 1) & 1, g, ST_TIMEOUT_PRODUCER, true, true)) {
-              ok = false;
-              break;
-            }
-            const uint32_t ab = (uint32_t)(tile & 1);
-            const uint32_t dst = sA + ab * g.a_bytes;
-            mbar_expect_tx(b_afull + 8 * ab, g.a_bytes);
-            for (int c = 0; c < g.nfull; c++) tma_load_2d(dst + c * kAChunkBytes, &tmA, b_afull + 8 * ab, c * kChunk, rb * kBM);
-            if (g.tail) tma_load_2d(dst + g.nfull * kAChunkBytes, &tmA64, b_afull + 8 * ab, g.nfull * kChunk, rb * kBM);
+          const int ya = (rb + (int)rank) * kBM;
+          for (int st = 0; st < g.nst; st++) {
+            // stage s is free once the MMAs that read it are complete
+            if (!mbar_wait(b_aempty + 8 * s, eph ^ 1, g, ST_TIMEOUT_PRODUCER, true, true)) { ok = false; break; }
+            mbar_expect_tx(b_afull + 8 * s, stage_bytes);
+            tma_load_3d(sA + s * stage_bytes, &tmU, b_afull + 8 * s, ya, st * g.sc);
             n_a++;
-          } else {
-            for (int kc = 0; kc < nkc; kc++) {
-              if (!mbar_wait(b_aempty + 8 * s, eph ^ 1, g, ST_TIMEOUT_PRODUCER, true, true)) { ok = false; break; }
-              if (kc < g.nfull) {
-                mbar_expect_tx(b_afull + 8 * s, kAChunkBytes);
-                tma_load_2d(sA + s * kAChunkBytes, &tmA, b_afull + 8 * s, kc * kChunk, rb * kBM);
-              } else {  // the 32-column tail
-                mbar_expect_tx(b_afull + 8 * s, kAChunkBytes / 2);
-                tma_load_2d(sA + s * kAChunkBytes, &tmA64, b_afull + 8 * s, kc * kChunk, rb * kBM);
-              }
-              n_a++;
-              if (++s == (uint32_t)S) {
-                s = 0;
-                eph ^= 1;
-              }
+            if (++s == (uint32_t)S) {
+              s = 0;
+              eph ^= 1;
             }
-            if (!ok) break;
           }
+          if (!ok) break;
           const uint32_t rsl = (uint32_t)(tile & (kRSlots - 1));
           if (!mbar_wait(b_rempty + 8 * rsl, ((tile / kRSlots) & 1) ^ 1, g, ST_TIMEOUT_PRODUCER, true, true)) { ok = false; break; }
           mbar_expect_tx(b_rfull + 8 * rsl, kRowFloats * 4);
-          bulk_load(sR + rsl * kRowFloats * 4, g.rowsoa + (size_t)rb * kRowFloats, kRowFloats * 4, b_rfull + 8 * rsl);
+          bulk_load(sR + rsl * kRowFloats * 4, g.rowsoa + (size_t)(rb + (int)rank) * kRowFloats, kRowFloats * 4,
+                    b_rfull + 8 * rsl);
           n_r++;
         }
       }
-      // Drain: every issued copy has landed before the CTA may exit.
+      // Drain: every copy this CTA issued has landed before the CTA may exit.
       if (item_i > 0) {
         mbar_wait(b_bfull, (item_i - 1) & 1, g, ST_TIMEOUT_DRAIN, false);
         for (uint32_t k = (item_i > 2 ? item_i - 2 : 0); k < item_i; k++)
@@ -1075,211 +1171,209 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       for (uint32_t k = (n_r > (uint32_t)kRSlots ? n_r - kRSlots : 0); k < n_r; k++)
         mbar_wait(b_rfull + 8 * (k % kRSlots), (k / kRSlots) & 1, g, ST_TIMEOUT_DRAIN, false);
-      const uint32_t ring = TR ? 2u : (uint32_t)S;
+      const uint32_t ring = (uint32_t)S;
       for (uint32_t k = (n_a > ring ? n_a - ring : 0); k < n_a; k++)
         mbar_wait(b_afull + 8 * (k % ring), (k / ring) & 1, g, ST_TIMEOUT_DRAIN, false);
     }
     __syncwarp();
-    role_exit(tmem, 2 * BN, false);
+    role_exit<CTAS>(tmem, false);
     return;
-  } else if (warp == kEpiWarps + 1) {
-    // ---------------------------------------------------------------- MMA
+  } else if (warp == 1) {
+    // -------------------------------------------------- MMA (CTA 0), relay (CTA 1)
     if (lane == 0) {
-      long long tile = 0;
-      uint32_t item_i = 0;
-      uint32_t s = 0, fph = 0;  // chunk ring: stage, parity of the round being consumed
-      // Operand descriptors: the start-address field counts 16-byte units, so
-      // a K step of 16 bf16 (32 B) adds 2 and a chunk or stage adds its size / 16.
-      const uint64_t a_desc0 = desc_sw128(sA), b_desc0 = desc_sw128(sB);
+      uint32_t tile = 0, item_i = 0;
+      uint32_t s = 0, fph = 0;  // ring: stage, parity of the round being consumed
       bool ok = true;
-      for (int phase = 0; ok && phase < 2; phase++)
-      for (ItemCursor cur = first_item(g); ok && cur.it < g.item1; cur.advance(g, gridDim.x)) {
-        int ct, rb0, rb1;
-        if (!cur.part(g, C::kM, BN, phase, ct, rb0, rb1)) continue;
-        if (!mbar_wait(b_bfull, item_i & 1, g, ST_TIMEOUT_MMA, true, true)) { ok = false; break; }
-        tc_fence_after();
-        item_i++;
-        for (int rb = rb0; ok && rb < rb1; rb++, tile++) {
-          const uint32_t b = (uint32_t)(tile & 1);
-          if (!mbar_wait(b_acce + 8 * b, ((tile >> 1) & 1) ^ 1, g, ST_TIMEOUT_MMA, true, true)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t d = tmem + b * BN;
-          if (TR) {
-            if (!mbar_wait(b_afull + 8 * b, (tile >> 1) & 1, g, ST_TIMEOUT_MMA, true, true)) { ok = false; break; }
-            tc_fence_after();
-            const uint64_t da0 = a_desc0 + (uint64_t)((b * g.a_bytes) >> 4);
-            for (int c = 0; c < g.nfull; c++) {
-#pragma unroll
-              for (int ks = 0; ks < kChunk / 16; ks++)
-                mma_bf16<BN>(d, da0 + (uint64_t)(c * (kAChunkBytes >> 4) + 2 * ks),
-                             b_desc0 + (uint64_t)(c * (C::kBChunkBytes >> 4) + 2 * ks), (c | ks) != 0);
-            }
-            if (g.tail) {
-              const uint64_t da = desc_sw64(sA + b * g.a_bytes + g.nfull * kAChunkBytes);
-              const uint64_t db = desc_sw64(sB + g.nfull * C::kBChunkBytes);
-              mma_bf16<BN>(d, da, db, g.nfull != 0);
-              mma_bf16<BN>(d, da + 2, db + 2, 1);
-            }
-            mma_commit(b_accf + 8 * b);
-            continue;
-          }
-          for (int kc = 0; kc < nkc; kc++) {
-            if (!mbar_wait(b_afull + 8 * s, fph, g, ST_TIMEOUT_MMA, true, true)) { ok = false; break; }
-            tc_fence_after();
-            if (kc < g.nfull) {
-              const uint64_t da = a_desc0 + (uint64_t)(s * (kAChunkBytes >> 4));
-              const uint64_t db = b_desc0 + (uint64_t)(kc * (C::kBChunkBytes >> 4));
-#pragma unroll
-              for (int ks = 0; ks < kChunk / 16; ks++) mma_bf16<BN>(d, da + 2 * ks, db + 2 * ks, (kc | ks) != 0);
-            } else {
-              const uint64_t da = desc_sw64(sA + s * kAChunkBytes);
-              const uint64_t db = desc_sw64(sB + g.nfull * C::kBChunkBytes);
-              mma_bf16<BN>(d, da, db, kc != 0);
-              mma_bf16<BN>(d, da + 2, db + 2, 1);
-            }
-            mma_commit(b_aempty + 8 * s);
+      if (rank == 1) {
+        // CTA 1's operands are in place: tell the issuer
+        for (int phase = 0; ok && phase < 2; phase++)
+        for (ItemCursor cur = first_item<CTAS>(g); ok && cur.it < g.item1; cur.advance(g, n_clusters)) {
+          int ct, rb0, rb1;
+          if (!cur.part(g, kBN / kBM, kBN, phase, ct, rb0, rb1)) continue;
+          if (!mbar_wait(b_bfull, item_i & 1, g, ST_TIMEOUT_MMA)) { ok = false; break; }
+          mbar_arrive_cluster(leader_addr(b_bfull));
+          item_i++;
+          for (int k = (rb1 - rb0 + M - 1) / M * g.nst; k > 0; k--) {
+            if (!mbar_wait(b_afull + 8 * s, fph, g, ST_TIMEOUT_MMA)) { ok = false; break; }
+            mbar_arrive_cluster(leader_addr(b_afull + 8 * s));
             if (++s == (uint32_t)S) {
               s = 0;
               fph ^= 1;
             }
           }
-          if (ok) mma_commit(b_accf + 8 * b);
         }
-        if (ok) mma_commit(b_bempty);  // the item's B tile is free once these MMAs complete
+      } else {
+        // This thread's instructions between MMAs are tensor time (an MMA takes 128
+        // clocks), so the operand offsets come from a table, one entry ahead.
+        const uint32_t a0 = desc_lo(sA), b0 = desc_lo(sB), stage_u = stage_bytes >> 4;
+        const int nst = g.nst, n_mma = 3 * g.nb + g.nt;
+        for (int phase = 0; ok && phase < 2; phase++)
+        for (ItemCursor cur = first_item<CTAS>(g); ok && cur.it < g.item1; cur.advance(g, n_clusters)) {
+          int ct, rb0, rb1;
+          if (!cur.part(g, kBN / kBM, kBN, phase, ct, rb0, rb1)) continue;
+          if (!mbar_wait(b_bfull, item_i & 1, g, ST_TIMEOUT_MMA)) { ok = false; break; }
+          tc_fence_after();
+          item_i++;
+          for (int rb = rb0; ok && rb < rb1; rb += M, tile++) {
+            const uint32_t b = tile & 1;
+            if (!mbar_wait(b_acce + 8 * b, ((tile >> 1) & 1) ^ 1, g, ST_TIMEOUT_MMA)) { ok = false; break; }
+            const uint32_t d = tmem + b * kBN;
+            uint32_t acc = 0;
+            int m = 0;
+            for (int st = 0; st < nst; st++) {
+              if (!mbar_wait(b_afull + 8 * s, fph, g, ST_TIMEOUT_MMA)) { ok = false; break; }
+              if (st == 0) tc_fence_after();
+              const uint32_t as = a0 + s * stage_u;
+              const int m1 = st + 1 == nst ? n_mma : (int)mma_end[st];
+              uint2 e = mma_tab[m];
+#pragma unroll 2
+              while (m < m1) {
+                const uint2 cur_e = e;
+                e = mma_tab[++m];
+                mma_f16<CTAS>(d, as + cur_e.x, b0 + cur_e.y, acc);
+                acc = 1;
+              }
+              // one commit a stage: the accumulator's also frees the tile's last stage
+              // (the epilogue passes it on), a second one held the MMAs up 240 clocks
+              mma_commit<CTAS>(st + 1 == nst ? b_accf + 8 * b : b_aempty + 8 * s);
+              if (++s == (uint32_t)S) {
+                s = 0;
+                fph ^= 1;
+              }
+            }
+          }
+          if (ok) mma_commit<CTAS>(b_bempty);  // the item's B tile is free once these MMAs complete
+        }
+        // All MMAs this thread issued are complete before TMEM is released and
+        // the CTAs exit.
+        mma_commit<CTAS>(b_done);
+        mbar_wait(b_done, 0, g, ST_TIMEOUT_DRAIN, false);
       }
-      // All MMAs this thread issued are complete before TMEM is released and
-      // the CTA exits.
-      mma_commit(b_done);
-      mbar_wait(b_done, 0, g, ST_TIMEOUT_DRAIN, false);
     }
     __syncwarp();
-    role_exit(tmem, 2 * BN, true);
+    role_exit<CTAS>(tmem, true);
     return;
   } else {
     // ---------------------------------------------------------------- epilogue
-    const int quarter = warp & 3, group = warp >> 2;
-    long long tile = 0;
-    uint32_t item_i = 0;
+    const int ew = warp - 2;  // epilogue warp; its TMEM lanes are 32 (warp % 4)..
+    const int quarter = warp & 3, part = (ew >> 2) & (4 / SETS - 1), set = SETS == 2 ? ew >> 3 : 0;
+    float* fs = scratch + ew * kScratch;
+    const uint32_t acce = CTAS == 2 ? leader_addr(b_acce) : b_acce;
+    uint32_t tile = 0, item_i = 0, st0 = 0;  // st0: ring stage of the tile's first operands
     bool ok = true;
     // One pass over the CTA's items per phase (ItemCursor::part): the full tiles with
     // the unmasked forms, then the masked tiles, each in a loop of its own.
     auto pass = [&](auto phase_tag) {
     constexpr int kPhase = decltype(phase_tag)::value;
-    for (ItemCursor cur = first_item(g); ok && cur.it < g.item1; cur.advance(g, gridDim.x)) {
+    for (ItemCursor cur = first_item<CTAS>(g); ok && cur.it < g.item1; cur.advance(g, n_clusters)) {
       int ct, rb0, rb1;
-      if (!cur.part(g, C::kM, BN, kPhase, ct, rb0, rb1)) continue;
+      if (!cur.part(g, kBN / kBM, kBN, kPhase, ct, rb0, rb1)) continue;
       const uint32_t cs = item_i & 1;
-      if (!mbar_wait(b_cfull + 8 * cs, (item_i >> 1) & 1, g, ST_TIMEOUT_EPI)) { ok = false; break; }
+      if (!warp_wait(b_cfull + 8 * cs, (item_i >> 1) & 1, g, ST_TIMEOUT_EPI)) { ok = false; break; }
       item_i++;
-      const float* csl = cslots + cs * C::kCSoa;
-      const float4 cg = *reinterpret_cast<const float4*>(csl + 4 * BN + 4 * group);
-      const int q0 = ct * BN + group * C::kColW;
+      const float* csl = cslots + cs * kColFloats;
+      const float* csw = csl + part * W;
+      // centre and half range of a and r over the slab's column groups
+      float4 cg = reinterpret_cast<const float4*>(csl + 4 * kBN)[SETS * part];
+      if (SETS == 2) {
+        const float4 u = cg, v = reinterpret_cast<const float4*>(csl + 4 * kBN)[SETS * part + 1];
+        const float lo = fminf(u.x - u.y, v.x - v.y), hi = fmaxf(u.x + u.y, v.x + v.y);
+        const float rl = fminf(u.z - u.w, v.z - v.w), rh = fmaxf(u.z + u.w, v.z + v.w);
+        const float bad = 0.0f * (u.x + v.x);  // NaN if either group has one
+        cg = make_float4(0.5f * (lo + hi) + bad, 0.5f * (hi - lo) * 1.000001f, 0.5f * (rl + rh),
+                         0.5f * (rh - rl) * 1.000001f);
+      }
+      const int q0 = ct * kBN + part * W;
       F2 cacc[CH][2];
 #pragma unroll
       for (int c = 0; c < CH; c++) cacc[c][0] = cacc[c][1] = f2(0.0f, 0.0f);
-      for (int rb = rb0; ok && rb < rb1; rb++, tile++) {
-        const uint32_t b = (uint32_t)(tile & 1);
-        const uint32_t rsl = (uint32_t)(tile & (kRSlots - 1));
-        if (!mbar_wait(b_rfull + 8 * rsl, (tile / kRSlots) & 1, g, ST_TIMEOUT_EPI) ||
-            !mbar_wait(b_accf + 8 * b, (tile >> 1) & 1, g, ST_TIMEOUT_EPI)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
+      bool any = false;  // this set had a tile of the item
+      for (int rb = rb0; ok && rb < rb1; rb += M, tile++) {
+        const uint32_t b = tile & 1;
+        const uint32_t last = st0 + g.nst - 1 < (uint32_t)S ? st0 + g.nst - 1 : st0 + g.nst - 1 - S;  // its last stage
+        st0 = last + 1 == (uint32_t)S ? 0 : last + 1;
+        if (SETS == 2 && (int)b != set) continue;
+        any = true;
+        const uint32_t rsl = tile & (kRSlots - 1);
+        if (!warp_wait(b_rfull + 8 * rsl, (tile / kRSlots) & 1, g, ST_TIMEOUT_EPI)) { ok = false; break; }
         const float* rsp = rslots + rsl * kRowFloats;
-        const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + b * BN + group * C::kColW;
-        const int p0 = rb * kBM;
-        const float* csw = csl + group * C::kColW;
+        const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + b * kBN + part * W;
+        const int p0 = (rb + (int)rank) * kBM;
+        int mode = kPure;
+        SlabC sc;
+        if constexpr (kPhase == 0 && weighted_num<METRIC>()) {
+          mode = slab_mode<METRIC>(*reinterpret_cast<const float4*>(rsp + kRowGrp + 4 * quarter), cg, g.ec, sc);
+          if (mode == kPure || mode == kFirst) {
+            slab_factors<METRIC>(rsp, csw, sc, fs, g.ec);
+            __syncwarp();
+          }
+        }
+        if (!warp_wait(b_accf + 8 * b, (tile >> 1) & 1, g, ST_TIMEOUT_EPI)) { ok = false; break; }
+        tc_fence_after();
+        if (ew == 8 * set && lane == 0) mbar_arrive_done_reading(b_aempty + 8 * last);
         float rsum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if constexpr (kPhase == 1) {
-          slab_pairs<METRIC, BN, true, true>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
-        } else if constexpr (!weighted_num<METRIC>()) {
-          slab_pairs<METRIC, BN, true, false>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
-        } else {
-          const float4 rg = *reinterpret_cast<const float4*>(rsp + kRowGrp + 4 * quarter);
-          float* fs = scratch + warp * C::kScratch;
-          const int mode = slab_mode<METRIC>(rg, cg, g.ec);
-          if (mode == kPure)
-            slab_factor<METRIC, BN, false>(taddr, rsp, csw, rg, cg, fs, cacc, g.ec, p0, q0, rsum);
-          else if (mode == kFirst)
-            slab_factor<METRIC, BN, true>(taddr, rsp, csw, rg, cg, fs, cacc, g.ec, p0, q0, rsum);
+        if constexpr (kPhase == 1 || METRIC == kDebugDot || METRIC == kDebugSum) {
+          tile_pairs<METRIC, true, kPhase == 1>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
+        } else if (mode == kPure) {
+          tile_factor<METRIC, false>(taddr, rsp, csw, sc, fs, cacc, g.ec, p0, q0, rsum);
+        } else if constexpr (weighted_num<METRIC>()) {
+          if (mode == kFirst) tile_factor<METRIC, true>(taddr, rsp, csw, sc, fs, cacc, g.ec, p0, q0, rsum);
           else if (METRIC == kPearson && mode == kPairFirst)
-            slab_pairs<METRIC, BN, false, false>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
+            tile_pairs<METRIC, false, false>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
           else if (mode == kPairExact)
-            slab_pairs<METRIC, BN, true, false>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
+            tile_pairs<METRIC, true, false>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
         }
+        // This warp's reads of the accumulator are complete: the MMA of the tile
+        // after the next may overwrite it while the row sums are finished.
         tc_fence_before();
-        // Row sums: 4 lanes per row, then the 4 column-group warps of this
-        // quarter through shared memory: the last of them to write its
-        // partials adds the four (fixed order) and issues one atomic per row
-        // and sum. It releases the accumulator only after reading, so no warp
-        // overwrites these partials (two tiles later) before they are read.
-        const float z = reduce_rows4(rsum);
+        __syncwarp();
+        if (lane == 0) mbar_arrive_done_reading(acce + 8 * b);
+        // Row sums: 4 lanes per row, then one FP64 atomic add per row and warp (256 a
+        // tile, a tenth of the rate the L2 sustains; combining the two halves' warps
+        // in shared memory first costs more issue slots than it saves).
+        float z = reduce_rows4(rsum);
         const int krow = 2 * (lane & 1) + ((lane >> 1) & 1);
-        float* rp = rowpart + b * (4 * kBM);
-        rp[group * kBM + quarter * 32 + (lane >> 2) + 8 * krow] = z;
-        __syncwarp();
-        unsigned last = 0;
-        if (lane == 0) {
-          // acquire-release at CTA scope: publishes this warp's partials and,
-          // for the fourth warp, makes the other three warps' partials visible
-          unsigned prev;
-          asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;"
-                       : "=r"(prev)
-                       : "r"(smem_u32(rowcnt + b * 4 + quarter))
-                       : "memory");
-          last = (prev & 3u) == 3u;
-        }
-        last = __shfl_sync(0xffffffffu, last, 0);
-        if (last) {
-          __syncwarp();
-          const int row = quarter * 32 + lane;
-          float sn = 0.0f;
-#pragma unroll
-          for (int gg = 0; gg < 4; gg++) sn += rp[gg * kBM + row];
-          const int p = p0 + row;
-          if (p < g.ec.n) atomicAdd(g.num + p, (double)sn);
-        }
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(b_acce + 8 * b);
-          mbar_arrive(b_rempty + 8 * rsl);
-        }
+        if (kPhase == 0 && weighted_num<METRIC>() && (mode == kPure || mode == kFirst)) z *= fs[4 * (lane >> 2) + krow];
+        const int p = p0 + quarter * 32 + (lane >> 2) + 8 * krow;
+        if (p < g.ec.n && !(kPhase == 0 && mode == kZero)) atomicAdd(g.num + p, (double)z);
+        __syncwarp();  // (the scratch is rewritten for the next tile)
+        if (lane == 0) mbar_arrive_done_reading(b_rempty + 8 * rsl);
       }
       if (!ok) break;
       // Column sums of the item.
-      float x[4 * CH];
+      if (any) {
+        float x[4 * CH];
 #pragma unroll
-      for (int c = 0; c < CH; c++)
+        for (int c = 0; c < CH; c++)
 #pragma unroll
-        for (int r = 0; r < 2; r++) f2_split(cacc[c][r], x[(c * 2 + r) * 2], x[(c * 2 + r) * 2 + 1]);
-      flush_columns<4 * CH>(x, q0, g.ec, g.num);
+          for (int r = 0; r < 2; r++) f2_split(cacc[c][r], x[(c * 2 + r) * 2], x[(c * 2 + r) * 2 + 1]);
+        flush_columns<4 * CH>(x, q0, g.ec, g.num);
+      }
       __syncwarp();
-      if (lane == 0) mbar_arrive(b_cempty + 8 * cs);
+      if (lane == 0) mbar_arrive_done_reading(b_cempty + 8 * cs);
     }
     };
     pass(std::integral_constant<int, 0>{});
     pass(std::integral_constant<int, 1>{});
-    role_exit(tmem, 2 * BN, false);
+    role_exit<CTAS>(tmem, false);
   }
 }
 
-// Column parameters of each BN-column tile, permuted so that thread t of an
+// Column parameters of each column tile, permuted so that thread t of an
 // epilogue warp finds its four columns of a 16-column chunk (2(t%4) + {0, 1}
 // and 8 + 2(t%4) + {0, 1}) in one float4 (col_soa_pos), and the row parameters
 // of each 128-row block, in order; each followed by the centre and half range
-// of a and r over its four groups (BN/4 columns, 32 rows), which the epilogue's
+// of a and r over its four groups (64 columns, 32 rows), which the epilogue's
 // slab forms are chosen by. A NaN makes its group's ranges NaN.
 // Blocks [0, n_ctp): column tiles; [n_ctp, n_ctp + n_rbp): row blocks.
-template <int BN>
 __global__ void k_sym_soa(const BlockParams* __restrict__ params, int n_ctp, float* __restrict__ colsoa,
                           float* __restrict__ rowsoa) {
   const int i = threadIdx.x;
   __shared__ float4 wm[8];
   const bool col = blockIdx.x < n_ctp;
-  const int width = col ? BN : kBM;
+  const int width = col ? kBN : kBM;
   const int tile = col ? blockIdx.x : blockIdx.x - n_ctp;
-  float* o = col ? colsoa + (size_t)tile * col_soa_floats(BN) : rowsoa + (size_t)tile * kRowSoaFloats;
+  float* o = col ? colsoa + (size_t)tile * kColFloats : rowsoa + (size_t)tile * kRowSoaFloats;
   if (i < width) {
     const BlockParams p = params[(size_t)tile * width + i];
     const int pos = col ? col_soa_pos(i) : i;
@@ -1327,65 +1421,70 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
   return fn;
 }
 
-// box_cols 64 (128-byte rows, SWIZZLE_128B) or 32 (64-byte rows, SWIZZLE_64B).
-bool make_map(CUtensorMap* m, const __nv_bfloat16* ptr, int kq, int rows, int box_rows, int box_cols = kChunk) {
+// U as [chunk][row][64 columns] (128-byte rows, SWIZZLE_128B), boxes of
+// box_rows rows of sc chunks. Where the pitch ends half way through the last chunk, its other half
+// reads the next row's first columns, which no MMA uses (the buffer has 64 bytes
+// past the last row).
+bool make_map(CUtensorMap* m, const __half* ptr, int pitch, int rows, int sc, int box_rows) {
   auto enc = get_encode();
   if (!enc) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)kq, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)kq * 2};
-  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(ptr), dims, strides, box,
-                   estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   box_cols == kChunk ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  cuuint64_t dims[3] = {(cuuint64_t)kChunk, (cuuint64_t)rows, (cuuint64_t)((pitch + kChunk - 1) / kChunk)};
+  cuuint64_t strides[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)kChunk * 2};
+  cuuint32_t box[3] = {(cuuint32_t)kChunk, (cuuint32_t)box_rows, (cuuint32_t)sc};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half*>(ptr), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
 
-size_t fixed_smem(int bn) {
-  return 1024 + 2 * (size_t)col_soa_floats(bn) * 4 + kRSlots * kRowFloats * 4 + kRowPartBytes +
-         (size_t)kEpiWarps * (32 + bn / 4) * 4 + kBarBytes;
-}
+constexpr size_t kFixedSmem =
+    (2 * (size_t)kColFloats + kRSlots * kRowFloats + (size_t)kEpiWarps * kScratch) * 4 + kBarBytes + kTabBytes;
 
 }  // namespace
 
-// Launch shape for a column tile width and A mode, if it fits: the whole-tile
-// mode needs two A tiles beside the B tile, the chunk ring at least three 16 KB
-// A stages (as many as fit, up to kMaxStages).
-bool plan_shape(int kq, int bn, bool tr, TcPlan* p) {
-  if (kq <= 0 || kq % 32 != 0 || (bn != 256 && bn != 128)) return false;
-  const size_t fixed = fixed_smem(bn);
-  const size_t a_bytes = (size_t)kBM * kq * 2, b_bytes = (size_t)bn * kq * 2;
-  if (tr) {
-    if (fixed + 2 * a_bytes + b_bytes > kSmemBudget) return false;
-    *p = TcPlan{bn, true, 2, fixed + 2 * a_bytes + b_bytes};
-    return true;
-  }
-  if (fixed + b_bytes + 3 * kAChunkBytes > kSmemBudget) return false;
-  const int st = (int)std::min<size_t>(kMaxStages, (kSmemBudget - fixed - b_bytes) / kAChunkBytes);
-  *p = TcPlan{bn, false, st, fixed + b_bytes + (size_t)st * kAChunkBytes};
+// Shape for K ellipse pixels: CTAs per tile, and a ring of stages of whole
+// row-block tiles (three or more) or of single chunks (three or more).
+bool plan_shape(int K, int ctas, bool whole, TcPlan* p) {
+  if (K <= 0) return false;
+  const SplitLayout l = split_layout(K);
+  const int nch = (l.pitch + kChunk - 1) / kChunk;
+  const int cols = nch * (kBN / kBM / ctas);  // chunks of 128 rows of the column tile in a CTA
+  const int chunks = (int)((kSmemBudget - kFixedSmem) / kChunkBytes) - cols;  // of the ring
+  const int sc = whole ? nch : 1;
+  if (chunks < 3 * sc) return false;
+  const int st = std::min(kMaxStages, chunks / sc);
+  *p = TcPlan{ctas, sc, st, kFixedSmem + (size_t)(cols + st * sc) * kChunkBytes};
   return true;
 }
 
-bool plan_gram_tc(int kq, TcPlan* p) {
-  // default: 256-column tiles (whole-tile A when it fits), else 128 (chunk ring)
-  return plan_shape(kq, 256, true, p) || plan_shape(kq, 256, false, p) || plan_shape(kq, 128, false, p);
+bool plan_gram_tc(int K, TcPlan* p) {
+  return plan_shape(K, 1, true, p) || plan_shape(K, 2, true, p) || plan_shape(K, 2, false, p);
 }
 
-int gram_tc_candidates(int kq, TcChoice* out, int cap) {
+// The shape a table entry names: whole-tile stages (tr 1) or single chunks.
+bool plan_choice(int K, const TcChoice& c, TcPlan* p) {
+  return c.tr ? plan_shape(K, 1, true, p) || plan_shape(K, 2, true, p) : plan_shape(K, 2, false, p);
+}
+
+int gram_tc_candidates(int K, TcChoice* out, int cap) {
   int n = 0;
   TcPlan p;
-  for (int bn : {256, 128})
-    for (int tr : {1, 0})
-      if (plan_shape(kq, bn, tr != 0, &p))
-        for (int L : {32, 16, 8, 4})
-          if (n < cap) out[n++] = TcChoice{bn, tr, L};
+  for (int tr : {1, 0})
+    if (plan_choice(K, TcChoice{kBN, tr, 128}, &p))
+      for (int L : {128, 32, 16, 8, 4})
+        if (n < cap) out[n++] = TcChoice{kBN, tr, L};
   return n;
 }
 
+bool gram_tc_valid(int K, const TcChoice& c) {
+  TcPlan p;
+  const bool L = c.L == 128 || c.L == 32 || c.L == 16 || c.L == 8 || c.L == 4;
+  return L && (c.bn == 256 || c.bn == 128) && (c.tr == 0 || c.tr == 1) && plan_choice(K, c, &p);
+}
+
 size_t gram_tc_soa_floats(int n_pad) {
-  // column tiles of 128 or 256 blocks plus one row-parameter block per 128 rows
-  return (size_t)(n_pad / 128) * col_soa_floats(128) + (size_t)(n_pad / 128) * kRowSoaFloats;
+  return (size_t)(n_pad / kBN) * kColFloats + (size_t)(n_pad / kBM) * kRowSoaFloats;
 }
 
 long long gram_tc_items(int n, int bn, int* L_out, int num_sms, int max_L) {
@@ -1396,45 +1495,42 @@ long long gram_tc_items(int n, int bn, int* L_out, int num_sms, int max_L) {
     return items_before_run(runs, n_ct, L / m);
   };
   int L = max_L > 0 && max_L < kMaxRun ? max_L : kMaxRun;
-  while (L > 2 && items(L) < 4LL * num_sms) L >>= 1;
+  while (L > 2 && items(L) < 16LL * num_sms) L >>= 1;
   if (L < m) L = m;
   if (L_out) *L_out = L;
   return items(L);
 }
 
-cudaError_t launch_gram_tc(const __nv_bfloat16* A, const __nv_bfloat16* B, int kq, int n_pad,
-                           const BlockParams* params, float* soa_ws, EpiConsts ec, double* num, int num_sms,
-                           int* status, cudaStream_t st, int shard, int n_shards,
+cudaError_t launch_gram_tc(const __half* U, int K, int n_pad, const BlockParams* params, float* soa_ws, EpiConsts ec,
+                           double* num, int num_sms, int* status, cudaStream_t st, int shard, int n_shards,
                            const TcDebug* dbg, const TcChoice* choice) {
   TcPlan plan;
-  const bool planned = choice && choice->bn ? plan_shape(kq, choice->bn, choice->tr != 0, &plan)
-                                            : plan_gram_tc(kq, &plan);
-  if (!planned || n_pad % 256 != 0 || n_shards < 1 || shard < 0 || shard >= n_shards) return cudaErrorInvalidValue;
+  const bool planned = (choice && choice->bn && plan_choice(K, *choice, &plan)) || plan_gram_tc(K, &plan);
+  if (!planned || n_pad % kBN != 0 || n_shards < 1 || shard < 0 || shard >= n_shards) return cudaErrorInvalidValue;
   if (ec.n <= 0) return cudaSuccess;
-  const int bn = plan.bn;
+  const SplitLayout l = split_layout(K);
   TcArgs g;
-  g.kq = kq;
-  g.nkc = (kq + kChunk - 1) / kChunk;  // nfull + tail
+  g.nb = l.nb;
+  g.nt = l.nt;
+  g.nch = (l.pitch + kChunk - 1) / kChunk;
+  g.sc = plan.sc;
+  g.nst = (g.nch + plan.sc - 1) / plan.sc;
   g.stages = plan.stages;
-  g.nfull = kq / kChunk;
-  g.tail = (kq % kChunk) ? 1 : 0;
-  g.a_bytes = (uint32_t)kBM * kq * 2;
-  g.b_bytes = (uint32_t)bn * kq * 2;
   g.n_rb = (ec.n + kBM - 1) / kBM;
-  g.n_ct = (ec.n + bn - 1) / bn;
+  g.n_ct = (ec.n + kBN - 1) / kBN;
   int L;
-  const long long items = gram_tc_items(ec.n, bn, &L, num_sms, choice ? choice->L : 0);
+  const long long items = gram_tc_items(ec.n, kBN, &L, num_sms, choice ? choice->L : 0);
   g.L = L;
-  g.h = L / (bn / kBM);
+  g.h = L / (kBN / kBM);
   g.n_runs = (g.n_rb + L - 1) / L;
-  // panels of column tiles whose B tiles (bn x K' bf16 each) fill at most 48 MB of L2
-  g.panel = std::max(1, (int)(((size_t)48 << 20) / g.b_bytes));
+  // panels of column tiles whose operands fill at most 48 MB of L2
+  g.panel = std::max(1, (int)(((size_t)48 << 20) / ((size_t)kBN * l.pitch * 2)));
   g.n_panels = (g.n_ct + g.panel - 1) / g.panel;
   g.item0 = items * shard / n_shards;
   g.item1 = items * (shard + 1) / n_shards;
-  const int n_ctp = n_pad / bn, n_rbp = n_pad / kBM;
+  const int n_ctp = n_pad / kBN, n_rbp = n_pad / kBM;
   float* colsoa = soa_ws;
-  float* rowsoa = soa_ws + (size_t)n_ctp * col_soa_floats(bn);
+  float* rowsoa = soa_ws + (size_t)n_ctp * kColFloats;
   g.colsoa = colsoa;
   g.rowsoa = rowsoa;
   g.ec = ec;
@@ -1442,42 +1538,51 @@ cudaError_t launch_gram_tc(const __nv_bfloat16* A, const __nv_bfloat16* B, int k
   g.status = status;
   g.timeout_ns = dbg && dbg->timeout_ns ? dbg->timeout_ns : 4000000000ull;
   g.withhold = dbg ? dbg->withhold_tile : -1;
-  if (bn == 256) k_sym_soa<256><<<n_ctp + n_rbp, 256, 0, st>>>(params, n_ctp, colsoa, rowsoa);
-  else k_sym_soa<128><<<n_ctp + n_rbp, 256, 0, st>>>(params, n_ctp, colsoa, rowsoa);
+  k_sym_soa<<<n_ctp + n_rbp, 256, 0, st>>>(params, n_ctp, colsoa, rowsoa);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (g.item0 >= g.item1) return cudaSuccess;
-  CUtensorMap mA, mB, mA64, mB64;
-  if (!make_map(&mA, A, kq, n_pad, kBM) || !make_map(&mB, B, kq, n_pad, bn)) return cudaErrorInvalidValue;
-  mA64 = mA;
-  mB64 = mB;
-  if (g.tail && (!make_map(&mA64, A, kq, n_pad, kBM, kChunk / 2) || !make_map(&mB64, B, kq, n_pad, bn, kChunk / 2)))
+  CUtensorMap mU, mB;
+  if (!make_map(&mU, U, l.pitch, n_pad, plan.sc, kBM) || !make_map(&mB, U, l.pitch, n_pad, plan.sc, kBN / plan.ctas))
     return cudaErrorInvalidValue;
-  const int grid = (int)std::min<long long>(g.item1 - g.item0, num_sms);
   const int smem = (int)plan.smem;
-#define SRED_TC3(M, BNV, TRV)                                                                            \
-  do {                                                                                                   \
-    e = cudaFuncSetAttribute(k_gram_tc<M, BNV, TRV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
-    if (e != cudaSuccess) return e;                                                                      \
-    k_gram_tc<M, BNV, TRV><<<grid, kThreads, smem, st>>>(mA, mB, mA64, mB64, g);                         \
-  } while (0)
-#define SRED_TC(M)                                   \
-  if (bn == 256 && plan.tr) SRED_TC3(M, 256, true);       \
-  else if (bn == 256) SRED_TC3(M, 256, false);       \
-  else if (plan.tr) SRED_TC3(M, 128, true);          \
-  else SRED_TC3(M, 128, false);
+  // one CTA per SM: as many CTAs or pairs of CTAs as can be resident at once
+  auto launch = [&](auto kern) -> cudaError_t {
+    cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (r != cudaSuccess) return r;
+    int groups = num_sms;
+    if (plan.ctas == 2) {
+      static std::atomic<int> resident[16];  // pairs per device, whatever the ring
+      int dev = 0;
+      if ((r = cudaGetDevice(&dev)) != cudaSuccess) return r;
+      groups = dev < 16 ? resident[dev].load() : 0;
+      if (groups == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(2 * std::max(1, num_sms / 2));
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        r = cudaOccupancyMaxActiveClusters(&groups, kern, &cfg);
+        if (r != cudaSuccess) return r;
+        groups = std::max(1, std::min(groups, num_sms / 2));
+        if (dev < 16) resident[dev].store(groups);
+      }
+    }
+    const int grid = plan.ctas * (int)std::min<long long>(g.item1 - g.item0, groups);
+    kern<<<grid, kThreads, smem, st>>>(mU, mB, g);
+    return cudaGetLastError();
+  };
+#define SRED_TC(M) return plan.ctas == 2 ? launch(k_gram_tc<M, 2>) : launch(k_gram_tc<M, 1>)
   switch (ec.metric) {
-    case kPearson: SRED_TC(kPearson); break;
-    case kSsim: SRED_TC(kSsim); break;
-    case kNrmse: SRED_TC(kNrmse); break;
-    case kNrmseW: SRED_TC(kNrmseW); break;
-    case kDebugDot: SRED_TC(kDebugDot); break;
-    case kDebugSum: SRED_TC(kDebugSum); break;
+    case kPearson: SRED_TC(kPearson);
+    case kSsim: SRED_TC(kSsim);
+    case kNrmse: SRED_TC(kNrmse);
+    case kNrmseW: SRED_TC(kNrmseW);
+    case kDebugDot: SRED_TC(kDebugDot);
+    case kDebugSum: SRED_TC(kDebugSum);
     default: return cudaErrorInvalidValue;
   }
 #undef SRED_TC
-#undef SRED_TC3
-  return cudaGetLastError();
 }
 
 }  // namespace sred

@@ -22,14 +22,12 @@ __global__ void k_count(const uint8_t* flags, size_t n, int2* counts);
 __global__ void k_scan(int2* counts, int nseg);
 __global__ void k_scatter(const uint8_t* flags, size_t n, const int2* offs, int* gram_pix, int* flat_pix,
                           int* slot);
-__global__ void k_pack(const float* img, int W, Ellipse e, const int* gram_pix, int n, float wscale, int mode,
-                       float* U, int kp, __nv_bfloat16* A, __nv_bfloat16* B, int kq, BlockParams* params,
-                       float* tile_rmax, double* sums, unsigned* arange);
+__global__ void k_pack(const float* img, int W, Ellipse e, const int* gram_pix, int n, float wscale, float* U, int kp,
+                       __half* S, BlockParams* params, float* tile_rmax, double* sums, unsigned* arange);
 __global__ void k_finalize(const int* slot, int W, int H, int rw, int rh, const double* num, const double* den,
                            const BlockParams* params, const double* sums, int n_flat, int metric, double sk,
                            double n_pixels, const float* mask, int apply_mask, float* out);
-__global__ void k_pack_vectors(const float* u, int n, int K, int mode, float* U, int kp, __nv_bfloat16* A,
-                               __nv_bfloat16* B, int kq);
+__global__ void k_pack_vectors(const float* u, int n, int K, float* U, int kp, __half* S);
 __global__ void k_minmax(const float* a, const float* mask, int W, int H, int bw_, int bh_, size_t plane,
                          unsigned* mm);
 __global__ void k_remap(float* a, const float* mask, int W, int H, int bw_, int bh_, size_t plane,

@@ -237,14 +237,11 @@ __global__ void k_scatter(const uint8_t* __restrict__ flags, size_t n, const int
 // The block sums are warp-wide reductions, one block after another; the
 // per-block scalar work (square roots, quotients, exp2, params) then runs on
 // lane k for block k of the 32, instead of on one lane per block while the
-// other 31 wait. mode 0: U only (fp32, row pitch kp). mode 1 / 2: the two- /
-// three-level split BF16 operands A, B (store_split; row pitch kq), and U as
-// well when U is given (tensor-core NRMSE). Rows [n, n_pad) are zero-filled by
-// the host.
+// other 31 wait. U: FP32 unit vectors (row pitch kp), S: the split FP16 operand
+// (store_split); either may be null. Rows [n, n_pad) are zero-filled by the host.
 // ---------------------------------------------------------------------------
 __global__ void k_pack(const float* __restrict__ img, int W, Ellipse e, const int* __restrict__ gram_pix,
-                       int n, float wscale, int mode, float* __restrict__ U, int kp,
-                       __nv_bfloat16* __restrict__ A, __nv_bfloat16* __restrict__ B, int kq,
+                       int n, float wscale, float* __restrict__ U, int kp, __half* __restrict__ S,
                        BlockParams* __restrict__ params, float* __restrict__ tile_rmax,
                        double* __restrict__ sums, unsigned* __restrict__ arange) {
   const unsigned full = 0xffffffffu;
@@ -252,6 +249,7 @@ __global__ void k_pack(const float* __restrict__ img, int W, Ellipse e, const in
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   const int K = e.k;
+  const SplitLayout lay = split_layout(K);
   const double sk = sqrt((double)(K - 1) / (double)K);
   const double rK = __drcp_rn((double)K);  // s / K as div_fixed: the correctly rounded quotient
   double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
@@ -312,16 +310,11 @@ __global__ void k_pack(const float* __restrict__ img, int W, Ellipse e, const in
       for (int i = lane; i < K; i += 32) {
         const double u = ((double)img[(size_t)(y + e.dy[i]) * W + (x + e.dx[i])] - mu_k) * inv_k;
         if (U) U[(size_t)j * kp + i] = (float)u;
-        if (mode != 0) store_split(A + (size_t)j * kq, B + (size_t)j * kq, K, i, u, mode + 1);
+        if (S) store_split(S + (size_t)j * lay.pitch, lay, i, u * (double)kSplitScale);
       }
       if (U)
         for (int i = K + lane; i < kp; i += 32) U[(size_t)j * kp + i] = 0.0f;
-      if (mode != 0) {
-        for (int i = (mode == 1 ? 3 : 6) * K + lane; i < kq; i += 32) {
-          A[(size_t)j * kq + i] = __float2bfloat16_rn(0.0f);
-          B[(size_t)j * kq + i] = __float2bfloat16_rn(0.0f);
-        }
-      }
+      if (S) store_split_pad(S + (size_t)j * lay.pitch, lay, lane);
     }
   }
   a_lo = __reduce_max_sync(full, a_lo);
@@ -347,30 +340,19 @@ __global__ void k_pack(const float* __restrict__ img, int W, Ellipse e, const in
 }
 
 // Diagnostics: pack caller-given vectors (n x K, FP32) as operands without
-// normalising them (one warp per row).
-__global__ void k_pack_vectors(const float* __restrict__ u, int n, int K, int mode, float* __restrict__ U, int kp,
-                               __nv_bfloat16* __restrict__ A, __nv_bfloat16* __restrict__ B, int kq) {
+// normalising or scaling them (one warp per row), as FP32 or split FP16.
+__global__ void k_pack_vectors(const float* __restrict__ u, int n, int K, float* __restrict__ U, int kp,
+                               __half* __restrict__ S) {
   const int lane = threadIdx.x & 31;
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
+  const SplitLayout lay = split_layout(K);
   for (int j = gw; j < n; j += nw) {
-    if (mode == 0) {
+    if (U)
       for (int i = lane; i < kp; i += 32) U[(size_t)j * kp + i] = i < K ? u[(size_t)j * K + i] : 0.0f;
-    } else {
-      for (int i = lane; i < kq; i += 32) {
-        A[(size_t)j * kq + i] = __float2bfloat16_rn(0.0f);
-        B[(size_t)j * kq + i] = __float2bfloat16_rn(0.0f);
-      }
-      __syncwarp();
-      for (int i = lane; i < K; i += 32) {
-        const float x = u[(size_t)j * K + i];
-        const __nv_bfloat16 hi = __float2bfloat16_rn(x);
-        const __nv_bfloat16 lo = __float2bfloat16_rn(x - __bfloat162float(hi));
-        __nv_bfloat16* a = A + (size_t)j * kq;
-        __nv_bfloat16* b = B + (size_t)j * kq;
-        a[i] = hi; a[K + i] = lo; a[2 * K + i] = hi;
-        b[i] = hi; b[K + i] = hi; b[2 * K + i] = lo;
-      }
+    if (S) {
+      for (int i = lane; i < K; i += 32) store_split(S + (size_t)j * lay.pitch, lay, i, (double)u[(size_t)j * K + i]);
+      store_split_pad(S + (size_t)j * lay.pitch, lay, lane);
     }
   }
 }

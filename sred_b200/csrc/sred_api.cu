@@ -29,7 +29,7 @@ using namespace sred;
 namespace {
 
 enum BufId {
-  B_IMG, B_MEANS, B_STDS, B_MASK, B_MASKIN, B_FLAGS, B_SLOT, B_GPIX, B_FPIX, B_COUNTS, B_U, B_A, B_B,
+  B_IMG, B_MEANS, B_STDS, B_MASK, B_MASKIN, B_FLAGS, B_SLOT, B_GPIX, B_FPIX, B_COUNTS, B_U, B_S,
   B_PARAMS, B_RMAX, B_NUM, B_DEN, B_SUMS, B_OUT, B_VARS, B_MM, B_NMASK, B_BAD, B_STATUS, B_STDS2, B_COLSOA,
   B_FEAT, B_SIG, B_FR, B_FI, B_GAT, B_OFF3, B_REF3, B_STAT, B_THR, B_KMX, B_KMD2, B_KMLAB, B_KMB, B_TBOX, B_TSTAT, B_TMEAN, B_TVAR, B_STKIN, B_STKOUT, B_SORT, B_NODES, B_SLICES,
   B_NBUF
@@ -47,7 +47,7 @@ struct GState {
   bool valid = false;
   bool vol = false;  // a 3D map (depth d, z radius rd)
   int d = 1, rd = 0;
-  int metric = 0, w = 0, h = 0, rw = 0, rh = 0, K = 0, n_g = 0, n_flat = 0, engine = 0, kp = 0, kq = 0;
+  int metric = 0, w = 0, h = 0, rw = 0, rh = 0, K = 0, n_g = 0, n_flat = 0, engine = 0, kp = 0;
   size_t n = 0, n_pad = 0;
   float nv = 0, thr = 0, npx = 0, relc = 0, wscale = 0;
   bool given = false, sorted = false;
@@ -102,15 +102,14 @@ std::map<TuneKey, TuneEntry> g_tune;
 // Size classes: up to 64 Ki blocks, up to 256 Ki, larger.
 int tune_nclass(int n) { return n < (1 << 16) ? 0 : n < (1 << 18) ? 1 : 2; }
 
-// Contraction engine and K' of a global map: Abs-diff needs no contraction
-// (the FP32 engine's kernel without a Gram); the other metrics run on the
-// context's engine, the tensor cores while the operands' B tile fits in
-// shared memory (NRMSE with the three-level split), else the FP32 engine.
-int pick_engine(const sred_ctx* c, int metric, int K, int* kq) {
-  *kq = split_cols_for(metric, K);
-  if (metric == kAbsDiff || c->engine != SRED_ENGINE_TC) return SRED_ENGINE_FP32;
+// Contraction engine of a global map: Abs-diff needs no contraction (the FP32
+// engine's kernel without a Gram); the other metrics run on the context's
+// engine. Blocks of more than kMaxGlobalK pixels have no engine (the FP32
+// engine's two tiles do not fit in shared memory, and its launch says so).
+int pick_engine(const sred_ctx* c, int metric, int K) {
+  if (metric == kAbsDiff || c->engine != SRED_ENGINE_TC || K > kMaxGlobalK) return SRED_ENGINE_FP32;
   TcPlan plan;
-  return plan_gram_tc(*kq, &plan) ? SRED_ENGINE_TC : SRED_ENGINE_FP32;
+  return plan_gram_tc(K, &plan) ? SRED_ENGINE_TC : SRED_ENGINE_FP32;
 }
 
 void log_msg(sred_ctx* c, const std::string& msg) {
@@ -336,12 +335,11 @@ sred_status global_prepare(sred_ctx* c, int metric, const float* d_img, int w, i
   const float npx = given ? given->n_pixels : java_float_count(nmask);
 
   // Operands and per-block parameters of the all-pairs contraction.
-  int kq;  // K' of the split-BF16 operands
-  const int engine = pick_engine(c, metric, K, &kq);
+  const int engine = pick_engine(c, metric, K);
   const size_t n_pad = round_up((size_t)std::max(n_g, 1), 256);
   const int kp = (int)round_up(K, 4);
   float* d_U = nullptr;
-  __nv_bfloat16 *d_A = nullptr, *d_B = nullptr;
+  __half* d_S = nullptr;
   BlockParams* d_params;
   float* d_rmax;
   double *d_num, *d_den, *d_sums;
@@ -355,10 +353,9 @@ sred_status global_prepare(sred_ctx* c, int metric, const float* d_img, int w, i
     CK(cudaMemsetAsync(d_U + (size_t)n_g * kp, 0, (n_pad - n_g) * kp * sizeof(float), st));
   }
   if (engine == SRED_ENGINE_TC) {
-    CKS(ensure(c, B_A, n_pad * kq, &d_A));
-    CKS(ensure(c, B_B, n_pad * kq, &d_B));
-    CK(cudaMemsetAsync(d_A + (size_t)n_g * kq, 0, (n_pad - n_g) * kq * sizeof(__nv_bfloat16), st));
-    CK(cudaMemsetAsync(d_B + (size_t)n_g * kq, 0, (n_pad - n_g) * kq * sizeof(__nv_bfloat16), st));
+    const size_t pitch = split_layout(K).pitch;
+    CKS(ensure(c, B_S, n_pad * pitch + kSplitSlack, &d_S));
+    CK(cudaMemsetAsync(d_S + n_g * pitch, 0, (n_pad - n_g) * pitch * sizeof(__half), st));
   }
   CK(cudaMemsetAsync(d_params + n_g, 0, (n_pad - n_g) * sizeof(BlockParams), st));
   CK(cudaMemsetAsync(d_rmax, 0, (n_pad / 128) * sizeof(float), st));
@@ -373,9 +370,8 @@ sred_status global_prepare(sred_ctx* c, int metric, const float* d_img, int w, i
   if (n_g > 0) {
     // one warp per group of 32 blocks
     const int pgrid = grid_for(((size_t)n_g + 31) / 32 * 32, 256, 8 * c->num_sms);
-    const int mode = engine == SRED_ENGINE_FP32 ? 0 : split_levels_for(metric, K) - 1;
-    k_pack<<<pgrid, 256, 0, st>>>(d_img, w, e, d_gpix, n_g, wscale, mode, d_U, kp, d_A, d_B, kq, d_params,
-                                  d_rmax, d_sums, reinterpret_cast<unsigned*>(d_sums + 4));
+    k_pack<<<pgrid, 256, 0, st>>>(d_img, w, e, d_gpix, n_g, wscale, d_U, kp, d_S, d_params, d_rmax, d_sums,
+                                  reinterpret_cast<unsigned*>(d_sums + 4));
     CK(cudaGetLastError());
   }
   if (engine == SRED_ENGINE_TC) {
@@ -393,7 +389,6 @@ sred_status global_prepare(sred_ctx* c, int metric, const float* d_img, int w, i
   gs->n_flat = n_flat;
   gs->engine = engine;
   gs->kp = kp;
-  gs->kq = kq;
   gs->n = n;
   gs->n_pad = n_pad;
   gs->nv = nv;
@@ -443,7 +438,9 @@ sred_status global_gram(sred_ctx* c, const GState& gs, cudaStream_t st, int shar
       ec.K = gs.K;
       ec.nrmse_near = kNrmseNear;
     }
+    if (gs.engine == SRED_ENGINE_TC) ec.gscale = kSplitGScale;
     ec.inv_wscale = 1.0f / gs.wscale;
+    ec.tau = kEps * gs.wscale * gs.wscale;
     ec.c2h = 0.5f * kC2 / ec.gscale;
     double* d_num = static_cast<double*>(c->buf[B_NUM].p);
     const BlockParams* d_params = static_cast<const BlockParams*>(c->buf[B_PARAMS].p);
@@ -457,8 +454,7 @@ sred_status global_gram(sred_ctx* c, const GState& gs, cudaStream_t st, int shar
       CKS(ensure(c, B_STATUS, 4, &d_status));
       auto run = [&](const TcChoice* ch) -> sred_status {
         CK(cudaMemsetAsync(d_status, 0, 4 * sizeof(int), st));
-        CK(launch_gram_tc(static_cast<const __nv_bfloat16*>(c->buf[B_A].p),
-                          static_cast<const __nv_bfloat16*>(c->buf[B_B].p), gs.kq, (int)gs.n_pad, d_params,
+        CK(launch_gram_tc(static_cast<const __half*>(c->buf[B_S].p), gs.K, (int)gs.n_pad, d_params,
                           static_cast<float*>(c->buf[B_COLSOA].p), ec, d_num, c->num_sms, d_status, st, shard,
                           n_shards, &c->tc_debug, ch));
         return SRED_OK;
@@ -467,7 +463,7 @@ sred_status global_gram(sred_ctx* c, const GState& gs, cudaStream_t st, int shar
       // that every shard partitions the work alike).
       TcChoice chosen;
       bool have = false;
-      const TuneKey key{gs.kq, ec.metric, tune_nclass(gs.n_g)};
+      const TuneKey key{split_cols(gs.K), ec.metric, tune_nclass(gs.n_g)};
       if (n_shards == 1) {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto f = g_tune.find(key);
@@ -482,7 +478,7 @@ sred_status global_gram(sred_ctx* c, const GState& gs, cudaStream_t st, int shar
         // on other streams at the same time perturb these timings, so a
         // tuning pass is best run on one context at a time.
         TcChoice cand[16];
-        const int nc = gram_tc_candidates(gs.kq, cand, 16);
+        const int nc = gram_tc_candidates(gs.K, cand, 16);
         float best = 3.4e38f;
         for (int i = 0; i < nc; i++) {
           CK(cudaMemsetAsync(d_num, 0, gs.n_pad * sizeof(double), st));
@@ -883,12 +879,11 @@ sred_status global3d_prepare(sred_ctx* c, int metric, const float* d_vol, int w,
   const int n_g = tot.x, n_flat = tot.y;
   const float npx = java_float_count(nmask);
 
-  int kq;
-  const int engine = pick_engine(c, metric, K, &kq);
+  const int engine = pick_engine(c, metric, K);
   const size_t n_pad = round_up((size_t)std::max(n_g, 1), 256);
   const int kp = (int)round_up(K, 4);
   float* d_U = nullptr;
-  __nv_bfloat16 *d_A = nullptr, *d_B = nullptr;
+  __half* d_S = nullptr;
   BlockParams* d_params;
   float* d_rmax;
   double *d_num, *d_den, *d_sums;
@@ -902,10 +897,9 @@ sred_status global3d_prepare(sred_ctx* c, int metric, const float* d_vol, int w,
     CK(cudaMemsetAsync(d_U + (size_t)n_g * kp, 0, (n_pad - n_g) * kp * sizeof(float), st));
   }
   if (engine == SRED_ENGINE_TC) {
-    CKS(ensure(c, B_A, n_pad * kq, &d_A));
-    CKS(ensure(c, B_B, n_pad * kq, &d_B));
-    CK(cudaMemsetAsync(d_A + (size_t)n_g * kq, 0, (n_pad - n_g) * kq * sizeof(__nv_bfloat16), st));
-    CK(cudaMemsetAsync(d_B + (size_t)n_g * kq, 0, (n_pad - n_g) * kq * sizeof(__nv_bfloat16), st));
+    const size_t pitch = split_layout(K).pitch;
+    CKS(ensure(c, B_S, n_pad * pitch + kSplitSlack, &d_S));
+    CK(cudaMemsetAsync(d_S + n_g * pitch, 0, (n_pad - n_g) * pitch * sizeof(__half), st));
   }
   CK(cudaMemsetAsync(d_params + n_g, 0, (n_pad - n_g) * sizeof(BlockParams), st));
   CK(cudaMemsetAsync(d_rmax, 0, (n_pad / 128) * sizeof(float), st));
@@ -918,8 +912,8 @@ sred_status global3d_prepare(sred_ctx* c, int metric, const float* d_vol, int w,
   const float wscale = (float)std::sqrt(1.4426950408889634 / (double)hden);
   if (n_g > 0) {
     k_pack3d<<<grid_for((size_t)n_g * 32, 256, 8 * c->num_sms), 256, 0, st>>>(
-        d_vol, v, d_off, d_gpix, n_g, wscale, engine == SRED_ENGINE_FP32 ? 0 : split_levels_for(metric, K) - 1, d_U, kp, d_A,
-        d_B, kq, d_params, d_rmax, reinterpret_cast<unsigned*>(d_sums + 4));
+        d_vol, v, d_off, d_gpix, n_g, wscale, d_U, kp, d_S, d_params, d_rmax,
+        reinterpret_cast<unsigned*>(d_sums + 4));
     CK(cudaGetLastError());
   }
   if (engine == SRED_ENGINE_TC) {
@@ -940,7 +934,6 @@ sred_status global3d_prepare(sred_ctx* c, int metric, const float* d_vol, int w,
   gs->n_flat = n_flat;
   gs->engine = engine;
   gs->kp = kp;
-  gs->kq = kq;
   gs->n = n;
   gs->n_pad = n_pad;
   gs->nv = nv;
@@ -1711,11 +1704,10 @@ sred_status reserve_global(sred_ctx* c, const sred_job* jobs, int n_jobs) {
     const size_t np = round_up(std::max<size_t>(inter, 1), 256);
     n = std::max(n, (size_t)j.w * j.h);
     n_pad = std::max(n_pad, np);
-    a = std::max(a, np * (size_t)split_cols_for(global_metric(j.metric), K));
+    a = std::max(a, np * (size_t)split_layout(K).pitch);
     u = std::max(u, np * round_up(K, 4));
     cols = std::max(cols, gram_tc_soa_floats((int)np));
-    int kq;
-    if (tc && pick_engine(c, global_metric(j.metric), K, &kq) == SRED_ENGINE_FP32) fp32 = true;
+    if (tc && pick_engine(c, global_metric(j.metric), K) == SRED_ENGINE_FP32) fp32 = true;
     if (global_metric(j.metric) == kNrmse) fp32 = true;  // U for the near-identical pairs
     if (global_metric(j.metric) == kAbsDiff) fp32 = true;
   }
@@ -1726,7 +1718,7 @@ sred_status reserve_global(sred_ctx* c, const sred_job* jobs, int n_jobs) {
   float2* f2;
   BlockParams* bp;
   double* d;
-  __nv_bfloat16* bf;
+  __half* hf;
   for (int id : {B_IMG, B_OUT, B_MEANS, B_STDS, B_MASK, B_MASKIN}) CKS(ensure(c, id, n, &f));
   CKS(ensure(c, B_FLAGS, n, &u8));
   for (int id : {B_SLOT, B_GPIX, B_FPIX}) CKS(ensure(c, id, n, &i32));
@@ -1739,8 +1731,7 @@ sred_status reserve_global(sred_ctx* c, const sred_job* jobs, int n_jobs) {
   CKS(ensure(c, B_SLICES, den_slices((int)n_pad), &f2));
   if (tc) {
     CKS(ensure(c, B_SORT, sort_workspace_ints((int)n_pad), &i32));
-    CKS(ensure(c, B_A, a, &bf));
-    CKS(ensure(c, B_B, a, &bf));
+    CKS(ensure(c, B_S, a + kSplitSlack, &hf));
     CKS(ensure(c, B_COLSOA, cols, &f));
   }
   if (fp32) CKS(ensure(c, B_U, u, &f));
@@ -2042,12 +2033,9 @@ int sred_gram_tuning_entries(int* entries, float* ms, int cap) {
 }
 
 sred_status sred_gram_tuning_set(int kq, int metric, int size_class, int bn, int tr, int max_l, float ms) {
-  TcPlan p;
-  TcChoice cand[16];
-  const int nc = gram_tc_candidates(kq, cand, 16);
-  bool ok = false;
-  for (int i = 0; i < nc; i++) ok |= cand[i].bn == bn && cand[i].tr == tr && cand[i].L == max_l;
-  if (!ok || size_class < 0 || size_class > 2 || !plan_gram_tc(kq, &p)) return SRED_ERR_ARG;
+  // (K' = 3K rounded up to 32: its largest K)
+  if (kq <= 0 || kq % 32 != 0 || size_class < 0 || size_class > 2 || !gram_tc_valid(kq / 3, TcChoice{bn, tr, max_l}))
+    return SRED_ERR_ARG;
   std::lock_guard<std::mutex> lk(g_tune_mu);
   g_tune[TuneKey{kq, metric, size_class}] = TuneEntry{TcChoice{bn, tr, max_l}, ms};
   return SRED_OK;
@@ -2076,9 +2064,10 @@ sred_status sred_debug_gram_rowdot(sred_ctx* c, int engine, const float* u, cons
   cudaSetDevice(c->device);
   cudaStream_t st = c->stream;
   const size_t n_pad = round_up((size_t)n, 256);
-  const int kp = (int)round_up(k, 4), kq = (int)round_up(3 * k, 32);
+  const int kp = (int)round_up(k, 4);
+  const size_t pitch = split_layout(k).pitch;
   float *d_u, *d_U = nullptr, *d_rmax;
-  __nv_bfloat16 *d_A = nullptr, *d_B = nullptr;
+  __half* d_S = nullptr;
   BlockParams* d_params;
   double *d_num, *d_den;
   CKS(ensure(c, B_IMG, (size_t)n * k, &d_u));
@@ -2090,10 +2079,8 @@ sred_status sred_debug_gram_rowdot(sred_ctx* c, int engine, const float* u, cons
     CKS(ensure(c, B_U, n_pad * kp, &d_U));
     CK(cudaMemsetAsync(d_U, 0, n_pad * kp * sizeof(float), st));
   } else {
-    CKS(ensure(c, B_A, n_pad * kq, &d_A));
-    CKS(ensure(c, B_B, n_pad * kq, &d_B));
-    CK(cudaMemsetAsync(d_A, 0, n_pad * kq * sizeof(__nv_bfloat16), st));
-    CK(cudaMemsetAsync(d_B, 0, n_pad * kq * sizeof(__nv_bfloat16), st));
+    CKS(ensure(c, B_S, n_pad * pitch + kSplitSlack, &d_S));
+    CK(cudaMemsetAsync(d_S, 0, n_pad * pitch * sizeof(__half), st));
   }
   std::vector<BlockParams> hp(n_pad);
   std::memset(hp.data(), 0, n_pad * sizeof(BlockParams));
@@ -2104,7 +2091,7 @@ sred_status sred_debug_gram_rowdot(sred_ctx* c, int engine, const float* u, cons
   CK(cudaMemsetAsync(d_num, 0, n_pad * sizeof(double), st));
   CK(cudaMemsetAsync(d_den, 0, n_pad * sizeof(double), st));
   k_pack_vectors<<<grid_for((size_t)n * 32, 256, 8 * c->num_sms), 256, 0, st>>>(
-      d_u, n, k, engine == SRED_ENGINE_FP32 ? 0 : 1, d_U, kp, d_A, d_B, kq);
+      d_u, n, k, d_U, kp, d_S);
   CK(cudaGetLastError());
   // num and den are two sums over the same schedule
   EpiConsts ec{kDebugDot, n, 1.0f, kC1, kC2}, ed{kDebugSum, n, 1.0f, kC1, kC2};
@@ -2118,11 +2105,9 @@ sred_status sred_debug_gram_rowdot(sred_ctx* c, int engine, const float* u, cons
     float* d_soa;
     CKS(ensure(c, B_COLSOA, gram_tc_soa_floats((int)n_pad), &d_soa));
     TcPlan plan;
-    if (!plan_gram_tc(kq, &plan)) return fail(c, SRED_ERR_ARG, "K too large for the tensor-core engine");
-    CK(launch_gram_tc(d_A, d_B, kq, (int)n_pad, d_params, d_soa, ec, d_num, c->num_sms, d_status, st, 0, 1,
-                      &c->tc_debug));
-    CK(launch_gram_tc(d_A, d_B, kq, (int)n_pad, d_params, d_soa, ed, d_den, c->num_sms, d_status, st, 0, 1,
-                      &c->tc_debug));
+    if (split_cols(k) > 576 || !plan_gram_tc(k, &plan)) return fail(c, SRED_ERR_ARG, "K too large for the tensor-core engine");
+    CK(launch_gram_tc(d_S, k, (int)n_pad, d_params, d_soa, ec, d_num, c->num_sms, d_status, st, 0, 1, &c->tc_debug));
+    CK(launch_gram_tc(d_S, k, (int)n_pad, d_params, d_soa, ed, d_den, c->num_sms, d_status, st, 0, 1, &c->tc_debug));
     int status = 0;
     CK(cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));

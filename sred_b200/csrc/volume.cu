@@ -293,20 +293,19 @@ __global__ void k_flags3d(const float* __restrict__ stds, Vol3 v, float thr, int
 }
 
 // One warp per listed block: FP64 moments of its ellipsoid vector, the unit
-// vector (x - mu) / |x - mu| as FP32 (mode 0, row pitch kp) or as the two- /
-// three-level split BF16 operands (mode 1 / 2, store_split, row pitch kq),
-// and the epilogue parameters; the same quantities as the 2D packing, over
-// linear offsets.
+// vector (x - mu) / |x - mu| as FP32 (U, row pitch kp) and as the split FP16
+// operand (S, store_split), either of which may be null, and the epilogue
+// parameters; the same quantities as the 2D packing, over linear offsets.
 __global__ void k_pack3d(const float* __restrict__ img, Vol3 v, const int* __restrict__ off,
-                         const int* __restrict__ gram_pix, int n, float wscale, int mode, float* __restrict__ U,
-                         int kp, __nv_bfloat16* __restrict__ A, __nv_bfloat16* __restrict__ B, int kq,
-                         BlockParams* __restrict__ params, float* __restrict__ tile_rmax,
+                         const int* __restrict__ gram_pix, int n, float wscale, float* __restrict__ U, int kp,
+                         __half* __restrict__ S, BlockParams* __restrict__ params, float* __restrict__ tile_rmax,
                          unsigned* __restrict__ arange) {
   unsigned a_lo = 0u, a_hi = 0u;  // ~bits of the smallest a, bits of the largest (launch_den, weights.cuh)
   const int lane = threadIdx.x & 31;
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   const int K = v.k;
+  const SplitLayout lay = split_layout(K);
   for (int j = gw; j < n; j += nw) {
     const float* c = img + (size_t)gram_pix[j];
     double s = 0.0;
@@ -325,16 +324,11 @@ __global__ void k_pack3d(const float* __restrict__ img, Vol3 v, const int* __res
     for (int i = lane; i < K; i += 32) {
       const double u = ((double)c[off[i]] - mu) * inv;
       if (U) U[(size_t)j * kp + i] = (float)u;
-      if (mode != 0) store_split(A + (size_t)j * kq, B + (size_t)j * kq, K, i, u, mode + 1);
+      if (S) store_split(S + (size_t)j * lay.pitch, lay, i, u * (double)kSplitScale);
     }
     if (U)
       for (int i = K + lane; i < kp; i += 32) U[(size_t)j * kp + i] = 0.0f;
-    if (mode != 0) {
-      for (int i = (mode == 1 ? 3 : 6) * K + lane; i < kq; i += 32) {
-        A[(size_t)j * kq + i] = __float2bfloat16_rn(0.0f);
-        B[(size_t)j * kq + i] = __float2bfloat16_rn(0.0f);
-      }
-    }
+    if (S) store_split_pad(S + (size_t)j * lay.pitch, lay, lane);
     if (lane == 0) {
       BlockParams bp;
       bp.a = (float)(sigma * (double)wscale);
