@@ -150,10 +150,11 @@ constexpr float kNrmseNear = 1.0f - 1.0f / 128.0f;
 // symmetric schedule as the tensor-core engine with 128 x 128 tiles.
 // U: n_pad x kp floats (unit vectors), params: n_pad entries, num: n
 // doubles (zeroed). The work items are split into n_shards equal ranges; this
-// launch runs range `shard`.
+// launch runs range `shard`. arange (Abs-diff): the range of a, by which the
+// kernel leaves the sums to launch_absdiff.
 cudaError_t launch_gram_fp32(const float* U, int kp, const BlockParams* params, const float* tile_rmax,
                              EpiConsts ec, double* num, int num_sms, cudaStream_t st, int shard = 0,
-                             int n_shards = 1);
+                             int n_shards = 1, const unsigned* arange = nullptr);
 
 // Column parameters of one BN-column tile as the tensor-core engine copies
 // them into shared memory: [a x BN | r x BN | sigma x BN | mu x BN | per group

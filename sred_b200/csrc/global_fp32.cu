@@ -21,6 +21,7 @@
 // cancellation for near-identical blocks.
 #include <algorithm>
 
+#include "absdiff.cuh"
 #include "common.cuh"
 #include "epilogue.cuh"
 
@@ -40,6 +41,7 @@ struct Fp32Args {
   EpiConsts ec;
   double* num;
   int n_rb;              // 128-blocks holding valid rows (= column tiles)
+  const unsigned* arange;  // Abs-diff: absdiff.cu has the sums where it has a table (nullptr: never)
   int L;                 // row blocks per item
   long long item0, item1;
 };
@@ -139,6 +141,10 @@ __global__ void __launch_bounds__(NT, 2) k_gram_fp32(Fp32Args g) {
   BlockParams* Bp = Ap + BM;                                                         // [BM]
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   const bool gram = METRIC != kAbsDiff;
+  if (METRIC == kAbsDiff && g.arange) {
+    double x0;
+    if (abs_grid(g.arange, (g.ec.n + kAbsSlice - 1) / kAbsSlice, &x0) > 0) return;
+  }
 
   for (long long it = g.item0 + blockIdx.x; it < g.item1; it += gridDim.x) {
     int ct, rb0, rb1;
@@ -226,7 +232,8 @@ __global__ void __launch_bounds__(NT, 2) k_gram_fp32(Fp32Args g) {
 }  // namespace
 
 cudaError_t launch_gram_fp32(const float* U, int kp, const BlockParams* params, const float* tile_rmax,
-                             EpiConsts ec, double* num, int num_sms, cudaStream_t st, int shard, int n_shards) {
+                             EpiConsts ec, double* num, int num_sms, cudaStream_t st, int shard, int n_shards,
+                             const unsigned* arange) {
   if (n_shards < 1 || shard < 0 || shard >= n_shards) return cudaErrorInvalidValue;
   if (ec.n <= 0) return cudaSuccess;
   Fp32Args g;
@@ -236,6 +243,7 @@ cudaError_t launch_gram_fp32(const float* U, int kp, const BlockParams* params, 
   g.tile_rmax = tile_rmax;
   g.ec = ec;
   g.num = num;
+  g.arange = arange;
   g.n_rb = (ec.n + BM - 1) / BM;
   // Items of up to 16 row blocks, fewer when that leaves under ~4 per SM slot.
   int L = 16;

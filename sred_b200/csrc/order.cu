@@ -1,14 +1,16 @@
-// Ordering of the relevant blocks by their standard deviation, for the
-// factorised weights of the tensor-core engine (global_tc.cu): a stable
-// two-pass radix sort of the compacted pixel list on the top 22 bits below the
-// sign of the FP32 local std (8 exponent and 14 mantissa bits, so neighbours
-// differ by less than 2^-14 relative beyond a true order), ties in raster
-// order. Deterministic: ranks come from counts in list order, never from the
-// order in which atomics land.
+// Ordering of the relevant blocks: a stable radix sort of an index list by
+// non-negative float keys, 11 bits a pass, ties in list order. Deterministic:
+// ranks come from counts in list order, never from the order in which atomics land.
+//   - the tensor-core engine's weights (global_tc.cu): the compacted pixel list by
+//     the top 22 bits below the sign of the FP32 local std (8 exponent and 14
+//     mantissa bits, so neighbours differ by less than 2^-14 relative beyond a true
+//     order), two passes;
+//   - Abs-diff (absdiff.cu): the blocks by all 31 bits of a, three passes.
 //
-// Cost: latency. 754,587 blocks: six launches, 24 bytes of traffic per block
-// and pass, about 60 us in a 70 ms map.
+// Bound by latency (a few CTAs' worth of work and three launches a pass).
 #include "order.cuh"
+
+#include <utility>
 
 namespace sred {
 
@@ -20,20 +22,20 @@ constexpr int kWarps = 8, kThreads = 32 * kWarps;
 constexpr int kPerWarp = kSortSpan / kWarps;
 constexpr int kScanBins = 32;  // bins per CTA of the scan
 
-// Key of a block: the float bits without the sign (a NaN std sorts last).
-__device__ __forceinline__ unsigned sort_digit(float s, int pass) {
-  return ((__float_as_uint(s) & 0x7fffffffu) >> (9 + kDigitBits * pass)) & (kBins - 1);
+// Digit of a key: the float bits without the sign (a NaN sorts last).
+__device__ __forceinline__ unsigned sort_digit(float s, int shift) {
+  return ((__float_as_uint(s) & 0x7fffffffu) >> shift) & (kBins - 1);
 }
 
 // table[bin][span]: blocks of each span with that digit; total[bin]: of all spans.
-__global__ void __launch_bounds__(kThreads) k_sort_count(const float* __restrict__ stds, const int* __restrict__ pix,
-                                                         int n, int pass, int nspan, int* __restrict__ table,
+__global__ void __launch_bounds__(kThreads) k_sort_count(const float* __restrict__ keys, const int* __restrict__ idx,
+                                                         int n, int shift, int nspan, int* __restrict__ table,
                                                          int* __restrict__ total) {
   __shared__ int h[kBins];
   for (int i = threadIdx.x; i < kBins; i += kThreads) h[i] = 0;
   __syncthreads();
   const int i0 = blockIdx.x * kSortSpan, i1 = min(n, i0 + kSortSpan);
-  for (int i = i0 + threadIdx.x; i < i1; i += kThreads) atomicAdd(h + sort_digit(stds[pix[i]], pass), 1);
+  for (int i = i0 + threadIdx.x; i < i1; i += kThreads) atomicAdd(h + sort_digit(keys[idx[i]], shift), 1);
   __syncthreads();
   for (int b = threadIdx.x; b < kBins; b += kThreads) {
     const int c = h[b];
@@ -84,8 +86,8 @@ __global__ void __launch_bounds__(kThreads) k_sort_scan(const int* __restrict__ 
 
 // Stable scatter of one span: every warp takes its part of the span in order;
 // blocks of equal digit in a warp's step are ranked by lane (match_any).
-__global__ void __launch_bounds__(kThreads) k_sort_scatter(const float* __restrict__ stds, const int* __restrict__ pix,
-                                                           int n, int pass, int nspan, const int* __restrict__ table,
+__global__ void __launch_bounds__(kThreads) k_sort_scatter(const float* __restrict__ keys, const int* __restrict__ idx,
+                                                           int n, int shift, int nspan, const int* __restrict__ table,
                                                            int* __restrict__ out, int* __restrict__ slot) {
   extern __shared__ int cnt[];  // [kWarps][kBins]
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -97,8 +99,8 @@ __global__ void __launch_bounds__(kThreads) k_sort_scatter(const float* __restri
 #pragma unroll
   for (int j = 0; j < kPerWarp / 32; j++) {
     const int i = i0 + 32 * j + lane;
-    px[j] = i < n ? pix[i] : -1;
-    dg[j] = px[j] >= 0 ? (int)sort_digit(stds[px[j]], pass) : -1;
+    px[j] = i < n ? idx[i] : -1;
+    dg[j] = px[j] >= 0 ? (int)sort_digit(keys[px[j]], shift) : -1;
     if (dg[j] >= 0) atomicAdd(mine + dg[j], 1);
   }
   __syncthreads();
@@ -132,27 +134,32 @@ __global__ void __launch_bounds__(kThreads) k_sort_scatter(const float* __restri
 
 size_t sort_workspace_ints(int n) {
   const size_t nspan = ((size_t)n + kSortSpan - 1) / kSortSpan;
-  return (size_t)kBins * nspan + 2 * kBins + (size_t)n;
+  return (size_t)kBins * nspan + 3 * kBins + (size_t)n;
 }
 
-cudaError_t launch_sort_blocks(const float* stds, int* pix, int n, int* ws, int* slot, cudaStream_t st) {
+cudaError_t launch_sort(const float* keys, int* idx, int n, int shift, int passes, int* ws, int* slot,
+                        const int** sorted, cudaStream_t st) {
+  if (sorted) *sorted = idx;
   if (n <= 0) return cudaSuccess;
   const int nspan = (n + kSortSpan - 1) / kSortSpan;
-  int* total = ws;                       // [2][kBins]
-  int* table = total + 2 * kBins;        // [kBins][nspan]
+  int* total = ws;                           // [passes][kBins]
+  int* table = total + 3 * kBins;            // [kBins][nspan]
   int* tmp = table + (size_t)kBins * nspan;  // [n]
   const int smem = kWarps * kBins * (int)sizeof(int);
   cudaError_t e = cudaFuncSetAttribute(k_sort_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(total, 0, 2 * kBins * sizeof(int), st);
+  e = cudaMemsetAsync(total, 0, passes * kBins * sizeof(int), st);
   if (e != cudaSuccess) return e;
-  for (int pass = 0; pass < 2; pass++) {
-    const int* in = pass ? tmp : pix;
-    int* out = pass ? pix : tmp;
-    k_sort_count<<<nspan, kThreads, 0, st>>>(stds, in, n, pass, nspan, table, total + pass * kBins);
+  int *in = idx, *out = tmp;
+  for (int pass = 0; pass < passes; pass++) {
+    const int sh = shift + kDigitBits * pass;
+    k_sort_count<<<nspan, kThreads, 0, st>>>(keys, in, n, sh, nspan, table, total + pass * kBins);
     k_sort_scan<<<kBins / kScanBins, kThreads, 0, st>>>(total + pass * kBins, nspan, table);
-    k_sort_scatter<<<nspan, kThreads, smem, st>>>(stds, in, n, pass, nspan, table, out, pass ? slot : nullptr);
+    k_sort_scatter<<<nspan, kThreads, smem, st>>>(keys, in, n, sh, nspan, table, out,
+                                                  pass + 1 == passes ? slot : nullptr);
+    std::swap(in, out);
   }
+  if (sorted) *sorted = in;
   return cudaGetLastError();
 }
 

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "absdiff.cuh"
 #include "kernels.cuh"
 #include "order.cuh"
 #include "shape.cuh"
@@ -31,7 +32,7 @@ namespace {
 enum BufId {
   B_IMG, B_MEANS, B_STDS, B_MASK, B_MASKIN, B_FLAGS, B_SLOT, B_GPIX, B_FPIX, B_COUNTS, B_U, B_S,
   B_PARAMS, B_RMAX, B_NUM, B_DEN, B_SUMS, B_OUT, B_VARS, B_MM, B_NMASK, B_BAD, B_STATUS, B_STDS2, B_COLSOA,
-  B_FEAT, B_SIG, B_FR, B_FI, B_GAT, B_OFF3, B_REF3, B_STAT, B_THR, B_KMX, B_KMD2, B_KMLAB, B_KMB, B_TBOX, B_TSTAT, B_TMEAN, B_TVAR, B_STKIN, B_STKOUT, B_SORT, B_NODES, B_SLICES,
+  B_FEAT, B_SIG, B_FR, B_FI, B_GAT, B_OFF3, B_REF3, B_STAT, B_THR, B_KMX, B_KMD2, B_KMLAB, B_KMB, B_TBOX, B_TSTAT, B_TMEAN, B_TVAR, B_STKIN, B_STKOUT, B_SORT, B_NODES, B_SLICES, B_KEYS, B_IDX, B_ABS,
   B_NBUF
 };
 
@@ -262,15 +263,30 @@ bool sort_for(int engine, int metric) {
 sred_status sort_blocks(sred_ctx* c, const float* d_stds, int n_g, cudaStream_t st) {
   int* d_ws;
   CKS(ensure(c, B_SORT, sort_workspace_ints(n_g), &d_ws));
-  CK(launch_sort_blocks(d_stds, static_cast<int*>(c->buf[B_GPIX].p), n_g, d_ws, static_cast<int*>(c->buf[B_SLOT].p),
-                        st));
+  CK(launch_sort(d_stds, static_cast<int*>(c->buf[B_GPIX].p), n_g, kStdShift, kStdPasses, d_ws,
+                 static_cast<int*>(c->buf[B_SLOT].p), nullptr, st));
   return SRED_OK;
 }
 
 // Kernels of a map between the statistics and the finalisation.
-int contraction_launches(int n_g, int engine, bool sorted) {
-  if (n_g == 0) return 0;
-  return (engine == SRED_ENGINE_TC ? 3 : 2) + kDenLaunches + (sorted ? kSortLaunches : 0);
+int contraction_launches(const GState& gs) {
+  if (gs.n_g == 0) return 0;
+  return (gs.engine == SRED_ENGINE_TC ? 3 : 2) + kDenLaunches + (gs.sorted ? 3 * kStdPasses : 0) +
+         (gs.metric == kAbsDiff ? kAbsLaunches : 0);
+}
+
+// The numerators of an Abs-diff map (shard 0's share of the sums, as the denominators).
+sred_status absdiff_sums(sred_ctx* c, const GState& gs, cudaStream_t st, const unsigned* arange) {
+  float* d_keys;
+  int *d_idx, *d_ws;
+  double* d_table;
+  CKS(ensure(c, B_KEYS, gs.n_g, &d_keys));
+  CKS(ensure(c, B_IDX, gs.n_g, &d_idx));
+  CKS(ensure(c, B_SORT, sort_workspace_ints(gs.n_g), &d_ws));
+  CKS(ensure(c, B_ABS, kAbsTable, &d_table));
+  CK(launch_absdiff(static_cast<const BlockParams*>(c->buf[B_PARAMS].p), gs.n_g, 1.0 / (double)gs.wscale, arange, d_keys,
+                    d_idx, d_ws, d_table, static_cast<double*>(c->buf[B_NUM].p), c->num_sms, st));
+  return SRED_OK;
 }
 
 // Phase 1: everything before the all-pairs contraction.
@@ -348,7 +364,8 @@ sred_status global_prepare(sred_ctx* c, int metric, const float* d_img, int w, i
   CKS(ensure(c, B_NUM, n_pad, &d_num));
   CKS(ensure(c, B_DEN, n_pad, &d_den));
   CKS(ensure(c, B_SUMS, 8, &d_sums));  // the flat blocks' sums, then the range of a
-  if (engine == SRED_ENGINE_FP32 || metric == kNrmse) {  // tensor-core NRMSE reads U for near-identical pairs
+  // tensor-core NRMSE reads U for near-identical pairs; Abs-diff correlates nothing
+  if ((engine == SRED_ENGINE_FP32 || metric == kNrmse) && metric != kAbsDiff) {
     CKS(ensure(c, B_U, n_pad * kp, &d_U));
     CK(cudaMemsetAsync(d_U + (size_t)n_g * kp, 0, (n_pad - n_g) * kp * sizeof(float), st));
   }
@@ -447,8 +464,10 @@ sred_status global_gram(sred_ctx* c, const GState& gs, cudaStream_t st, int shar
     const float* d_rmax = static_cast<const float*>(c->buf[B_RMAX].p);
     CKS(denominators(c, gs, st, shard));
     if (gs.engine == SRED_ENGINE_FP32) {
+      const unsigned* arange = reinterpret_cast<const unsigned*>(static_cast<double*>(c->buf[B_SUMS].p) + 4);
+      if (gs.metric == kAbsDiff && shard == 0) CKS(absdiff_sums(c, gs, st, arange));
       CK(launch_gram_fp32(static_cast<const float*>(c->buf[B_U].p), gs.kp, d_params, d_rmax, ec, d_num, c->num_sms,
-                          st, shard, n_shards));
+                          st, shard, n_shards, arange));
     } else {
       int* d_status;
       CKS(ensure(c, B_STATUS, 4, &d_status));
@@ -546,7 +565,7 @@ sred_status global_finish(sred_ctx* c, const GState& gs, cudaStream_t st, int no
     info->ms_gram = t12;
     info->ms_finalize = t23;
     info->ms_total = t03;
-    info->launches = (gs.given ? 0 : 2) + 4 + contraction_launches(gs.n_g, gs.engine, gs.sorted) + 1 +
+    info->launches = (gs.given ? 0 : 2) + 4 + contraction_launches(gs) + 1 +
                      (normalize ? 3 : 0);
   }
   if (c->log_cb) {
@@ -892,7 +911,8 @@ sred_status global3d_prepare(sred_ctx* c, int metric, const float* d_vol, int w,
   CKS(ensure(c, B_NUM, n_pad, &d_num));
   CKS(ensure(c, B_DEN, n_pad, &d_den));
   CKS(ensure(c, B_SUMS, 8, &d_sums));  // the range of a, after the 2D maps' sums
-  if (engine == SRED_ENGINE_FP32 || metric == kNrmse) {  // tensor-core NRMSE reads U for near-identical pairs
+  // tensor-core NRMSE reads U for near-identical pairs; Abs-diff correlates nothing
+  if ((engine == SRED_ENGINE_FP32 || metric == kNrmse) && metric != kAbsDiff) {
     CKS(ensure(c, B_U, n_pad * kp, &d_U));
     CK(cudaMemsetAsync(d_U + (size_t)n_g * kp, 0, (n_pad - n_g) * kp * sizeof(float), st));
   }
@@ -990,7 +1010,7 @@ sred_status global3d_finish(sred_ctx* c, const GState& gs, cudaStream_t st, int 
     info->ms_gram = t12;
     info->ms_finalize = t23;
     info->ms_total = t03;
-    info->launches = 5 + contraction_launches(gs.n_g, gs.engine, gs.sorted) + 1 + (normalize ? 3 : 0);
+    info->launches = 5 + contraction_launches(gs) + 1 + (normalize ? 3 : 0);
   }
   if (c->log_cb) {
     float t03 = 0;
@@ -1693,7 +1713,7 @@ sred_status sred_global_map_2d(sred_ctx* c, const char* metric, const float* img
 // thereby synchronises the device, while other workers' kernels run.
 sred_status reserve_global(sred_ctx* c, const sred_job* jobs, int n_jobs) {
   size_t n = 1, n_pad = 256, a = 1, u = 1, cols = 1;
-  bool fp32 = c->engine == SRED_ENGINE_FP32, tc = c->engine == SRED_ENGINE_TC;
+  bool fp32 = c->engine == SRED_ENGINE_FP32, tc = c->engine == SRED_ENGINE_TC, absdiff = false;
   for (int i = 0; i < n_jobs; i++) {
     const sred_job& j = jobs[i];
     Ellipse e;
@@ -1709,7 +1729,7 @@ sred_status reserve_global(sred_ctx* c, const sred_job* jobs, int n_jobs) {
     cols = std::max(cols, gram_tc_soa_floats((int)np));
     if (tc && pick_engine(c, global_metric(j.metric), K) == SRED_ENGINE_FP32) fp32 = true;
     if (global_metric(j.metric) == kNrmse) fp32 = true;  // U for the near-identical pairs
-    if (global_metric(j.metric) == kAbsDiff) fp32 = true;
+    if (global_metric(j.metric) == kAbsDiff) absdiff = true;
   }
   float* f;
   uint8_t* u8;
@@ -1729,8 +1749,13 @@ sred_status reserve_global(sred_ctx* c, const sred_job* jobs, int n_jobs) {
   CKS(ensure(c, B_DEN, n_pad, &d));
   CKS(ensure(c, B_NODES, kDenNodes, &d));
   CKS(ensure(c, B_SLICES, den_slices((int)n_pad), &f2));
+  if (absdiff) {
+    CKS(ensure(c, B_KEYS, n_pad, &f));
+    CKS(ensure(c, B_IDX, n_pad, &i32));
+    CKS(ensure(c, B_ABS, kAbsTable, &d));
+  }
+  if (tc || absdiff) CKS(ensure(c, B_SORT, sort_workspace_ints((int)n_pad), &i32));
   if (tc) {
-    CKS(ensure(c, B_SORT, sort_workspace_ints((int)n_pad), &i32));
     CKS(ensure(c, B_S, a + kSplitSlack, &hf));
     CKS(ensure(c, B_COLSOA, cols, &f));
   }

@@ -26,22 +26,9 @@ namespace sred {
 
 namespace {
 
-constexpr double kH = 0.125;
-constexpr int kPad = 6;            // nodes below the smallest a
 constexpr int kThreads = 256;
 constexpr int kPer = kDenSlice / kThreads;
 constexpr int kGroup = 8;          // nodes per step
-constexpr float kFar = 14.0f;
-
-// Node grid of the a-range (arange: see launch_den): first node and count (0: no grid).
-__device__ __forceinline__ int node_grid(const unsigned* __restrict__ arange, double* x0) {
-  const unsigned lo = ~arange[0], hi = arange[1];
-  if (hi >= 0x7f800000u) return 0;  // infinite or NaN (either sign)
-  const double a0 = (double)__uint_as_float(lo), a1 = (double)__uint_as_float(hi);
-  *x0 = a0 - kPad * kH;
-  const double m = floor((a1 - a0) / kH) + 2 * kPad + 2;
-  return m <= (double)kDenNodes ? (int)m : 0;
-}
 
 __global__ void __launch_bounds__(kThreads) k_den_nodes(const BlockParams* __restrict__ params, int n,
                                                         const unsigned* __restrict__ arange,
@@ -56,7 +43,7 @@ __global__ void __launch_bounds__(kThreads) k_den_nodes(const BlockParams* __res
 #pragma unroll
   for (int j = 0; j < kPer; j++) {
     const int i = i0 + j * kThreads + threadIdx.x;
-    v[j] = i < n ? params[i].a : 3.4e38f;  // past the end: further than kFar from every node
+    v[j] = i < n ? params[i].a : 3.4e38f;  // past the end: further than kNodeFar from every node
     if (i < n) {
       lo = fminf(lo, v[j]);
       hi = fmaxf(hi, v[j]);
@@ -83,19 +70,19 @@ __global__ void __launch_bounds__(kThreads) k_den_nodes(const BlockParams* __res
   double x0;
   const int m = node_grid(arange, &x0);
   if (m == 0) return;
-  const int g0 = max(0, (int)floor(((double)lo - kFar - x0) / (kH * kGroup)));
-  const int g1 = min((m - 1) / kGroup, (int)floor(((double)hi + kFar - x0) / (kH * kGroup)));
-  const double q = exp2(-2.0 * kH * kH);
+  const int g0 = max(0, (int)floor(((double)lo - kNodeFar - x0) / (kNodeH * kGroup)));
+  const int g1 = min((m - 1) / kGroup, (int)floor(((double)hi + kNodeFar - x0) / (kNodeH * kGroup)));
+  const double q = exp2(-2.0 * kNodeH * kNodeH);
   for (int g = g0; g <= g1; g++) {
-    const double xb = x0 + (double)(g * kGroup) * kH;
+    const double xb = x0 + (double)(g * kGroup) * kNodeH;
     double acc[kGroup];
 #pragma unroll
     for (int k = 0; k < kGroup; k++) acc[k] = 0.0;
 #pragma unroll
     for (int j = 0; j < kPer; j++) {
       const double d = xb - (double)v[j];
-      if (fabs(d + 0.5 * kH * kGroup) > (double)kFar) continue;  // (2^-182 at most)
-      double e = exp2(-d * d), r = exp2(-(2.0 * d + kH) * kH);
+      if (fabs(d + 0.5 * kNodeH * kGroup) > (double)kNodeFar) continue;  // (2^-182 at most)
+      double e = exp2(-d * d), r = exp2(-(2.0 * d + kNodeH) * kNodeH);
 #pragma unroll
       for (int k = 0; k < kGroup; k++) {
         acc[k] += e;
@@ -126,13 +113,6 @@ __global__ void __launch_bounds__(kThreads) k_den_nodes(const BlockParams* __res
   }
 }
 
-// 1 / prod_{j != k} (k - j) for the nodes 0..11.
-__device__ __forceinline__ double lagrange_scale(int k) {
-  const double f[12] = {1.0, 1.0, 2.0, 6.0, 24.0, 120.0, 720.0, 5040.0, 40320.0, 362880.0, 3628800.0, 39916800.0};
-  const double v = 1.0 / (f[k] * f[11 - k]);
-  return (k & 1) ? v : -v;  // sign (-1)^(11 - k)
-}
-
 __global__ void __launch_bounds__(kThreads) k_den_eval(const BlockParams* __restrict__ params, int n,
                                                        const unsigned* __restrict__ arange,
                                                        const double* __restrict__ nodes,
@@ -142,20 +122,7 @@ __global__ void __launch_bounds__(kThreads) k_den_eval(const BlockParams* __rest
   double x0;
   if (node_grid(arange, &x0) > 0) {
     if (i >= n) return;
-    const double t = ((double)params[i].a - x0) / kH;
-    const int k0 = (int)floor(t) - (kPad - 1);
-    const double s = t - (double)k0;  // in [5, 6)
-    double suf[12];
-    suf[11] = 1.0;
-#pragma unroll
-    for (int k = 11; k > 0; k--) suf[k - 1] = suf[k] * (s - (double)k);
-    double pre = 1.0, sum = 0.0;
-#pragma unroll
-    for (int k = 0; k < 12; k++) {
-      sum += lagrange_scale(k) * pre * suf[k] * nodes[k0 + k];
-      pre *= s - (double)k;
-    }
-    den[i] = sum;
+    den[i] = interpolate12((double)params[i].a, x0, nodes, 1);
     return;
   }
   __shared__ float sa[kThreads];
@@ -177,7 +144,7 @@ __global__ void __launch_bounds__(kThreads) k_den_eval(const BlockParams* __rest
   double sum = 0.0;
   for (int s = 0; s < nslices; s++) {
     const float2 r = slices[s];
-    if (!any_bad && (r.x - hi > kFar || lo - r.y > kFar)) continue;  // (a NaN range is not skipped)
+    if (!any_bad && (r.x - hi > kNodeFar || lo - r.y > kNodeFar)) continue;  // (a NaN range is not skipped)
     const int q0 = s * kDenSlice, q1 = min(n, q0 + kDenSlice);
     for (int qb = q0; qb < q1; qb += kThreads) {
       const int m = min(kThreads, q1 - qb);

@@ -7,6 +7,47 @@ namespace sred {
 constexpr int kDenSlice = 2048;    // blocks per CTA of the node sums
 constexpr int kDenNodes = 16384;   // node table (doubles)
 
+// Functions of a block's a as sums over all blocks: nodes kNodeH apart and a
+// 12-point Lagrange polynomial between them (weights.cu: how accurate).
+constexpr double kNodeH = 0.125;
+constexpr int kNodePad = 6;        // nodes below the smallest a
+constexpr float kNodeFar = 14.0f;  // terms further off (2^-169) are left out
+
+// Node grid of the a-range (arange: see launch_den): first node and count (0: no grid).
+__device__ __forceinline__ int node_grid(const unsigned* __restrict__ arange, double* x0) {
+  const unsigned lo = ~arange[0], hi = arange[1];
+  if (hi >= 0x7f800000u) return 0;  // infinite or NaN (either sign)
+  const double a0 = (double)__uint_as_float(lo), a1 = (double)__uint_as_float(hi);
+  *x0 = a0 - kNodePad * kNodeH;
+  const double m = floor((a1 - a0) / kNodeH) + 2 * kNodePad + 2;
+  return m <= (double)kDenNodes ? (int)m : 0;
+}
+
+// 1 / prod_{j != k} (k - j) for the nodes 0..11.
+__device__ __forceinline__ double lagrange_scale(int k) {
+  const double f[12] = {1.0, 1.0, 2.0, 6.0, 24.0, 120.0, 720.0, 5040.0, 40320.0, 362880.0, 3628800.0, 39916800.0};
+  const double v = 1.0 / (f[k] * f[11 - k]);
+  return (k & 1) ? v : -v;  // sign (-1)^(11 - k)
+}
+
+// The function at a from its node values (stride between nodes).
+__device__ __forceinline__ double interpolate12(double a, double x0, const double* __restrict__ nodes, size_t stride) {
+  const double t = (a - x0) / kNodeH;
+  const int k0 = (int)floor(t) - (kNodePad - 1);
+  const double s = t - (double)k0;  // in [5, 6)
+  double suf[12];
+  suf[11] = 1.0;
+#pragma unroll
+  for (int k = 11; k > 0; k--) suf[k - 1] = suf[k] * (s - (double)k);
+  double pre = 1.0, sum = 0.0;
+#pragma unroll
+  for (int k = 0; k < 12; k++) {
+    sum += lagrange_scale(k) * pre * suf[k] * nodes[(size_t)(k0 + k) * stride];
+    pre *= s - (double)k;
+  }
+  return sum;
+}
+
 int den_slices(int n);
 
 // den[p] = sum_q 2^-(a_p - a_q)^2 over the n blocks of params. arange: the

@@ -17,19 +17,20 @@ def ctx():
     return _lib.Context(0, "tc")
 
 
-def _sums(ctx, engine, img, b, relc):
-    """[num | den] of the unsharded map and the run info (shard 0 of 1)."""
+def _sums(ctx, engine, img, b, relc, metric="Pearson's R"):
+    """num and den of the unsharded map and the run info (shard 0 of 1)."""
     import torch
     ctx.set_engine(engine)
     h, w = img.shape
     d = torch.from_numpy(img).cuda()
     part = torch.zeros(2 * w * h, dtype=torch.float64, device="cuda")
     info = _lib.RunInfo()
-    ctx.check(ctx._L.sred_global_map_2d_shard_sums(ctx.h, b"Pearson's R", C.c_void_p(d.data_ptr()), w, h, b, b, relc, 0,
+    ctx.check(ctx._L.sred_global_map_2d_shard_sums(ctx.h, metric.encode(), C.c_void_p(d.data_ptr()), w, h, b, b, relc, 0,
                                                    1, C.c_void_p(part.data_ptr()), 2 * w * h, None, C.byref(info)),
               "shard_sums")
     n = int(info.n_relevant - info.n_flat)
-    return part.cpu().numpy()[n:2 * n], info
+    part = part.cpu().numpy()
+    return part[:n], part[n:2 * n], info
 
 
 def _expected_a(img, b, info):
@@ -47,18 +48,23 @@ def _expected_a(img, b, info):
     return s[use], (s64[use] * np.float64(ws)).astype(np.float32)
 
 
+def _weights_image(w, h, bright):
+    if not bright:
+        return synth.normalize_input(synth.spot_image(w, h, 4, seed=w))
+    rng = np.random.default_rng(5)
+    img = (1e-6 * rng.random((h, w))).astype(np.float32)
+    img[40:60, 40:70] = 4 * rng.random((20, 30), dtype=np.float32)
+    return img
+
+
 # Images whose listed blocks number one slice of 2,048 or less, a slice and a few, several
 # slices; and with a bright square on a nearly silent background (the a-range beyond the
 # node table: direct sums).
 @pytest.mark.parametrize("w,h,b,bright", [(21, 19, 3, 0), (50, 46, 5, 0), (130, 97, 9, 0), (150, 140, 5, 1)])
 @pytest.mark.parametrize("engine", ["tc", "fp32"])
 def test_denominators_and_block_order(ctx, engine, w, h, b, bright):
-    img = synth.normalize_input(synth.spot_image(w, h, 4, seed=w))
-    if bright:
-        rng = np.random.default_rng(5)
-        img = (1e-6 * rng.random((h, w))).astype(np.float32)
-        img[40:60, 40:70] = 4 * rng.random((20, 30), dtype=np.float32)
-    den, info = _sums(ctx, engine, img, b, 0.0)
+    img = _weights_image(w, h, bright)
+    _, den, info = _sums(ctx, engine, img, b, 0.0)
     s, a = _expected_a(img, b, info)
     assert den.size == a.size
     if bright:
@@ -70,6 +76,21 @@ def test_denominators_and_block_order(ctx, engine, w, h, b, bright):
     # nodes: 6e-11 relative, plus an FP32 rounding of an argument that falls the other way
     # (2 ln2 d da 2^-24, below 1e-6); direct sums: ex2.approx (2^-22) and FP32 arguments
     np.testing.assert_allclose(den, exp, rtol=4e-6 if bright else 1e-6)
+
+
+# The same sizes; the slices of Abs-diff hold 512 blocks.
+@pytest.mark.parametrize("w,h,b", [(21, 19, 3), (34, 18, 3), (50, 46, 5), (130, 97, 9)])
+def test_absdiff_numerators(ctx, w, h, b):
+    img = _weights_image(w, h, 0)
+    num, den, info = _sums(ctx, "tc", img, b, 0.0, "Abs. diff. of StdDevs")
+    _, a = _expected_a(img, b, info)
+    a = a.astype(np.float64)
+    d = np.abs(a[:, None] - a[None])
+    wt = np.exp2(-d * d)
+    ws = np.sqrt(1.4426950408889634 / np.float64(np.float32(np.float32(info.noise_var) + np.float32(1e-7))))
+    np.testing.assert_allclose(den, wt.sum(1), rtol=1e-6)
+    # within a slice ex2.approx (2^-22) and FP32 sums of 32
+    np.testing.assert_allclose(num, (d * wt).sum(1) / ws, rtol=2e-6)
 
 
 # Contrast from all slabs factorised to slabs whose every weight underflows; both bars as in
