@@ -9,12 +9,81 @@
 // Nrmse,AbsDiffStds}2D.cl, with cl/kernelGetLocalStatistics2D.cl for the
 // moments) bit for bit. The image tile and its halo are staged in shared
 // memory so every pixel is read from HBM once.
+//
+// The host steps that follow (java/CLUtils.java:788-821, 936-960, and the
+// normalisation) are one read-modify-write pass each, k_plane_pass: the range a
+// pass needs is taken by the kernel that wrote the values.
+#include <algorithm>
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
 namespace sred {
 
-constexpr int kTileX = 32, kTileY = 16, kThreadsY = 8;  // each thread: rows y and y + 8 of the tile
+namespace {
+
+constexpr int kThreadsY = 8;         // thread rows of a CTA (one warp each)
+constexpr int kTileY = 2 * kThreadsY;  // a thread's pixels: rows y and y + 8 of the tile
+
+using f2 = unsigned long long;  // two floats: rows y (low) and y + 8
+
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
+  f2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// The rounded product, as a b + nz with nz = (-0, -0) a kernel argument: the
+// compiler merges a packed multiplication, or a multiply-add of a -0 that it can
+// see, with the addition that follows into one rounding, even with .rn on both.
+__device__ __forceinline__ f2 mul2(f2 a, f2 b, f2 nz) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(nz));
+  return r;
+}
+constexpr f2 kNegZero2 = 0x8000000080000000ull;
+__device__ __forceinline__ f2 pack2(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f2 v, float* a, float* b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(*a), "=f"(*b) : "l"(v));
+}
+
+// Order-preserving key of a float (-0 below +0), and back.
+__device__ __forceinline__ unsigned ord_bits(float f) {
+  const unsigned u = __float_as_uint(f);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float ord_float(unsigned u) {
+  return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
+}
+
+// A CTA's smallest and largest key into mm (all threads of the CTA call it).
+__device__ __forceinline__ void cta_minmax(unsigned lo, unsigned hi, unsigned* mm) {
+  __shared__ unsigned s_lo[8], s_hi[8];
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0) {
+    s_lo[threadIdx.x >> 5] = lo;
+    s_hi[threadIdx.x >> 5] = hi;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    lo = __reduce_min_sync(0xffffffffu, s_lo[threadIdx.x & 7]);
+    hi = __reduce_max_sync(0xffffffffu, s_hi[threadIdx.x & 7]);
+    if (threadIdx.x == 0 && lo <= hi) {
+      atomicMin(mm, lo);
+      atomicMax(mm + 1, hi);
+    }
+  }
+}
 
 // The metric of one pixel from its block sums (reference order, explicitly
 // rounded), and its local std.
@@ -37,105 +106,234 @@ __device__ __forceinline__ float block_metric_value(int metric, int K, float mea
   return fmaxf(0.0f, __fdiv_rn(__fmul_rn(a, b), __fmul_rn(cc, dd)));
 }
 
-__global__ void __launch_bounds__(kTileX* kThreadsY)
-    k_block_map(const float* __restrict__ img_all, int W, int H, int frames, Ellipse e, RefBlock rb,
-                int metric, float* __restrict__ out_all, float* __restrict__ stds_out) {
-  // shared: the image tile (kTileY + 2rh) x (kTileX + 2rw), then the ellipse
-  // as linear tile offsets (K ints) and the reference block (K floats). Each
-  // thread evaluates two pixels, rows y and y + 8, so every broadcast load of
-  // an offset or a reference value serves both; each pixel keeps the
-  // reference's sequential order.
-  extern __shared__ float tile[];
-  const int f = blockIdx.z;
-  const float* img = img_all + (size_t)f * W * H;
-  float* out = out_all + (size_t)f * W * H;
-  const int tw = kTileX + 2 * e.rw, th = kTileY + 2 * e.rh;
-  int* s_off = reinterpret_cast<int*>(tile + tw * th);
-  float* s_ref = reinterpret_cast<float*>(s_off + e.k);
-  const int x0 = blockIdx.x * kTileX - e.rw, y0 = blockIdx.y * kTileY - e.rh;
-  const int tid = threadIdx.y * kTileX + threadIdx.x;
-  for (int i = tid; i < tw * th; i += kTileX * kThreadsY) {
-    const int ty = i / tw, tx = i - ty * tw;
-    const int gx = x0 + tx, gy = y0 + ty;
-    tile[i] = (gx >= 0 && gx < W && gy >= 0 && gy < H) ? img[(size_t)gy * W + gx] : 0.0f;
+// The ellipse by rows: row r holds the columns -hw[r] .. hw[r].
+struct BlockRows {
+  int k, rw, rh;
+  short hw[kMaxK];
+};
+
+// Visits the block of a thread's 2 PX pixels in the reference's order: f(i, w)
+// for element i with w(q) the value pair of pixel column q. Neighbouring pixels
+// share all but one value of an element, so a window of PX pairs slides along
+// each row: one shared-memory load an element for 2 PX pixels. Column c of the
+// tile lies at (c % PX) p + c / PX, which keeps the loads of a warp contiguous.
+template <int PX, class F>
+__device__ __forceinline__ void sweep(const f2* base, int p, int pitch, const BlockRows& e, F f) {
+  int i = 0;
+  for (int r = 0; r <= 2 * e.rh; r++, base += pitch) {
+    const int hw = e.hw[r], s = e.rw - hw;
+    int o[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) o[q] = ((s + q) % PX) * p + (s + q) / PX;
+    f2 w[PX];
+#pragma unroll
+    for (int q = 0; q < PX - 1; q++) w[q] = base[o[q]];
+    auto element = [&](auto jc) {
+      constexpr int j = decltype(jc)::value;
+      constexpr int c = PX - 1 + j;  // the column that enters the window
+      w[c % PX] = base[o[c & 3] + (c >> 2) * (4 / PX)];
+      f(i + j, [&](int q) { return w[(j + q) % PX]; });
+    };
+    int n = 2 * hw + 1;
+    for (; n >= 4; n -= 4, i += 4) {
+      element(std::integral_constant<int, 0>());
+      element(std::integral_constant<int, 1>());
+      element(std::integral_constant<int, 2>());
+      element(std::integral_constant<int, 3>());
+#pragma unroll
+      for (int q = 0; q < 4; q++) o[q] += 4 / PX;
+    }
+    // (n is odd: 1 or 3 left)
+    element(std::integral_constant<int, 0>());
+    if (n == 3) {
+      element(std::integral_constant<int, 1>());
+      element(std::integral_constant<int, 2>());
+    }
+    i += n;
   }
-  for (int i = tid; i < e.k; i += kTileX * kThreadsY) {
-    s_off[i] = e.dy[i] * tw + e.dx[i];
-    s_ref[i] = rb.px[i];
+}
+
+// The tile of PX: columns, values per column class, f2 per row.
+template <int PX>
+struct Tile {
+  static constexpr int kX = 32 * PX;
+  __host__ __device__ static int cols(int rw) { return kX + 2 * rw; }
+  // p = 4 mod 8: the classes of neighbouring columns fall on different banks
+  __host__ __device__ static int p(int rw) { return PX == 1 ? cols(rw) : ((cols(rw) + PX - 1) / PX + 11) / 8 * 8 - 4; }
+  __host__ __device__ static int pitch(int rw) { return PX * p(rw); }
+  static size_t smem(int rw, int rh, int k) {
+    return sizeof(f2) * ((size_t)pitch(rw) * (kThreadsY + 2 * rh) + k);
+  }
+};
+
+// MODE: kPearson (also SSIM), kNrmse, kCosine, kAbsDiff. Bound by FP32 issue: a
+// pixel's element is 6 operations that may not be merged (sum; difference, two
+// products, two sums), in packed pairs of two rows, and the window leaves 1/4 load
+// a pixel. 16 frames of 1024x1024, 15x15 (177 elements), normalised: 1365 us with one
+// load an element and pass and a thread per two pixels, 720 now (480 at one scalar
+// operation a lane and clock).
+template <int MODE, int PX>
+__global__ void __launch_bounds__(32 * kThreadsY)
+    k_block_map(const float* __restrict__ img_all, int W, int H, const __grid_constant__ BlockRows e,
+                const __grid_constant__ RefBlock rb, int metric, f2 nz, float* __restrict__ out_all,
+                float* __restrict__ stds_all, unsigned* __restrict__ mm) {
+  // shared: pair row r of the tile = its rows r and r + 8 side by side, for r in
+  // [0, 8 + 2 rh); then the reference block, each value twice.
+  extern __shared__ f2 tile[];
+  const size_t plane = (size_t)W * H * blockIdx.z;
+  const float* img = img_all + plane;
+  float* out = out_all + plane;
+  float* stds = stds_all ? stds_all + plane : nullptr;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int cols = Tile<PX>::cols(e.rw), p = Tile<PX>::p(e.rw), pitch = PX * p;
+  const int pr = kThreadsY + 2 * e.rh, K = e.k;
+  f2* s_ref = tile + (size_t)pitch * pr;
+  {
+    const int x0 = blockIdx.x * Tile<PX>::kX - e.rw, y0 = blockIdx.y * kTileY - e.rh;
+    float* t = reinterpret_cast<float*>(tile);
+    for (int r = ty; r < pr + kThreadsY; r += kThreadsY) {
+      const int gy = y0 + r;
+      const bool row_in = gy >= 0 && gy < H;
+      for (int c = tx; c < cols; c += 32) {
+        const int gx = x0 + c;
+        const float v = row_in && gx >= 0 && gx < W ? img[(size_t)gy * W + gx] : 0.0f;
+        const int o = (c % PX) * p + c / PX;
+        if (r < pr) t[2 * (r * pitch + o)] = v;
+        if (r >= kThreadsY) t[2 * ((r - kThreadsY) * pitch + o) + 1] = v;
+      }
+    }
+    for (int i = threadIdx.x; i < K; i += 32 * kThreadsY) s_ref[i] = pack2(rb.px[i], rb.px[i]);
   }
   __syncthreads();
-  const int x = blockIdx.x * kTileX + threadIdx.x;
-  const int ya = blockIdx.y * kTileY + threadIdx.y, yb = ya + kThreadsY;
-  if (x >= W || ya >= H) return;
-  const bool has_b = yb < H;
-  const bool in_x = x >= e.rw && x < W - e.rw;
-  const bool in_a = in_x && ya >= e.rh && ya < H - e.rh;
-  const bool in_b = has_b && in_x && yb >= e.rh && yb < H - e.rh;
-  const size_t pa = (size_t)ya * W + x, pb = (size_t)yb * W + x;
-  if (!in_a && !in_b) {
-    out[pa] = 0.0f;
-    if (stds_out) stds_out[(size_t)f * W * H + pa] = 0.0f;
-    if (has_b) {
-      out[pb] = 0.0f;
-      if (stds_out) stds_out[(size_t)f * W * H + pb] = 0.0f;
+  const int x = blockIdx.x * Tile<PX>::kX + PX * tx, y = blockIdx.y * kTileY + ty;
+  unsigned lo = 0xffffffffu, hi = 0u;
+  // (a pixel outside the interior is evaluated on the zero-padded tile and discarded)
+  const bool some = x < W - e.rw && x + PX > e.rw && y < H - e.rh && y + kThreadsY >= e.rh;
+  float val[PX][2], sd[PX][2];
+#pragma unroll
+  for (int q = 0; q < PX; q++) val[q][0] = val[q][1] = sd[q][0] = sd[q][1] = 0.0f;
+  if (some) {
+    const f2* base = tile + ty * pitch + tx;
+    f2 m[PX], v[PX], a[PX], xx[PX], rr = 0;
+#pragma unroll
+    for (int q = 0; q < PX; q++) m[q] = v[q] = a[q] = xx[q] = 0;
+    sweep<PX>(base, p, pitch, e, [&](int, auto w) {
+#pragma unroll
+      for (int q = 0; q < PX; q++) m[q] = add2(m[q], w(q));
+    });
+#pragma unroll
+    for (int q = 0; q < PX; q++) {
+      float s0, s1;
+      unpack2(m[q], &s0, &s1);
+      m[q] = pack2(__fdiv_rn(s0, (float)K), __fdiv_rn(s1, (float)K));
     }
-    return;
+    sweep<PX>(base, p, pitch, e, [&](int i, auto w) {
+      const f2 ref = MODE == kAbsDiff ? 0 : s_ref[i];
+#pragma unroll
+      for (int q = 0; q < PX; q++) {
+        const f2 d = sub2(w(q), m[q]);
+        v[q] = add2(v[q], mul2(d, d, nz));
+        if (MODE == kNrmse) {
+          const f2 t = sub2(ref, d);
+          a[q] = add2(a[q], mul2(t, t, nz));
+        } else if (MODE == kCosine) {
+          a[q] = add2(a[q], mul2(ref, w(q), nz));
+          xx[q] = add2(xx[q], mul2(w(q), w(q), nz));
+        } else if (MODE == kPearson) {
+          a[q] = add2(a[q], mul2(ref, d, nz));
+        }
+      }
+      if (MODE == kCosine) rr = add2(rr, mul2(ref, ref, nz));
+    });
+    float r0, r1;
+    unpack2(rr, &r0, &r1);
+#pragma unroll
+    for (int q = 0; q < PX; q++) {
+      float ms[2], vs[2], as[2], xs[2];
+      unpack2(m[q], &ms[0], &ms[1]);
+      unpack2(v[q], &vs[0], &vs[1]);
+      unpack2(a[q], &as[0], &as[1]);
+      unpack2(xx[q], &xs[0], &xs[1]);
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        float s;
+        const float o = block_metric_value(metric, K, ms[h], vs[h], as[h], r0, xs[h], rb.mean, rb.std, &s);
+        const int px = x + q, py = y + h * kThreadsY;
+        if (px >= e.rw && px < W - e.rw && py >= e.rh && py < H - e.rh) {
+          val[q][h] = o;
+          sd[q][h] = s;
+          lo = min(lo, ord_bits(o));
+          hi = max(hi, ord_bits(o));
+        }
+      }
+    }
   }
-  // (a pixel outside the interior is evaluated on the zero-padded tile and
-  // discarded)
-  const float* ca = tile + (threadIdx.y + e.rh) * tw + (threadIdx.x + e.rw);
-  const float* cb = ca + kThreadsY * tw;
-  const int K = e.k;
-  float sa = 0.0f, sb = 0.0f;
-  for (int i = 0; i < K; i++) {
-    const int o = s_off[i];
-    sa = __fadd_rn(sa, ca[o]);
-    sb = __fadd_rn(sb, cb[o]);
-  }
-  const float ma = __fdiv_rn(sa, (float)K), mb = __fdiv_rn(sb, (float)K);
-  float va = 0.0f, aa = 0.0f, ra = 0.0f, xa = 0.0f;
-  float vb = 0.0f, ab = 0.0f, rb2 = 0.0f, xb = 0.0f;
-  for (int i = 0; i < K; i++) {
-    const int o = s_off[i];
-    const float ref = s_ref[i];
-    const float pxa = ca[o], pxb = cb[o];
-    const float da = __fsub_rn(pxa, ma), db = __fsub_rn(pxb, mb);
-    va = __fadd_rn(va, __fmul_rn(da, da));
-    vb = __fadd_rn(vb, __fmul_rn(db, db));
-    if (metric == kNrmse) {
-      const float ta = __fsub_rn(ref, da), tb = __fsub_rn(ref, db);
-      aa = __fadd_rn(aa, __fmul_rn(ta, ta));
-      ab = __fadd_rn(ab, __fmul_rn(tb, tb));
-    } else if (metric == kCosine) {
-      aa = __fadd_rn(aa, __fmul_rn(ref, pxa));
-      ab = __fadd_rn(ab, __fmul_rn(ref, pxb));
-      ra = __fadd_rn(ra, __fmul_rn(ref, ref));
-      rb2 = __fadd_rn(rb2, __fmul_rn(ref, ref));
-      xa = __fadd_rn(xa, __fmul_rn(pxa, pxa));
-      xb = __fadd_rn(xb, __fmul_rn(pxb, pxb));
+  const bool wide = PX == 4 && (W & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 &&
+                    (reinterpret_cast<uintptr_t>(stds) & 15) == 0;
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int py = y + h * kThreadsY;
+    if (x >= W || py >= H) continue;
+    const size_t o = (size_t)py * W + x;
+    if (PX == 4 && wide) {
+      *reinterpret_cast<float4*>(out + o) = make_float4(val[0][h], val[1 % PX][h], val[2 % PX][h], val[3 % PX][h]);
+      if (stds)
+        *reinterpret_cast<float4*>(stds + o) = make_float4(sd[0][h], sd[1 % PX][h], sd[2 % PX][h], sd[3 % PX][h]);
     } else {
-      aa = __fadd_rn(aa, __fmul_rn(ref, da));
-      ab = __fadd_rn(ab, __fmul_rn(ref, db));
+#pragma unroll
+      for (int q = 0; q < PX; q++)
+        if (x + q < W) {
+          out[o + q] = val[q][h];
+          if (stds) stds[o + q] = sd[q][h];
+        }
     }
   }
-  float sd;
-  const float r_a = block_metric_value(metric, K, ma, va, aa, ra, xa, rb.mean, rb.std, &sd);
-  out[pa] = in_a ? r_a : 0.0f;
-  if (stds_out) stds_out[(size_t)f * W * H + pa] = in_a ? sd : 0.0f;
-  if (has_b) {
-    const float r_b = block_metric_value(metric, K, mb, vb, ab, rb2, xb, rb.mean, rb.std, &sd);
-    out[pb] = in_b ? r_b : 0.0f;
-    if (stds_out) stds_out[(size_t)f * W * H + pb] = in_b ? sd : 0.0f;
+  if (mm) cta_minmax(lo, hi, mm + 2 * blockIdx.z);
+}
+
+template <int MODE, int PX>
+cudaError_t launch_mode(const float* img, int w, int h, int frames, const BlockRows& e, const RefBlock& rb, int metric,
+                        float* out, float* stds, unsigned* mm, cudaStream_t st) {
+  const size_t smem = Tile<PX>::smem(e.rw, e.rh, e.k);
+  if (smem > 48 * 1024) {
+    const cudaError_t err =
+        cudaFuncSetAttribute(k_block_map<MODE, PX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return err;
+  }
+  const dim3 grid((w + Tile<PX>::kX - 1) / Tile<PX>::kX, (h + kTileY - 1) / kTileY, frames);
+  k_block_map<MODE, PX><<<grid, 32 * kThreadsY, smem, st>>>(img, w, h, e, rb, metric, kNegZero2, out, stds, mm);
+  return cudaGetLastError();
+}
+
+template <int PX>
+cudaError_t launch_px(const float* img, int w, int h, int frames, const BlockRows& e, const RefBlock& rb, int metric,
+                      float* out, float* stds, unsigned* mm, cudaStream_t st) {
+  switch (metric) {
+    case kNrmse: return launch_mode<kNrmse, PX>(img, w, h, frames, e, rb, metric, out, stds, mm, st);
+    case kCosine: return launch_mode<kCosine, PX>(img, w, h, frames, e, rb, metric, out, stds, mm, st);
+    case kAbsDiff: return launch_mode<kAbsDiff, PX>(img, w, h, frames, e, rb, metric, out, stds, mm, st);
+    default: return launch_mode<kPearson, PX>(img, w, h, frames, e, rb, metric, out, stds, mm, st);
   }
 }
 
-size_t block_map_smem(const Ellipse& e) {
-  return sizeof(float) * (size_t)(kTileX + 2 * e.rw) * (kTileY + 2 * e.rh) + (sizeof(int) + sizeof(float)) * (size_t)e.k;
-}
+}  // namespace
 
-void block_map_launch_shape(int w, int h, int frames, dim3* grid, dim3* block) {
-  *grid = dim3((w + kTileX - 1) / kTileX, (h + kTileY - 1) / kTileY, frames);
-  *block = dim3(kTileX, kThreadsY);
+cudaError_t launch_block_map(const float* img, int w, int h, int frames, const Ellipse& e, const RefBlock& rb,
+                             int metric, float* out, float* stds, unsigned* mm, int num_sms, cudaStream_t st) {
+  BlockRows rows;
+  rows.k = e.k;
+  rows.rw = e.rw;
+  rows.rh = e.rh;
+  for (int i = 0; i < e.k; i++) rows.hw[e.dy[i] + e.rh] = e.dx[i];  // the last column of a row stays
+  // Four pixel columns a thread where that still gives 1.5 CTAs an SM and the
+  // 128-column tiles pad the width to no more than 1.5 times what 32-column tiles do;
+  // else one. At 1024x1024 15x15 four take 80 us where one takes 94 (700x700: 55 and
+  // 61), at 400x300 15x15 (76 CTAs against 247) 44 and 40, at 513x512 9x9 40 and 37.
+  const int tiles = (w + Tile<4>::kX - 1) / Tile<4>::kX, ys = (h + kTileY - 1) / kTileY;
+  const bool four = (long long)tiles * ys * frames * 2 >= 3LL * num_sms &&
+                    2 * tiles * Tile<4>::kX <= 3 * ((w + 31) / 32 * 32);
+  if (four) return launch_px<4>(img, w, h, frames, rows, rb, metric, out, stds, mm, st);
+  return launch_px<1>(img, w, h, frames, rows, rb, metric, out, stds, mm, st);
 }
 
 __global__ void k_init_minmax(unsigned* mm, int planes) {
@@ -145,53 +343,104 @@ __global__ void k_init_minmax(unsigned* mm, int planes) {
   }
 }
 
-__device__ __forceinline__ float ord_to_float(unsigned u) {
-  return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
+namespace {
+
+struct PlaneArgs {
+  float* a;
+  const float* mask;  // null: the whole interior
+  int W, H, rw, rh;
+  const unsigned* mm_in;
+  unsigned* mm_out;  // the range of the results, or null
+};
+
+// One pass over the interior (where mask > 0): see PlanePass. VEC floats a load;
+// the thread's column and row advance with its index, without divisions.
+template <int OP, int VEC>
+__global__ void __launch_bounds__(256) k_plane_pass(const PlaneArgs g) {
+  const size_t n = (size_t)g.W * g.H, step = (size_t)gridDim.x * 256 * VEC;
+  float* a = g.a + n * blockIdx.y;
+  const float* mask = g.mask ? g.mask + n * blockIdx.y : nullptr;
+  float mn = 0.0f, d = 1.0f;
+  bool remap = false;
+  if (OP != kPassRange && OP != kPassInvert) {
+    const unsigned k0 = g.mm_in[2 * blockIdx.y], k1 = g.mm_in[2 * blockIdx.y + 1];
+    remap = k1 != 0u || OP == kPassAbsDiff;  // nothing selected: the reference remaps nothing either
+    mn = ord_float(k0);
+    float mx = ord_float(k1);
+    if (OP == kPassAbsDiff) mx = fmaxf(mx, 1.4e-45f);
+    d = __fadd_rn(__fsub_rn(mx, mn), kEps);
+  }
+  size_t p = ((size_t)blockIdx.x * 256 + threadIdx.x) * VEC;
+  int x = (int)(p % g.W), y = (int)(p / g.W);
+  const int sx = (int)(step % g.W), sy = (int)(step / g.W);
+  unsigned lo = 0xffffffffu, hi = 0u;
+  for (; p < n; p += step) {
+    float v[VEC], m[VEC];
+    if (VEC == 4) {
+      const float4 t = *reinterpret_cast<const float4*>(a + p);
+      v[0] = t.x, v[1 % VEC] = t.y, v[2 % VEC] = t.z, v[3 % VEC] = t.w;
+      if (mask) {
+        const float4 u = *reinterpret_cast<const float4*>(mask + p);
+        m[0] = u.x, m[1 % VEC] = u.y, m[2 % VEC] = u.z, m[3 % VEC] = u.w;
+      }
+    } else {
+      v[0] = a[p];
+      if (mask) m[0] = mask[p];
+    }
+    int xx = x, yy = y;
+    bool any = false;
+#pragma unroll
+    for (int q = 0; q < VEC; q++) {
+      if (xx >= g.rw && xx < g.W - g.rw && yy >= g.rh && yy < g.H - g.rh && (!mask || m[q] > 0.0f)) {
+        if (remap) v[q] = __fdiv_rn(__fsub_rn(v[q], mn), d);
+        if (OP == kPassAbsDiff) v[q] = __fsub_rn(1.0f, v[q]);
+        if (OP == kPassInvert || OP == kPassRemapInvert) v[q] = (v[q] == 0.0f) ? 1.0f : __fdiv_rn(1.0f, v[q]);
+        lo = min(lo, ord_bits(v[q]));
+        hi = max(hi, ord_bits(v[q]));
+        any = true;
+      }
+      if (++xx == g.W) xx = 0, yy++;
+    }
+    if (OP != kPassRange && any) {
+      if (VEC == 4) *reinterpret_cast<float4*>(a + p) = make_float4(v[0], v[1 % VEC], v[2 % VEC], v[3 % VEC]);
+      else a[p] = v[0];
+    }
+    x += sx;
+    y += sy;
+    if (x >= g.W) x -= g.W, y++;
+  }
+  if (g.mm_out) cta_minmax(lo, hi, g.mm_out + 2 * blockIdx.y);
 }
 
-// Abs-diff post-processing, java/CLUtils.java:936-960: min-max over the
-// interior with the maximum starting at Float.MIN_VALUE, then 1 - x.
-__global__ void k_block_absdiff_post(float* __restrict__ a_all, int W, int H, int rw, int rh, size_t plane,
-                                     const unsigned* __restrict__ mm_all) {
-  float* a = a_all + plane * blockIdx.y;
-  const unsigned* mm = mm_all + 2 * blockIdx.y;
-  const float mn = ord_to_float(mm[0]);
-  const float mx = fmaxf(ord_to_float(mm[1]), 1.4e-45f);
-  const float d = __fadd_rn(__fsub_rn(mx, mn), kEps);
-  for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < (size_t)W * H;
-       p += (size_t)gridDim.x * blockDim.x) {
-    const int x = (int)(p % W), y = (int)(p / W);
-    if (x < rw || x >= W - rw || y < rh || y >= H - rh) continue;
-    a[p] = __fsub_rn(1.0f, __fdiv_rn(__fsub_rn(a[p], mn), d));
+template <int VEC>
+void launch_pass(PlanePass op, const PlaneArgs& g, dim3 grid, cudaStream_t st) {
+  switch (op) {
+    case kPassRange: k_plane_pass<kPassRange, VEC><<<grid, 256, 0, st>>>(g); break;
+    case kPassRemap: k_plane_pass<kPassRemap, VEC><<<grid, 256, 0, st>>>(g); break;
+    case kPassRemapInvert: k_plane_pass<kPassRemapInvert, VEC><<<grid, 256, 0, st>>>(g); break;
+    case kPassInvert: k_plane_pass<kPassInvert, VEC><<<grid, 256, 0, st>>>(g); break;
+    case kPassAbsDiff: k_plane_pass<kPassAbsDiff, VEC><<<grid, 256, 0, st>>>(g); break;
   }
 }
 
-// NRMSE with relevance constant 0: the interior is the mask (java/CLUtils.java:788-797).
-__global__ void k_interior_mask(float* __restrict__ mask_all, int W, int H, int rw, int rh, size_t plane) {
-  float* mask = mask_all + plane * blockIdx.y;
-  for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < (size_t)W * H;
-       p += (size_t)gridDim.x * blockDim.x) {
-    const int x = (int)(p % W), y = (int)(p / W);
-    mask[p] = (x < rw || x >= W - rw || y < rh || y >= H - rh) ? 0.0f : 1.0f;
-  }
+}  // namespace
+
+void launch_plane_pass(PlanePass op, float* a, const float* mask, int w, int h, int rw, int rh, int planes,
+                       const unsigned* mm_in, unsigned* mm_out, int num_sms, cudaStream_t st) {
+  const PlaneArgs g{a, mask, w, h, rw, rh, mm_in, mm_out};
+  const size_t n = (size_t)w * h;
+  // float4 where every plane and quad is aligned
+  const bool vec = n % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(mask)) & 15) == 0;
+  const size_t per = 256 * (vec ? 4 : 1), want = (n + per - 1) / per;
+  const size_t cap = std::max<size_t>(1, (size_t)16 * num_sms / planes);
+  const dim3 grid((unsigned)std::min(want, cap), planes);
+  if (vec) launch_pass<4>(op, g, grid, st);
+  else launch_pass<1>(op, g, grid, st);
 }
 
 __global__ void k_apply_mask(float* __restrict__ a, const float* __restrict__ mask, size_t n) {
   for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x)
     a[p] = __fmul_rn(a[p], mask[p]);
-}
-
-// NRMSE inversion on mask > 0, java/CLUtils.java:809-821.
-__global__ void k_invert_masked(float* __restrict__ a_all, const float* __restrict__ mask_all, int W, int H,
-                                int rw, int rh, size_t plane) {
-  float* a = a_all + plane * blockIdx.y;
-  const float* mask = mask_all + plane * blockIdx.y;
-  for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < (size_t)W * H;
-       p += (size_t)gridDim.x * blockDim.x) {
-    const int x = (int)(p % W), y = (int)(p / W);
-    if (x < rw || x >= W - rw || y < rh || y >= H - rh) continue;
-    if (mask[p] > 0.0f) a[p] = (a[p] == 0.0f) ? 1.0f : __fdiv_rn(1.0f, a[p]);
-  }
 }
 
 }  // namespace sred

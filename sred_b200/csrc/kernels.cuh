@@ -28,25 +28,29 @@ __global__ void k_finalize(const int* slot, int W, int H, int rw, int rh, const 
                            const BlockParams* params, const double* sums, int n_flat, int metric, double sk,
                            double n_pixels, const float* mask, int apply_mask, float* out);
 __global__ void k_pack_vectors(const float* u, int n, int K, float* U, int kp, __half* S);
-__global__ void k_minmax(const float* a, const float* mask, int W, int H, int bw_, int bh_, size_t plane,
-                         unsigned* mm);
-__global__ void k_remap(float* a, const float* mask, int W, int H, int bw_, int bh_, size_t plane,
-                        const unsigned* mm);
-// Per-plane min/max words before k_minmax: {ordered +inf, ordered -inf} per plane
+// Per-plane min/max words before a range is taken: {ordered +inf, ordered -inf} per plane
 // (a kernel rather than a copy from pageable host memory, which would wait
 // for the stream to drain).
 __global__ void k_init_minmax(unsigned* mm, int planes);
 
 // block_map.cu
-__global__ void k_block_map(const float* img, int W, int H, int frames, Ellipse e, RefBlock rb, int metric,
-                            float* out, float* stds_out);
-// Dynamic shared memory and launch shape of k_block_map.
-size_t block_map_smem(const Ellipse& e);
-void block_map_launch_shape(int w, int h, int frames, dim3* grid, dim3* block);
-__global__ void k_block_absdiff_post(float* a, int W, int H, int rw, int rh, size_t plane, const unsigned* mm);
-__global__ void k_interior_mask(float* mask, int W, int H, int rw, int rh, size_t plane);
+// The map of a reference block (all metrics of block_metric_value), the local stds
+// (stds, or null) and the range of the interior (mm, or null: 2 words per frame).
+cudaError_t launch_block_map(const float* img, int w, int h, int frames, const Ellipse& e, const RefBlock& rb,
+                             int metric, float* out, float* stds, unsigned* mm, int num_sms, cudaStream_t st);
+// One pass over the interior of every plane (where mask > 0, if there is one), with
+// the range mm_in of its values; mm_out (or null) receives the range of the results.
+// Normalisation (java/Utils.java:985-1031) is kPassRange and kPassRemap.
+enum PlanePass {
+  kPassRange,        // the range alone
+  kPassRemap,        // (v - min) / (max - min + eps) in FP32
+  kPassRemapInvert,  // remap, then the NRMSE inversion (java/CLUtils.java:809-821)
+  kPassInvert,       // the inversion alone
+  kPassAbsDiff       // 1 - remap, the maximum starting at Float.MIN_VALUE (java/CLUtils.java:936-960)
+};
+void launch_plane_pass(PlanePass op, float* a, const float* mask, int w, int h, int rw, int rh, int planes,
+                       const unsigned* mm_in, unsigned* mm_out, int num_sms, cudaStream_t st);
 __global__ void k_apply_mask(float* a, const float* mask, size_t n);
-__global__ void k_invert_masked(float* a, const float* mask, int W, int H, int rw, int rh, size_t plane);
 
 // gat.cu
 __global__ void k_gat(float* img, size_t n, double gain, double c);

@@ -398,57 +398,4 @@ __global__ void k_finalize(const int* __restrict__ slot, int W, int H, int rw, i
   out[p] = o;
 }
 
-// ---------------------------------------------------------------------------
-// Normalisation, java/Utils.java:985-1031: min/max over mask > 0 on the
-// interior (or the whole interior when mask is NULL), then
-// (v - min) / (max - min + eps) in FP32.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned ord_bits(float f) {
-  unsigned u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float ord_float(unsigned u) {
-  return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
-}
-
-__global__ void k_minmax(const float* __restrict__ a, const float* __restrict__ mask, int W, int H,
-                         int bw_, int bh_, size_t plane, unsigned* __restrict__ mm) {
-  const float* img = a + plane * blockIdx.y;
-  const float* msk = mask ? mask + plane * blockIdx.y : nullptr;
-  unsigned* m = mm + 2 * blockIdx.y;
-  unsigned lo = 0xffffffffu, hi = 0u;
-  size_t n = (size_t)W * H;
-  for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-    int x = (int)(p % W), y = (int)(p / W);
-    if (x < bw_ || x >= W - bw_ || y < bh_ || y >= H - bh_) continue;
-    if (msk && !(msk[p] > 0.0f)) continue;
-    unsigned b = ord_bits(img[p]);
-    lo = min(lo, b);
-    hi = max(hi, b);
-  }
-  lo = __reduce_min_sync(0xffffffffu, lo);
-  hi = __reduce_max_sync(0xffffffffu, hi);
-  if ((threadIdx.x & 31) == 0) {
-    atomicMin(m, lo);
-    atomicMax(m + 1, hi);
-  }
-}
-
-__global__ void k_remap(float* __restrict__ a, const float* __restrict__ mask, int W, int H, int bw_,
-                        int bh_, size_t plane, const unsigned* __restrict__ mm) {
-  float* img = a + plane * blockIdx.y;
-  const float* msk = mask ? mask + plane * blockIdx.y : nullptr;
-  const unsigned* m = mm + 2 * blockIdx.y;
-  if (m[1] == 0u) return;  // nothing selected: the reference remaps nothing either
-  float mn = ord_float(m[0]), mx = ord_float(m[1]);
-  float d = __fadd_rn(__fsub_rn(mx, mn), kEps);
-  size_t n = (size_t)W * H;
-  for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-    int x = (int)(p % W), y = (int)(p / W);
-    if (x < bw_ || x >= W - bw_ || y < bh_ || y >= H - bh_) continue;
-    if (msk && !(msk[p] > 0.0f)) continue;
-    img[p] = __fdiv_rn(__fsub_rn(img[p], mn), d);
-  }
-}
-
 }  // namespace sred

@@ -5,9 +5,8 @@
 // must not touch the allocator once started. For them this entry point
 // computes the same block map as sred_block_map_2d_device without allocating
 // anything: the little device scratch it needs (the per-frame min/max words
-// of the normalisation and, for NRMSE, the interior mask) lives in one
-// file-scope __device__ array of fixed size that every GPU loading this
-// library holds until exit. The call synchronises its stream before it
+// of the host steps) lives in one file-scope __device__ array of fixed size
+// that every GPU loading this library holds until exit. The call synchronises its stream before it
 // returns; the caller's buffers are complete then.
 //
 // Host code must not use the array's name as a device address (there it is
@@ -26,9 +25,10 @@
 
 namespace {
 
-constexpr size_t kNoAllocMaskFloats = 1u << 20;  // NRMSE interior mask: frames * w * h <= 1,048,576
-constexpr int kNoAllocMaxFrames = 4096;          // normalisation min/max words: 2 per frame
-constexpr size_t kNoAllocScratchBytes = kNoAllocMaskFloats * sizeof(float) + 2 * kNoAllocMaxFrames * sizeof(unsigned);
+constexpr size_t kNoAllocNrmseFloats = 1u << 20;  // NRMSE: frames * w * h <= 1,048,576
+constexpr int kNoAllocMaxFrames = 4096;           // min/max words: two ranges of 2 per frame
+constexpr size_t kNoAllocTileBytes = 48 * 1024;   // FP32 tile of 32 x 16 pixels with halo, and 8 bytes per element
+constexpr size_t kNoAllocScratchBytes = 4 * kNoAllocMaxFrames * sizeof(unsigned);
 constexpr int kMaxDevices = 64;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
@@ -87,19 +87,19 @@ extern "C" sred_status sred_block_map_2d_device_noalloc(const char* metric, cons
   Ellipse e;
   if (build_ellipse(bw, bh, &e) != block_size || block_size < 2 || block_size > kMaxK) return SRED_ERR_ARG;
   const size_t plane = (size_t)w * h, n = plane * frames;
-  // Sizes beyond the fixed scratch are refused, not truncated.
+  // Sizes beyond the documented limits are refused, not truncated.
   if (frames > kNoAllocMaxFrames) return SRED_ERR_ARG;
-  if (m == kNrmse && n > kNoAllocMaskFloats) return SRED_ERR_ARG;
-  const size_t tile_smem = block_map_smem(e);
-  if (tile_smem > 48 * 1024) return SRED_ERR_ARG;
+  if (m == kNrmse && n > kNoAllocNrmseFloats) return SRED_ERR_ARG;
+  if (sizeof(float) * (size_t)(32 + 2 * e.rw) * (16 + 2 * e.rh) + 8 * (size_t)e.k > kNoAllocTileBytes)
+    return SRED_ERR_ARG;
 
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return SRED_ERR_NODEV;
   unsigned char* scratch = nullptr;
   sred_status st = scratch_address(dev, &scratch);
   if (st != SRED_OK) return st;
-  float* d_mask = reinterpret_cast<float*>(scratch);
-  unsigned* d_mm = reinterpret_cast<unsigned*>(scratch + kNoAllocMaskFloats * sizeof(float));
+  unsigned* mm = reinterpret_cast<unsigned*>(scratch);
+  unsigned* mm2 = mm + 2 * frames;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -126,38 +126,21 @@ extern "C" sred_status sred_block_map_2d_device_noalloc(const char* metric, cons
     phase_reference_dft(ref_pixels, ref_std, bw, bh, &pr);
     launch_block_phase(d_img, w, h, frames, e, bw, bh, pr, d_out, nullptr, s);
   } else {
-    dim3 grid, blk;
-    block_map_launch_shape(w, h, frames, &grid, &blk);
-    k_block_map<<<grid, blk, tile_smem, s>>>(d_img, w, h, frames, e, rb, m, d_out, nullptr);
+    k_init_minmax<<<grid_of((size_t)2 * frames, 256, 64), 256, 0, s>>>(mm, 2 * frames);
+    if (launch_block_map(d_img, w, h, frames, e, rb, m, d_out, nullptr, mm, sms, s) != cudaSuccess)
+      return SRED_ERR_LAUNCH;
   }
-  const dim3 pg(grid_of(plane, 256, 4 * sms), frames);
-  const int ig = grid_of((size_t)frames, 256, 64);
-  // The relevance constant is 0 here: the mask is the interior for NRMSE
-  // (java/CLUtils.java:788-797) and absent otherwise.
-  if (m == kNrmse) {
-    k_interior_mask<<<pg, 256, 0, s>>>(d_mask, w, h, rw, rh, plane);
-    k_apply_mask<<<grid_of(n, 256, 8 * sms), 256, 0, s>>>(d_out, d_mask, n);
-    k_init_minmax<<<ig, 256, 0, s>>>(d_mm, frames);
-    k_minmax<<<pg, 256, 0, s>>>(d_out, d_mask, w, h, rw, rh, plane, d_mm);
-    k_remap<<<pg, 256, 0, s>>>(d_out, d_mask, w, h, rw, rh, plane, d_mm);
-    k_invert_masked<<<pg, 256, 0, s>>>(d_out, d_mask, w, h, rw, rh, plane);
-    if (normalize_output) {
-      k_init_minmax<<<ig, 256, 0, s>>>(d_mm, frames);
-      k_minmax<<<pg, 256, 0, s>>>(d_out, d_mask, w, h, rw, rh, plane, d_mm);
-      k_remap<<<pg, 256, 0, s>>>(d_out, d_mask, w, h, rw, rh, plane, d_mm);
-    }
-  } else {
-    if (m == kAbsDiff) {
-      k_init_minmax<<<ig, 256, 0, s>>>(d_mm, frames);
-      k_minmax<<<pg, 256, 0, s>>>(d_out, nullptr, w, h, rw, rh, plane, d_mm);
-      k_block_absdiff_post<<<pg, 256, 0, s>>>(d_out, w, h, rw, rh, plane, d_mm);
-    }
-    if (normalize_output) {
-      k_init_minmax<<<ig, 256, 0, s>>>(d_mm, frames);
-      k_minmax<<<pg, 256, 0, s>>>(d_out, nullptr, w, h, rw, rh, plane, d_mm);
-      k_remap<<<pg, 256, 0, s>>>(d_out, nullptr, w, h, rw, rh, plane, d_mm);
-    }
+  // The relevance constant is 0 here: no mask but the interior.
+  const bool shape = m == kHu || m == kHu7 || m == kPhase;
+  if (m == kNrmse || m == kAbsDiff) {
+    launch_plane_pass(m == kNrmse ? kPassRemapInvert : kPassAbsDiff, d_out, nullptr, w, h, rw, rh, frames, mm,
+                      normalize_output ? mm2 : nullptr, sms, s);
+    mm = mm2;
+  } else if (shape && normalize_output) {
+    k_init_minmax<<<grid_of((size_t)frames, 256, 64), 256, 0, s>>>(mm, frames);
+    launch_plane_pass(kPassRange, d_out, nullptr, w, h, rw, rh, frames, nullptr, mm, sms, s);
   }
+  if (normalize_output) launch_plane_pass(kPassRemap, d_out, nullptr, w, h, rw, rh, frames, mm, nullptr, sms, s);
   if (cudaGetLastError() != cudaSuccess) return SRED_ERR_LAUNCH;
   if (cudaStreamSynchronize(s) != cudaSuccess) return SRED_ERR_LAUNCH;
   return SRED_OK;

@@ -238,9 +238,8 @@ sred_status normalize_dev(sred_ctx* c, float* d_a, const float* d_mask, int w, i
   unsigned* mm;
   CKS(ensure(c, B_MM, 2 * planes, &mm));
   k_init_minmax<<<grid_for((size_t)planes, 256, 64), 256, 0, st>>>(mm, planes);
-  dim3 g(grid_for((size_t)w * h, 256, 4 * c->num_sms), planes);
-  k_minmax<<<g, 256, 0, st>>>(d_a, d_mask, w, h, rw, rh, (size_t)w * h, mm);
-  k_remap<<<g, 256, 0, st>>>(d_a, d_mask, w, h, rw, rh, (size_t)w * h, mm);
+  launch_plane_pass(kPassRange, d_a, d_mask, w, h, rw, rh, planes, nullptr, mm, c->num_sms, st);
+  launch_plane_pass(kPassRemap, d_a, d_mask, w, h, rw, rh, planes, mm, nullptr, c->num_sms, st);
   CK(cudaGetLastError());
   return SRED_OK;
 }
@@ -634,24 +633,24 @@ sred_status block_core(sred_ctx* c, int metric, const float* d_img, int w, int h
   rb.mean = ref_mean;
   rb.std = ref_std;
   std::memcpy(rb.px, ref_pixels, sizeof(float) * e.k);
-  const bool need_mask = (metric == kNrmse) || relc > 0.0f;
   float* d_stds = nullptr;
-  if (need_mask) CKS(ensure(c, B_STDS2, n, &d_stds));
+  if (relc > 0.0f) CKS(ensure(c, B_STDS2, n, &d_stds));
+  // Ranges of the map (by its own kernel) and of the first host step's results.
+  unsigned *mm, *ranged = nullptr;
+  CKS(ensure(c, B_MM, (size_t)4 * frames, &mm));
+  unsigned* mm2 = mm + 2 * frames;
   if (metric == kHu || metric == kHu7 || metric == kPhase) {
     CKS(block_shape_launch(c, metric, d_img, w, h, frames, e, ref_pixels, bw, bh, ref_std, d_out, d_stds, st));
   } else {
-    dim3 grid, blk;
-    block_map_launch_shape(w, h, frames, &grid, &blk);
-    const size_t smem = block_map_smem(e);
-    if (smem > 200 * 1024) return fail(c, SRED_ERR_ARG, "block too large for the streaming tile");
-    if (smem > 48 * 1024)
-      CK(cudaFuncSetAttribute(k_block_map, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_block_map<<<grid, blk, smem, st>>>(d_img, w, h, frames, e, rb, metric, d_out, d_stds);
+    if (metric == kNrmse || metric == kAbsDiff || normalize) {
+      k_init_minmax<<<grid_for((size_t)2 * frames, 256, 64), 256, 0, st>>>(mm, 2 * frames);
+      ranged = mm;
+    }
+    CK(launch_block_map(d_img, w, h, frames, e, rb, metric, d_out, d_stds, ranged, c->num_sms, st));
   }
   CK(cudaGetLastError());
 
   float* d_mask = nullptr;
-  const dim3 pg(grid_for(plane, 256, 4 * c->num_sms), frames);
   auto relevance_masks = [&]() -> sred_status {
     float* d_m;
     uint8_t* d_flags;
@@ -670,31 +669,33 @@ sred_status block_core(sred_ctx* c, int metric, const float* d_img, int w, int h
     return SRED_OK;
   };
 
-  if (metric == kNrmse) {
-    if (relc == 0.0f) {
-      CKS(ensure(c, B_MASK, n, &d_mask));
-      k_interior_mask<<<pg, 256, 0, st>>>(d_mask, w, h, rw, rh, plane);
-    } else {
-      CKS(relevance_masks());
-    }
-    k_apply_mask<<<grid_for(n, 256, 8 * c->num_sms), 256, 0, st>>>(d_out, d_mask, n);
-    CKS(normalize_dev(c, d_out, d_mask, w, h, rw, rh, frames, st));
-    k_invert_masked<<<pg, 256, 0, st>>>(d_out, d_mask, w, h, rw, rh, plane);
-    if (normalize) CKS(normalize_dev(c, d_out, d_mask, w, h, rw, rh, frames, st));
-  } else {
-    if (metric == kAbsDiff) {
-      unsigned* mm;
-      CKS(ensure(c, B_MM, 2 * frames, &mm));
-      k_init_minmax<<<grid_for((size_t)frames, 256, 64), 256, 0, st>>>(mm, frames);
-      k_minmax<<<pg, 256, 0, st>>>(d_out, nullptr, w, h, rw, rh, plane, mm);
-      k_block_absdiff_post<<<pg, 256, 0, st>>>(d_out, w, h, rw, rh, plane, mm);
-    }
-    if (relc > 0.0f) {
-      CKS(relevance_masks());
-      k_apply_mask<<<grid_for(n, 256, 8 * c->num_sms), 256, 0, st>>>(d_out, d_mask, n);
-    }
-    if (normalize) CKS(normalize_dev(c, d_out, d_mask, w, h, rw, rh, frames, st));
+  auto pass = [&](PlanePass op, const unsigned* in, unsigned* out) {
+    launch_plane_pass(op, d_out, d_mask, w, h, rw, rh, frames, in, out, c->num_sms, st);
+  };
+  if (metric == kAbsDiff) {
+    // (relevance masks come after the transform)
+    pass(kPassAbsDiff, mm, relc > 0.0f ? nullptr : mm2);
+    ranged = mm2;
   }
+  if (relc > 0.0f) {
+    CKS(relevance_masks());
+    k_apply_mask<<<grid_for(n, 256, 8 * c->num_sms), 256, 0, st>>>(d_out, d_mask, n);
+    if (metric == kNrmse || normalize) {
+      k_init_minmax<<<grid_for((size_t)2 * frames, 256, 64), 256, 0, st>>>(mm, 2 * frames);
+      pass(kPassRange, nullptr, mm);
+      ranged = mm;
+    }
+  } else if (!ranged && normalize) {  // shape metrics
+    k_init_minmax<<<grid_for((size_t)frames, 256, 64), 256, 0, st>>>(mm, frames);
+    pass(kPassRange, nullptr, mm);
+    ranged = mm;
+  }
+  if (metric == kNrmse) {
+    // the mask is the interior without a relevance constant (java/CLUtils.java:788-797)
+    pass(kPassRemapInvert, mm, normalize ? mm2 : nullptr);
+    ranged = mm2;
+  }
+  if (normalize) pass(kPassRemap, ranged, nullptr);
   CK(cudaGetLastError());
   return SRED_OK;  // enqueued on st; the callers decide when to wait
 }
