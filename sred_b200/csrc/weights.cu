@@ -15,10 +15,13 @@
 // nodes of a block follow from two multiplications,
 //   2^-(x + h - a)^2 = 2^-(x - a)^2 * r,  r = 2^-(2 (x - a) h + h^2),  r' = r 2^(-2 h^2),
 // and one FP64 atomic add per node and CTA. Nodes further than 14 from every
-// block of the slice (terms below 2^-169) are skipped.
+// block of the slice (terms below 2^-169) are skipped. Few slices share their nodes
+// out among several CTAs each: 6.5 us instead of 26 for 9,810 blocks.
 // k_den_eval: one thread per block. Where the range of a does not fit the node
 // table (2,046 at h = 1/8) or is not finite, the same kernel sums the pair terms
 // directly (FP32 terms, FP64 sums of 256), slice by slice within that distance.
+#include <algorithm>
+
 #include "epilogue.cuh"
 #include "weights.cuh"
 
@@ -29,6 +32,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kPer = kDenSlice / kThreads;
 constexpr int kGroup = 8;          // nodes per step
+constexpr int kDenCtas = 148;      // CTAs that few slices are spread over
 
 __global__ void __launch_bounds__(kThreads) k_den_nodes(const BlockParams* __restrict__ params, int n,
                                                         const unsigned* __restrict__ arange,
@@ -66,14 +70,14 @@ __global__ void __launch_bounds__(kThreads) k_den_nodes(const BlockParams* __res
     hi = fmaxf(hi, wr[k].y);
   }
   if (bad) lo = hi = nanf("");
-  if (threadIdx.x == 0) slices[blockIdx.x] = make_float2(lo, hi);
+  if (threadIdx.x == 0 && blockIdx.y == 0) slices[blockIdx.x] = make_float2(lo, hi);
   double x0;
   const int m = node_grid(arange, &x0);
   if (m == 0) return;
   const int g0 = max(0, (int)floor(((double)lo - kNodeFar - x0) / (kNodeH * kGroup)));
   const int g1 = min((m - 1) / kGroup, (int)floor(((double)hi + kNodeFar - x0) / (kNodeH * kGroup)));
   const double q = exp2(-2.0 * kNodeH * kNodeH);
-  for (int g = g0; g <= g1; g++) {
+  for (int g = g0 + blockIdx.y; g <= g1; g += gridDim.y) {
     const double xb = x0 + (double)(g * kGroup) * kNodeH;
     double acc[kGroup];
 #pragma unroll
@@ -172,7 +176,8 @@ cudaError_t launch_den(const BlockParams* params, int n, const unsigned* arange,
   const cudaError_t e = cudaMemsetAsync(nodes, 0, kDenNodes * sizeof(double), st);
   if (e != cudaSuccess) return e;
   const int ns = den_slices(n);
-  k_den_nodes<<<ns, kThreads, 0, st>>>(params, n, arange, nodes, slices);
+  const int parts = std::max(1, std::min(32, kDenCtas / ns));
+  k_den_nodes<<<dim3(ns, parts), kThreads, 0, st>>>(params, n, arange, nodes, slices);
   k_den_eval<<<(n + kThreads - 1) / kThreads, kThreads, 0, st>>>(params, n, arange, nodes, slices, ns, den);
   return cudaGetLastError();
 }
