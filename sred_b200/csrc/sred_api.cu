@@ -727,27 +727,23 @@ dim3 vol_grid(const Vol3& v) { return dim3((v.W + 31) / 32, (v.H + 3) / 4, v.D);
 // java/Utils.java:1463-1498 (getMeanNoiseVar3D): the mean of the local
 // variances over the interior, summed in FP32 in raster order with a float
 // count, as the reference does on the host.
-float noise_var_3d(const Vol3& v, const float* stds) {
-  float s = 0.0f, n = 0.0f;
-  for (int z = v.rd; z < v.D - v.rd; z++)
-    for (int y = v.rh; y < v.H - v.rh; y++)
-      for (int x = v.rw; x < v.W - v.rw; x++) {
-        const float sd = stds[((size_t)z * v.H + y) * v.W + x];
-        s += sd * sd;
-        n += 1.0f;
-      }
-  return s / n;
+sred_status noise_var_3d(sred_ctx* c, const Vol3& v, const float* d_stds, cudaStream_t st, float* out) {
+  float *d_sum, sum;
+  CKS(ensure(c, B_VARS, 1, &d_sum));
+  CK(launch_noise3d(d_stds, v, d_sum, st));
+  CK(cudaMemcpyAsync(&sum, d_sum, sizeof(float), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  const double n = (double)std::max(0, v.W - 2 * v.rw) * std::max(0, v.H - 2 * v.rh) * std::max(0, v.D - 2 * v.rd);
+  *out = sum / (float)std::min(n, 16777216.0);  // a float counting by ones stops there
+  return SRED_OK;
 }
 
-// Relevance mask of a volume from device local stds (the noise variance on
-// the host from a copy of them); map, if not null, is multiplied by the mask.
+// Relevance mask of a volume from device local stds; map, if not null, is
+// multiplied by the mask.
 sred_status mask_3d(sred_ctx* c, const Vol3& v, const float* d_stds, float relc, float* d_mask, float* d_map,
                     cudaStream_t st, float* noise_var) {
-  const size_t n = (size_t)v.W * v.H * v.D;
-  std::vector<float> h_stds(n);
-  CK(cudaMemcpyAsync(h_stds.data(), d_stds, n * sizeof(float), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  const float nv = noise_var_3d(v, h_stds.data());
+  float nv;
+  CKS(noise_var_3d(c, v, d_stds, st, &nv));
   k_mask3d<<<vol_grid(v), dim3(32, 4), 0, st>>>(d_stds, v, nv * relc, d_mask, d_map);
   CK(cudaGetLastError());
   if (noise_var) *noise_var = nv;
@@ -864,10 +860,8 @@ sred_status global3d_prepare(sred_ctx* c, int metric, const float* d_vol, int w,
   const dim3 grid = vol_grid(v), blk(32, 4);
   k_local_stats3d<<<grid, blk, sizeof(int) * K, st>>>(d_vol, v, d_off, d_means, d_stds);
   CK(cudaGetLastError());
-  std::vector<float> h_stds(n);
-  CK(cudaMemcpyAsync(h_stds.data(), d_stds, n * sizeof(float), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  const float nv = noise_var_3d(v, h_stds.data());
+  float nv;
+  CKS(noise_var_3d(c, v, d_stds, st, &nv));
   const bool has_interior = w > 2 * v.rw && h > 2 * v.rh && d > 2 * v.rd;
   if (has_interior && !std::isfinite(nv))
     return fail(c, SRED_ERR_INVALID_INPUT, "Input contains invalid (NaN or Infinite) values.");
