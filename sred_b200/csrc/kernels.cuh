@@ -22,8 +22,11 @@ __global__ void k_count(const uint8_t* flags, size_t n, int2* counts);
 __global__ void k_scan(int2* counts, int nseg);
 __global__ void k_scatter(const uint8_t* flags, size_t n, const int2* offs, int* gram_pix, int* flat_pix,
                           int* slot);
-__global__ void k_pack(const float* img, int W, Ellipse e, const int* gram_pix, int n, float wscale, float* U, int kp,
-                       __half* S, BlockParams* params, float* tile_rmax, double* sums, unsigned* arange);
+// The listed blocks' parameters and operands; off: the block's linear offsets (3D), or
+// null for e on an image W wide.
+cudaError_t launch_pack(const float* img, int W, const Ellipse& e, const int* off, int K, const int* gram_pix, int n,
+                        float wscale, float* U, int kp, __half* S, BlockParams* params, float* tile_rmax, double* sums,
+                        unsigned* arange, int num_sms, cudaStream_t st);
 __global__ void k_finalize(const int* slot, int W, int H, int rw, int rh, const double* num, const double* den,
                            const BlockParams* params, const double* sums, int n_flat, int metric, double sk,
                            double n_pixels, const float* mask, int apply_mask, float* out);

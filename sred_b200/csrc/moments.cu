@@ -7,6 +7,8 @@
 // they agree bit for bit with an IEEE-754 evaluation of the reference code.
 // Everything that feeds the all-pairs sums (block moments, unit vectors,
 // weights' arguments, the per-pixel division) is FP64.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -226,64 +228,95 @@ __global__ void k_scatter(const uint8_t* __restrict__ flags, size_t n, const int
 }
 
 // ---------------------------------------------------------------------------
-// Operand packing: each warp takes 32 consecutive gram blocks at a time (their
-// pixels overlap, so the passes hit L1). FP64 moments of the ellipse vector,
-// unit vector u = (x - mu) / |x - mu|, per-block epilogue params, and the
-// closed-form sums the flat blocks need:
+// Operand packing of the 2D and 3D maps. FP64 moments of the block's vector, unit
+// vector u = (x - mu) / |x - mu|, per-block epilogue params, and the closed-form sums
+// the flat blocks need (2D; sums may be null):
 //   sums[0] = sum_q 2^-(a_q)^2           (weight of a pair with a flat block)
 //   sums[1] = sum_q sqrt((K-1)/K) sigma_q (NRMSE against a flat block)
 //   sums[2] = sum_q sigma_q 2^-(a_q)^2     (Abs-diff against a flat block)
-// and the range of a (arange: launch_den, weights.cuh).
-// The block sums are warp-wide reductions, one block after another; the
-// per-block scalar work (square roots, quotients, exp2, params) then runs on
-// lane k for block k of the 32, instead of on one lane per block while the
-// other 31 wait. U: FP32 unit vectors (row pitch kp), S: the split FP16 operand
-// (store_split); either may be null. Rows [n, n_pad) are zero-filled by the host.
+// and the range of a (arange: launch_den, weights.cuh). U: FP32 unit vectors (row
+// pitch kp), S: the split FP16 operand (store_split); either may be null. Rows
+// [n, n_pad) are zero-filled by the host.
+//
+// A warp takes NB consecutive blocks at a time; a lane holds elements lane, lane + 32,
+// ... (R of them) of each in registers as FP64, so an image value is read and
+// converted once, its offset once per kernel. The NB sums are reduced together (NB / 2
+// + ... + 1 exchanges and the rest of the five steps, instead of five each) and leave
+// lane l with the scalars of block l % NB. Bound by conversions and FP64 issue; a map
+// of few blocks by latency, which many short groups spread over all SMs: 16,851 blocks
+// of 137 elements took 206 us with a warp per 32 blocks, three reads of the image and
+// a per-lane load of the kernel's parameters each, and 18 now; 53,600 of 33 (a
+// 256x256 map) about 100 us and 50.
 // ---------------------------------------------------------------------------
-__global__ void k_pack(const float* __restrict__ img, int W, Ellipse e, const int* __restrict__ gram_pix,
-                       int n, float wscale, float* __restrict__ U, int kp, __half* __restrict__ S,
-                       BlockParams* __restrict__ params, float* __restrict__ tile_rmax,
-                       double* __restrict__ sums, unsigned* __restrict__ arange) {
+template <int NB>
+__device__ __forceinline__ double reduce_blocks(double (&s)[NB], int lane) {
+  // step t: lane bit t keeps the odd or even half, so lane l ends with index l % NB
+#pragma unroll
+  for (int t = 0, m = NB; m > 1; t++, m >>= 1) {
+    const bool up = (lane >> t) & 1;
+#pragma unroll
+    for (int k = 0; k < m / 2; k++) {
+      const double keep = up ? s[2 * k + 1] : s[2 * k], send = up ? s[2 * k] : s[2 * k + 1];
+      s[k] = keep + __shfl_xor_sync(0xffffffffu, send, 1 << t);
+    }
+  }
+#pragma unroll
+  for (int o = NB; o < 32; o <<= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+  return s[0];
+}
+
+template <int NB, int R>
+__global__ void __launch_bounds__(256)
+    k_pack(const float* __restrict__ img, int W, const __grid_constant__ Ellipse e, const int* __restrict__ off, int K,
+           const int* __restrict__ gram_pix, int n, float wscale, float* __restrict__ U, int kp,
+           __half* __restrict__ S, BlockParams* __restrict__ params, float* __restrict__ tile_rmax,
+           double* __restrict__ sums, unsigned* __restrict__ arange) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
-  const int K = e.k;
   const SplitLayout lay = split_layout(K);
   const double sk = sqrt((double)(K - 1) / (double)K);
   const double rK = __drcp_rn((double)K);  // s / K as div_fixed: the correctly rounded quotient
+  int o[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const int i = lane + 32 * r;
+    o[r] = i >= K ? 0 : off ? off[i] : e.dy[i] * W + e.dx[i];
+  }
   double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
   unsigned a_lo = 0u, a_hi = 0u;  // ~bits of the smallest a, bits of the largest
-  for (long long j0 = 32LL * gw; j0 < n; j0 += 32LL * nw) {
-    const int nb = (int)min(32LL, (long long)n - j0);
-    // The sum and centred sum of squares of each block; lane k keeps block k's.
-    double my_s = 0.0, my_v = 0.0;
-    for (int k = 0; k < nb; k++) {
-      const int p = gram_pix[j0 + k];
-      const int x = p % W, y = p / W;
-      double s = 0.0;
-      for (int i = lane; i < K; i += 32) s += (double)img[(size_t)(y + e.dy[i]) * W + (x + e.dx[i])];
-      for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(full, s, o);
-      const double mu = div_fixed(s, (double)K, rK);
-      double v = 0.0;
-      for (int i = lane; i < K; i += 32) {
-        const double d = (double)img[(size_t)(y + e.dy[i]) * W + (x + e.dx[i])] - mu;
-        v += d * d;
-      }
-      for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(full, v, o);
-      if (lane == k) {
-        my_s = s;
-        my_v = v;
+  for (long long j0 = (long long)NB * gw; j0 < n; j0 += (long long)NB * nw) {
+    const int nb = (int)min((long long)NB, (long long)n - j0);
+    const int pix = gram_pix[j0 + min(lane % NB, nb - 1)];
+    double d[NB][R], s[NB];
+#pragma unroll
+    for (int k = 0; k < NB; k++) {
+      const float* c = img + __shfl_sync(full, pix, k);
+      s[k] = 0.0;
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        d[k][r] = lane + 32 * r < K ? (double)c[o[r]] : 0.0;
+        s[k] += d[k][r];
       }
     }
-    // Block j0 + lane's scalars.
-    double mu = 0.0, inv = 0.0;
+    const double mu = div_fixed(reduce_blocks<NB>(s, lane), (double)K, rK);
+#pragma unroll
+    for (int k = 0; k < NB; k++) {
+      const double m = __shfl_sync(full, mu, k);
+      s[k] = 0.0;
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        d[k][r] = lane + 32 * r < K ? d[k][r] - m : 0.0;
+        s[k] += d[k][r] * d[k][r];
+      }
+    }
+    const double v = reduce_blocks<NB>(s, lane);
+    const double nrm = sqrt(v);
+    const double inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
     if (lane < nb) {
       const long long j = j0 + lane;
-      mu = div_fixed(my_s, (double)K, rK);
-      const double nrm = sqrt(my_v);
-      inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
-      const double sigma = sqrt(my_v / (K - 1));
+      const double sigma = sqrt(v / (K - 1));
       BlockParams bp;
       bp.a = (float)(sigma * (double)wscale);
       bp.e = sigma > 0.0 ? (float)((double)kEps / sigma) : 0.0f;
@@ -295,22 +328,28 @@ __global__ void k_pack(const float* __restrict__ img, int W, Ellipse e, const in
       a_lo = max(a_lo, ~__float_as_uint(bp.a));
       a_hi = max(a_hi, __float_as_uint(bp.a));
       atomicMax(reinterpret_cast<int*>(tile_rmax) + (j >> 7), __float_as_int(bp.r));
-      const double a = sigma * (double)wscale;
-      const double w0 = exp2(-(a * a));
-      acc0 += w0;
-      acc1 += sk * sigma;
-      acc2 += sigma * w0;
+      if (sums) {
+        const double a = sigma * (double)wscale;
+        const double w0 = exp2(-(a * a));
+        acc0 += w0;
+        acc1 += sk * sigma;
+        acc2 += sigma * w0;
+      }
     }
-    // Unit vectors and operands, block by block.
-    for (int k = 0; k < nb; k++) {
+    if (!U && !S) continue;
+#pragma unroll
+    for (int k = 0; k < NB; k++) {
+      const double f = __shfl_sync(full, inv, k);
+      if (k >= nb) break;
       const long long j = j0 + k;
-      const double mu_k = __shfl_sync(full, mu, k), inv_k = __shfl_sync(full, inv, k);
-      const int p = gram_pix[j];
-      const int x = p % W, y = p / W;
-      for (int i = lane; i < K; i += 32) {
-        const double u = ((double)img[(size_t)(y + e.dy[i]) * W + (x + e.dx[i])] - mu_k) * inv_k;
-        if (U) U[(size_t)j * kp + i] = (float)u;
-        if (S) store_split(S + (size_t)j * lay.pitch, lay, i, u * (double)kSplitScale);
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const int i = lane + 32 * r;
+        if (i < K) {
+          const double u = d[k][r] * f;
+          if (U) U[(size_t)j * kp + i] = (float)u;
+          if (S) store_split(S + (size_t)j * lay.pitch, lay, i, u * (double)kSplitScale);
+        }
       }
       if (U)
         for (int i = K + lane; i < kp; i += 32) U[(size_t)j * kp + i] = 0.0f;
@@ -319,14 +358,15 @@ __global__ void k_pack(const float* __restrict__ img, int W, Ellipse e, const in
   }
   a_lo = __reduce_max_sync(full, a_lo);
   a_hi = __reduce_max_sync(full, a_hi);
-  if (lane == 0) {
+  if (lane == 0 && (a_lo | a_hi)) {
     atomicMax(arange, a_lo);
     atomicMax(arange + 1, a_hi);
   }
-  for (int o = 16; o; o >>= 1) {
-    acc0 += __shfl_xor_sync(full, acc0, o);
-    acc1 += __shfl_xor_sync(full, acc1, o);
-    acc2 += __shfl_xor_sync(full, acc2, o);
+  if (!sums) return;
+  for (int t = 16; t; t >>= 1) {
+    acc0 += __shfl_xor_sync(full, acc0, t);
+    acc1 += __shfl_xor_sync(full, acc1, t);
+    acc2 += __shfl_xor_sync(full, acc2, t);
   }
   __shared__ double red[3][32];
   const int wi = threadIdx.x >> 5;
@@ -337,6 +377,24 @@ __global__ void k_pack(const float* __restrict__ img, int W, Ellipse e, const in
     for (int i = 0; i < (int)(blockDim.x >> 5); i++) t += red[threadIdx.x][i];
     atomicAdd(sums + threadIdx.x, t);
   }
+}
+
+cudaError_t launch_pack(const float* img, int W, const Ellipse& e, const int* off, int K, const int* gram_pix, int n,
+                        float wscale, float* U, int kp, __half* S, BlockParams* params, float* tile_rmax, double* sums,
+                        unsigned* arange, int num_sms, cudaStream_t st) {
+  // registers hold NB x R values; past 224 elements (Abs-diff alone) NB is 2
+  const int nb = K <= 128 ? 8 : K <= 224 ? 4 : 2;
+  const int groups = (n + nb - 1) / nb, grid = std::min((groups + 7) / 8, 8 * num_sms);
+  auto run = [&](auto kernel) {
+    kernel<<<grid, 256, 0, st>>>(img, W, e, off, K, gram_pix, n, wscale, U, kp, S, params, tile_rmax, sums, arange);
+  };
+  if (K <= 32) run(k_pack<8, 1>);
+  else if (K <= 64) run(k_pack<8, 2>);
+  else if (K <= 128) run(k_pack<8, 4>);
+  else if (K <= 160) run(k_pack<4, 5>);
+  else if (K <= 224) run(k_pack<4, 7>);
+  else run(k_pack<2, 16>);
+  return cudaGetLastError();
 }
 
 // Diagnostics: pack caller-given vectors (n x K, FP32) as operands without

@@ -384,11 +384,8 @@ sred_status global_prepare(sred_ctx* c, int metric, const float* d_img, int w, i
   const float hden = nv + kEps;
   const float wscale = (float)std::sqrt(1.4426950408889634 / (double)hden);
   if (n_g > 0) {
-    // one warp per group of 32 blocks
-    const int pgrid = grid_for(((size_t)n_g + 31) / 32 * 32, 256, 8 * c->num_sms);
-    k_pack<<<pgrid, 256, 0, st>>>(d_img, w, e, d_gpix, n_g, wscale, d_U, kp, d_S, d_params, d_rmax, d_sums,
-                                  reinterpret_cast<unsigned*>(d_sums + 4));
-    CK(cudaGetLastError());
+    CK(launch_pack(d_img, w, e, nullptr, e.k, d_gpix, n_g, wscale, d_U, kp, d_S, d_params, d_rmax, d_sums,
+                   reinterpret_cast<unsigned*>(d_sums + 4), c->num_sms, st));
   }
   if (engine == SRED_ENGINE_TC) {
     float* d_soa;
@@ -926,10 +923,8 @@ sred_status global3d_prepare(sred_ctx* c, int metric, const float* d_vol, int w,
   const float hden = nv + kEps;
   const float wscale = (float)std::sqrt(1.4426950408889634 / (double)hden);
   if (n_g > 0) {
-    k_pack3d<<<grid_for((size_t)n_g * 32, 256, 8 * c->num_sms), 256, 0, st>>>(
-        d_vol, v, d_off, d_gpix, n_g, wscale, d_U, kp, d_S, d_params, d_rmax,
-        reinterpret_cast<unsigned*>(d_sums + 4));
-    CK(cudaGetLastError());
+    CK(launch_pack(d_vol, 0, Ellipse(), d_off, K, d_gpix, n_g, wscale, d_U, kp, d_S, d_params, d_rmax, nullptr,
+                   reinterpret_cast<unsigned*>(d_sums + 4), c->num_sms, st));
   }
   if (engine == SRED_ENGINE_TC) {
     float* d_soa;

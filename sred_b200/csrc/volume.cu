@@ -292,63 +292,6 @@ __global__ void k_flags3d(const float* __restrict__ stds, Vol3 v, float thr, int
   if ((threadIdx.x & 31) == 0 && wc) atomicAdd(n_mask, (unsigned long long)wc);
 }
 
-// One warp per listed block: FP64 moments of its ellipsoid vector, the unit
-// vector (x - mu) / |x - mu| as FP32 (U, row pitch kp) and as the split FP16
-// operand (S, store_split), either of which may be null, and the epilogue
-// parameters; the same quantities as the 2D packing, over linear offsets.
-__global__ void k_pack3d(const float* __restrict__ img, Vol3 v, const int* __restrict__ off,
-                         const int* __restrict__ gram_pix, int n, float wscale, float* __restrict__ U, int kp,
-                         __half* __restrict__ S, BlockParams* __restrict__ params, float* __restrict__ tile_rmax,
-                         unsigned* __restrict__ arange) {
-  unsigned a_lo = 0u, a_hi = 0u;  // ~bits of the smallest a, bits of the largest (launch_den, weights.cuh)
-  const int lane = threadIdx.x & 31;
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
-  const int K = v.k;
-  const SplitLayout lay = split_layout(K);
-  for (int j = gw; j < n; j += nw) {
-    const float* c = img + (size_t)gram_pix[j];
-    double s = 0.0;
-    for (int i = lane; i < K; i += 32) s += (double)c[off[i]];
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    const double mu = s / K;
-    double var = 0.0;
-    for (int i = lane; i < K; i += 32) {
-      const double d = (double)c[off[i]] - mu;
-      var += d * d;
-    }
-    for (int o = 16; o; o >>= 1) var += __shfl_xor_sync(0xffffffffu, var, o);
-    const double nrm = sqrt(var);
-    const double inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
-    const double sigma = sqrt(var / (K - 1));
-    for (int i = lane; i < K; i += 32) {
-      const double u = ((double)c[off[i]] - mu) * inv;
-      if (U) U[(size_t)j * kp + i] = (float)u;
-      if (S) store_split(S + (size_t)j * lay.pitch, lay, i, u * (double)kSplitScale);
-    }
-    if (U)
-      for (int i = K + lane; i < kp; i += 32) U[(size_t)j * kp + i] = 0.0f;
-    if (S) store_split_pad(S + (size_t)j * lay.pitch, lay, lane);
-    if (lane == 0) {
-      BlockParams bp;
-      bp.a = (float)(sigma * (double)wscale);
-      bp.e = sigma > 0.0 ? (float)((double)kEps / sigma) : 0.0f;
-      bp.r = sigma > 0.0 ? (float)(1.0 / sigma) : 0.0f;
-      bp.sigma = (float)sigma;
-      bp.mu = (float)mu;
-      bp.pad0 = bp.pad1 = bp.pad2 = 0.0f;
-      params[j] = bp;
-      a_lo = max(a_lo, ~__float_as_uint(bp.a));
-      a_hi = max(a_hi, __float_as_uint(bp.a));
-      atomicMax(reinterpret_cast<int*>(tile_rmax) + (j >> 7), __float_as_int(bp.r));
-    }
-  }
-  if (lane == 0 && a_hi | a_lo) {
-    atomicMax(arange, a_lo);
-    atomicMax(arange + 1, a_hi);
-  }
-}
-
 // num / (den nPixels + eps) in FP64 over the interior, with the flat test
 // blocks' closed-form share: n_flat pairs of weight 2^-(a_p^2) each, and for
 // NRMSE a term sqrt((K-1)/K) sigma_p per pair times that weight (the flat

@@ -40,8 +40,6 @@ __global__ void k_remap3d(float* a, const float* mask, Vol3 v, const unsigned* m
 // 3D global map (the 2D pair engines run on the compacted block lists).
 __global__ void k_flags3d(const float* stds, Vol3 v, float thr, int flat_columns, float* mask, uint8_t* flags,
                           unsigned long long* n_mask);
-__global__ void k_pack3d(const float* img, Vol3 v, const int* off, const int* gram_pix, int n, float wscale,
-                         float* U, int kp, __half* S, BlockParams* params, float* tile_rmax, unsigned* arange);
 __global__ void k_finalize3d(const int* slot, Vol3 v, const double* num, const double* den,
                              const BlockParams* params, int n_flat, int metric, double sk, double n_pixels,
                              const float* mask, int apply_mask, float* out);
