@@ -18,6 +18,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "ranges.cuh"
 
 namespace sred {
 
@@ -54,35 +55,6 @@ __device__ __forceinline__ f2 pack2(float a, float b) {
 }
 __device__ __forceinline__ void unpack2(f2 v, float* a, float* b) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(*a), "=f"(*b) : "l"(v));
-}
-
-// Order-preserving key of a float (-0 below +0), and back.
-__device__ __forceinline__ unsigned ord_bits(float f) {
-  const unsigned u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float ord_float(unsigned u) {
-  return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
-}
-
-// A CTA's smallest and largest key into mm (all threads of the CTA call it).
-__device__ __forceinline__ void cta_minmax(unsigned lo, unsigned hi, unsigned* mm) {
-  __shared__ unsigned s_lo[8], s_hi[8];
-  lo = __reduce_min_sync(0xffffffffu, lo);
-  hi = __reduce_max_sync(0xffffffffu, hi);
-  if ((threadIdx.x & 31) == 0) {
-    s_lo[threadIdx.x >> 5] = lo;
-    s_hi[threadIdx.x >> 5] = hi;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    lo = __reduce_min_sync(0xffffffffu, s_lo[threadIdx.x & 7]);
-    hi = __reduce_max_sync(0xffffffffu, s_hi[threadIdx.x & 7]);
-    if (threadIdx.x == 0 && lo <= hi) {
-      atomicMin(mm, lo);
-      atomicMax(mm + 1, hi);
-    }
-  }
 }
 
 // The metric of one pixel from its block sums (reference order, explicitly
@@ -351,6 +323,7 @@ struct PlaneArgs {
   int W, H, rw, rh;
   const unsigned* mm_in;
   unsigned* mm_out;  // the range of the results, or null
+  int own;           // 1: a range per plane, 0: one for all (the slices of a volume)
 };
 
 // One pass over the interior (where mask > 0): see PlanePass. VEC floats a load;
@@ -363,7 +336,7 @@ __global__ void __launch_bounds__(256) k_plane_pass(const PlaneArgs g) {
   float mn = 0.0f, d = 1.0f;
   bool remap = false;
   if (OP != kPassRange && OP != kPassInvert) {
-    const unsigned k0 = g.mm_in[2 * blockIdx.y], k1 = g.mm_in[2 * blockIdx.y + 1];
+    const unsigned k0 = g.mm_in[2 * g.own * blockIdx.y], k1 = g.mm_in[2 * g.own * blockIdx.y + 1];
     remap = k1 != 0u || OP == kPassAbsDiff;  // nothing selected: the reference remaps nothing either
     mn = ord_float(k0);
     float mx = ord_float(k1);
@@ -409,7 +382,7 @@ __global__ void __launch_bounds__(256) k_plane_pass(const PlaneArgs g) {
     y += sy;
     if (x >= g.W) x -= g.W, y++;
   }
-  if (g.mm_out) cta_minmax(lo, hi, g.mm_out + 2 * blockIdx.y);
+  if (g.mm_out) cta_minmax(lo, hi, g.mm_out + 2 * g.own * blockIdx.y);
 }
 
 template <int VEC>
@@ -426,8 +399,9 @@ void launch_pass(PlanePass op, const PlaneArgs& g, dim3 grid, cudaStream_t st) {
 }  // namespace
 
 void launch_plane_pass(PlanePass op, float* a, const float* mask, int w, int h, int rw, int rh, int planes,
-                       const unsigned* mm_in, unsigned* mm_out, int num_sms, cudaStream_t st) {
-  const PlaneArgs g{a, mask, w, h, rw, rh, mm_in, mm_out};
+                       const unsigned* mm_in, unsigned* mm_out, int num_sms, cudaStream_t st, bool shared_range) {
+  if (planes < 1) return;
+  const PlaneArgs g{a, mask, w, h, rw, rh, mm_in, mm_out, shared_range ? 0 : 1};
   const size_t n = (size_t)w * h;
   // float4 where every plane and quad is aligned
   const bool vec = n % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(mask)) & 15) == 0;

@@ -42,7 +42,8 @@ __global__ void k_init_minmax(unsigned* mm, int planes);
 cudaError_t launch_block_map(const float* img, int w, int h, int frames, const Ellipse& e, const RefBlock& rb,
                              int metric, float* out, float* stds, unsigned* mm, int num_sms, cudaStream_t st);
 // One pass over the interior of every plane (where mask > 0, if there is one), with
-// the range mm_in of its values; mm_out (or null) receives the range of the results.
+// the range mm_in of its values; mm_out (or null) receives the range of the results;
+// shared_range: one range for all planes (the interior slices of a volume).
 // Normalisation (java/Utils.java:985-1031) is kPassRange and kPassRemap.
 enum PlanePass {
   kPassRange,        // the range alone
@@ -52,7 +53,8 @@ enum PlanePass {
   kPassAbsDiff       // 1 - remap, the maximum starting at Float.MIN_VALUE (java/CLUtils.java:936-960)
 };
 void launch_plane_pass(PlanePass op, float* a, const float* mask, int w, int h, int rw, int rh, int planes,
-                       const unsigned* mm_in, unsigned* mm_out, int num_sms, cudaStream_t st);
+                       const unsigned* mm_in, unsigned* mm_out, int num_sms, cudaStream_t st,
+                       bool shared_range = false);
 __global__ void k_apply_mask(float* a, const float* mask, size_t n);
 
 // gat.cu

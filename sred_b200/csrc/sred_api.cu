@@ -713,9 +713,21 @@ sred_status prepare_volume(sred_ctx* c, int w, int h, int d, int bw, int bh, int
   std::vector<int> off(kMaxK3);
   const int k = build_ellipsoid(bw, bh, bd, w, h, off.data());
   if (k < 2 || k > kMaxK3) return fail(c, SRED_ERR_ARG, "ellipsoid block size out of range");
-  CKS(ensure(c, B_OFF3, k, d_off));
-  CK(cudaMemcpyAsync(*d_off, off.data(), sizeof(int) * k, cudaMemcpyHostToDevice, st));
+  // behind the offsets, from an even index on: the block's rows, {first offset, voxels}
+  off.resize(k + (k & 1));
+  int nrows = 0;
+  for (int i = 0; i < k; i++) {
+    if (i == 0 || off[i] != off[i - 1] + 1) {
+      off.push_back(off[i]);
+      off.push_back(0);
+      nrows++;
+    }
+    off.back()++;
+  }
+  CKS(ensure(c, B_OFF3, off.size(), d_off));
+  CK(cudaMemcpyAsync(*d_off, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice, st));
   *v = Vol3{w, h, d, bw / 2, bh / 2, bd / 2, k};
+  v->nrows = nrows;
   return SRED_OK;
 }
 
@@ -747,6 +759,19 @@ sred_status mask_3d(sred_ctx* c, const Vol3& v, const float* d_stds, float relc,
   return SRED_OK;
 }
 
+// java/Utils.java:1572-1630 (normalizeImage3D) over the interior (where mask > 0 when a
+// mask is given): the passes of the 2D maps over the interior slices, with one range
+// (mm, initialised; ranged: it holds the range already).
+void normalize3(sred_ctx* c, const Vol3& v, float* d_a, const float* d_mask, unsigned* mm, bool ranged,
+                cudaStream_t st) {
+  const size_t o = (size_t)v.rd * v.W * v.H;
+  const float* m = d_mask ? d_mask + o : nullptr;
+  const int slices = v.D - 2 * v.rd;
+  if (!ranged)
+    launch_plane_pass(kPassRange, d_a + o, m, v.W, v.H, v.rw, v.rh, slices, nullptr, mm, c->num_sms, st, true);
+  launch_plane_pass(kPassRemap, d_a + o, m, v.W, v.H, v.rw, v.rh, slices, mm, nullptr, c->num_sms, st, true);
+}
+
 // With h_vol, d_vol is filled from host memory here, in slabs of slices on
 // the context's upload stream, and each slab's local statistics and map run
 // as soon as the slices they read have landed, so the upload overlaps the
@@ -762,22 +787,20 @@ sred_status block3d_core(sred_ctx* c, int metric, const float* d_vol, int w, int
   CKS(prepare_volume(c, w, h, d, bw, bh, bd, st, &v, &d_off));
   if (block_size != v.k) return fail(c, SRED_ERR_ARG, "block_size does not match the ellipsoid of bw x bh x bd");
   const size_t n = (size_t)w * h * d;
-  float *d_ref, *d_means, *d_stds;
+  float *d_ref, *d_stds = nullptr;
+  unsigned* mm;
   CKS(ensure(c, B_REF3, v.k, &d_ref));
-  CKS(ensure(c, B_MEANS, n, &d_means));
-  CKS(ensure(c, B_STDS, n, &d_stds));
+  CKS(ensure(c, B_MM, 2, &mm));
+  if (relc > 0.0f) CKS(ensure(c, B_STDS, n, &d_stds));
+  const bool ranged = normalize && !(relc > 0.0f);  // the map's kernels take its range
+  if (normalize) k_init_minmax<<<1, 32, 0, st>>>(mm, 1);
   CK(cudaMemcpyAsync(d_ref, ref_pixels, sizeof(float) * v.k, cudaMemcpyHostToDevice, st));
-  const dim3 grid = vol_grid(v), blk(32, 4);
-  // slices [z0, z1): local statistics, map, metric transform
   auto slab = [&](int z0, int z1) -> sred_status {
     if (z1 <= z0) return SRED_OK;
     Vol3 vs = v;
     vs.z0 = z0;
-    const dim3 gs(grid.x, grid.y, z1 - z0);
-    k_local_stats3d<<<gs, blk, sizeof(int) * v.k, st>>>(d_vol, vs, d_off, d_means, d_stds);
-    CK(launch_block_map3d(d_vol, vs, d_off, d_ref, ref_mean, ref_std, metric, d_means, d_stds, d_out, st, z1));
-    if (metric == kNrmse || metric == kAbsDiff) k_block3d_post<<<gs, blk, 0, st>>>(d_out, vs, metric);
-    CK(cudaGetLastError());
+    CK(launch_block_map3d(d_vol, vs, d_off, d_ref, ref_mean, ref_std, metric, d_out, d_stds, ranged ? mm : nullptr, st,
+                          z1));
     return SRED_OK;
   };
   if (!h_vol) {
@@ -820,14 +843,8 @@ sred_status block3d_core(sred_ctx* c, int metric, const float* d_vol, int w, int
     CKS(ensure(c, B_MASK, n, &d_mask));
     CKS(mask_3d(c, v, d_stds, relc, d_mask, d_out, st, nullptr));
   }
-  if (normalize) {
-    unsigned* mm;
-    CKS(ensure(c, B_MM, 2, &mm));
-    k_init_minmax<<<1, 32, 0, st>>>(mm, 1);
-    k_minmax3d<<<grid_for((size_t)v.W * v.H * v.D, 256, 4 * c->num_sms), 256, 0, st>>>(d_out, d_mask, v, mm);
-    k_remap3d<<<grid, blk, 0, st>>>(d_out, d_mask, v, mm);
-    CK(cudaGetLastError());
-  }
+  if (normalize) normalize3(c, v, d_out, d_mask, mm, ranged, st);
+  CK(cudaGetLastError());
   CK(cudaStreamSynchronize(st));
   return SRED_OK;
 }
@@ -974,8 +991,7 @@ sred_status global3d_finish(sred_ctx* c, const GState& gs, cudaStream_t st, int 
     unsigned* mm;
     CKS(ensure(c, B_MM, 2, &mm));
     k_init_minmax<<<1, 32, 0, st>>>(mm, 1);
-    k_minmax3d<<<grid_for((size_t)v.W * v.H * v.D, 256, 4 * c->num_sms), 256, 0, st>>>(d_out, d_mask, v, mm);
-    k_remap3d<<<grid, blk, 0, st>>>(d_out, d_mask, v, mm);
+    normalize3(c, v, d_out, d_mask, mm, false, st);
     CK(cudaGetLastError());
   }
   CK(cudaEventRecord(c->ev[3], st));

@@ -5,13 +5,13 @@
 //
 // FP32 in the reference kernels' evaluation order (cl/kernelGetLocalStatistics3D.cl,
 // cl/kernelGetBlock{Pearson,Ssim,Nrmse,AbsDiffStds}3D.cl); compiled with
-// -fmad=false so that no multiply-add is fused. One thread per voxel, threads
-// of a warp on consecutive x so that every gather of the block is coalesced;
-// the block offsets (and reference voxels) sit in shared memory and the
-// Pearson chain re-reads the block through L1 instead of holding it in a
-// local array.
+// -fmad=false so that no multiply-add is fused.
 #include <float.h>
 
+#include <algorithm>
+#include <type_traits>
+
+#include "ranges.cuh"
 #include "volume.cuh"
 
 namespace sred {
@@ -31,16 +31,6 @@ __device__ __forceinline__ bool voxel(const Vol3& v, int* x, int* y, int* z, siz
   if (*x >= v.W || *y >= v.H) return false;
   *p = ((size_t)*z * v.H + *y) * v.W + *x;
   return true;
-}
-
-// Order-preserving key of a float for atomicMin/atomicMax on unsigned ints
-// (-0 orders below +0, as Math.min / Math.max do).
-__device__ __forceinline__ unsigned f2key(float f) {
-  const unsigned u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float key2f(unsigned k) {
-  return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
 }  // namespace
@@ -73,111 +63,220 @@ __global__ void __launch_bounds__(128)
   stds[p] = sqrtf(var / (float)(K - 1));
 }
 
-template <bool CACHE>
-__global__ void __launch_bounds__(128)
-    k_block_map3d_t(const float* __restrict__ img, Vol3 v, const int* __restrict__ off,
-                    const float* __restrict__ ref, float ref_mean, float ref_std, int metric,
-                    const float* __restrict__ means, const float* __restrict__ stds, float* __restrict__ out) {
-  extern __shared__ int s_off[];
-  float* s_ref = reinterpret_cast<float*>(s_off + v.k);
-  float* s_t = s_ref + v.k;  // CACHE: [K][128] normalised block values of the Pearson chain
-  for (int i = threadIdx.y * blockDim.x + threadIdx.x; i < v.k; i += blockDim.x * blockDim.y) {
-    s_off[i] = off[i];
-    s_ref[i] = ref[i];
-  }
-  __syncthreads();
-  int x, y, z;
-  size_t p;
-  if (!voxel(v, &x, &y, &z, &p)) return;
-  if (!interior3(x, y, z, v)) {
-    out[p] = 0.0f;
-    return;
-  }
-  const float tstd = stds[p];
-  const float* c = img + p;
-  const int K = v.k;
-  if (metric == kAbsDiff) {  // cl/kernelGetBlockAbsDiffStds3D.cl
-    out[p] = fabsf(ref_std - tstd);
-    return;
-  }
-  const float tmean = means[p];
-  if (metric == kPearson) {
-    // cl/kernelGetBlockPearson3D.cl: min-max of the block, minus its mean,
-    // min-max again, then the covariance with the reference. Every division of
-    // a pass shares its divisor (div_fixed: correctly rounded, as the
-    // kernel's own divisions); with CACHE the first normalisation is kept in
-    // shared memory for the last pass instead of being computed again.
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    float mn = FLT_MAX, mx = -FLT_MAX;
-    for (int i = 0; i < K; i++) {
-      const float t = c[s_off[i]];
-      mn = fminf(mn, t);
-      mx = fmaxf(mx, t);
+// ---------------------------------------------------------------------------
+// The block map. A thread takes PX voxels of a row; neighbours share all but one
+// value of each row of the block, so a window of PX values slides along it: one load
+// (through L1) serves PX voxels, and an element's offset and reference value are
+// fetched once for PX. The local statistics are the first sweeps of the same kernel,
+// the metric transform and the range its last step, and Pearson's first normalisation
+// is computed again in the last sweep (five operations) rather than kept.
+// Bound by FP32 issue, 24 operations an element and voxel for Pearson: 199 us for
+// 256x256x64, 5x5x5 (33 elements), normalised, where one voxel a thread in four
+// kernels took 330.
+// ---------------------------------------------------------------------------
+namespace {
+
+// Visits the block in the reference's order: f(i, w), w(q) the value of voxel column q.
+// A window at the end of a row holds values of the next one, which only discarded voxels
+// see; with LAST (the slice whose blocks reach the end of the volume) it repeats the row's
+// last value instead. room: columns from the first voxel to the last of the row.
+template <int PX, bool LAST, class F>
+__device__ __forceinline__ void sweep3(const float* c, const int2* rows, int nrows, int room, F f) {
+  int i = 0;
+  for (int r = 0; r < nrows; r++) {
+    const int2 row = rows[r];  // offset of its first voxel, voxels (odd)
+    const float* p = c + row.x;
+    int n = row.y, last = room + (n >> 1);
+    float w[PX];
+#pragma unroll
+    for (int q = 0; q < PX - 1; q++) w[q] = p[LAST ? min(q, last) : q];
+    auto element = [&](auto jc) {
+      constexpr int j = decltype(jc)::value;
+      w[(j + PX - 1) % PX] = p[LAST ? min(j + PX - 1, last) : j + PX - 1];
+      f(i + j, [&](int q) { return w[(j + q) % PX]; });
+    };
+    for (; n >= 4; n -= 4, i += 4, p += 4, last -= 4) {
+      element(std::integral_constant<int, 0>());
+      element(std::integral_constant<int, 1>());
+      element(std::integral_constant<int, 2>());
+      element(std::integral_constant<int, 3>());
     }
-    const float d1 = mx - mn + kEps, y1 = __frcp_rn(d1);
-    float mn2 = FLT_MAX, mx2 = -FLT_MAX;
-    for (int i = 0; i < K; i++) {
-      const float t = div_fixed(c[s_off[i]] - mn, d1, y1) - tmean;
-      if (CACHE) s_t[i * 128 + tid] = t;
-      mn2 = fminf(mn2, t);
-      mx2 = fmaxf(mx2, t);
+    element(std::integral_constant<int, 0>());
+    if (n == 3) {
+      element(std::integral_constant<int, 1>());
+      element(std::integral_constant<int, 2>());
     }
-    const float d2 = mx2 - mn2 + kEps, y2 = __frcp_rn(d2);
-    float cov = 0.0f;
-    for (int i = 0; i < K; i++) {
-      const float t = CACHE ? s_t[i * 128 + tid] : div_fixed(c[s_off[i]] - mn, d1, y1) - tmean;
-      cov += s_ref[i] * div_fixed(t - mn2, d2, y2);
-    }
-    cov /= (float)(K - 1);
-    if (ref_std == 0.0f && tstd == 0.0f) out[p] = 1.0f;
-    else if (ref_std == 0.0f || tstd == 0.0f) out[p] = 0.0f;
-    else out[p] = fmaxf(0.0f, cov / ((ref_std * tstd) + kEps));
-    return;
+    i += n;
   }
-  if (metric == kSsim) {  // cl/kernelGetBlockSsim3D.cl
-    float cov = 0.0f;
-    for (int i = 0; i < K; i++) cov += s_ref[i] * (c[s_off[i]] - tmean);
-    cov /= (float)(K - 1);
-    if (ref_std == 0.0f && tstd == 0.0f) {
-      out[p] = 1.0f;
-    } else if (ref_std == 0.0f || tstd == 0.0f) {
-      out[p] = 0.0f;
-    } else {
-      const float ssim = ((2.0f * ref_mean * tmean + kC1) * (2.0f * cov + kC2)) /
-                         (((ref_mean * ref_mean) + (tmean * tmean) + kC1) * ((ref_std * ref_std) + (tstd * tstd) + kC2));
-      out[p] = fmaxf(0.0f, ssim);
-    }
-    return;
-  }
-  // NRMSE, cl/kernelGetBlockNrmse3D.cl
-  float mse = 0.0f;
-  for (int i = 0; i < K; i++) {
-    const float d = s_ref[i] - (c[s_off[i]] - tmean);
-    mse += d * d;
-  }
-  mse /= (float)K;
-  out[p] = sqrtf(mse);
 }
 
-cudaError_t launch_block_map3d(const float* img, Vol3 v, const int* off, const float* ref, float ref_mean,
-                               float ref_std, int metric, const float* means, const float* stds, float* out,
-                               cudaStream_t st, int z1) {
-  const dim3 grid((v.W + 31) / 32, (v.H + 3) / 4, (z1 < 0 ? v.D : z1) - v.z0), blk(32, 4);
-  // The Pearson chain caches its first normalisation (K x 128 floats) while
-  // that fits in 96 KB of shared memory; past it, it recomputes.
-  const size_t smem_base = 2 * sizeof(int) * (size_t)v.k;
-  const size_t smem_cache = smem_base + sizeof(float) * 128 * (size_t)v.k;
-  if (metric == kPearson && smem_cache <= 96 * 1024) {
-    if (smem_cache > 48 * 1024) {
-      const cudaError_t e =
-          cudaFuncSetAttribute(k_block_map3d_t<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cache);
-      if (e != cudaSuccess) return e;
+constexpr int kRows3 = 8;  // rows of a CTA, one warp each
+
+// The voxels x .. x + PX - 1 (of which those right of the interior are discarded): their
+// values, local stds and range.
+template <int METRIC, int PX, bool LAST>
+__device__ __forceinline__ void map_voxels(const float* c, int x, const Vol3& v, const int2* rows, const float* s_ref,
+                                           float ref_mean, float ref_std, float (&val)[PX], float (&sd)[PX],
+                                           unsigned& lo, unsigned& hi) {
+  const int K = v.k, room = v.W - 1 - x;
+  float mean[PX], var[PX], acc[PX], mn[PX], mx[PX];
+#pragma unroll
+  for (int q = 0; q < PX; q++) {
+    mean[q] = var[q] = acc[q] = 0.0f;
+    mn[q] = FLT_MAX;
+    mx[q] = -FLT_MAX;
+  }
+  sweep3<PX, LAST>(c, rows, v.nrows, room, [&](int, auto w) {
+#pragma unroll
+    for (int q = 0; q < PX; q++) {
+      mean[q] += w(q);
+      if (METRIC == kPearson) {
+        mn[q] = fminf(mn[q], w(q));
+        mx[q] = fmaxf(mx[q], w(q));
+      }
     }
-    k_block_map3d_t<true><<<grid, blk, smem_cache, st>>>(img, v, off, ref, ref_mean, ref_std, metric, means, stds,
-                                                         out);
-  } else {
-    k_block_map3d_t<false><<<grid, blk, smem_base, st>>>(img, v, off, ref, ref_mean, ref_std, metric, means, stds,
-                                                          out);
+  });
+  // cl/kernelGetBlockPearson3D.cl: min-max of the block, minus its mean, min-max
+  // again, then the covariance with the reference. Every division of a sweep shares
+  // its divisor (div_fixed: correctly rounded, as the kernel's own divisions).
+  float d1[PX], y1[PX], mn2[PX], mx2[PX];
+#pragma unroll
+  for (int q = 0; q < PX; q++) {
+    mean[q] /= (float)K;
+    d1[q] = mx[q] - mn[q] + kEps;
+    y1[q] = METRIC == kPearson ? __frcp_rn(d1[q]) : 0.0f;
+    mn2[q] = FLT_MAX;
+    mx2[q] = -FLT_MAX;
+  }
+  sweep3<PX, LAST>(c, rows, v.nrows, room, [&](int i, auto w) {
+    const float rf = METRIC == kSsim || METRIC == kNrmse ? s_ref[i] : 0.0f;
+#pragma unroll
+    for (int q = 0; q < PX; q++) {
+      const float d = w(q) - mean[q];
+      var[q] += d * d;
+      if (METRIC == kPearson) {
+        const float t = div_fixed(w(q) - mn[q], d1[q], y1[q]) - mean[q];
+        mn2[q] = fminf(mn2[q], t);
+        mx2[q] = fmaxf(mx2[q], t);
+      } else if (METRIC == kSsim) {  // cl/kernelGetBlockSsim3D.cl
+        acc[q] += rf * d;
+      } else if (METRIC == kNrmse) {  // cl/kernelGetBlockNrmse3D.cl
+        const float e = rf - d;
+        acc[q] += e * e;
+      }
+    }
+  });
+  if (METRIC == kPearson) {
+#pragma unroll
+    for (int q = 0; q < PX; q++) {
+      mx2[q] = mx2[q] - mn2[q] + kEps;
+      mx[q] = __frcp_rn(mx2[q]);
+    }
+    sweep3<PX, LAST>(c, rows, v.nrows, room, [&](int i, auto w) {
+      const float rf = s_ref[i];
+#pragma unroll
+      for (int q = 0; q < PX; q++) {
+        const float t = div_fixed(w(q) - mn[q], d1[q], y1[q]) - mean[q];
+        acc[q] += rf * div_fixed(t - mn2[q], mx2[q], mx[q]);
+      }
+    });
+  }
+#pragma unroll
+  for (int q = 0; q < PX; q++) {
+    if (x + q >= v.W - v.rw) break;
+    const float s = sqrtf(var[q] / (float)(K - 1));
+    float o;
+    if (METRIC == kAbsDiff) {  // cl/kernelGetBlockAbsDiffStds3D.cl, java/CLUtils.java:1590-1600
+      o = 1.0f - fabsf(ref_std - s);
+    } else if (METRIC == kNrmse) {  // java/CLUtils.java:1459-1471
+      o = sqrtf(acc[q] / (float)K);
+      o = o == 0.0f ? 1.0f : 1.0f / o;
+    } else if (ref_std == 0.0f && s == 0.0f) {
+      o = 1.0f;
+    } else if (ref_std == 0.0f || s == 0.0f) {
+      o = 0.0f;
+    } else if (METRIC == kPearson) {
+      o = fmaxf(0.0f, acc[q] / (float)(K - 1) / ((ref_std * s) + kEps));
+    } else {
+      const float cov = acc[q] / (float)(K - 1);
+      o = fmaxf(0.0f, ((2.0f * ref_mean * mean[q] + kC1) * (2.0f * cov + kC2)) /
+                          (((ref_mean * ref_mean) + (mean[q] * mean[q]) + kC1) *
+                           ((ref_std * ref_std) + (s * s) + kC2)));
+    }
+    val[q] = o;
+    sd[q] = s;
+    lo = min(lo, ord_bits(o));
+    hi = max(hi, ord_bits(o));
+  }
+}
+
+template <int METRIC, int PX>
+__global__ void __launch_bounds__(32 * kRows3)
+    k_block_map3d(const float* __restrict__ img, Vol3 v, const int* __restrict__ off, const float* __restrict__ ref,
+                  float ref_mean, float ref_std, float* __restrict__ out, float* __restrict__ stds,
+                  unsigned* __restrict__ mm) {
+  extern __shared__ int2 s_rows[];
+  float* s_ref = reinterpret_cast<float*>(s_rows + v.nrows);
+  const int2* rows = reinterpret_cast<const int2*>(off + v.k + (v.k & 1));
+  for (int i = threadIdx.x; i < v.nrows; i += 32 * kRows3) s_rows[i] = rows[i];
+  for (int i = threadIdx.x; i < v.k; i += 32 * kRows3) s_ref[i] = ref[i];
+  __syncthreads();
+  // the tiles start at the first interior column; the first one also owns those before it
+  const int lane = threadIdx.x & 31, x0 = v.rw + blockIdx.x * 32 * PX, x = x0 + lane * PX;
+  const int y = blockIdx.y * kRows3 + (threadIdx.x >> 5), z = blockIdx.z + v.z0;
+  const size_t base = ((size_t)z * v.H + y) * v.W;
+  unsigned lo = 0xffffffffu, hi = 0u;
+  float val[PX], sd[PX];
+#pragma unroll
+  for (int q = 0; q < PX; q++) val[q] = sd[q] = 0.0f;
+  if (interior3(x, y, z, v)) {
+    if (z == v.D - 1 - v.rd)
+      map_voxels<METRIC, PX, true>(img + base + x, x, v, s_rows, s_ref, ref_mean, ref_std, val, sd, lo, hi);
+    else
+      map_voxels<METRIC, PX, false>(img + base + x, x, v, s_rows, s_ref, ref_mean, ref_std, val, sd, lo, hi);
+  }
+  if (y < v.H) {
+#pragma unroll
+    for (int q = 0; q < PX; q++)
+      if (x + q < v.W) {
+        out[base + x + q] = val[q];
+        if (stds) stds[base + x + q] = sd[q];
+      }
+    if (blockIdx.x == 0)
+      for (int i = lane; i < min(v.rw, v.W); i += 32) {
+        out[base + i] = 0.0f;
+        if (stds) stds[base + i] = 0.0f;
+      }
+  }
+  if (mm) cta_minmax(lo, hi, mm);
+}
+
+template <int METRIC>
+void launch_map3d(const float* img, const Vol3& v, const int* off, const float* ref, float ref_mean, float ref_std,
+                  float* out, float* stds, unsigned* mm, cudaStream_t st, int slices) {
+  const size_t smem = sizeof(int2) * v.nrows + sizeof(float) * v.k;
+  const int iw = v.W - 2 * v.rw;
+  auto run = [&](auto kernel, int px) {
+    const dim3 grid(std::max(1, (v.W - v.rw + 32 * px - 1) / (32 * px)), (v.H + kRows3 - 1) / kRows3, slices);
+    kernel<<<grid, 32 * kRows3, smem, st>>>(img, v, off, ref, ref_mean, ref_std, out, stds, mm);
+  };
+  // the widest window whose warps the interior fills at least half
+  if (iw > 64) run(k_block_map3d<METRIC, 4>, 4);
+  else if (iw > 32) run(k_block_map3d<METRIC, 2>, 2);
+  else run(k_block_map3d<METRIC, 1>, 1);
+}
+
+}  // namespace
+
+cudaError_t launch_block_map3d(const float* img, Vol3 v, const int* off, const float* ref, float ref_mean,
+                               float ref_std, int metric, float* out, float* stds, unsigned* mm, cudaStream_t st,
+                               int z1) {
+  const int n = z1 - v.z0;
+  switch (metric) {
+    case kPearson: launch_map3d<kPearson>(img, v, off, ref, ref_mean, ref_std, out, stds, mm, st, n); break;
+    case kSsim: launch_map3d<kSsim>(img, v, off, ref, ref_mean, ref_std, out, stds, mm, st, n); break;
+    case kNrmse: launch_map3d<kNrmse>(img, v, off, ref, ref_mean, ref_std, out, stds, mm, st, n); break;
+    default: launch_map3d<kAbsDiff>(img, v, off, ref, ref_mean, ref_std, out, stds, mm, st, n); break;
   }
   return cudaGetLastError();
 }
@@ -196,16 +295,6 @@ __global__ void k_divide_fixed64(const double* __restrict__ a, size_t n, double 
     out[i] = div_fixed(a[i], b, y);
 }
 
-// Host steps on the interior (java/CLUtils.java:1459-1471, 1590-1600): NRMSE
-// inverted (0 -> 1), Abs-diff turned into 1 - x.
-__global__ void k_block3d_post(float* __restrict__ a, Vol3 v, int metric) {
-  int x, y, z;
-  size_t p;
-  if (!voxel(v, &x, &y, &z, &p) || !interior3(x, y, z, v)) return;
-  if (metric == kNrmse) a[p] = a[p] == 0.0f ? 1.0f : 1.0f / a[p];
-  else if (metric == kAbsDiff) a[p] = 1.0f - a[p];
-}
-
 // java/Utils.java:1501-1525 (getRelevanceMask3D) for the threshold
 // noise_var * c; map (if not null) is multiplied by the mask (applyMask3D).
 __global__ void k_mask3d(const float* __restrict__ stds, Vol3 v, float thr, float* __restrict__ mask,
@@ -217,42 +306,6 @@ __global__ void k_mask3d(const float* __restrict__ stds, Vol3 v, float thr, floa
   if (interior3(x, y, z, v)) m = (stds[p] * stds[p]) <= thr ? 0.0f : 1.0f;
   mask[p] = m;
   if (map) map[p] *= m;
-}
-
-// java/Utils.java:1572-1630 (normalizeImage3D): min and max over the interior
-// (where mask > 0 when a mask is given); mm = {min key, max key}. Grid-stride
-// over the volume (a grid of a few CTAs per SM) so that each warp issues one
-// pair of atomics for many voxels.
-__global__ void k_minmax3d(const float* __restrict__ a, const float* __restrict__ mask, Vol3 v,
-                           unsigned* __restrict__ mm) {
-  const size_t n = (size_t)v.W * v.H * v.D, plane = (size_t)v.W * v.H;
-  unsigned lo = 0xffffffffu, hi = 0u;
-  for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-    const int z = (int)(p / plane), y = (int)((p % plane) / v.W), x = (int)(p % v.W);
-    if (interior3(x, y, z, v) && (!mask || mask[p] > 0.0f)) {
-      const unsigned k = f2key(a[p]);
-      lo = min(lo, k);
-      hi = max(hi, k);
-    }
-  }
-  for (int o = 16; o; o >>= 1) {
-    lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-  }
-  if ((threadIdx.x & 31) == 0 && lo != 0xffffffffu) {
-    atomicMin(mm, lo);
-    atomicMax(mm + 1, hi);
-  }
-}
-
-__global__ void k_remap3d(float* __restrict__ a, const float* __restrict__ mask, Vol3 v,
-                          const unsigned* __restrict__ mm) {
-  if (mm[0] == 0xffffffffu) return;  // no voxel selected: the reference changes nothing
-  int x, y, z;
-  size_t p;
-  if (!voxel(v, &x, &y, &z, &p) || !interior3(x, y, z, v) || (mask && !(mask[p] > 0.0f))) return;
-  const float mn = key2f(mm[0]), mx = key2f(mm[1]);
-  a[p] = (a[p] - mn) / (mx - mn + kEps);
 }
 
 // ---------------------------------------------------------------------------

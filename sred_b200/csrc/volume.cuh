@@ -13,6 +13,7 @@ struct Vol3 {
   int rw, rh, rd;
   int k;
   int z0 = 0;  // first slice of a launch over slices [z0, z0 + gridDim.z) of the per-voxel kernels
+  int nrows = 0;  // rows of the ellipsoid
 };
 
 // Host: linear offsets (z W H + y W + x) of the voxels of the ellipsoid
@@ -20,22 +21,19 @@ struct Vol3 {
 // float arithmetic). Writes at most kMaxK3 offsets; returns the voxel count.
 int build_ellipsoid(int bw, int bh, int bd, int W, int H, int* off);
 
-// One thread per voxel; dynamic shared memory: k ints (stats), k ints + k
-// floats (block map).
+// One thread per voxel; dynamic shared memory: k ints.
 __global__ void k_local_stats3d(const float* img, Vol3 v, const int* off, float* means, float* stds);
-// The raw 3D block map (one thread per voxel; the dynamic shared memory it
-// needs is chosen here) over slices [v.z0, z1) (z1 < 0: to the last slice).
+// The 3D block map over slices [v.z0, z1), NRMSE inverted and Abs-diff turned into
+// 1 - x; the local stds (stds, or null) and the range of the interior (mm, or null).
+// off: the block's offsets and rows (prepare_volume).
 cudaError_t launch_block_map3d(const float* img, Vol3 v, const int* off, const float* ref, float ref_mean,
-                               float ref_std, int metric, const float* means, const float* stds, float* out,
-                               cudaStream_t st, int z1 = -1);
+                               float ref_std, int metric, float* out, float* stds, unsigned* mm, cudaStream_t st,
+                               int z1);
 __global__ void k_divide_fixed(const float* a, size_t n, float b, float* out);
 __global__ void k_divide_fixed64(const double* a, size_t n, double b, double* out);
-__global__ void k_block3d_post(float* a, Vol3 v, int metric);
 // The FP32 sum of sigma^2 over the interior in raster order (0 without an interior).
 cudaError_t launch_noise3d(const float* stds, Vol3 v, float* sum, cudaStream_t st);
 __global__ void k_mask3d(const float* stds, Vol3 v, float thr, float* mask, float* map);
-__global__ void k_minmax3d(const float* a, const float* mask, Vol3 v, unsigned* mm);
-__global__ void k_remap3d(float* a, const float* mask, Vol3 v, const unsigned* mm);
 
 // 3D global map (the 2D pair engines run on the compacted block lists).
 __global__ void k_flags3d(const float* stds, Vol3 v, float thr, int flat_columns, float* mask, uint8_t* flags,

@@ -89,3 +89,22 @@ def test_block_map_bits(ctx, metric, w, h, frames, bw, bh):
         for f in range(frames):
             exp = _expected(metric, img[f], ref, offs, bw // 2, bh // 2, normalize)
             assert np.array_equal(got[f], exp), (f, normalize, float(np.abs(got[f] - exp).max()))
+
+
+@pytest.mark.parametrize("w,h,d,bw,bh,bd", [(37, 9, 5, 5, 3, 3), (38, 10, 6, 5, 5, 3), (69, 9, 8, 5, 3, 7), (70, 11, 5, 5, 3, 3),
+                                            (133, 17, 4, 3, 5, 3), (260, 9, 9, 9, 7, 5), (9, 9, 9, 9, 3, 3)])
+@pytest.mark.parametrize("metric", clutils.BLOCK_METRICS)
+def test_block_map_3d_bits(ctx, metric, w, h, d, bw, bh, bd):
+    """Interiors of 33, 34, 65, 66, 131 and 252 columns (windows of 2 and 4, whole and ragged
+    last ones, two tiles) and of one; with and without normalisation and relevance mask."""
+    import oracle
+    rng = np.random.default_rng(w + h)
+    vol = rng.random((d, h, w), dtype=F)
+    z, y, x = d // 2, h // 2, w // 2
+    rb = utils.get_reference_block_3d(vol[z - bd // 2:z + bd // 2 + 1, y - bh // 2:y + bh // 2 + 1,
+                                          x - bw // 2:x + bw // 2 + 1])
+    for c, normalize in ((0.0, True), (0.0, False), (1.0, True)):
+        exp = oracle.block_map3d(metric, vol, rb.pixels, bw, bh, bd, rb.mean, rb.std, c, normalize)["map"]
+        got = clutils.calculate_block_repetition_map_3d(metric, utils.InputImage3D(vol.ravel(), w, h, d), rb, c, normalize,
+                                                        ctx=ctx)
+        assert np.array_equal(got, exp.ravel(), equal_nan=True), (c, normalize)
