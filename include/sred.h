@@ -319,7 +319,7 @@ sred_status sred_phase_correlation_map_2d(sred_ctx *ctx, const float *img, const
  * Same result as sred_block_map_2d_device with relevance_constant 0; needs no
  * context. Runs on the current device and on `stream` (NULL = the default
  * stream) and synchronises that stream before it returns, so the map is
- * complete then. Scratch is a fixed device array of about 4 MiB that every
+ * complete then. Scratch is a fixed device array of 64 KiB that every
  * GPU loading this library holds until exit; the limits are frames <= 4096,
  * for NRMSE frames * w * h <= 1,048,576, and a block whose image tile with
  * halo fits in 48 KB of shared memory (every block up to 25 x 25; a 3 x 401

@@ -141,8 +141,8 @@ struct Tile {
 // MODE: kPearson (also SSIM), kNrmse, kCosine, kAbsDiff. Bound by FP32 issue: a
 // pixel's element is 6 operations that may not be merged (sum; difference, two
 // products, two sums), in packed pairs of two rows, and the window leaves 1/4 load
-// a pixel. 16 frames of 1024x1024, 15x15 (177 elements), normalised: 1365 us with one
-// load an element and pass and a thread per two pixels, 720 now (480 at one scalar
+// a pixel. 16 frames of 1024x1024, 15x15 (149 elements), normalised: 1365 us with one
+// load an element and pass and a thread per two pixels, 720 now (403 at one scalar
 // operation a lane and clock).
 template <int MODE, int PX>
 __global__ void __launch_bounds__(32 * kThreadsY)

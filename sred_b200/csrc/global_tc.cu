@@ -307,7 +307,7 @@ __device__ __forceinline__ void tmem_wait_batch(uint32_t (&v)[2][8]) {
 // ---------------------------------------------------------------------------
 // Epilogue arithmetic on f32x2 pairs (two neighbouring columns of one row).
 //
-// The blocks are ordered by sigma, so the 32 rows and BN/4 columns of a warp's
+// The blocks are ordered by sigma, so the 32 rows and 64 or 128 columns of a warp's
 // slab have nearly equal a (the weight's argument). With a_p = alpha + dp and
 // a_q = beta + dq (alpha, beta: the slab's group centres),
 //   2^-(a_p - a_q)^2 = 2^-(a_p - beta)^2 * 2^(dq (2 (alpha - beta) - dq)) * 2^(2 dp dq)

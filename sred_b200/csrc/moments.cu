@@ -244,8 +244,8 @@ __global__ void k_scatter(const uint8_t* __restrict__ flags, size_t n, const int
 // + ... + 1 exchanges and the rest of the five steps, instead of five each) and leave
 // lane l with the scalars of block l % NB. Bound by conversions and FP64 issue; a map
 // of few blocks by latency, which many short groups spread over all SMs: 16,851 blocks
-// of 137 elements took 206 us with a warp per 32 blocks, three reads of the image and
-// a per-lane load of the kernel's parameters each, and 18 now; 53,600 of 33 (a
+// of 113 elements took 206 us with a warp per 32 blocks, three reads of the image and
+// a per-lane load of the kernel's parameters each, and 18 now; 63,500 of 13 (a
 // 256x256 map) about 100 us and 50.
 // ---------------------------------------------------------------------------
 template <int NB>

@@ -255,7 +255,13 @@ struct GivenStats {
 // The tensor-core engine's weighted metrics run on blocks in order of sigma
 // (their weights factorise, global_tc.cu); unweighted NRMSE and the FP32 engine
 // take the blocks in raster order, whose pixels overlap while packing.
-bool sort_for(int engine, int metric) {
+// So do maps of fewer than 28,000 blocks, where the sort's six launches (57 us) take more
+// than the exponential a pair that they save: 6,500 blocks, 5x5 Pearson 271 us sorted and
+// 229 not; 23,100, 9x9 Pearson 414 and 384; 33,000, 9x9 SSIM 620 and 616; 46,700, 5x5
+// Pearson 609 and 758.
+constexpr int kSortMin = 28000;
+bool sort_for(int engine, int metric, int n) {
+  if (n < kSortMin) return false;
   return engine == SRED_ENGINE_TC && (metric == kPearson || metric == kSsim || metric == kNrmseW);
 }
 
@@ -377,7 +383,7 @@ sred_status global_prepare(sred_ctx* c, int metric, const float* d_img, int w, i
   CK(cudaMemsetAsync(d_rmax, 0, (n_pad / 128) * sizeof(float), st));
   CK(cudaMemsetAsync(d_num, 0, n_pad * sizeof(double), st));
   CK(cudaMemsetAsync(d_sums, 0, 8 * sizeof(double), st));
-  const bool sorted = sort_for(engine, metric);
+  const bool sorted = sort_for(engine, metric, n_g);
   if (sorted) CKS(sort_blocks(c, d_stds, n_g, st));
   // weight = exp(-(s_p - s_q)^2 / (FILTER_PARAM + EPSILON)) = 2^-(a_p - a_q)^2,
   // FILTER_PARAM + EPSILON summed in FP32 as the reference kernel does.
@@ -630,8 +636,10 @@ sred_status block_core(sred_ctx* c, int metric, const float* d_img, int w, int h
   rb.mean = ref_mean;
   rb.std = ref_std;
   std::memcpy(rb.px, ref_pixels, sizeof(float) * e.k);
+  // (NRMSE without a relevance constant has the interior as its mask, java/CLUtils.java:788-797)
+  const bool masked = relc > 0.0f || (metric == kNrmse && relc != 0.0f);
   float* d_stds = nullptr;
-  if (relc > 0.0f) CKS(ensure(c, B_STDS2, n, &d_stds));
+  if (masked) CKS(ensure(c, B_STDS2, n, &d_stds));
   // Ranges of the map (by its own kernel) and of the first host step's results.
   unsigned *mm, *ranged = nullptr;
   CKS(ensure(c, B_MM, (size_t)4 * frames, &mm));
@@ -639,7 +647,7 @@ sred_status block_core(sred_ctx* c, int metric, const float* d_img, int w, int h
   if (metric == kHu || metric == kHu7 || metric == kPhase) {
     CKS(block_shape_launch(c, metric, d_img, w, h, frames, e, ref_pixels, bw, bh, ref_std, d_out, d_stds, st));
   } else {
-    if (metric == kNrmse || metric == kAbsDiff || normalize) {
+    if (metric == kAbsDiff || (!masked && (metric == kNrmse || normalize))) {
       k_init_minmax<<<grid_for((size_t)2 * frames, 256, 64), 256, 0, st>>>(mm, 2 * frames);
       ranged = mm;
     }
@@ -671,10 +679,10 @@ sred_status block_core(sred_ctx* c, int metric, const float* d_img, int w, int h
   };
   if (metric == kAbsDiff) {
     // (relevance masks come after the transform)
-    pass(kPassAbsDiff, mm, relc > 0.0f ? nullptr : mm2);
+    pass(kPassAbsDiff, mm, masked ? nullptr : mm2);
     ranged = mm2;
   }
-  if (relc > 0.0f) {
+  if (masked) {
     CKS(relevance_masks());
     k_apply_mask<<<grid_for(n, 256, 8 * c->num_sms), 256, 0, st>>>(d_out, d_mask, n);
     if (metric == kNrmse || normalize) {
@@ -688,7 +696,6 @@ sred_status block_core(sred_ctx* c, int metric, const float* d_img, int w, int h
     ranged = mm;
   }
   if (metric == kNrmse) {
-    // the mask is the interior without a relevance constant (java/CLUtils.java:788-797)
     pass(kPassRemapInvert, mm, normalize ? mm2 : nullptr);
     ranged = mm2;
   }
@@ -735,13 +742,30 @@ dim3 vol_grid(const Vol3& v) { return dim3((v.W + 31) / 32, (v.H + 3) / 4, v.D);
 
 // java/Utils.java:1463-1498 (getMeanNoiseVar3D): the mean of the local
 // variances over the interior, summed in FP32 in raster order with a float
-// count, as the reference does on the host.
+// count, as the reference does on the host. Volumes of up to 65,536 voxels are summed
+// here: 84x45x13 (a global map) takes 281 us so and 324 with k_noise3d, which gains from
+// there on (86x58x24: 436 and 412; 128x128x48: 5.1 ms and 4.2).
+constexpr size_t kNoiseHostVoxels = 65536;
 sred_status noise_var_3d(sred_ctx* c, const Vol3& v, const float* d_stds, cudaStream_t st, float* out) {
-  float *d_sum, sum;
-  CKS(ensure(c, B_VARS, 1, &d_sum));
-  CK(launch_noise3d(d_stds, v, d_sum, st));
-  CK(cudaMemcpyAsync(&sum, d_sum, sizeof(float), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+  const size_t all = (size_t)v.W * v.H * v.D;
+  float sum = 0.0f;
+  if (all <= kNoiseHostVoxels) {
+    std::vector<float> h(all);
+    CK(cudaMemcpyAsync(h.data(), d_stds, all * sizeof(float), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    for (int z = v.rd; z < v.D - v.rd; z++)
+      for (int y = v.rh; y < v.H - v.rh; y++)
+        for (int x = v.rw; x < v.W - v.rw; x++) {
+          const float sd = h[((size_t)z * v.H + y) * v.W + x];
+          sum += sd * sd;
+        }
+  } else {
+    float* d_sum;
+    CKS(ensure(c, B_VARS, 1, &d_sum));
+    CK(launch_noise3d(d_stds, v, d_sum, st));
+    CK(cudaMemcpyAsync(&sum, d_sum, sizeof(float), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+  }
   const double n = (double)std::max(0, v.W - 2 * v.rw) * std::max(0, v.H - 2 * v.rh) * std::max(0, v.D - 2 * v.rd);
   *out = sum / (float)std::min(n, 16777216.0);  // a float counting by ones stops there
   return SRED_OK;
@@ -934,7 +958,7 @@ sred_status global3d_prepare(sred_ctx* c, int metric, const float* d_vol, int w,
   CK(cudaMemsetAsync(d_rmax, 0, (n_pad / 128) * sizeof(float), st));
   CK(cudaMemsetAsync(d_num, 0, n_pad * sizeof(double), st));
   CK(cudaMemsetAsync(d_sums, 0, 8 * sizeof(double), st));
-  const bool sorted = sort_for(engine, metric == kNrmse ? kNrmseW : metric);
+  const bool sorted = sort_for(engine, metric == kNrmse ? kNrmseW : metric, n_g);
   if (sorted) CKS(sort_blocks(c, d_stds, n_g, st));
   // weight = exp(-(s_p - s_q)^2 / (FILTER_PARAM + EPSILON)) = 2^-(a_p - a_q)^2
   const float hden = nv + kEps;
@@ -1016,7 +1040,7 @@ sred_status global3d_finish(sred_ctx* c, const GState& gs, cudaStream_t st, int 
     info->ms_gram = t12;
     info->ms_finalize = t23;
     info->ms_total = t03;
-    info->launches = 5 + contraction_launches(gs) + 1 + (normalize ? 3 : 0);
+    info->launches = 6 + contraction_launches(gs) + 1 + (normalize ? 3 : 0);
   }
   if (c->log_cb) {
     float t03 = 0;

@@ -400,9 +400,9 @@ int build_ellipsoid(int bw, int bh, int bd, int W, int H, int* off) {
 // adds the whole number nearest to x / ulp; a tie goes by the parity of S. An element,
 // and any run of elements, is then a function of S's parity: two whole increments, and
 // those compose associatively. So 16,384 elements at a time are 1,024 threads' runs and
-// a scan. Where S reaches 2^24 the thread that holds the element adds its run one by
-// one in FP32 (the sum's binade rises at most 253 times), and the others continue from
-// there. Subnormal sums share the lowest binade's ulp; a sum past the largest float is
+// a scan of the warps' sums. Where S reaches 2^24 the warp that holds the element steps
+// through its 512 by itself, the run that ends the binade in FP32 (the binade rises at
+// most 253 times), and the others continue from there. Subnormal sums share the lowest binade's ulp; a sum past the largest float is
 // Inf or NaN for good. Bound by the one SM's issue slots: 0.26 ms for
 // 128x128x48 (676,000 elements), where the copy to the host and the serial sum there
 // added 1.0 ms to the map.
@@ -427,12 +427,94 @@ __device__ __forceinline__ Step shfl_up(Step a, int d) {
   return Step{__shfl_up_sync(0xffffffffu, a.e, d), __shfl_up_sync(0xffffffffu, a.o, d)};
 }
 
+// s = S ulp with a whole S (below kSumTop unless s is not finite), x / ulp in two exact
+// steps of f1 and f2: ulp = 2^(e - 150) for e = max(1, the biased exponent of s).
+struct Grid {
+  int S;
+  float f1, f2;
+  __device__ __forceinline__ explicit Grid(float s) {
+    const unsigned bits = __float_as_uint(s);
+    const int e = max(1, (int)(bits >> 23)), up = 150 - e, u1 = min(up, 127);  // up: -104 .. 149
+    S = (bits >> 23) ? (int)((bits & 0x7fffffu) | 0x800000u) : (int)bits;
+    f1 = __uint_as_float((unsigned)(u1 + 127) << 23);
+    f2 = __uint_as_float((unsigned)(up - u1 + 127) << 23);
+  }
+  __device__ __forceinline__ float at(int n) const { return (float)n / f2 / f1; }
+};
+
+// A run's increment where no element ties or is 2^22 ulp or more; with one that does, or
+// a NaN, *odd is set and run_steps gives it. Rounds by adding 1.5 2^23 (conversions issue
+// at an eighth of the rate).
+__device__ __forceinline__ int run_increment(const float* run, const Grid& g, bool* odd) {
+  const float magic = 12582912.0f;
+  int sum = 0;
+  bool o = false;
+#pragma unroll
+  for (int j = 0; j < kSumRun; j++) {
+    const float t = run[j] * g.f1 * g.f2, m = t + magic;
+    o |= !(t < 4194304.0f) || fabsf(t - (m - magic)) == 0.5f;
+    sum += (int)(__float_as_uint(m) & 0x7fffffu);
+  }
+  *odd = o;
+  return sum - kSumRun * 0x400000;
+}
+__device__ __noinline__ Step run_steps(const float* run, float f1, float f2) {
+  Step a{0, 0};
+  for (int j = 0; j < kSumRun; j++) {
+    const float t = run[j] * f1 * f2, fl = floorf(t), fr = t - fl;
+    if (!(t < (float)kSumTop)) return Step{kSumTop, kSumTop};  // (a NaN too: the FP32 additions meet it)
+    const int k = (int)fl;
+    a = then(a, fr == 0.5f ? Step{k + (k & 1), k + !(k & 1)} : Step{k + (fr > 0.5f), k + (fr > 0.5f)});
+  }
+  return a;
+}
+// Inclusive composition over the lanes.
+__device__ __forceinline__ Step scan_steps(Step a, int lane) {
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const Step b = shfl_up(a, d);
+    if (lane >= d) a = then(b, a);
+  }
+  return a;
+}
+
+// The sum after a warp's 32 runs: lanes' increments while the binade lasts, and the run
+// that ends it in FP32.
+__device__ float warp_sum(float s, const float* run, int lane) {
+  for (int first = 0; first < 32;) {
+    if (!(s <= 3.402823466e38f)) {  // Inf stays, unless a NaN follows
+      bool nan = s != s;
+      for (int j = 0; j < kSumRun; j++) nan |= run[j] != run[j] && lane >= first;
+      return __any_sync(0xffffffffu, nan) ? nanf("") : s;
+    }
+    const Grid g(s);
+    bool tie;
+    Step a;
+    a.e = a.o = run_increment(run, g, &tie);
+    if (tie) a = run_steps(run, g.f1, g.f2);
+    if (lane < first) a = Step{0, 0};
+    a = scan_steps(a, lane);
+    const int end = g.S + ((g.S & 1) ? a.o : a.e);
+    const unsigned past = __ballot_sync(0xffffffffu, end >= kSumTop);
+    int begin = __shfl_up_sync(0xffffffffu, end, 1);
+    if (lane == 0) begin = g.S;
+    if (!past) return g.at(__shfl_sync(0xffffffffu, end, 31));
+    first = __ffs(past);
+    float t = g.at(begin);
+    if (lane == first - 1) {
+#pragma unroll
+      for (int j = 0; j < kSumRun; j++) t += run[j];
+    }
+    s = __shfl_sync(0xffffffffu, t, first - 1);
+  }
+  return s;
+}
+
 __global__ void __launch_bounds__(kSumThreads) k_noise3d(const float* __restrict__ stds, Vol3 v,
                                                          float* __restrict__ sum) {
   extern __shared__ float s_x[];
   __shared__ Step s_warp[32];
   __shared__ float s_sum;
-  __shared__ int s_next, s_total;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const unsigned iw = v.W - 2 * v.rw, ih = v.H - 2 * v.rh;
   const size_t n = (size_t)iw * ih * (v.D - 2 * v.rd);
@@ -458,6 +540,7 @@ __global__ void __launch_bounds__(kSumThreads) k_noise3d(const float* __restrict
   };
   load();
   float s = 0.0f;
+  const float* run = s_x + tid * (kSumRun + 1);
   const size_t chunks = (n + kSumChunk - 1) / kSumChunk;
   for (size_t c = 0; c < chunks; c++) {
     __syncthreads();
@@ -468,101 +551,66 @@ __global__ void __launch_bounds__(kSumThreads) k_noise3d(const float* __restrict
     }
     __syncthreads();
     if (c + 1 < chunks) load();
-    const float* run = s_x + tid * (kSumRun + 1);
-    int first = 0;  // the runs before it are in s
-    while (first < kSumThreads) {
-      if (!(s <= 3.402823466e38f)) {  // Inf stays, unless a NaN follows
+    int first = 0;  // the warps before it are in s
+    if (c == 0) {   // half of the binades end in the first warp's 512 elements
+      if (w == 0) {
+        const float t = warp_sum(0.0f, run, lane);
+        if (lane == 0) s_sum = t;
+      }
+      __syncthreads();
+      s = s_sum;
+      first = 1;
+    }
+    while (first < 32) {
+      if (!(s <= 3.402823466e38f)) {
         bool nan = s != s;
-        for (int j = 0; j < kSumRun; j++) nan |= run[j] != run[j] && tid >= first;
+        for (int j = 0; j < kSumRun; j++) nan |= run[j] != run[j] && w >= first;
         if (__syncthreads_or(nan)) s = nanf("");
         break;
       }
-      // s = S 2^(e - 150) with e = max(1, its biased exponent); x / ulp in two exact steps
-      const unsigned bits = __float_as_uint(s);
-      const int e = max(1, (int)(bits >> 23));
-      const int S = (bits >> 23) ? (int)((bits & 0x7fffffu) | 0x800000u) : (int)bits;
-      const int up = 150 - e, u1 = min(up, 127), u2 = up - u1;  // up: -104 .. 149
-      const float f1 = __uint_as_float((unsigned)(u1 + 127) << 23), f2 = __uint_as_float((unsigned)(u2 + 127) << 23);
-      int sum = 0;
-      bool tie = false, big = false;  // (a NaN counts as big: the FP32 additions meet it)
-#pragma unroll
-      for (int j = 0; j < kSumRun; j++) {
-        const float t = run[j] * f1 * f2, q = rintf(t);
-        big |= !(t < (float)kSumTop);
-        tie |= fabsf(t - q) == 0.5f;
-        sum += (int)q;
+      const Grid g(s);
+      bool tie;
+      Step a;
+      a.e = a.o = run_increment(run, g, &tie);
+      if (w < first) {
+        a = Step{0, 0};
+        tie = false;
       }
-      Step a{0, 0};
-      if (tid >= first) a.e = a.o = big ? kSumTop : min(sum, kSumTop);
-      tie = tie && !big && tid >= first;
-      if (tid == 0) s_next = kSumThreads;
-      Step before, after;
+      Step all;  // after warp `lane`
       if (__syncthreads_or(tie)) {
-        if (tie) {
-          a = Step{0, 0};
-          for (int j = 0; j < kSumRun; j++) {
-            const float t = run[j] * f1 * f2, fl = floorf(t), fr = t - fl;
-            const int k = (int)fl;
-            a = then(a, fr == 0.5f ? Step{k + (k & 1), k + !(k & 1)} : Step{k + (fr > 0.5f), k + (fr > 0.5f)});
-          }
-        }
-        Step in = a;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const Step b = shfl_up(in, d);
-          if (lane >= d) in = then(b, in);
-        }
-        if (lane == 31) s_warp[w] = in;
+        if (tie) a = run_steps(run, g.f1, g.f2);
+        a = scan_steps(a, lane);
+        if (lane == 31) s_warp[w] = a;
         __syncthreads();
-        Step pre = s_warp[lane];
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const Step b = shfl_up(pre, d);
-          if (lane >= d) pre = then(b, pre);
-        }
-        pre = Step{__shfl_sync(0xffffffffu, pre.e, (w + 31) & 31), __shfl_sync(0xffffffffu, pre.o, (w + 31) & 31)};
-        if (w == 0) pre = Step{0, 0};
-        const Step ex = shfl_up(in, 1);
-        before = lane == 0 ? pre : then(pre, ex);
-        after = then(pre, in);
+        all = scan_steps(s_warp[lane], lane);
       } else {  // one increment for both parities
-        int in = a.e;
+        const int t = __reduce_add_sync(0xffffffffu, a.e);  // below 2^31
+        if (lane == 0) s_warp[w].e = min(t, kSumTop);
+        __syncthreads();
+        int in = s_warp[lane].e;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
           const int b = __shfl_up_sync(0xffffffffu, in, d);
           if (lane >= d) in = min(in + b, kSumTop);
         }
-        if (lane == 31) s_warp[w].e = in;
-        __syncthreads();
-        int pre = s_warp[lane].e;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const int b = __shfl_up_sync(0xffffffffu, pre, d);
-          if (lane >= d) pre = min(pre + b, kSumTop);
+        all.e = all.o = in;
+      }
+      const int end = g.S + ((g.S & 1) ? all.o : all.e);
+      const unsigned past = __ballot_sync(0xffffffffu, end >= kSumTop);
+      if (past) {
+        const int hit = __ffs(past) - 1;  // the binade ends in this warp
+        int begin = __shfl_sync(0xffffffffu, end, max(hit - 1, 0));
+        if (hit == 0) begin = g.S;
+        if (w == hit) {
+          const float t = warp_sum(g.at(begin), run, lane);
+          if (lane == 0) s_sum = t;
         }
-        pre = __shfl_sync(0xffffffffu, pre, (w + 31) & 31);
-        if (w == 0) pre = 0;
-        const int ex = __shfl_up_sync(0xffffffffu, in, 1);
-        before.e = before.o = lane == 0 ? pre : min(pre + ex, kSumTop);
-        after.e = after.o = min(pre + in, kSumTop);
-      }
-      const int s0 = S + ((S & 1) ? before.o : before.e), s1 = S + ((S & 1) ? after.o : after.e);
-      if (s0 < kSumTop && s1 >= kSumTop) {  // at most one thread: the binade ends in its run
-        float t = (float)s0;
-        t = u2 ? t / f2 / f1 : t / f1;
-#pragma unroll
-        for (int j = 0; j < kSumRun; j++) t += run[j];
-        s_sum = t;
-        s_next = tid + 1;
-      }
-      if (tid == kSumThreads - 1) s_total = s1;
-      __syncthreads();
-      first = s_next;
-      if (s_total < kSumTop) {
-        const float t = (float)s_total;
-        s = u2 ? t / f2 / f1 : t / f1;
-      } else {
+        __syncthreads();
         s = s_sum;
+        first = hit + 1;
+      } else {
+        s = g.at(__shfl_sync(0xffffffffu, end, 31));
+        first = 32;
       }
       __syncthreads();
     }

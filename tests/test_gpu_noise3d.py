@@ -1,6 +1,7 @@
 """The noise variance of a volume against its serial FP32 sum (java/Utils.java:1467-1483),
 bit for bit: both round every partial sum, so no tolerance is due. Interiors of one
-voxel, of one column, around a whole number of the kernel's 16,384-voxel steps; values
+voxel, of one column, whole numbers of the kernel's 16,384-voxel steps and not, on both
+sides of the 65,536 voxels from which the kernel sums; values
 that tie on half an ulp, that leap over binades, that are subnormal, zero or not finite."""
 import numpy as np
 import pytest
@@ -38,7 +39,8 @@ def _values(kind, n, rng):
 
 
 @pytest.mark.parametrize("w,h,d", [(1, 1, 1), (1, 5000, 7), (31, 33, 1), (32, 32, 16), (113, 29, 5), (32, 32, 17),
-                                   (17, 1, 1025), (128, 120, 41)])
+                                   (17, 1, 1025), (128, 120, 41), (64, 64, 20), (63, 13, 101), (1, 5000, 14),
+                                   (64, 128, 10)])
 @pytest.mark.parametrize("kind", ["random", "ties", "halves", "leaps", "subnormal", "zeros", "overflow", "inf",
                                   "inf nan"])
 def test_noise_variance_3d_bits(ctx, kind, w, h, d):
