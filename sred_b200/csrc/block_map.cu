@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(256) k_plane_pass(const PlaneArgs g) {
   const float* mask = g.mask ? g.mask + n * blockIdx.y : nullptr;
   float mn = 0.0f, d = 1.0f;
   bool remap = false;
-  if (OP != kPassRange && OP != kPassInvert) {
+  if (OP == kPassRemap || OP == kPassRemapInvert || OP == kPassAbsDiff) {
     const unsigned k0 = g.mm_in[2 * g.own * blockIdx.y], k1 = g.mm_in[2 * g.own * blockIdx.y + 1];
     remap = k1 != 0u || OP == kPassAbsDiff;  // nothing selected: the reference remaps nothing either
     mn = ord_float(k0);
@@ -364,10 +364,15 @@ __global__ void __launch_bounds__(256) k_plane_pass(const PlaneArgs g) {
     bool any = false;
 #pragma unroll
     for (int q = 0; q < VEC; q++) {
-      if (xx >= g.rw && xx < g.W - g.rw && yy >= g.rh && yy < g.H - g.rh && (!mask || m[q] > 0.0f)) {
+      const bool in = xx >= g.rw && xx < g.W - g.rw && yy >= g.rh && yy < g.H - g.rh;
+      if (OP == kPassMask && in) {  // (a map is 0 outside its interior)
+        v[q] = __fmul_rn(v[q], m[q]);
+        any = true;
+      }
+      if (in && (!mask || m[q] > 0.0f)) {
         if (remap) v[q] = __fdiv_rn(__fsub_rn(v[q], mn), d);
         if (OP == kPassAbsDiff) v[q] = __fsub_rn(1.0f, v[q]);
-        if (OP == kPassInvert || OP == kPassRemapInvert) v[q] = (v[q] == 0.0f) ? 1.0f : __fdiv_rn(1.0f, v[q]);
+        if (OP == kPassRemapInvert) v[q] = (v[q] == 0.0f) ? 1.0f : __fdiv_rn(1.0f, v[q]);
         lo = min(lo, ord_bits(v[q]));
         hi = max(hi, ord_bits(v[q]));
         any = true;
@@ -391,7 +396,7 @@ void launch_pass(PlanePass op, const PlaneArgs& g, dim3 grid, cudaStream_t st) {
     case kPassRange: k_plane_pass<kPassRange, VEC><<<grid, 256, 0, st>>>(g); break;
     case kPassRemap: k_plane_pass<kPassRemap, VEC><<<grid, 256, 0, st>>>(g); break;
     case kPassRemapInvert: k_plane_pass<kPassRemapInvert, VEC><<<grid, 256, 0, st>>>(g); break;
-    case kPassInvert: k_plane_pass<kPassInvert, VEC><<<grid, 256, 0, st>>>(g); break;
+    case kPassMask: k_plane_pass<kPassMask, VEC><<<grid, 256, 0, st>>>(g); break;
     case kPassAbsDiff: k_plane_pass<kPassAbsDiff, VEC><<<grid, 256, 0, st>>>(g); break;
   }
 }
@@ -410,11 +415,6 @@ void launch_plane_pass(PlanePass op, float* a, const float* mask, int w, int h, 
   const dim3 grid((unsigned)std::min(want, cap), planes);
   if (vec) launch_pass<4>(op, g, grid, st);
   else launch_pass<1>(op, g, grid, st);
-}
-
-__global__ void k_apply_mask(float* __restrict__ a, const float* __restrict__ mask, size_t n) {
-  for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x)
-    a[p] = __fmul_rn(a[p], mask[p]);
 }
 
 }  // namespace sred

@@ -49,13 +49,12 @@ enum PlanePass {
   kPassRange,        // the range alone
   kPassRemap,        // (v - min) / (max - min + eps) in FP32
   kPassRemapInvert,  // remap, then the NRMSE inversion (java/CLUtils.java:809-821)
-  kPassInvert,       // the inversion alone
+  kPassMask,         // v times the mask
   kPassAbsDiff       // 1 - remap, the maximum starting at Float.MIN_VALUE (java/CLUtils.java:936-960)
 };
 void launch_plane_pass(PlanePass op, float* a, const float* mask, int w, int h, int rw, int rh, int planes,
                        const unsigned* mm_in, unsigned* mm_out, int num_sms, cudaStream_t st,
                        bool shared_range = false);
-__global__ void k_apply_mask(float* a, const float* mask, size_t n);
 
 // gat.cu
 __global__ void k_gat(float* img, size_t n, double gain, double c);

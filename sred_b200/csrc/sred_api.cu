@@ -684,12 +684,10 @@ sred_status block_core(sred_ctx* c, int metric, const float* d_img, int w, int h
   }
   if (masked) {
     CKS(relevance_masks());
-    k_apply_mask<<<grid_for(n, 256, 8 * c->num_sms), 256, 0, st>>>(d_out, d_mask, n);
-    if (metric == kNrmse || normalize) {
-      k_init_minmax<<<grid_for((size_t)2 * frames, 256, 64), 256, 0, st>>>(mm, 2 * frames);
-      pass(kPassRange, nullptr, mm);
-      ranged = mm;
-    }
+    const bool range = metric == kNrmse || normalize;
+    if (range) k_init_minmax<<<grid_for((size_t)2 * frames, 256, 64), 256, 0, st>>>(mm, 2 * frames);
+    pass(kPassMask, nullptr, range ? mm : nullptr);
+    ranged = mm;
   } else if (!ranged && normalize) {  // shape metrics
     k_init_minmax<<<grid_for((size_t)frames, 256, 64), 256, 0, st>>>(mm, frames);
     pass(kPassRange, nullptr, mm);
