@@ -995,6 +995,14 @@ __device__ __forceinline__ void group_sync() {
   else __syncthreads();
 }
 
+// Ring stage of a tile's last operands: st0 is the stage of its first ones, back =
+// (stages per tile - 1) % S. (A tile may take more stages than the ring has: K = 197 takes
+// seven of a ring of five.)
+__host__ __device__ inline uint32_t ring_last(uint32_t st0, uint32_t back, uint32_t S) {
+  const uint32_t s = st0 + back;  // both below S
+  return s < S ? s : s - S;
+}
+
 // End of a role: all warps (of both CTAs of a pair) meet (no CTA leaves while the
 // other may still arrive on its barriers or an MMA reads its shared memory), then
 // the MMA warps free TMEM.
@@ -1260,6 +1268,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
     float* fs = scratch + ew * kScratch;
     const uint32_t acce = CTAS == 2 ? leader_addr(b_acce) : b_acce;
     uint32_t tile = 0, item_i = 0, st0 = 0;  // st0: ring stage of the tile's first operands
+    const uint32_t back = (uint32_t)(g.nst - 1) % (uint32_t)S;
     bool ok = true;
     // One pass over the CTA's items per phase (ItemCursor::part): the full tiles with
     // the unmasked forms, then the masked tiles, each in a loop of its own.
@@ -1290,7 +1299,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
       bool any = false;  // this set had a tile of the item
       for (int rb = rb0; ok && rb < rb1; rb += M, tile++) {
         const uint32_t b = tile & 1;
-        const uint32_t last = st0 + g.nst - 1 < (uint32_t)S ? st0 + g.nst - 1 : st0 + g.nst - 1 - S;  // its last stage
+        const uint32_t last = ring_last(st0, back, S);  // its last stage
         st0 = last + 1 == (uint32_t)S ? 0 : last + 1;
         if (SETS == 2 && (int)b != set) continue;
         any = true;
