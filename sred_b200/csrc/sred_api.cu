@@ -285,10 +285,10 @@ sred_status absdiff_sums(sred_ctx* c, const GState& gs, cudaStream_t st, const u
   float* d_keys;
   int *d_idx, *d_ws;
   double* d_table;
-  CKS(ensure(c, B_KEYS, gs.n_g, &d_keys));
-  CKS(ensure(c, B_IDX, gs.n_g, &d_idx));
+  CKS(ensure(c, B_KEYS, abs_keys(gs.n_g), &d_keys));
+  CKS(ensure(c, B_IDX, abs_keys(gs.n_g), &d_idx));
   CKS(ensure(c, B_SORT, sort_workspace_ints(gs.n_g), &d_ws));
-  CKS(ensure(c, B_ABS, kAbsTable, &d_table));
+  CKS(ensure(c, B_ABS, abs_table_doubles(gs.n_g), &d_table));
   CK(launch_absdiff(static_cast<const BlockParams*>(c->buf[B_PARAMS].p), gs.n_g, 1.0 / (double)gs.wscale, arange, d_keys,
                     d_idx, d_ws, d_table, static_cast<double*>(c->buf[B_NUM].p), c->num_sms, st));
   return SRED_OK;
@@ -1778,9 +1778,9 @@ sred_status reserve_global(sred_ctx* c, const sred_job* jobs, int n_jobs) {
   CKS(ensure(c, B_NODES, kDenNodes, &d));
   CKS(ensure(c, B_SLICES, den_slices((int)n_pad), &f2));
   if (absdiff) {
-    CKS(ensure(c, B_KEYS, n_pad, &f));
-    CKS(ensure(c, B_IDX, n_pad, &i32));
-    CKS(ensure(c, B_ABS, kAbsTable, &d));
+    CKS(ensure(c, B_KEYS, abs_keys((int)n_pad), &f));
+    CKS(ensure(c, B_IDX, abs_keys((int)n_pad), &i32));
+    CKS(ensure(c, B_ABS, abs_table_doubles((int)n_pad), &d));
   }
   if (tc || absdiff) CKS(ensure(c, B_SORT, sort_workspace_ints((int)n_pad), &i32));
   if (tc) {

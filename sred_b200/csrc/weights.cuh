@@ -23,29 +23,45 @@ __device__ __forceinline__ int node_grid(const unsigned* __restrict__ arange, do
   return m <= (double)kDenNodes ? (int)m : 0;
 }
 
-// 1 / prod_{j != k} (k - j) for the nodes 0..11.
+// 1 / prod_{j != k} (k - j) for the nodes 0..N-1 (N even).
+template <int N>
 __device__ __forceinline__ double lagrange_scale(int k) {
   const double f[12] = {1.0, 1.0, 2.0, 6.0, 24.0, 120.0, 720.0, 5040.0, 40320.0, 362880.0, 3628800.0, 39916800.0};
-  const double v = 1.0 / (f[k] * f[11 - k]);
-  return (k & 1) ? v : -v;  // sign (-1)^(11 - k)
+  const double v = 1.0 / (f[k] * f[N - 1 - k]);
+  return (k & 1) ? v : -v;  // sign (-1)^(N - 1 - k)
 }
 
-// The function at a from its node values (stride between nodes).
-__device__ __forceinline__ double interpolate12(double a, double x0, const double* __restrict__ nodes, size_t stride) {
-  const double t = (a - x0) / kNodeH;
-  const int k0 = (int)floor(t) - (kNodePad - 1);
-  const double s = t - (double)k0;  // in [5, 6)
-  double suf[12];
-  suf[11] = 1.0;
+// The polynomial through the values f[0..N-1] at the nodes 0..N-1, at s.
+template <int N>
+__device__ __forceinline__ double lagrange(double s, const double* f) {
+  double suf[N];
+  suf[N - 1] = 1.0;
 #pragma unroll
-  for (int k = 11; k > 0; k--) suf[k - 1] = suf[k] * (s - (double)k);
+  for (int k = N - 1; k > 0; k--) suf[k - 1] = suf[k] * (s - (double)k);
   double pre = 1.0, sum = 0.0;
 #pragma unroll
-  for (int k = 0; k < 12; k++) {
-    sum += lagrange_scale(k) * pre * suf[k] * nodes[(size_t)(k0 + k) * stride];
+  for (int k = 0; k < N; k++) {
+    sum += lagrange_scale<N>(k) * pre * suf[k] * f[k];
     pre *= s - (double)k;
   }
   return sum;
+}
+
+// The 12 node values around a (stride between nodes), and a's place among them (in [5, 6)).
+__device__ __forceinline__ double node_values(double a, double x0, const double* __restrict__ nodes, size_t stride,
+                                              double (&f)[12]) {
+  const double t = (a - x0) / kNodeH;
+  const int k0 = (int)floor(t) - (kNodePad - 1);
+#pragma unroll
+  for (int k = 0; k < 12; k++) f[k] = nodes[(size_t)(k0 + k) * stride];
+  return t - (double)k0;
+}
+
+// The function at a from its node values.
+__device__ __forceinline__ double interpolate12(double a, double x0, const double* __restrict__ nodes, size_t stride) {
+  double f[12];
+  const double s = node_values(a, x0, nodes, stride, f);
+  return lagrange<12>(s, f);
 }
 
 int den_slices(int n);
