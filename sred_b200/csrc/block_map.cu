@@ -78,9 +78,10 @@ __device__ __forceinline__ float block_metric_value(int metric, int K, float mea
   return fmaxf(0.0f, __fdiv_rn(__fmul_rn(a, b), __fmul_rn(cc, dd)));
 }
 
-// The ellipse by rows: row r holds the columns -hw[r] .. hw[r].
+// The ellipse by rows: row r holds the columns -hw[r] .. hw[r]; the first and the last
+// `single` rows hold one element each.
 struct BlockRows {
-  int k, rw, rh;
+  int k, rw, rh, single;
   short hw[kMaxK];
 };
 
@@ -89,10 +90,25 @@ struct BlockRows {
 // share all but one value of an element, so a window of PX pairs slides along
 // each row: one shared-memory load an element for 2 PX pixels. Column c of the
 // tile lies at (c % PX) p + c / PX, which keeps the loads of a warp contiguous.
+// The rows of one element, most of a narrow block's, take a loop without a window
+// (3x101 at 1024x1024, PX = 1: 160 us without it, 96 so).
 template <int PX, class F>
 __device__ __forceinline__ void sweep(const f2* base, int p, int pitch, const BlockRows& e, F f) {
   int i = 0;
-  for (int r = 0; r <= 2 * e.rh; r++, base += pitch) {
+  auto single = [&]() {
+    int o[PX];
+#pragma unroll
+    for (int q = 0; q < PX; q++) o[q] = ((e.rw + q) % PX) * p + (e.rw + q) / PX;
+#pragma unroll 4
+    for (int r = 0; r < e.single; r++, i++, base += pitch) {
+      f2 w[PX];
+#pragma unroll
+      for (int q = 0; q < PX; q++) w[q] = base[o[q]];
+      f(i, [&](int q) { return w[q]; });
+    }
+  };
+  single();
+  for (int r = e.single; r <= 2 * e.rh - e.single; r++, base += pitch) {
     const int hw = e.hw[r], s = e.rw - hw;
     int o[4];
 #pragma unroll
@@ -123,6 +139,7 @@ __device__ __forceinline__ void sweep(const f2* base, int p, int pitch, const Bl
     }
     i += n;
   }
+  single();
 }
 
 // The tile of PX: columns, values per column class, f2 per row.
@@ -263,13 +280,19 @@ __global__ void __launch_bounds__(32 * kThreadsY)
   if (mm) cta_minmax(lo, hi, mm + 2 * blockIdx.z);
 }
 
+// Shared memory of a tile at most: the tallest block's (3x509) takes 140 KB of it.
+constexpr size_t kMaxTile = 144 * 1024;
+// Of the four-column tile: two CTAs an SM.
+constexpr size_t kMaxTile4 = 113 * 1024;
+
 template <int MODE, int PX>
 cudaError_t launch_mode(const float* img, int w, int h, int frames, const BlockRows& e, const RefBlock& rb, int metric,
                         float* out, float* stds, unsigned* mm, cudaStream_t st) {
   const size_t smem = Tile<PX>::smem(e.rw, e.rh, e.k);
-  if (smem > 48 * 1024) {
+  if (smem > kMaxTile) return cudaErrorInvalidValue;
+  if (smem > 48 * 1024) {  // (the same value in every call: another thread's launch may lie between)
     const cudaError_t err =
-        cudaFuncSetAttribute(k_block_map<MODE, PX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_block_map<MODE, PX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxTile);
     if (err != cudaSuccess) return err;
   }
   const dim3 grid((w + Tile<PX>::kX - 1) / Tile<PX>::kX, (h + kTileY - 1) / kTileY, frames);
@@ -297,13 +320,18 @@ cudaError_t launch_block_map(const float* img, int w, int h, int frames, const E
   rows.rw = e.rw;
   rows.rh = e.rh;
   for (int i = 0; i < e.k; i++) rows.hw[e.dy[i] + e.rh] = e.dx[i];  // the last column of a row stays
-  // Four pixel columns a thread where that still gives 1.5 CTAs an SM and the
-  // 128-column tiles pad the width to no more than 1.5 times what 32-column tiles do;
-  // else one. At 1024x1024 15x15 four take 80 us where one takes 94 (700x700: 55 and
-  // 61), at 400x300 15x15 (76 CTAs against 247) 44 and 40, at 513x512 9x9 40 and 37.
+  rows.single = 0;
+  while (rows.single < e.rh && rows.hw[rows.single] == 0) rows.single++;
+  // Four pixel columns a thread where that still gives 1.5 CTAs an SM, the
+  // 128-column tiles pad the width to no more than 1.5 times what 32-column tiles do, and
+  // two tiles fit an SM; else one. At 1024x1024 15x15 four take 80 us where one takes 94
+  // (700x700: 55 and 61), at 400x300 15x15 (76 CTAs against 247) 44 and 40, at 513x512 9x9
+  // 40 and 37; of tall blocks at 1024x1024, 3x81 (two tiles an SM) 88 and 93, 3x101 (one)
+  // 122 and 102, and from 3x195 on the tile fits no SM.
   const int tiles = (w + Tile<4>::kX - 1) / Tile<4>::kX, ys = (h + kTileY - 1) / kTileY;
   const bool four = (long long)tiles * ys * frames * 2 >= 3LL * num_sms &&
-                    2 * tiles * Tile<4>::kX <= 3 * ((w + 31) / 32 * 32);
+                    2 * tiles * Tile<4>::kX <= 3 * ((w + 31) / 32 * 32) &&
+                    Tile<4>::smem(e.rw, e.rh, e.k) <= kMaxTile4;
   if (four) return launch_px<4>(img, w, h, frames, rows, rb, metric, out, stds, mm, st);
   return launch_px<1>(img, w, h, frames, rows, rb, metric, out, stds, mm, st);
 }
