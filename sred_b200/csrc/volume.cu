@@ -442,9 +442,9 @@ struct Grid {
   __device__ __forceinline__ float at(int n) const { return (float)n / f2 / f1; }
 };
 
-// A run's increment where no element ties or is 2^22 ulp or more; with one that does, or
-// a NaN, *odd is set and run_steps gives it. Rounds by adding 1.5 2^23 (conversions issue
-// at an eighth of the rate).
+// A run's increment where no element ties or rounds to 2^22 ulp or more; with one that does,
+// or a NaN, *odd is set and run_steps gives it. Rounds by adding 1.5 2^23 (conversions issue
+// at an eighth of the rate); from 2^22 - 0.5 on that sum is 2^24, past the low 23 bits.
 __device__ __forceinline__ int run_increment(const float* run, const Grid& g, bool* odd) {
   const float magic = 12582912.0f;
   int sum = 0;
@@ -452,7 +452,7 @@ __device__ __forceinline__ int run_increment(const float* run, const Grid& g, bo
 #pragma unroll
   for (int j = 0; j < kSumRun; j++) {
     const float t = run[j] * g.f1 * g.f2, m = t + magic;
-    o |= !(t < 4194304.0f) || fabsf(t - (m - magic)) == 0.5f;
+    o |= !(t < 4194303.5f) || fabsf(t - (m - magic)) == 0.5f;
     sum += (int)(__float_as_uint(m) & 0x7fffffu);
   }
   *odd = o;
