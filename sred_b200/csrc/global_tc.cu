@@ -140,12 +140,21 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// The epilogue's arrivals only say that this warp's reads of a buffer are done
-// (their values are in registers), so they are relaxed: a releasing arrive waits
-// for the warp's row-sum atomics in flight to reach L2, 550 clocks a tile at CTA
-// scope and 1,500 at cluster scope.
-__device__ __forceinline__ void mbar_arrive_done_reading(uint32_t bar) {
+// The epilogue's arrivals hand a buffer that this warp has read to the copies or MMAs that
+// overwrite it.
+// The accumulator's: tensor memory, whose reads tcgen05.wait::ld completes and
+// tcgen05.fence::before_thread_sync orders before the arrival, so that one is relaxed (a release
+// at cluster scope cost 1,500 clocks a tile).
+__device__ __forceinline__ void mbar_arrive_tmem(uint32_t bar) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// The shared-memory buffers' (barriers of this CTA): one fence orders the warp's reads before
+// them, the lanes' by the __syncwarp that precedes it. It waits for the warp's row-sum
+// atomics in flight to reach L2 too, so it stands before a tile's, when the previous tile's
+// are long there: behind them it cost 550 clocks a tile.
+__device__ __forceinline__ void fence_reads() { asm volatile("fence.acq_rel.cta;" ::: "memory"); }
+__device__ __forceinline__ void mbar_arrive_fenced(uint32_t bar) {
+  asm volatile("mbarrier.arrive.relaxed.cta.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 __device__ __forceinline__ void cluster_sync() {
@@ -1319,7 +1328,6 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
         }
         if (!warp_wait(b_accf + 8 * b, (tile >> 1) & 1, g, ST_TIMEOUT_EPI)) { ok = false; break; }
         tc_fence_after();
-        if (ew == 8 * set && lane == 0) mbar_arrive_done_reading(b_aempty + 8 * last);
         float rsum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if constexpr (kPhase == 1 || METRIC == kDebugDot || METRIC == kDebugSum) {
           tile_pairs<METRIC, true, kPhase == 1>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
@@ -1332,11 +1340,27 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
           else if (mode == kPairExact)
             tile_pairs<METRIC, true, false>(taddr, rsp, csw, cacc, p0, q0, g.ec, rsum);
         }
-        // This warp's reads of the accumulator are complete: the MMA of the tile
-        // after the next may overwrite it while the row sums are finished.
+        // This warp's reads of the accumulator are complete: the MMA of the tile after the next
+        // may overwrite it while the row sums are finished. So are its reads of the row (and,
+        // at this set's last tile of the item, the column) parameters, and the MMAs that read
+        // the tile's last operands, which a warp passes on. One set of 16 warps gives back two slots
+        // of row parameters at a time and takes turns at passing on, for fewer fences: every tile
+        // SSIM took 1.2% longer with them and NRMSE 6%, so 1% and 0.5%. Two sets hide a fence a
+        // tile (0.5-1%; 2% at 256x256 5x5).
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_done_reading(acce + 8 * b);
+        const bool pass_on = SETS == 2 ? ew == 8 * set : tile % EW == (uint32_t)ew;
+        const bool rows_read = SETS == 2 || b == 1, cols_read = rb + SETS * M >= rb1;
+        if (lane == 0) {
+          mbar_arrive_tmem(acce + 8 * b);
+          if (rows_read || cols_read || pass_on) {
+            fence_reads();
+            if (rows_read) mbar_arrive_fenced(b_rempty + 8 * rsl);
+            if (SETS == 1 && rows_read) mbar_arrive_fenced(b_rempty + 8 * (rsl - 1));
+            if (cols_read) mbar_arrive_fenced(b_cempty + 8 * cs);
+            if (pass_on) mbar_arrive_fenced(b_aempty + 8 * last);
+          }
+        }
         // Row sums: 4 lanes per row, then one FP64 atomic add per row and warp (256 a
         // tile, a tenth of the rate the L2 sustains; combining the two halves' warps
         // in shared memory first costs more issue slots than it saves).
@@ -1346,11 +1370,15 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
         const int p = p0 + quarter * 32 + (lane >> 2) + 8 * krow;
         if (p < g.ec.n && !(kPhase == 0 && mode == kZero)) atomicAdd(g.num + p, (double)z);
         __syncwarp();  // (the scratch is rewritten for the next tile)
-        if (lane == 0) mbar_arrive_done_reading(b_rempty + 8 * rsl);
       }
       if (!ok) break;
-      // Column sums of the item.
-      if (any) {
+      if (!any) {  // (the slot's ranges were read all the same)
+        __syncwarp();
+        if (lane == 0) {
+          fence_reads();
+          mbar_arrive_fenced(b_cempty + 8 * cs);
+        }
+      } else {  // column sums of the item
         float x[4 * CH];
 #pragma unroll
         for (int c = 0; c < CH; c++)
@@ -1358,8 +1386,6 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
           for (int r = 0; r < 2; r++) f2_split(cacc[c][r], x[(c * 2 + r) * 2], x[(c * 2 + r) * 2 + 1]);
         flush_columns<4 * CH>(x, q0, g.ec, g.num);
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive_done_reading(b_cempty + 8 * cs);
     }
     };
     pass(std::integral_constant<int, 0>{});
