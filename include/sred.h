@@ -33,7 +33,8 @@ typedef enum {
 } sred_status;
 
 /* Contraction engine of the global map. SRED_ENGINE_TC: split-FP16 tcgen05
- * tensor-core Gram with FP32 accumulation (u = hi + mid, 22 significand bits);
+ * tensor-core Gram with FP32 accumulation (u = hi + mid to 2^-23, and a third part while
+ * 6 K <= 128);
  * SRED_ENGINE_FP32: plain FP32 CUDA-core Gram.
  * Both share moments, the symmetric schedule (each unordered block pair
  * evaluated once), the pair terms and the denominators. Abs-diff needs no

@@ -53,23 +53,32 @@ struct BlockParams {
   float pad0, pad1, pad2;
 };
 
-// Split-FP16 operand of the tensor-core engine: u = hi + mid, hi = fp16(u 2^14) and
-// mid = fp16(u 2^14 - hi) (|u| <= 1, so hi <= 2^14 and every mid down to u = 2^-16
-// keeps its 11 bits). Dot products hi.hi + mid.hi + hi.mid carry 22 significand
-// bits; G = 2^-28 of the accumulated value.
+// Split-FP16 operand of the tensor-core engine: u = hi + mid (+ lo), hi = fp16(u 2^14),
+// mid = fp16(u 2^14 - hi), lo = fp16(u 2^14 - hi - mid) (|u| <= 1, so hi <= 2^14 and every
+// mid down to u = 2^-16 keeps its 11 bits); G = 2^-28 of the accumulated value.
+//   two parts:   hi.hi + hi.mid + mid.hi; an element is off by up to 2^-23 of its binade and the
+//                product by mid.mid (2^-22 at most)
+//   three parts: hi.hi + hi.mid + mid.hi + mid.mid + hi.lo + lo.hi: FP32-level elements. While
+//                6 K <= 128, where a tile's time is its epilogue's (split_parts).
 //
 // A row holds each part once. The row and the column operand are the same array:
 // the MMAs pair blocks of 16 elements of one with blocks of the other. K = 16 nb + r:
-//   [hi: nb blocks | mid: nb blocks | row tail: nt | column tail: nt],
+//   [hi: nb blocks | mid: nb blocks | lo: nb blocks | row tail: nt | column tail: nt],
 // the tails holding the last r elements of every part side by side, as
-// [hi|mid|hi] in the row tail and [hi|hi|mid] in the column tail, nt = ceil(3r / 16)
-// blocks: 3 nb + nt steps of 16 instead of 3 ceil(K / 16).
+// [mid|hi|hi] in the row tail and [hi|mid|hi] in the column tail ([lo|mid|hi|mid|hi|hi] and
+// [hi|mid|lo|hi|mid|hi] of three parts: smallest products first), nt blocks: 3 nb + nt steps
+// of 16 instead of 3 ceil(K / 16) (6 nb + nt of 6 ceil(K / 16)).
 struct SplitLayout {
-  int nb, r, nt, pitch;  // pitch: fp16 per row, a multiple of 32
+  int parts, nb, r, nt, pitch;  // pitch: fp16 per row, a multiple of 32
+  __host__ __device__ int steps() const { return parts * (parts + 1) / 2 * nb + nt; }
 };
+__host__ __device__ inline int split_parts(int K) { return 6 * K <= 128 ? 3 : 2; }
 __host__ __device__ inline SplitLayout split_layout(int K) {
-  const int nb = K / 16, r = K % 16, nt = (3 * r + 15) / 16;
-  return SplitLayout{nb, r, nt, 32 * (nb + nt)};
+  const int parts = split_parts(K);
+  int nb = K / 16, r = K % 16;
+  if (parts == 3 && r > 5) nb++, r = 0;  // (a padded block: fewer columns than a tail of six r)
+  const int nt = (parts * (parts + 1) / 2 * r + 15) / 16;
+  return SplitLayout{parts, nb, r, nt, (16 * (parts * nb + 2 * nt) + 31) / 32 * 32};
 }
 constexpr float kSplitScale = 16384.0f;
 constexpr float kSplitGScale = 1.0f / (16384.0f * 16384.0f);
@@ -81,27 +90,34 @@ inline bool nrmse_metric(int m) { return m == 2 /* kNrmse */ || m == 8 /* kNrmse
 // Element i of a block's vector (already scaled) into its row.
 __device__ __forceinline__ void store_split(__half* row, const SplitLayout& l, int i, double u) {
   const __half hi = __float2half_rn((float)u);
-  const __half mid = __float2half_rn((float)(u - (double)__half2float(hi)));
-  if (i < 16 * l.nb) {
+  const double rest = u - (double)__half2float(hi);
+  const __half mid = __float2half_rn((float)rest);
+  const __half lo = __float2half_rn((float)(rest - (double)__half2float(mid)));
+  const int n = 16 * l.nb;
+  if (i < n) {
     row[i] = hi;
-    row[16 * l.nb + i] = mid;
+    row[n + i] = mid;
+    if (l.parts == 3) row[2 * n + i] = lo;
+    return;
+  }
+  __half* a = row + l.parts * n + (i - n);
+  __half* b = a + 16 * l.nt;
+  const int r = l.r;
+  if (l.parts == 2) {
+    a[0] = mid, a[r] = hi, a[2 * r] = hi;
+    b[0] = hi, b[r] = mid, b[2 * r] = hi;
   } else {
-    __half* a = row + 32 * l.nb + (i - 16 * l.nb);
-    __half* b = a + 16 * l.nt;
-    a[0] = hi;
-    a[l.r] = mid;
-    a[2 * l.r] = hi;
-    b[0] = hi;
-    b[l.r] = hi;
-    b[2 * l.r] = mid;
+    a[0] = lo, a[r] = mid, a[2 * r] = hi, a[3 * r] = mid, a[4 * r] = hi, a[5 * r] = hi;
+    b[0] = hi, b[r] = mid, b[2 * r] = lo, b[3 * r] = hi, b[4 * r] = mid, b[5 * r] = hi;
   }
 }
-// The zeros behind the tails, one of 32 lanes' share.
-__device__ __forceinline__ void store_split_pad(__half* row, const SplitLayout& l, int lane) {
-  for (int i = 3 * l.r + lane; i < 16 * l.nt; i += 32) {
-    row[32 * l.nb + i] = __float2half_rn(0.0f);
-    row[32 * l.nb + 16 * l.nt + i] = __float2half_rn(0.0f);
-  }
+// The zeros behind the tails and behind the last block's elements, one of 32 lanes' share.
+__device__ __forceinline__ void store_split_pad(__half* row, const SplitLayout& l, int K, int lane) {
+  const __half zero = __float2half_rn(0.0f);
+  __half* tail = row + 16 * l.parts * l.nb;
+  for (int i = l.parts * (l.parts + 1) / 2 * l.r + lane; i < 16 * l.nt; i += 32) tail[i] = tail[16 * l.nt + i] = zero;
+  for (int i = K + lane; i < 16 * l.nb; i += 32)
+    for (int p = 0; p < l.parts; p++) row[16 * l.nb * p + i] = zero;
 }
 
 // a / b, correctly rounded, for many a and one b: y = RN(1/b) once, then

@@ -1,9 +1,10 @@
 // Split-FP16 tcgen05 engine of the global repetition map (sm_100a).
 //
 // G = <u_p, u_q> on the 5th-generation tensor cores, where each block's FP64 unit
-// vector u is split into two fp16 parts, u = hi + mid (common.cuh: SplitLayout),
-// and G = hi.hi + mid.hi + hi.mid with FP32 accumulation: an FP32-accurate dot
-// product (what is left out is below 2^-22 |u_p| |u_q|).
+// vector u is split into fp16 parts, u = hi + mid, and lo for small blocks (common.cuh:
+// SplitLayout), and G = hi.hi + mid.hi + hi.mid (+ mid.mid + lo.hi + hi.lo) with FP32
+// accumulation: what two parts leave out is below 3 2^-22 |u_p| |u_q| (mid.mid, and the
+// rounding of each mid).
 //
 // Symmetric schedule. Every per-pair term of the global map (weight, Pearson,
 // global SSIM, NRMSE; epilogue.cuh) is symmetric in (p, q), so each unordered
@@ -69,7 +70,7 @@ constexpr int kRowFloats = kRowSoaFloats;         // one 128-row block's paramet
 constexpr int kColFloats = col_soa_floats(kBN);   // one column tile's parameters
 constexpr int kMaxRun = 128;                      // row blocks per run (work item), at most
 constexpr int kBarBytes = 512;
-constexpr int kMaxMma = 64;                       // entries of the MMA table (3 nb + nt + 1 at most 58)
+constexpr int kMaxMma = 64;                       // entries of the MMA table (SplitLayout::steps() + 1 at most 58)
 constexpr int kTabBytes = kMaxMma * 8 + 16 * 4;
 constexpr size_t kSmemBudget = 227 * 1024;
 
@@ -94,7 +95,7 @@ struct Cfg {
 constexpr int kScratch = 32 + 128;                  // floats of f and g per epilogue warp
 
 struct TcArgs {
-  int nb, nt;                   // blocks of 16 per part and tail blocks (SplitLayout)
+  int parts, nb, nt;            // parts, blocks of 16 per part and tail blocks (SplitLayout)
   int nch, sc, nst, stages;     // chunks per tile, chunks per stage, stages per tile, ring depth
   int n_rb, n_ct;               // row blocks holding valid rows, column tiles
   int L, h;                     // row blocks per item (a run), L / (BN / 128)
@@ -1082,32 +1083,47 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // Operand offsets (16-byte units, within a stage and the column tile) of the
-  // tile's MMAs, in the order of the row operand's blocks: hi blocks with hi and
-  // mid, mid blocks with hi, row tails with column tails. A block of 16 fp16 is 32 B,
-  // four to a chunk.
+  // tile's MMAs. A block of 16 fp16 is 32 B, four to a chunk. Row part P meets the column parts
+  // 0 .. parts - 1 - P, in the order of the row operand's blocks: hi with hi and mid, mid with
+  // hi, row tails with column tails. Every MMA truncates the accumulator, so the products of
+  // three parts go smallest first where one stage holds the tile (5x5 Pearson: numerators off
+  // by -1.6e-7 +- 4.8e-8 in the order of the blocks, by -4.7e-8 +- 4.0e-8 so; two parts: 9x9
+  // SSIM takes 1% longer so).
   uint2* mma_tab = reinterpret_cast<uint2*>(sbase + (sBar + kBarBytes - base));
   uint32_t* mma_end = reinterpret_cast<uint32_t*>(mma_tab + kMaxMma);  // MMAs up to the end of each stage
   if (warp == 2) {
-    const int nb = g.nb, nt = g.nt, n = 3 * nb + nt;
+    const int parts = g.parts, nb = g.nb, nt = g.nt, n_full = parts * (parts + 1) / 2 * nb, n = n_full + nt;
     constexpr uint32_t kChunkU = kChunkBytes >> 4;
     for (int m = lane; m <= n; m += 32) {  // (entry n: read ahead, never used)
-      int qa, qb;
-      if (m < 2 * nb) {
-        qa = m >> 1;
-        qb = (m & 1) ? nb + qa : qa;
-      } else if (m < 3 * nb) {
-        qa = m - nb;
-        qb = qa - nb;
+      int qa = 0, qb = 0;
+      if (parts == 3 && g.nst == 1) {
+        if (m >= n - nb && m < n) {  // hi.hi
+          qa = qb = m - (n - nb);
+        } else if (m >= n_full - nb) {
+          qa = parts * nb + min(m - (n_full - nb), max(nt - 1, 0));
+          qb = qa + nt;
+        } else {
+          int s = parts - 1, i = m;  // the products of parts P + Q = s
+          while (i >= (s + 1) * nb) i -= (s + 1) * nb, s--;
+          qa = i / nb * nb + i % nb;
+          qb = (s - i / nb) * nb + i % nb;
+        }
+      } else if (m < n_full) {
+        int P = 0, i = m;
+        while (i >= (parts - P) * nb) i -= (parts - P) * nb, P++;
+        qa = P * nb + i / (parts - P);
+        qb = i % (parts - P) * nb + i / (parts - P);
       } else {
-        qa = min(m - nb, 2 * nb + nt - 1);
+        qa = parts * nb + min(m - n_full, max(nt - 1, 0));
         qb = qa + nt;
       }
       const uint32_t ca = (uint32_t)(qa >> 2) % (uint32_t)g.sc, cb = (uint32_t)(qb >> 2);
       mma_tab[m] = make_uint2(ca * kChunkU + 2 * (qa & 3), cb * (BH * kChunkU) + 2 * (qb & 3));
     }
     for (int st = lane; st < g.nst; st += 32) {
-      const int q1 = min(2 * nb + nt, 4 * (st + 1) * g.sc);
-      mma_end[st] = q1 <= nb ? 2 * q1 : q1 + nb;
+      int q = min(parts * nb + nt, 4 * (st + 1) * g.sc), m = max(q - parts * nb, 0);
+      for (int P = 0; P < parts; P++) m += (parts - P) * min(max(q - P * nb, 0), nb);
+      mma_end[st] = m;
     }
   }
   if (warp == 1) {  // the MMA warps of both CTAs own the TMEM allocation
@@ -1223,7 +1239,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
         // This thread's instructions between MMAs are tensor time (an MMA takes 128
         // clocks), so the operand offsets come from a table, one entry ahead.
         const uint32_t a0 = desc_lo(sA), b0 = desc_lo(sB), stage_u = stage_bytes >> 4;
-        const int nst = g.nst, n_mma = 3 * g.nb + g.nt;
+        const int nst = g.nst, n_mma = g.parts * (g.parts + 1) / 2 * g.nb + g.nt;
         for (int phase = 0; ok && phase < 2; phase++)
         for (ItemCursor cur = first_item<CTAS>(g); ok && cur.it < g.item1; cur.advance(g, n_clusters)) {
           int ct, rb0, rb1;
@@ -1545,6 +1561,7 @@ cudaError_t launch_gram_tc(const __half* U, int K, int n_pad, const BlockParams*
   if (ec.n <= 0) return cudaSuccess;
   const SplitLayout l = split_layout(K);
   TcArgs g;
+  g.parts = l.parts;
   g.nb = l.nb;
   g.nt = l.nt;
   g.nch = (l.pitch + kChunk - 1) / kChunk;

@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(256)
       }
       if (U)
         for (int i = K + lane; i < kp; i += 32) U[(size_t)j * kp + i] = 0.0f;
-      if (S) store_split_pad(S + (size_t)j * lay.pitch, lay, lane);
+      if (S) store_split_pad(S + (size_t)j * lay.pitch, lay, K, lane);
     }
   }
   a_lo = __reduce_max_sync(full, a_lo);
@@ -410,7 +410,7 @@ __global__ void k_pack_vectors(const float* __restrict__ u, int n, int K, float*
       for (int i = lane; i < kp; i += 32) U[(size_t)j * kp + i] = i < K ? u[(size_t)j * K + i] : 0.0f;
     if (S) {
       for (int i = lane; i < K; i += 32) store_split(S + (size_t)j * lay.pitch, lay, i, (double)u[(size_t)j * K + i]);
-      store_split_pad(S + (size_t)j * lay.pitch, lay, lane);
+      store_split_pad(S + (size_t)j * lay.pitch, lay, K, lane);
     }
   }
 }
