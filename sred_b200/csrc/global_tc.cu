@@ -363,6 +363,16 @@ struct SlabC {
   float alpha, beta, cf, sf, eg, kc;
 };
 
+// SSIM's 1/(sigma_p^2 + sigma_q^2 + c2): whether the mixed curvature of its logarithm,
+// h = 4 x y / (x^2 + y^2 + c2)^2 at x = sigma_p and y = sigma_q, stays near its value at the
+// slab's centres, which e = h ra rb holds. Over relative half ranges u and v of up to 1/16 it
+// changes by at most 6 (u + v) of itself, so the first-order term neglects at most
+// 6 (u + v) e: below 2^-22 here.
+__host__ __device__ inline bool ssim_split_bounded(float a, float ra, float b, float rb, float e) {
+  const float ab = a * b, x = ra * b, y = rb * a;  // u a b, v a b
+  return 16.0f * fmaxf(x, y) <= ab && e * (x + y) <= 3.8e-8f * ab;
+}
+
 // The form a slab takes. rg, cg: {centre of a, half range of a, centre of r, half range of r}.
 template <int METRIC>
 __device__ __forceinline__ int slab_mode(const float4& rg, const float4& cg, const EpiConsts& ec, SlabC& sc) {
@@ -390,8 +400,10 @@ __device__ __forceinline__ int slab_mode(const float4& rg, const float4& cg, con
     // derivative joins the first-order term. 2 sp sq G + c2 = 2 sp sq (G + c2/2 rp rq)
     // needs sigma > 0 and no overflow.
     const float sa = rg.x * ec.inv_wscale, sb = cg.x * ec.inv_wscale;
-    const float S = fmaf(sa, sa, fmaf(sb, sb, ec.c2));
-    sc.kc += 4.0f * sa * sb * ec.inv_wscale * ec.inv_wscale / (S * S);
+    const float S = rcp_approx(fmaf(sa, sa, fmaf(sb, sb, ec.c2))) * ec.inv_wscale;
+    const float h = 4.0f * (sa * S) * (sb * S);
+    sc.kc += h;
+    ok = ok && ssim_split_bounded(rg.x, rg.y, cg.x, cg.y, h * rg.y * cg.y);
     ok = ok && rg.z - rg.w > 0.0f && cg.z - cg.w > 0.0f && (rg.z + rg.w) * (cg.z + cg.w) < 1e25f;
   }
   const float e = sc.kc * rg.y * cg.y;
