@@ -373,6 +373,11 @@ __host__ __device__ inline bool ssim_split_bounded(float a, float ra, float b, f
   return 16.0f * fmaxf(x, y) <= ab && e * (x + y) <= 3.8e-8f * ab;
 }
 
+// Whether the row factors 2^-(a_p - beta)^2 of a slab, D between the centres, stay normal numbers.
+// One that flushes to 0 takes weights of up to 2^-78 with it (g reaches 2^48); they matter to
+// weighted NRMSE alone, whose self pair is 0: of a block among equal ones they are the whole sum.
+__host__ __device__ inline bool row_factors_normal(float D, float ra) { return fabsf(D) + ra <= 11.2f; }
+
 // The form a slab takes. rg, cg: {centre of a, half range of a, centre of r, half range of r}.
 template <int METRIC>
 __device__ __forceinline__ int slab_mode(const float4& rg, const float4& cg, const EpiConsts& ec, SlabC& sc) {
@@ -385,6 +390,7 @@ __device__ __forceinline__ int slab_mode(const float4& rg, const float4& cg, con
   sc.kc = 1.3862944f;  // 2 ln2
   if (fabsf(D) - rg.y - cg.y > kZeroDist) return kZero;
   bool ok = fabsf(D) * cg.y <= 24.0f;
+  if (METRIC == kNrmseW) ok = ok && row_factors_normal(D, rg.y);
   if (METRIC == kPearson) {
     const float ra = rcp_approx(rg.x), rb = rcp_approx(cg.x);
     const float t0 = ec.tau * ra * rb, c = rcp_approx(1.0f + t0), u = 1.442695f * t0 * c;

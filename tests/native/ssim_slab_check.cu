@@ -1,8 +1,9 @@
-// Host-side check of the bound that lets a slab of SSIM pairs take the factorised form: for
+// Host-side check of the bounds that let a slab of pairs take the factorised form. SSIM's: for
 // random slabs (centres and half ranges of the weight argument a over many decades), the form's
 // value against the exact one in 64 bits, in the slab's corners and along its edges. Prints
-// the slabs tried, the slabs accepted and the largest relative error of an accepted one. Built and
-// run by tests/test_ssim_slab.py.
+// the slabs tried, the slabs accepted, those with a wide range and the largest relative error of an
+// accepted one. Weighted NRMSE's: no row factor is subnormal (exit code 1 otherwise). Built and run by
+// tests/test_ssim_slab.py.
 #include "../../sred_b200/csrc/global_tc.cu"
 
 #include <cmath>
@@ -36,6 +37,14 @@ int main() {
       worst = std::fmax(worst, std::fabs(split * (x * x + y * y + c2) / std::exp2(2 * dp * dq) - 1));
     }
   }
+  // Row factors of accepted slabs: the smallest one, in the FP32 arithmetic of the kernel.
+  float least = 1.0f;
+  for (int i = 0; i < 1000000; i++) {
+    const float D = (float)uni(-13, 13), ra = (float)(i % 2 ? uni(0, 4) : decades(-6, 0));
+    if (!row_factors_normal(D, ra)) continue;
+    for (float d : {D - ra, D + ra}) least = std::fmin(least, std::exp2(-d * d));
+  }
+  if (!(least >= 1.17549435e-38f)) return 1;
   std::printf("%lld %lld %lld %.3e\n", tried, accepted, wide, worst);
   return 0;
 }

@@ -1,6 +1,7 @@
 """What SSIM's factorised slabs neglect is bounded (global_tc.cu, ssim_split_bounded, compiled
 for the host): 2^-21 for the weight without its first-order term or (6.9e-4)^2 / 2 with it, and
-2^-22 for the curvature of 1/(sigma_p^2 + sigma_q^2 + c2). No GPU is used."""
+2^-22 for the curvature of 1/(sigma_p^2 + sigma_q^2 + c2); weighted NRMSE's row factors are
+normal numbers (row_factors_normal). No GPU is used."""
 import shutil
 import subprocess
 from pathlib import Path
