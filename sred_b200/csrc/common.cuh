@@ -196,6 +196,18 @@ struct TcPlan {
 };
 bool plan_gram_tc(int K, TcPlan* plan);
 
+// What a status word of the tensor-core kernel other than 0 means (kTcUnaligned: shared memory
+// not on the 1,024-byte boundary the swizzled tiles need; the others: the role whose wait ran out).
+constexpr int kTcUnaligned = 5;
+inline sred_status tc_status_error(int status, const char** msg) {
+  if (status == kTcUnaligned) {
+    *msg = "tensor-core kernel: shared memory not aligned to 1,024 bytes";
+    return SRED_ERR_LAUNCH;
+  }
+  *msg = "tensor-core pipeline wait exceeded its bound";
+  return SRED_ERR_TIMEOUT;
+}
+
 // Test hooks of the tensor-core engine: a wait limit (0: 4 s) and a tile whose
 // operand copies the producer never issues (-1: none), so that the pipeline
 // waits run out with nothing in flight.

@@ -74,7 +74,7 @@ constexpr int kMaxMma = 64;                       // entries of the MMA table (S
 constexpr int kTabBytes = kMaxMma * 8 + 16 * 4;
 constexpr size_t kSmemBudget = 227 * 1024;
 
-enum { ST_OK = 0, ST_TIMEOUT_PRODUCER = 1, ST_TIMEOUT_MMA = 2, ST_TIMEOUT_EPI = 3, ST_TIMEOUT_DRAIN = 4, ST_ALIGNMENT = 5 };
+enum { ST_OK = 0, ST_TIMEOUT_PRODUCER = 1, ST_TIMEOUT_MMA = 2, ST_TIMEOUT_EPI = 3, ST_TIMEOUT_DRAIN = 4, ST_ALIGNMENT = kTcUnaligned };
 
 // Epilogue sets. Two: warps 0-7 take the even tiles, warps 8-15 the odd ones, each
 // warp 32 rows x 128 columns, so that one set's fixed work per tile (waits, row

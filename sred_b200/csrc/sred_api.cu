@@ -526,7 +526,11 @@ sred_status global_gram(sred_ctx* c, const GState& gs, cudaStream_t st, int shar
       int status = 0;
       CK(cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));
-      if (status) return fail(c, SRED_ERR_TIMEOUT, "tensor-core pipeline wait exceeded its bound");
+      if (status) {
+        const char* msg;
+        const sred_status e = tc_status_error(status, &msg);
+        return fail(c, e, msg);
+      }
     }
   }
   CK(cudaEventRecord(c->ev[2], st));
@@ -2168,7 +2172,11 @@ sred_status sred_debug_gram_rowdot(sred_ctx* c, int engine, const float* u, cons
     int status = 0;
     CK(cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (status) return fail(c, SRED_ERR_TIMEOUT, "tensor-core pipeline wait exceeded its bound");
+    if (status) {
+      const char* msg;
+      const sred_status e = tc_status_error(status, &msg);
+      return fail(c, e, msg);
+    }
   }
   CK(cudaMemcpyAsync(num, d_num, n * sizeof(double), cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(den, d_den, n * sizeof(double), cudaMemcpyDeviceToHost, st));
