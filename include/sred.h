@@ -337,8 +337,9 @@ sred_status sred_block_map_2d_device_noalloc(const char *metric, const float *d_
  * for caller-given vectors u (n x k, row-major) and weights w1, w2,
  * num[p] = sum_q <u_p, u_q> w1[p] w1[q] and den[p] = sum_q (w2[p] + w2[q]),
  * symmetric pair terms like the maps' own, computed by the
- * chosen engine's all-pairs kernel (the tensor-core engine splits u into
- * fp16 hi/mid without normalising or scaling it: |u| below 65504). */
+ * chosen engine's all-pairs kernel (the tensor-core engine splits u into fp16
+ * parts without normalising it, scaled by the power of two that brings its
+ * largest element to 2^13: vectors below 2^-16 of it lose bits). */
 sred_status sred_debug_gram_rowdot(sred_ctx *ctx, int engine, const float *u, const float *w1,
                                    const float *w2, int n, int k, double *num, double *den);
 

@@ -30,7 +30,7 @@ cudaError_t launch_pack(const float* img, int W, const Ellipse& e, const int* of
 __global__ void k_finalize(const int* slot, int W, int H, int rw, int rh, const double* num, const double* den,
                            const BlockParams* params, const double* sums, int n_flat, int metric, double sk,
                            double n_pixels, const float* mask, int apply_mask, float* out);
-__global__ void k_pack_vectors(const float* u, int n, int K, float* U, int kp, __half* S);
+__global__ void k_pack_vectors(const float* u, int n, int K, float scale, float* U, int kp, __half* S);
 // Per-plane min/max words before a range is taken: {ordered +inf, ordered -inf} per plane
 // (a kernel rather than a copy from pageable host memory, which would wait
 // for the stream to drain).

@@ -398,8 +398,8 @@ cudaError_t launch_pack(const float* img, int W, const Ellipse& e, const int* of
 }
 
 // Diagnostics: pack caller-given vectors (n x K, FP32) as operands without
-// normalising or scaling them (one warp per row), as FP32 or split FP16.
-__global__ void k_pack_vectors(const float* __restrict__ u, int n, int K, float* __restrict__ U, int kp,
+// normalising them (one warp per row), as FP32 or, scaled, as split FP16.
+__global__ void k_pack_vectors(const float* __restrict__ u, int n, int K, float scale, float* __restrict__ U, int kp,
                                __half* __restrict__ S) {
   const int lane = threadIdx.x & 31;
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -409,7 +409,7 @@ __global__ void k_pack_vectors(const float* __restrict__ u, int n, int K, float*
     if (U)
       for (int i = lane; i < kp; i += 32) U[(size_t)j * kp + i] = i < K ? u[(size_t)j * K + i] : 0.0f;
     if (S) {
-      for (int i = lane; i < K; i += 32) store_split(S + (size_t)j * lay.pitch, lay, i, (double)u[(size_t)j * K + i]);
+      for (int i = lane; i < K; i += 32) store_split(S + (size_t)j * lay.pitch, lay, i, (double)u[(size_t)j * K + i] * (double)scale);
       store_split_pad(S + (size_t)j * lay.pitch, lay, K, lane);
     }
   }

@@ -2146,16 +2146,25 @@ sred_status sred_debug_gram_rowdot(sred_ctx* c, int engine, const float* u, cons
   std::vector<BlockParams> hp(n_pad);
   std::memset(hp.data(), 0, n_pad * sizeof(BlockParams));
   for (int i = 0; i < n; i++) { hp[i].a = w1[i]; hp[i].r = w2[i]; }
+  // the tensor-core engine's FP16 parts: the largest |u| to [2^13, 2^14), by a power of two
+  int e2 = 0;
+  if (engine == SRED_ENGINE_TC) {
+    float m = 0.0f;
+    for (size_t i = 0; i < (size_t)n * k; i++)
+      if (std::isfinite(u[i])) m = std::max(m, std::fabs(u[i]));
+    if (m > 0.0f) e2 = std::min(60, std::max(-60, 13 - std::ilogb(m)));
+  }
   CK(cudaMemcpyAsync(d_u, u, (size_t)n * k * sizeof(float), cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_params, hp.data(), n_pad * sizeof(BlockParams), cudaMemcpyHostToDevice, st));
   CK(cudaMemsetAsync(d_rmax, 0, (n_pad / 128) * sizeof(float), st));
   CK(cudaMemsetAsync(d_num, 0, n_pad * sizeof(double), st));
   CK(cudaMemsetAsync(d_den, 0, n_pad * sizeof(double), st));
   k_pack_vectors<<<grid_for((size_t)n * 32, 256, 8 * c->num_sms), 256, 0, st>>>(
-      d_u, n, k, d_U, kp, d_S);
+      d_u, n, k, std::ldexp(1.0f, e2), d_U, kp, d_S);
   CK(cudaGetLastError());
   // num and den are two sums over the same schedule
   EpiConsts ec{kDebugDot, n, 1.0f, kC1, kC2}, ed{kDebugSum, n, 1.0f, kC1, kC2};
+  ec.gscale = std::ldexp(1.0f, -2 * e2);
   if (engine == SRED_ENGINE_FP32) {
     CK(launch_gram_fp32(d_U, kp, d_params, d_rmax, ec, d_num, c->num_sms, st));
     CK(launch_gram_fp32(d_U, kp, d_params, d_rmax, ed, d_den, c->num_sms, st));
