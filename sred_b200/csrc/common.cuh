@@ -13,6 +13,7 @@ constexpr float kC1 = 0.0001f;      // cl/kernelGetGlobalSsim2D.cl:102
 constexpr float kC2 = 0.0009f;      // cl/kernelGetGlobalSsim2D.cl:104
 constexpr int kMaxK = 512;          // largest ellipse block size accepted
 constexpr int kMaxGlobalK = 212;    // largest block of a global map with a contraction
+constexpr size_t kMaxSmem = 227 * 1024;  // shared memory of a CTA
 
 enum Metric { kPearson = 0, kSsim = 1, kNrmse = 2, kAbsDiff = 3, kCosine = 4,
               kDebugDot = 5 /* diagnostics: num += G a_p a_q */,

@@ -255,10 +255,11 @@ cudaError_t launch_gram_fp32(const float* U, int kp, const BlockParams* params, 
   if (g.item0 >= g.item1) return cudaSuccess;
   size_t smem = (size_t)2 * kp * (BM + 4) * sizeof(float) + 2 * BM * sizeof(BlockParams);
   const int grid = (int)std::min<long long>(g.item1 - g.item0, 2LL * num_sms);
-  cudaError_t e;
-#define SRED_LAUNCH(M)                                                                           \
-  e = cudaFuncSetAttribute(k_gram_fp32<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-  if (e != cudaSuccess) return e;                                                                \
+  if (smem > kMaxSmem) return cudaErrorInvalidValue;
+  cudaError_t e;  // (the same attribute in every call: another thread's launch may lie between)
+#define SRED_LAUNCH(M)                                                                               \
+  e = cudaFuncSetAttribute(k_gram_fp32<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem); \
+  if (e != cudaSuccess) return e;                                                                    \
   k_gram_fp32<M><<<grid, NT, smem, st>>>(g);
   switch (ec.metric) {
     case kPearson: SRED_LAUNCH(kPearson); break;

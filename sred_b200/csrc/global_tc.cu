@@ -72,7 +72,6 @@ constexpr int kMaxRun = 128;                      // row blocks per run (work it
 constexpr int kBarBytes = 512;
 constexpr int kMaxMma = 64;                       // entries of the MMA table (SplitLayout::steps() + 1 at most 58)
 constexpr int kTabBytes = kMaxMma * 8 + 16 * 4;
-constexpr size_t kSmemBudget = 227 * 1024;
 
 enum { ST_OK = 0, ST_TIMEOUT_PRODUCER = 1, ST_TIMEOUT_MMA = 2, ST_TIMEOUT_EPI = 3, ST_TIMEOUT_DRAIN = 4, ST_ALIGNMENT = kTcUnaligned };
 
@@ -1519,7 +1518,7 @@ bool plan_shape(int K, int ctas, bool whole, TcPlan* p) {
   const SplitLayout l = split_layout(K);
   const int nch = (l.pitch + kChunk - 1) / kChunk;
   const int cols = nch * (kBN / kBM / ctas);  // chunks of 128 rows of the column tile in a CTA
-  const int chunks = (int)((kSmemBudget - kFixedSmem) / kChunkBytes) - cols;  // of the ring
+  const int chunks = (int)((kMaxSmem - kFixedSmem) / kChunkBytes) - cols;  // of the ring
   const int sc = whole ? nch : 1;
   if (chunks < 3 * sc) return false;
   const int st = std::min(kMaxStages, chunks / sc);
@@ -1618,7 +1617,8 @@ cudaError_t launch_gram_tc(const __half* U, int K, int n_pad, const BlockParams*
   const int smem = (int)plan.smem;
   // one CTA per SM: as many CTAs or pairs of CTAs as can be resident at once
   auto launch = [&](auto kern) -> cudaError_t {
-    cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // (the same value in every call: another thread's launch may lie between)
+    cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
     if (r != cudaSuccess) return r;
     int groups = num_sms;
     if (plan.ctas == 2) {
