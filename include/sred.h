@@ -217,8 +217,9 @@ sred_status sred_block_map_2d_device(sred_ctx *ctx, const char *metric, const fl
  * loop): img and out are frames*w*h floats in host memory, each frame mapped
  * and normalised on its own, exactly as sred_block_map_2d_device maps them.
  * The stack moves in chunks of chunk_frames frames (0: an eighth of the
- * stack, in 2 to 32 MiB) through two device slots, so the upload of one chunk, the map of the
- * previous one and the download of the one before run at the same time; with
+ * stack, in 2 to 32 MiB, or 32 MiB if out is not page-locked) through two
+ * device slots, so the upload of one chunk, the map of the previous one and
+ * the download of the one before run at the same time; with
  * page-locked host buffers the copies run concurrently with the kernels.
  * Returns when out is complete (or, on an error, when no copy touches img or
  * out any more). */

@@ -1975,13 +1975,12 @@ sred_status sred_block_map_2d_stack(sred_ctx* c, const char* metric, const float
   if (w <= 0 || h <= 0) return fail(c, SRED_ERR_ARG, "bad dimensions");
   if (frames < 1 || chunk_frames < 0) return fail(c, SRED_ERR_ARG, "frames must be >= 1 and chunk_frames >= 0");
   const size_t plane = (size_t)w * h;
-  // default chunk: an eighth of the stack, in 2 to 32 MiB: only the first upload
-  // and the last download overlap nothing, and a chunk's copies stay long against
-  // its launches (24 frames of 512x512, 11x11 NRMSE: 1182 us in one chunk, 804 in chunks)
   size_t chunk = chunk_frames;
   if (!chunk) {
-    const size_t bytes = std::min<size_t>(std::max<size_t>((size_t)frames * plane / 2, (size_t)2 << 20), (size_t)32 << 20);
-    chunk = bytes / (plane * sizeof(float));
+    cudaPointerAttributes at;
+    const bool pageable = cudaPointerGetAttributes(&at, out) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    chunk = stack_chunk(frames, plane, pageable);
   }
   chunk = std::max<size_t>(1, std::min<size_t>(chunk, std::min(frames, 65535)));
   const int nchunks = (int)((frames + chunk - 1) / chunk);
