@@ -17,9 +17,11 @@
 // A block adds nothing to its own numerator, so one whose nearest neighbours are far, or
 // equal, has a sum as small as their weight, while the polynomial's error goes with all that
 // is near: 6e-11 of the blocks within a few units, 2e-6 of a sum over blocks 5.5 away, 7e-4
-// at 7.5. The 10-point polynomial on the same nodes tells: it is off by 2 to 25 times as much
-// wherever the 12-point one is off by more than 1e-7, and where the two differ by more than kAbsTol of the
-// numerator, k_abs_direct takes the block.
+// at 7.5. The 10-point polynomial on the same nodes tells: wherever the 12-point one is off by
+// more than 1e-7 the two differ by 2 (blocks 11 away) to 25 times that error (5 away; 12 times
+// among equal ones), and where they differ by more than kAbsTol of the numerator, k_abs_direct
+// takes the block: an error of 2.5e-6 at most, 4e-7 where terms are not about to vanish; an FP32
+// pair term is off by 3e-6.
 // n x (nodes + 512) terms instead of n^2 / 2: a map of 500x381, 7x7 (115,000 blocks)
 // took 5.6 ms with the pair kernel and takes 0.37. A range of a without a node table (weights.cuh), or one
 // whose node-by-slice table exceeds kAbsTable, takes the pair kernel
@@ -36,7 +38,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kPer = kAbsSlice / kThreads;
 constexpr int kGroup = 8;  // nodes per step
-constexpr double kAbsTol = 5e-7;
+constexpr double kAbsTol = 5e-6;
 constexpr int kFlagWords = kAbsSlice / 32;
 constexpr int kParts = 32;  // shares of the slices that a flagged slice's sums are cut into
 constexpr int kBlocks = 8;  // flagged blocks at a time
@@ -224,11 +226,13 @@ __global__ void __launch_bounds__(kThreads) k_abs_direct(const float* __restrict
     }
     __syncthreads();
     for (int k0 = 0; k0 < m; k0 += kBlocks) {
-      float a[kBlocks];
+      float a[kBlocks], some[kBlocks];  // sums of up to 8 terms
       double acc[kBlocks];
+      int steps = 0;
 #pragma unroll
       for (int k = 0; k < kBlocks; k++) {
         a[k] = sorted[at[min(k0 + k, m - 1)]];
+        some[k] = 0.0f;
         acc[k] = 0.0;
       }
       for (int t = part; t < ns; t += kParts) {
@@ -243,15 +247,22 @@ __global__ void __launch_bounds__(kThreads) k_abs_direct(const float* __restrict
         }
 #pragma unroll
         for (int k = 0; k < kBlocks; k++) {
-          float sum = 0.0f;
 #pragma unroll
           for (int j = 0; j < kPer; j++) {
             const float d = a[k] - q[j];
-            sum = fmaf(fabsf(d), ex2_approx(-d * d), sum);
+            some[k] = fmaf(fabsf(d), ex2_approx(-d * d), some[k]);
           }
-          acc[k] += (double)sum;
+        }
+        if ((++steps & 3) == 0) {
+#pragma unroll
+          for (int k = 0; k < kBlocks; k++) {
+            acc[k] += (double)some[k];
+            some[k] = 0.0f;
+          }
         }
       }
+#pragma unroll
+      for (int k = 0; k < kBlocks; k++) acc[k] += (double)some[k];
       // 8 sums over 32 lanes: lane l ends with sum l & 7
 #pragma unroll
       for (int r = 0; r < 3; r++) {
@@ -281,7 +292,7 @@ __global__ void __launch_bounds__(kThreads) k_abs_direct(const float* __restrict
 int abs_slices(int n) { return (n + kAbsSlice - 1) / kAbsSlice; }
 
 size_t abs_table_doubles(int n) {
-  return 2 * std::min<size_t>(kAbsTable, (size_t)kDenNodes * std::max(1, abs_slices(n)));
+  return 2 * std::min<size_t>(kAbsTable, (size_t)kAbsNodes * std::max(1, abs_slices(n)));
 }
 
 // (the flags of the slices and their list follow the keys' use: kFlagWords + 1 words a slice, and the count)

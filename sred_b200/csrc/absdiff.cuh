@@ -7,11 +7,12 @@ namespace sred {
 
 constexpr int kAbsSlice = 512;         // blocks per slice, in order of a
 constexpr int kAbsTable = 4 << 20;     // doubles of one node-by-slice table, at most
+constexpr int kAbsNodes = 1 << 16;     // nodes of the tables, at most
 
 // Nodes of the tables for ns slices and its first node (0: the pair kernel runs instead).
 __device__ __forceinline__ int abs_grid(const unsigned* __restrict__ arange, int ns, double* x0) {
   const int m = node_grid(arange, x0);
-  return (long long)m * ns <= kAbsTable ? m : 0;
+  return m <= kAbsNodes && (long long)m * ns <= kAbsTable ? m : 0;
 }
 
 int abs_slices(int n);

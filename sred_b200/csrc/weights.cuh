@@ -5,7 +5,7 @@
 namespace sred {
 
 constexpr int kDenSlice = 2048;    // blocks per CTA of the node sums
-constexpr int kDenNodes = 16384;   // node table (doubles)
+constexpr int kDenNodes = 1 << 18; // node table (doubles): a-ranges of up to 32,766
 
 // Functions of a block's a as sums over all blocks: nodes kNodeH apart and a
 // 12-point Lagrange polynomial between them (weights.cu: how accurate).
