@@ -12,7 +12,7 @@ constexpr float kEps = 0.0000001f;  // java/Utils.java:20 (Utils.EPSILON)
 constexpr float kC1 = 0.0001f;      // cl/kernelGetGlobalSsim2D.cl:102
 constexpr float kC2 = 0.0009f;      // cl/kernelGetGlobalSsim2D.cl:104
 constexpr int kMaxK = 512;          // largest ellipse block size accepted
-constexpr int kMaxGlobalK = 212;    // largest block of a global map with a contraction
+constexpr int kMaxGlobalK = 212;    // largest block of a global map
 constexpr size_t kMaxSmem = 227 * 1024;  // shared memory of a CTA
 
 enum Metric { kPearson = 0, kSsim = 1, kNrmse = 2, kAbsDiff = 3, kCosine = 4,
@@ -93,20 +93,24 @@ __device__ __forceinline__ void store_split(__half* row, const SplitLayout& l, i
   const __half hi = __float2half_rn((float)u);
   const double rest = u - (double)__half2float(hi);
   const __half mid = __float2half_rn((float)rest);
+  const int n = 16 * l.nb, r = l.r;
+  __half* a = row + l.parts * n + (i - n);  // (i in the tail)
+  __half* b = a + 16 * l.nt;
+  if (l.parts == 2) {
+    if (i < n) {
+      row[i] = hi;
+      row[n + i] = mid;
+    } else {
+      a[0] = mid, a[r] = hi, a[2 * r] = hi;
+      b[0] = hi, b[r] = mid, b[2 * r] = hi;
+    }
+    return;
+  }
   const __half lo = __float2half_rn((float)(rest - (double)__half2float(mid)));
-  const int n = 16 * l.nb;
   if (i < n) {
     row[i] = hi;
     row[n + i] = mid;
-    if (l.parts == 3) row[2 * n + i] = lo;
-    return;
-  }
-  __half* a = row + l.parts * n + (i - n);
-  __half* b = a + 16 * l.nt;
-  const int r = l.r;
-  if (l.parts == 2) {
-    a[0] = mid, a[r] = hi, a[2 * r] = hi;
-    b[0] = hi, b[r] = mid, b[2 * r] = hi;
+    row[2 * n + i] = lo;
   } else {
     a[0] = lo, a[r] = mid, a[2 * r] = hi, a[3 * r] = mid, a[4 * r] = hi, a[5 * r] = hi;
     b[0] = hi, b[r] = mid, b[2 * r] = lo, b[3 * r] = hi, b[4 * r] = mid, b[5 * r] = hi;
@@ -117,8 +121,9 @@ __device__ __forceinline__ void store_split_pad(__half* row, const SplitLayout& 
   const __half zero = __float2half_rn(0.0f);
   __half* tail = row + 16 * l.parts * l.nb;
   for (int i = l.parts * (l.parts + 1) / 2 * l.r + lane; i < 16 * l.nt; i += 32) tail[i] = tail[16 * l.nt + i] = zero;
-  for (int i = K + lane; i < 16 * l.nb; i += 32)
-    for (int p = 0; p < l.parts; p++) row[16 * l.nb * p + i] = zero;
+  if (l.parts == 3)  // (two parts pad no block)
+    for (int i = K + lane; i < 16 * l.nb; i += 32)
+      for (int p = 0; p < 3; p++) row[16 * l.nb * p + i] = zero;
 }
 
 // a / b, correctly rounded, for many a and one b: y = RN(1/b) once, then
@@ -189,7 +194,7 @@ constexpr int kRowSoaFloats = 4 * 128 + 16;
 
 // Ring shape of the tensor-core engine for K ellipse pixels: stages of whole
 // row-block tiles or of single 64-column chunks (sc chunks each), dynamic shared
-// memory. False if the operands do not fit in shared memory (K above 288).
+// memory. False if the operands do not fit in shared memory (K = 267-271, 278-287, above 288).
 struct TcPlan {
   int ctas;  // CTAs that share a tile (1 or 2)
   int sc, stages;

@@ -275,7 +275,8 @@ __global__ void __launch_bounds__(256)
   const int lane = threadIdx.x & 31;
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
-  const SplitLayout lay = split_layout(K);
+  SplitLayout lay = split_layout(K);
+  if (R > 1) lay.parts = 2;  // (known when compiled: three parts are for K <= 21)
   const double sk = sqrt((double)(K - 1) / (double)K);
   const double rK = __drcp_rn((double)K);  // s / K as div_fixed: the correctly rounded quotient
   int o[R];
