@@ -13,26 +13,28 @@
 // below the diagonal are masked in the diagonal tiles, and each pair's term is
 // added to the sums of both blocks (the self pair once).
 //
-// Work item = (column tile ct, a run of up to L row blocks). A cluster of two
-// CTAs (two SMs) works on an item together: row blocks go in pairs, CTA r of the
-// cluster takes row block rb + r, and one M = 256 tcgen05.mma (cta_group::2)
-// computes both CTAs' 128 x 256 tiles. Each CTA keeps half of the column tile's
-// operand (128 rows of U) in its shared memory for the whole item and streams its
-// own row blocks through a ring of stages. One CTA per tile (M = 128) read 96 bytes
-// of shared memory per clock for the MMAs alone, of 128 there are, and wrote 32 more
-// for the row blocks; the pair reads 64. Items are ordered panel-major
+// Work item = (column tile ct, a run of up to L row blocks). The column tile's operand
+// stays in shared memory for the whole item, the row blocks stream through a ring of
+// stages. Where the operand and three whole row-block tiles fit one CTA (K up to 42,
+// and 48-53, 64), a CTA works on an item by itself with M = 128 MMAs. Else a cluster of
+// two CTAs (two SMs) does: row blocks go in pairs, CTA r of the cluster takes row block
+// rb + r, one M = 256 tcgen05.mma (cta_group::2) computes both CTAs' 128 x 256 tiles,
+// and each CTA keeps half of the column tile's operand (128 rows of U), with whole row
+// blocks as stages or, from K = 97 on (and for some from 75), chunks of 64 columns. One
+// CTA per tile reads 96 bytes of shared memory per clock for the MMAs alone, of 128 there
+// are, and writes 32 more for the row blocks; the pair reads 64. Items are ordered panel-major
 // (decode_item): all clusters work on the same row blocks at a time and share them
 // in L2, and a panel's column tiles stay in L2 while the runs pass over them.
-// Each cluster walks its items twice: first their full tiles, then their masked
+// Each cluster (or CTA) walks its items twice: first their full tiles, then their masked
 // ones (diagonal and ragged tiles, about 0.2% of all), so that the masked
 // epilogue form sits in a loop of its own (with it in the main loop the full
 // tiles ran 3% slower).
 // Warp roles (one CTA per SM, persistent):
-//   warp 16     TMA producer (one thread)
-//   warp 17     CTA 0: MMA issuer (one thread): tcgen05.mma M=256 N=256 K=16 into
-//               one of two TMEM accumulators, tcgen05.commit to both CTAs'
+//   warp 0      TMA producer (one thread)
+//   warp 1      CTA 0: MMA issuer (one thread): tcgen05.mma M=128 or 256, N=256, K=16
+//               into one of two TMEM accumulators, tcgen05.commit to both CTAs'
 //               barriers. CTA 1: relays its producer's arrivals to CTA 0.
-//   warps 0-15  epilogue: tcgen05.ld.16x256b gives each thread 4 rows x 4 columns
+//   warps 2-17  epilogue: tcgen05.ld.16x256b gives each thread 4 rows x 4 columns
 //               of a 32 x 16 block; the fused per-pair metric runs on f32x2 pairs
 //               of neighbouring columns. Column sums of the item stay in registers
 //               and leave once per item (a butterfly over the 8 lanes that share
@@ -366,10 +368,12 @@ struct SlabC {
 // h = 4 x y / (x^2 + y^2 + c2)^2 at x = sigma_p and y = sigma_q, stays near its value at the
 // slab's centres, which e = h ra rb holds. Over relative half ranges u and v of up to 1/16 it
 // changes by at most 6 (u + v) of itself, so the first-order term neglects at most
-// 6 (u + v) e: below 2^-22 here.
-__host__ __device__ inline bool ssim_split_bounded(float a, float ra, float b, float rb, float e) {
-  const float ab = a * b, x = ra * b, y = rb * a;  // u a b, v a b
-  return 16.0f * fmaxf(x, y) <= ab && e * (x + y) <= 3.8e-8f * ab;
+// 6 (u + v) e: below 2^-22 here. u and v are also those of r = 1 / sigma, whose test includes
+// that no sigma of the slab is 0. (The bound costs 1% of a 512x512 9x9 map.)
+__host__ __device__ inline bool ssim_split_bounded(const float4& rg, const float4& cg, float e) {
+  const bool ok = rg.z > 16.0f * rg.w && cg.z > 16.0f * cg.w;
+  if (e <= 3e-7f) return ok;
+  return ok && e * (rg.y * cg.x + cg.y * rg.x) <= 3.8e-8f * (rg.x * cg.x);
 }
 
 // Whether the row factors 2^-(a_p - beta)^2 of a slab, D between the centres, stay normal numbers.
@@ -408,8 +412,7 @@ __device__ __forceinline__ int slab_mode(const float4& rg, const float4& cg, con
     const float S = rcp_approx(fmaf(sa, sa, fmaf(sb, sb, ec.c2))) * ec.inv_wscale;
     const float h = 4.0f * (sa * S) * (sb * S);
     sc.kc += h;
-    ok = ok && ssim_split_bounded(rg.x, rg.y, cg.x, cg.y, h * rg.y * cg.y);
-    ok = ok && rg.z - rg.w > 0.0f && cg.z - cg.w > 0.0f && (rg.z + rg.w) * (cg.z + cg.w) < 1e25f;
+    ok = ok && ssim_split_bounded(rg, cg, h * rg.y * cg.y) && (rg.z + rg.w) * (cg.z + cg.w) < 1e25f;
   }
   const float e = sc.kc * rg.y * cg.y;
   if (ok && e <= kFirstTol) return e <= kPureTol ? kPure : kFirst;

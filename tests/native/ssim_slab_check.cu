@@ -26,7 +26,11 @@ int main() {
     const double h = 4 * x0 * y0 * iw * iw / (S0 * S0), e = (1.3862944 + h) * ra * rb;
     tried++;
     if (e > kFirstTol) continue;
-    if (!ssim_split_bounded((float)a, (float)ra, (float)b, (float)rb, (float)(h * ra * rb))) continue;
+    auto group = [&](double c, double r) {  // centre and half range of a and of 1 / sigma, as the kernel keeps them
+      const double lo = 1 / ((c + r) * iw), hi = 1 / ((c - r) * iw);
+      return make_float4((float)c, (float)r, (float)(0.5 * (lo + hi)), (float)(0.5 * (hi - lo)));
+    };
+    if (!ssim_split_bounded(group(a, ra), group(b, rb), (float)(h * ra * rb))) continue;
     accepted++;
     wide += ra > 0.03 * a || rb > 0.03 * b;
     for (int u = 0; u < 25; u++) {
