@@ -38,9 +38,10 @@ typedef enum {
  * SRED_ENGINE_FP32: plain FP32 CUDA-core Gram.
  * Both share moments, the symmetric schedule (each unordered block pair
  * evaluated once), the pair terms and the denominators. Abs-diff needs no
- * contraction and runs on the FP32 engine's kernel. On the FP32 engine NRMSE
- * accumulates |u_p - u_q|^2 directly. The other metrics' blocks are limited to
- * K = 212 pixels on either engine (SRED_ERR_LAUNCH above). */
+ * contraction and takes the FP32 engine's kernel where its node sums do not
+ * serve. On the FP32 engine NRMSE accumulates |u_p - u_q|^2 directly. Blocks are
+ * limited to K = 212 pixels on either engine and for every metric
+ * (SRED_ERR_LAUNCH above). */
 typedef enum { SRED_ENGINE_TC = 0, SRED_ENGINE_FP32 = 1 } sred_engine;
 
 typedef struct sred_ctx sred_ctx;

@@ -326,8 +326,8 @@ cudaError_t launch_block_map(const float* img, int w, int h, int frames, const E
   // 128-column tiles pad the width to no more than 1.5 times what 32-column tiles do, and
   // two tiles fit an SM; else one. At 1024x1024 15x15 four take 80 us where one takes 94
   // (700x700: 55 and 61), at 400x300 15x15 (76 CTAs against 247) 44 and 40, at 513x512 9x9
-  // 40 and 37; of tall blocks at 1024x1024, 3x81 (two tiles an SM) 88 and 93, 3x101 (one)
-  // 122 and 102, and from 3x195 on the tile fits no SM.
+  // 40 and 37; of tall blocks at 1024x1024, 5x61 (two tiles an SM) 119 and 131 and 3x81 (two) 88
+  // and 85, 3x101 (one) 121 and 97, 5x101 (one) 210 and 180, and from 3x195 on the tile fits no SM.
   const int tiles = (w + Tile<4>::kX - 1) / Tile<4>::kX, ys = (h + kTileY - 1) / kTileY;
   const bool four = (long long)tiles * ys * frames * 2 >= 3LL * num_sms &&
                     2 * tiles * Tile<4>::kX <= 3 * ((w + 31) / 32 * 32) &&
