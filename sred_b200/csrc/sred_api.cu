@@ -1978,9 +1978,9 @@ sred_status sred_block_map_2d_stack(sred_ctx* c, const char* metric, const float
   size_t chunk = chunk_frames;
   if (!chunk) {
     cudaPointerAttributes at;
-    const bool pageable = cudaPointerGetAttributes(&at, out) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
-    cudaGetLastError();
-    chunk = stack_chunk(frames, plane, pageable);
+    const cudaError_t e = cudaPointerGetAttributes(&at, out);
+    if (e != cudaSuccess) cudaGetLastError();
+    chunk = stack_chunk(frames, plane, e != cudaSuccess || at.type == cudaMemoryTypeUnregistered);
   }
   chunk = std::max<size_t>(1, std::min<size_t>(chunk, std::min(frames, 65535)));
   const int nchunks = (int)((frames + chunk - 1) / chunk);
