@@ -69,5 +69,6 @@ def test_isolated_and_equal_blocks(ctx, kind, w, h, seed):
         d = np.abs(a[i:i + 1024, None] - a[None])
         exp[i:i + 1024] = (d * np.exp2(-d * d)).sum(1) / np.float64(ws)
     # FP32 pair terms: d^2 (half an ulp below 128, times ln 2: 2.7e-6), ex2.approx (2^-22), sums of
-    # 32 (1.9e-6); nodes 5e-7; weights below 2^-126 flush to 0
+    # 32 (1.9e-6), together 4.9e-6; nodes 4e-7, up to 2.5e-6 of terms about to vanish; weights below
+    # 2^-126 flush to 0
     np.testing.assert_allclose(num, exp, rtol=5.5e-6, atol=12 * 2.0 ** -126 * a.size / np.float64(ws))
